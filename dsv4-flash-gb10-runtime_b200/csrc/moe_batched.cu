@@ -5,9 +5,11 @@
 // Pipeline on the caller's stream: pairs grouped by expert; grouped GEMM 1 (gate/up + SwiGLU) and grouped GEMM 2
 // (down, router weight applied) on tcgen05 tensor cores; per-token sum in the router's order.  Two tensor-core
 // paths: block-scaled MXFP4 MMAs fed with the packed weights as stored (moe_gemm_mxf4.cuh; activations as three
-// MXFP4 terms; the default), and fp16 MMAs with in-kernel dequantisation (moe_gemm_kernel.cuh; exact operands).
+// MXFP4 terms; the default), and fp16 MMAs with the weights dequantised into tensor memory (moe_gemm_kernel.cuh; exact
+// operands).
 // Nothing is allocated; all scratch lives in the caller's workspace.
 #include "moe_gemm_kernel.cuh"
+#include "moe_prep_kernel.cuh"
 #include "moe_gemm_mxf4.cuh"
 #include "moe_mma_rate.cuh"
 
@@ -24,29 +26,36 @@ struct Carve {
 };
 
 struct WorkspaceMap {
-    size_t xh, xexp, offsets, tiles_up, tiles_down, slot_pair, pair_slot, mid, y, xq, xs, midf, mq, ms, total;
+    size_t offsets, tiles_up, tiles_down, pair_slot, slot_w, y;      // both paths
+    size_t xq, xs, mq, ms;                                          // block-scaled path
+    size_t xh, xexp, typical, mid, mid_exp;                         // fp16 path (the same bytes)
+    size_t total;
 };
 
 WorkspaceMap map_workspace(long long T, int k, int K, int H, int O, int E) {
     const long long P = T * k;
     Carve c;
     WorkspaceMap m;
-    m.xh = c.take((size_t)T * K * 2);
-    m.xexp = c.take((size_t)T * 4);
     m.offsets = c.take((size_t)(E + 1) * 4);
     m.tiles_up = c.take((size_t)(E + 1) * 4);
     m.tiles_down = c.take((size_t)(E + 1) * 4);
-    m.slot_pair = c.take((size_t)P * 4);
     m.pair_slot = c.take((size_t)P * 4);
-    m.mid = c.take((size_t)P * H * 2);
+    m.slot_w = c.take((size_t)P * 4);
     m.y = c.take((size_t)P * O * 4);
-    // block-scaled path: three MXFP4 terms of x and of the FP32 intermediate
-    m.xq = c.take((size_t)3 * T * K / 2);
-    m.xs = c.take((size_t)3 * T * K / 32);
-    m.midf = c.take((size_t)P * H * 4);
+    const size_t shared = c.off;
+    // three MXFP4 terms of x (a row per pair) and of the intermediate
+    m.xq = c.take((size_t)3 * P * K / 2);
+    m.xs = c.take((size_t)3 * P * K / 32);
     m.mq = c.take((size_t)3 * P * H / 2);
     m.ms = c.take((size_t)3 * P * H / 32);
-    m.total = c.off;
+    const size_t mxf4_end = c.off;
+    c.off = shared;
+    m.xh = c.take((size_t)P * K * 2);
+    m.xexp = c.take((size_t)P * 8);
+    m.typical = c.take((size_t)E * 4);
+    m.mid = c.take((size_t)P * H * 2);
+    m.mid_exp = c.take((size_t)P * 4);
+    m.total = c.off > mxf4_end ? c.off : mxf4_end;
     return m;
 }
 
@@ -84,28 +93,86 @@ bool pdl_enabled() {
     return v == 1;
 }
 
-// Every kernel of this library starts with griddepcontrol.launch_dependents and reads or writes global memory only
+// Every kernel of this library executes griddepcontrol.launch_dependents early and reads or writes global memory only
 // after griddepcontrol.wait, so consecutive kernels are launched with programmatic stream serialisation: the
 // next kernel's CTAs are scheduled while the previous kernel drains, and its prologue (barrier set-up, tensor
 // memory allocation) overlaps the tail.
 template <class... Params, class... Args>
-cudaError_t launch_k(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+cudaError_t launch_k(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster,
                      Args&&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
+    int n = 0;
+    if (pdl_enabled()) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = cluster;
+        attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
+        ++n;
+    }
     cfg.attrs = attr;
-    cfg.numAttrs = pdl_enabled() ? 1 : 0;
+    cfg.numAttrs = n;
     return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 
-// Stage timing (diagnostic; off by default): when switched on, the block-scaled path records an event before its
-// first kernel and after each of its kernels; mxfp4_moe_stage_times turns them into microseconds.  Events between
+// Row-major tensors seen in boxes of 128 bytes of the innermost axis, 128-byte swizzle.  The encoder is a
+// driver function without side effects on the device; it is looked up once.
+typedef CUresult (*EncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                                const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+cudaError_t box_map(CUtensorMap* map, CUtensorMapDataType type, int elem, const void* base, int rank, const cuuint64_t* dim,
+                    const cuuint32_t* box) {
+    static EncodeTiled encode = [] {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult res;
+        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &res) != cudaSuccess) p = nullptr;
+        return reinterpret_cast<EncodeTiled>(p);
+    }();
+    if (!encode) return cudaErrorNotSupported;
+    const cuuint64_t stride[2] = {dim[0] * elem, dim[0] * elem * dim[1]};
+    const cuuint32_t step[3] = {1, 1, 1};
+    const CUresult r = encode(map, type, (cuuint32_t)rank, const_cast<void*>(base), dim, stride, box, step,
+                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+}
+// packed weights [rows, K / 2]: 128 rows
+cudaError_t weight_map(CUtensorMap* map, const uint8_t* base, long long rows, int K) {
+    const cuuint64_t dim[2] = {(cuuint64_t)(K / 2), (cuuint64_t)rows};
+    const cuuint32_t box[2] = {128, kMoeTileRows};
+    return box_map(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, base, 2, dim, box);
+}
+// three MXFP4 terms [3][P][K / 2]: half a tile's columns of every term
+cudaError_t term_maps(CUtensorMap (&map)[kMoeWidths], const uint8_t* base, long long P, int K) {
+    cudaError_t err = cudaSuccess;
+    for (int i = 0; i < kMoeWidths && err == cudaSuccess; ++i) {
+        const cuuint64_t dim[3] = {(cuuint64_t)(K / 2), (cuuint64_t)P, kQTerms};
+        const cuuint32_t box[3] = {128, (cuuint32_t)moe_width(i, kQTok) / 2, kQTerms};
+        err = box_map(&map[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, base, 3, dim, box);
+    }
+    return err;
+}
+// fp16 activations [P, K]: a tile's columns
+cudaError_t half_maps(CUtensorMap (&map)[kMoeWidths], const __half* base, long long P, int K) {
+    cudaError_t err = cudaSuccess;
+    for (int i = 0; i < kMoeWidths && err == cudaSuccess; ++i) {
+        const cuuint64_t dim[2] = {(cuuint64_t)K, (cuuint64_t)P};
+        const cuuint32_t box[2] = {kTmKBlock, (cuuint32_t)moe_width(i, kMoeTileTokens)};
+        err = box_map(&map[i], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, base, 2, dim, box);
+    }
+    return err;
+}
+
+// Stage timing (diagnostic; off by default): when switched on, a call records an event before its
+// first kernel and after each of its stages (grouping and quantising x share a launch, and the intermediate is quantised
+// inside the gate/up GEMM: those two stages read as the time between two events); mxfp4_moe_stage_times turns them into microseconds.  Events between
 // the launches take away the overlap of programmatic dependent launch, so a timed call is slower than a normal one.
 constexpr int kStageMarks = 7;      // start, group, quantise x, gate/up GEMM, quantise intermediate, down GEMM, combine
 bool g_stage_timing = false;
@@ -177,7 +244,6 @@ static int moe_forward_impl(int path, const __nv_bfloat16* x, const uint8_t* ban
         std::fprintf(stderr, "%s: null pointer or a tensor that is not 16-byte aligned\n", who);
         return -2;
     }
-    static int up_done[64] = {0}, down_done[64] = {0};
     uint8_t* ws = reinterpret_cast<uint8_t*>(workspace);
     const WorkspaceMap m = map_workspace(n_tokens, k, K_in, hidden, out_dim, n_experts);
     const int P = n_tokens * k;
@@ -185,110 +251,99 @@ static int moe_forward_impl(int path, const __nv_bfloat16* x, const uint8_t* ban
     g.offsets = reinterpret_cast<int*>(ws + m.offsets);
     g.tiles_up = reinterpret_cast<int*>(ws + m.tiles_up);
     g.tiles_down = reinterpret_cast<int*>(ws + m.tiles_down);
-    g.slot_pair = reinterpret_cast<int*>(ws + m.slot_pair);
     g.pair_slot = reinterpret_cast<int*>(ws + m.pair_slot);
-    __half* xh = reinterpret_cast<__half*>(ws + m.xh);
-    int* xexp = reinterpret_cast<int*>(ws + m.xexp);
-    __half* mid = reinterpret_cast<__half*>(ws + m.mid);
+    g.slot_w = reinterpret_cast<float*>(ws + m.slot_w);
     float* y = reinterpret_cast<float*>(ws + m.y);
 
     int* status = nullptr;
     cudaGetSymbolAddress(reinterpret_cast<void**>(&status), g_device_status);
     stage_mark(stream, 0);
-    if (path == 1)
-        launch_k(moe_group_kernel, dim3(1), dim3(1024), 0, stream, ids, P, n_experts, hidden / kMoeTileRows,
-                 (out_dim + kQRowsDown - 1) / kQRowsDown, kQTokUp, kQTokDown, g, status);
-    else
-        launch_k(moe_group_kernel, dim3(1), dim3(1024), 0, stream, ids, P, n_experts, hidden / kMoeTileRows,
-                 out_dim / kMoeTileRows, kMoeTileTokens, kMoeTileTokens, g, status);
-    stage_mark(stream, 1);
     const int grid = sm_count();
 
-    if (path == 1) {
-        // ---- block-scaled MXFP4 tensor-core path
-        static int qup_done[64] = {0}, qdown_done[64] = {0};
-        uint8_t* xq = ws + m.xq; uint8_t* xs = ws + m.xs;
-        uint8_t* mq = ws + m.mq; uint8_t* ms = ws + m.ms;
-        float* midf = reinterpret_cast<float*>(ws + m.midf);
-        const int qgrid = 4 * grid;
-        // a token none of whose experts is in this bank (expert parallel: they all live on other ranks) is not read
-        const int* no_rows = nullptr;
-        if (peer_in)
-            launch_k(moe_quantize_mxfp4x3_kernel<__nv_bfloat16, true>, dim3(qgrid), dim3(256), 0, stream, x,
-                     (long long)n_tokens, K_in, xq, xs, *peer_in, no_rows, ids, k);
-        else
-            launch_k(moe_quantize_mxfp4x3_kernel<__nv_bfloat16, false>, dim3(qgrid), dim3(256), 0, stream, x,
-                     (long long)n_tokens, K_in, xq, xs, MoePeerIn{}, no_rows, ids, k);
-        stage_mark(stream, 2);
-        MoeQGemmArgs qu;
-        qu.wa_p = bank_W1_packed; qu.wb_p = bank_W3_packed; qu.wa_s = bank_W1_scale; qu.wb_s = bank_W3_scale;
-        qu.stride_p = (long long)hidden * (K_in / 2); qu.stride_s = (long long)hidden * (K_in / 32);
-        qu.rows = hidden; qu.K = K_in; qu.n_experts = n_experts; qu.k_top = k;
-        qu.act_q = xq; qu.act_s = xs; qu.act_rows = n_tokens; qu.pair_w = weights; qu.g = g; qu.mid = midf; qu.y = nullptr;
-        cudaError_t qerr = allow_smem(moe_gemm_mxf4_kernel<0>, MoeQGemmLayout<0>::kBytes, qup_done);
-        if (qerr == cudaSuccess) {
-            launch_k(moe_gemm_mxf4_kernel<0>, dim3(grid), dim3(kGemmThreads), MoeQGemmLayout<0>::kBytes, stream, qu);
-            stage_mark(stream, 3);
-            // only the rows that exist: the pairs of this bank's experts fill slots [0, offsets[n_experts])
-            const int* used = g.offsets + n_experts;
-            const int* no_ids = nullptr;
-            launch_k(moe_quantize_mxfp4x3_kernel<float, false>, dim3(qgrid), dim3(256), 0, stream, midf, (long long)P,
-                     hidden, mq, ms, MoePeerIn{}, used, no_ids, 0);
-            stage_mark(stream, 4);
-            qerr = cudaGetLastError();
-        }
-        MoeQGemmArgs qd = qu;
-        qd.wa_p = bank_W2_packed; qd.wb_p = nullptr; qd.wa_s = bank_W2_scale; qd.wb_s = nullptr;
-        qd.stride_p = (long long)out_dim * (hidden / 2); qd.stride_s = (long long)out_dim * (hidden / 32);
-        qd.rows = out_dim; qd.K = hidden; qd.act_q = mq; qd.act_s = ms; qd.act_rows = P; qd.mid = nullptr; qd.y = y;
-        if (qerr == cudaSuccess) qerr = allow_smem(moe_gemm_mxf4_kernel<1>, MoeQGemmLayout<1>::kBytes, qdown_done);
-        if (qerr == cudaSuccess) {
-            launch_k(moe_gemm_mxf4_kernel<1>, dim3(grid), dim3(kGemmThreads), MoeQGemmLayout<1>::kBytes, stream, qd);
-            stage_mark(stream, 5);
-            dim3 cgrid((out_dim / 4 + 127) / 128, n_tokens < 65535 ? n_tokens : 65535);
-            if (peer)
-                launch_k(moe_combine_peer_kernel, dim3(cgrid), dim3(128), 0, stream, y, g.pair_slot, n_tokens, k, out_dim, *peer);
-            else
-                launch_k(moe_combine_kernel, dim3(cgrid), dim3(128), 0, stream, y, g.pair_slot, n_tokens, k, out_dim, out);
-            stage_mark(stream, 6);
-            qerr = cudaGetLastError();
-        }
-        if (qerr != cudaSuccess) {
-            std::fprintf(stderr, "%s: launch failed: %s\n", who, cudaGetErrorString(qerr));
-            return -3;
-        }
-        return 0;
-    }
+    MoeGroupArgs ga;
+    ga.ids = ids; ga.weights = weights; ga.n_pairs = P; ga.n_experts = n_experts; ga.g = g; ga.status = status;
+    const int rows_up = path == 1 ? kQTileRowsUp : kMoeTileRows, rows_down = path == 1 ? kQTileRowsDown : 2 * kMoeTileRows;
+    ga.m_tiles_up = hidden / rows_up; ga.m_tiles_down = (out_dim + rows_down - 1) / rows_down;
+    ga.tile_tokens = path == 1 ? kQTok : kMoeTileTokens;
+    launch_k(moe_group_kernel, dim3(P > kGroupOneBlockPairs ? kGroupCluster : 1), dim3(kPrepThreads), 0, stream, P > kGroupOneBlockPairs ? kGroupCluster : 1, ga);
+    stage_mark(stream, 1);
 
-    // ---- fp16 tensor-core path with in-kernel dequantisation
-    launch_k(moe_token_fp16_kernel, dim3((n_tokens + 7) / 8), dim3(256), 0, stream, x, n_tokens, K_in, xh, xexp);
-    MoeGemmArgs up;
-    up.wa_p = bank_W1_packed; up.wb_p = bank_W3_packed; up.wa_s = bank_W1_scale; up.wb_s = bank_W3_scale;
-    up.stride_p = (long long)hidden * (K_in / 2); up.stride_s = (long long)hidden * (K_in / 32);
-    up.rows = hidden; up.K = K_in; up.n_experts = n_experts; up.k_top = k;
-    up.act = xh; up.xexp = xexp; up.pair_w = weights; up.g = g; up.mid = mid; up.y = nullptr;
-    const size_t smem_up = MoeGemmLayout<0>::bytes(K_in);
-    cudaError_t err = allow_smem(moe_gemm_kernel<0>, smem_up, up_done);
-    if (err == cudaSuccess) {
-        launch_k(moe_gemm_kernel<0>, dim3(grid), dim3(kGemmThreads), smem_up, stream, up);
-        err = cudaGetLastError();
+    MoeActArgs aa;
+    aa.x = x; aa.pair_slot = g.pair_slot; aa.n_tokens = n_tokens; aa.k = k; aa.K = K_in; aa.n_pairs = P;
+    aa.q = ws + m.xq; aa.s = ws + m.xs; aa.xh = reinterpret_cast<__half*>(ws + m.xh);
+    aa.xexp = reinterpret_cast<int2*>(ws + m.xexp); aa.typical = reinterpret_cast<int*>(ws + m.typical);
+    aa.w1_s = bank_W1_scale; aa.w3_s = bank_W3_scale; aa.hidden = hidden; aa.n_experts = n_experts;
+    const MoePeerIn no_peers = {};
+    const MoePeerIn& pin = peer_in ? *peer_in : no_peers;
+    cudaError_t err = cudaSuccess;
+    if (path == 1) {
+        // ---- block-scaled MXFP4 tensor-core path; a warp per 256 elements, at most eight blocks of eight warps per SM
+        static int qup_done[64] = {0}, qdown_done[64] = {0};
+        const long long blocks = ((long long)n_tokens * (K_in / 256) + 7) / 8;
+        const dim3 agrid((unsigned)(blocks < 8LL * grid ? blocks : 8LL * grid)), ablock(256);
+        launch_k(peer_in ? moe_act_mxf4_kernel<true> : moe_act_mxf4_kernel<false>, agrid, ablock, 0, stream, 1, aa, pin);
+        stage_mark(stream, 2);
+        MoeQMaps up_maps, down_maps;
+        err = weight_map(&up_maps.wa, bank_W1_packed, (long long)n_experts * hidden, K_in);
+        if (err == cudaSuccess) err = weight_map(&up_maps.wb, bank_W3_packed, (long long)n_experts * hidden, K_in);
+        if (err == cudaSuccess) err = term_maps(up_maps.act, aa.q, P, K_in);
+        if (err == cudaSuccess) err = weight_map(&down_maps.wa, bank_W2_packed, (long long)n_experts * out_dim, hidden);
+        down_maps.wb = down_maps.wa;
+        if (err == cudaSuccess) err = term_maps(down_maps.act, ws + m.mq, P, hidden);
+        MoeQGemmArgs qu;
+        qu.wa_s = bank_W1_scale; qu.wb_s = bank_W3_scale; qu.rows = hidden; qu.K = K_in; qu.n_experts = n_experts;
+        qu.act_s = aa.s; qu.n_pairs = P; qu.g = g; qu.mid_q = ws + m.mq; qu.mid_s = ws + m.ms; qu.y = nullptr;
+        MoeQGemmArgs qd = qu;
+        qd.wa_s = bank_W2_scale; qd.wb_s = nullptr; qd.rows = out_dim; qd.K = hidden; qd.act_s = ws + m.ms; qd.y = y;
+        const uint32_t smem = moe_q_smem_bytes(n_experts);
+        if (err == cudaSuccess) err = allow_smem(moe_gemm_mxf4_kernel<0>, smem, qup_done);
+        if (err == cudaSuccess) err = allow_smem(moe_gemm_mxf4_kernel<1>, smem, qdown_done);
+        if (err == cudaSuccess) {
+            launch_k(moe_gemm_mxf4_kernel<0>, dim3(grid & ~1), dim3(kQThreads), smem, stream, 2, up_maps, qu);
+            stage_mark(stream, 3);
+            stage_mark(stream, 4);
+            launch_k(moe_gemm_mxf4_kernel<1>, dim3(grid & ~1), dim3(kQThreads), smem, stream, 2, down_maps, qd);
+        }
+    } else {
+        // ---- fp16 tensor-core path: weights dequantised into tensor memory
+        static int up_done[64] = {0}, down_done[64] = {0};
+        const int blocks = (n_tokens + kActRows - 1) / kActRows;
+        const dim3 agrid((n_experts + 31) / 32 + (blocks < 2 * grid ? blocks : 2 * grid)), ablock(kPrepThreads);
+        launch_k(peer_in ? moe_act_fp16_kernel<true> : moe_act_fp16_kernel<false>, agrid, ablock, 0, stream, 1, aa, pin);
+        stage_mark(stream, 2);
+        __half* mid = reinterpret_cast<__half*>(ws + m.mid);
+        MoeMaps up_maps, down_maps;
+        err = weight_map(&up_maps.wa, bank_W1_packed, (long long)n_experts * hidden, K_in);
+        if (err == cudaSuccess) err = weight_map(&up_maps.wb, bank_W3_packed, (long long)n_experts * hidden, K_in);
+        if (err == cudaSuccess) err = half_maps(up_maps.act, aa.xh, P, K_in);
+        if (err == cudaSuccess) err = weight_map(&down_maps.wa, bank_W2_packed, (long long)n_experts * out_dim, hidden);
+        down_maps.wb = down_maps.wa;
+        if (err == cudaSuccess) err = half_maps(down_maps.act, mid, P, hidden);
+        MoeGemmArgs up;
+        up.wa_s = bank_W1_scale; up.wb_s = bank_W3_scale; up.rows = hidden; up.K = K_in; up.n_experts = n_experts;
+        up.xexp = aa.xexp; up.typical = aa.typical; up.g = g;
+        up.mid_log = 2;
+        while ((2 << (up.mid_log - 2)) <= K_in) ++up.mid_log;                // floor(log2(K)) + 2
+        up.mid = mid; up.mid_exp = reinterpret_cast<int*>(ws + m.mid_exp); up.y = y;
+        MoeGemmArgs down = up;
+        down.wa_s = bank_W2_scale; down.wb_s = nullptr; down.rows = out_dim; down.K = hidden;
+        if (err == cudaSuccess) err = allow_smem(moe_gemm_kernel<0>, kTmSmem, up_done);
+        if (err == cudaSuccess) err = allow_smem(moe_gemm_kernel<1>, kTmSmem, down_done);
+        if (err == cudaSuccess) {
+            launch_k(moe_gemm_kernel<0>, dim3(grid), dim3(kTmThreads), kTmSmem, stream, 1, up_maps, up);
+            stage_mark(stream, 3);
+            stage_mark(stream, 4);
+            launch_k(moe_gemm_kernel<1>, dim3(grid), dim3(kTmThreads), kTmSmem, stream, 1, down_maps, down);
+        }
     }
-    MoeGemmArgs down = up;
-    down.wa_p = bank_W2_packed; down.wb_p = nullptr; down.wa_s = bank_W2_scale; down.wb_s = nullptr;
-    down.stride_p = (long long)out_dim * (hidden / 2); down.stride_s = (long long)out_dim * (hidden / 32);
-    down.rows = out_dim; down.K = hidden; down.act = mid; down.mid = nullptr; down.y = y;
-    const size_t smem_down = MoeGemmLayout<1>::bytes(hidden);
-    if (err == cudaSuccess) err = allow_smem(moe_gemm_kernel<1>, smem_down, down_done);
     if (err == cudaSuccess) {
-        launch_k(moe_gemm_kernel<1>, dim3(grid), dim3(kGemmThreads), smem_down, stream, down);
-        err = cudaGetLastError();
-    }
-    if (err == cudaSuccess) {
+        stage_mark(stream, 5);
         dim3 cgrid((out_dim / 4 + 127) / 128, n_tokens < 65535 ? n_tokens : 65535);
         if (peer)
-            launch_k(moe_combine_peer_kernel, dim3(cgrid), dim3(128), 0, stream, y, g.pair_slot, n_tokens, k, out_dim, *peer);
+            launch_k(moe_combine_peer_kernel, dim3(cgrid), dim3(128), 0, stream, 1, y, g.pair_slot, n_tokens, k, out_dim, *peer);
         else
-            launch_k(moe_combine_kernel, dim3(cgrid), dim3(128), 0, stream, y, g.pair_slot, n_tokens, k, out_dim, out);
+            launch_k(moe_combine_kernel, dim3(cgrid), dim3(128), 0, stream, 1, y, g.pair_slot, n_tokens, k, out_dim, out);
+        stage_mark(stream, 6);
         err = cudaGetLastError();
     }
     if (err != cudaSuccess) {
@@ -298,18 +353,23 @@ static int moe_forward_impl(int path, const __nv_bfloat16* x, const uint8_t* ban
     return 0;
 }
 
-// Default path: block-scaled MXFP4 MMAs; DSV4_B200_MOE_PATH=fp16 in the environment selects the fp16 path.
-DSV4_API int mxfp4_moe_forward(const __nv_bfloat16* x, const uint8_t* bank_W1_packed, const uint8_t* bank_W3_packed,
-                               const uint8_t* bank_W2_packed, const uint8_t* bank_W1_scale,
-                               const uint8_t* bank_W3_scale, const uint8_t* bank_W2_scale, const int* ids,
-                               const float* weights, int n_tokens, int n_experts, int K_in, int hidden, int out_dim,
-                               int k, __nv_bfloat16* out, void* workspace, cudaStream_t stream) {
+// The tensor-core path of the entries that leave it to the library: block-scaled MXFP4 MMAs; DSV4_B200_MOE_PATH=fp16 in
+// the environment selects the fp16 path.
+static int default_path() {
     static int path = -1;
     if (path < 0) {
         const char* e = std::getenv("DSV4_B200_MOE_PATH");
         path = (e && e[0] == 'f') ? 0 : 1;
     }
-    return moe_forward_impl(path, x, bank_W1_packed, bank_W3_packed, bank_W2_packed, bank_W1_scale, bank_W3_scale,
+    return path;
+}
+
+DSV4_API int mxfp4_moe_forward(const __nv_bfloat16* x, const uint8_t* bank_W1_packed, const uint8_t* bank_W3_packed,
+                               const uint8_t* bank_W2_packed, const uint8_t* bank_W1_scale,
+                               const uint8_t* bank_W3_scale, const uint8_t* bank_W2_scale, const int* ids,
+                               const float* weights, int n_tokens, int n_experts, int K_in, int hidden, int out_dim,
+                               int k, __nv_bfloat16* out, void* workspace, cudaStream_t stream) {
+    return moe_forward_impl(default_path(), x, bank_W1_packed, bank_W3_packed, bank_W2_packed, bank_W1_scale, bank_W3_scale,
                             bank_W2_scale, ids, weights, n_tokens, n_experts, K_in, hidden, out_dim, k, out, workspace,
                             stream);
 }
@@ -363,12 +423,7 @@ DSV4_API int mxfp4_moe_forward_ep(const __nv_bfloat16* x, const uint8_t* bank_W1
         peer.recv[r] = reinterpret_cast<__nv_bfloat16*>(recv_ptrs[r]);
     }
     peer.world = world; peer.my_rank = my_rank; peer.tokens_per_rank = tokens_per_rank;
-    static int path = -1;
-    if (path < 0) {
-        const char* e = std::getenv("DSV4_B200_MOE_PATH");
-        path = (e && e[0] == 'f') ? 0 : 1;
-    }
-    return moe_forward_impl(path, x, bank_W1_packed, bank_W3_packed, bank_W2_packed, bank_W1_scale, bank_W3_scale,
+    return moe_forward_impl(default_path(), x, bank_W1_packed, bank_W3_packed, bank_W2_packed, bank_W1_scale, bank_W3_scale,
                             bank_W2_scale, ids, weights, n_tokens, n_experts, K_in, hidden, out_dim, k, nullptr,
                             workspace, stream, &peer);
 }
@@ -388,7 +443,7 @@ DSV4_API int mxfp4_moe_ep_sum(const __nv_bfloat16* recv, const int* ids, int k, 
     const long long n4 = (long long)n_tokens * out_dim / 4;
     long long grid = (n4 + 255) / 256;
     if (grid > 8LL * sm_count()) grid = 8LL * sm_count();
-    launch_k(moe_ep_sum_kernel, dim3((unsigned)grid), dim3(256), 0, stream, recv, ids, k, experts_per_rank, world,
+    launch_k(moe_ep_sum_kernel, dim3((unsigned)grid), dim3(256), 0, stream, 1, recv, ids, k, experts_per_rank, world,
              n_tokens, out_dim, out);
     return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
@@ -400,7 +455,7 @@ DSV4_API int mxfp4_moe_ep_sum(const __nv_bfloat16* recv, const int* ids, int k, 
 // published ids into this rank's view (local index, -1 for experts of other ranks), the activation quantiser reads
 // every token's row from the rank that published it (plain loads over NVLink), and the combine kernel stores the
 // partial rows into the home ranks' receive buffers as in mxfp4_moe_forward_ep.  x_ptrs / ids_ptrs / w_ptrs /
-// recv_ptrs: HOST arrays of `world` device pointers.  Block-scaled tensor-core path only.  workspace:
+// recv_ptrs: HOST arrays of `world` device pointers.  workspace:
 // mxfp4_moe_forward_ep2_workspace_bytes.  Return codes as mxfp4_moe_forward_ep.
 DSV4_API size_t mxfp4_moe_forward_ep2_workspace_bytes(int world, int tokens_per_rank, int k, int K_in, int hidden,
                                                       int out_dim, int n_experts_local) {
@@ -440,9 +495,9 @@ DSV4_API int mxfp4_moe_forward_ep2(void* const* x_ptrs, void* const* ids_ptrs, v
     int* ids_local = reinterpret_cast<int*>(ws + base);
     float* w_local = reinterpret_cast<float*>(ws + base + (((size_t)n_tokens * k * 4 + 255) & ~size_t(255)));
     const int n_meta = n_tokens * k;
-    launch_k(moe_ep_gather_meta_kernel, dim3((unsigned)((n_meta + 255) / 256)), dim3(256), 0, stream, in, k, ids_local,
+    launch_k(moe_ep_gather_meta_kernel, dim3((unsigned)((n_meta + 255) / 256)), dim3(256), 0, stream, 1, in, k, ids_local,
              w_local);
-    return moe_forward_impl(1, nullptr, bank_W1_packed, bank_W3_packed, bank_W2_packed, bank_W1_scale, bank_W3_scale,
+    return moe_forward_impl(default_path(), nullptr, bank_W1_packed, bank_W3_packed, bank_W2_packed, bank_W1_scale, bank_W3_scale,
                             bank_W2_scale, ids_local, w_local, n_tokens, n_experts_local, K_in, hidden, out_dim, k,
                             nullptr, workspace, stream, &peer, &in);
 }

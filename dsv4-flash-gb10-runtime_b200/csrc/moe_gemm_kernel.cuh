@@ -1,228 +1,411 @@
-// The tensor-core kernel of the batched routed-expert path (see moe_gemm.cuh for the design).
+// Grouped GEMMs of the fp16 path: fp16 tcgen05 MMAs whose A operand, the dequantised weight tile, lives in TENSOR
+// MEMORY (number formats: moe_gemm.cuh).
+//
+// What bounds it.  A weight tile of 128 rows x 64 K-elements is 4 KB in HBM.  Written to shared memory as fp16 it is
+// 16 KB, written and read through the port the MMAs also fetch the tokens from; a kernel that did so was bound there
+// (348 TFLOP/s at 4096 tokens).  Here the tile goes registers -> tensor memory (tcgen05.st, 128 lanes x 32 columns), which
+// costs shared memory nothing, and the MMA (A from tensor memory, B = tokens from shared memory) runs at N / 2 clocks
+// per 128 x N x 16: 4 N clocks for the two matrices and 64 K-elements of a stage.  Dequantisation takes about 280 clocks
+// of each scheduler for the same stage (E2M1 conversion + one half-rate multiply per two weights), so tiles of
+// 80 .. 128 tokens are bound by the tensor pipe and tiles of a few tokens by HBM (8.7 KB per stage and SM).
+//
+// A tile: 128 rows of two matrices (gate/up: the same rows of W1 and W3; down: two row blocks of W2) x up to 128 tokens.
+// CTA = 20 warps (five per scheduler: 96 registers a thread), persistent grid, one CTA per SM, tiles by static striding:
+//   warps 0..15  dequantise: warp = (K-block parity, matrix, lane quadrant); a thread owns one weight row, takes 32
+//                bytes and two scale bytes of it per K-block of 64 and writes 32 tensor-memory columns.  They also drain the
+//                finished accumulators, after the first stages of the NEXT tile are in tensor memory, so that the MMAs
+//                continue as soon as the accumulators have been read.
+//   warp 16      token rows -> shared memory (one TMA box per K-block, the rows of a tile being neighbours), six ahead
+//   warp 17      packed weights -> shared memory (TMA, 256 K-elements = 16 KB per matrix and stage) and their scales
+//   warp 18      issues the MMAs
+//   warp 19      a tile ahead: token tables, and the largest scale byte of every row
+// Tensor memory: columns 0..255 two accumulators of 128, 256..511 four stages of two 128 x 64 fp16 tiles.
+// Every wait is bounded (stream_ring.cuh).
 #pragma once
 
 #include "moe_gemm.cuh"
 
 namespace dsv4 {
 
+constexpr int kTmDequantWarps = 16;
+constexpr int kTmTokenWarp = kTmDequantWarps, kTmWeightWarp = kTmTokenWarp + 1;
+constexpr int kTmMmaWarp = kTmWeightWarp + 1, kTmAuxWarp = kTmMmaWarp + 1;
+constexpr int kTmThreads = (kTmAuxWarp + 1) * 32;
+constexpr int kTmKBlock = 64;                         // K-elements per tensor-memory / token stage
+constexpr int kTmWBlock = 256;                        // K-elements per packed-weight stage (128 bytes per row)
+constexpr int kTmWStages = 3, kTmAStages = 4, kTmBStages = 6, kTmTables = 3;
+constexpr uint32_t kTmWTile = 128 * 128;              // packed weights of one matrix and stage
+constexpr uint32_t kTmWScale = 128 * 8;               // scale bytes of one matrix and stage
+constexpr uint32_t kTmWStage = 2 * kTmWTile + 2 * kTmWScale;
+constexpr uint32_t kTmBStage = kMoeTileTokens * 128;
+constexpr uint32_t kTmOffB = kTmWStages * 2 * kTmWTile;                       // every tile 1024-byte aligned
+constexpr uint32_t kTmOffS = kTmOffB + kTmBStages * kTmBStage;
+constexpr uint32_t kTmSmem = kTmOffS + kTmWStages * 2 * kTmWScale + 1024;
+
+struct MoeGemmArgs {
+    const uint8_t* wa_s; const uint8_t* wb_s;   // E8M0 scales: up W1, W3; down W2 (wb unused)
+    int rows;                                   // weight rows per expert
+    int K;                                      // reduction length (multiple of 256)
+    int n_experts;
+    const int2* xexp;                           // [P] {e_t, q_t} of a slot's token (up)
+    const int* typical;                         // [E] c1 | c3 << 8 (up)
+    int mid_log;                                // L (up)
+    MoeGroups g;
+    __half* mid;                                // up output [P, rows]
+    int* mid_exp;                               // [P] power of two taken out of a slot's mid (up writes, down reads)
+    float* y;                                   // down output [P, rows]
+};
+// Weight boxes of 128 rows x 128 bytes; activation boxes of a tile's columns x 64 fp16 values, one per column count.
+struct MoeMaps { CUtensorMap wa, wb, act[kMoeWidths]; };
+
+struct MoeTile { int e, slot0, n_valid, width, m0, mats; };
+
 template <int MODE>
-__global__ void __launch_bounds__(kGemmThreads, 1) moe_gemm_kernel(const MoeGemmArgs a) {
-    using L = MoeGemmLayout<MODE>;
-    constexpr int S = L::kStages;
-    constexpr int MATS = L::kMats;
+__device__ __forceinline__ MoeTile moe_tile_decode(const int* tiles, const int* offsets, int n_experts, int m_tiles, int rows,
+                                                   int tile) {
+    int lo = 0, hi = n_experts;                 // last expert with tiles[e] <= tile
+    while (hi - lo > 1) {
+        const int md = (lo + hi) >> 1;
+        if (tiles[md] <= tile) lo = md; else hi = md;
+    }
+    MoeTile t;
+    t.e = lo;
+    const int local = tile - tiles[lo], nt = local / m_tiles, n = offsets[lo + 1] - offsets[lo];
+    const int per = moe_tokens_per_tile(n, kMoeTileTokens);
+    t.slot0 = offsets[lo] + nt * per;
+    t.n_valid = min(per, offsets[lo + 1] - t.slot0);
+    t.width = moe_width_index(t.n_valid);
+    t.m0 = (local - nt * m_tiles) * (MODE == 0 ? kMoeTileRows : 2 * kMoeTileRows);
+    t.mats = (MODE == 1 && t.m0 + kMoeTileRows >= rows) ? 1 : 2;       // a last, half down tile
+    return t;
+}
+
+// 2^(s - c) (c >= s) as two equal fp16 halves: exact down to 2^-24, 0 below and for s == 255.
+__device__ __forceinline__ uint32_t half2_pow2(int s, int c) {
+    const float f = __uint_as_float((uint32_t)max(s - c + 127, 1) << 23);
+    uint32_t h;
+    asm("cvt.rn.f16x2.f32 %0, %1, %1;" : "=r"(h) : "f"(s == 255 ? 0.f : f));
+    return h;
+}
+
+// 16 packed bytes (one scale block) -> 16 registers of two fp16 values times `mult`.
+__device__ __forceinline__ void dequant_block(const uint4& w, uint32_t mult, uint32_t (&out)[16]) {
+    const uint32_t word[4] = {w.x, w.y, w.z, w.w};
+    const __half2 m = *reinterpret_cast<const __half2*>(&mult);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        __half2 h[4];
+        e2m1x8_to_h2x4(word[i], h);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const __half2 v = __hmul2(h[j], m);
+            out[4 * i + j] = *reinterpret_cast<const uint32_t*>(&v);
+        }
+    }
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(kTmThreads, 1) moe_gemm_kernel(const __grid_constant__ MoeMaps maps, const MoeGemmArgs a) {
     extern __shared__ __align__(1024) uint8_t gemm_smem[];
-    __shared__ __align__(8) uint64_t bar_full[S], bar_empty[S], bar_accum;
+    __shared__ __align__(8) uint64_t w_full[kTmWStages], w_empty[kTmWStages], a_full[kTmAStages], a_empty[kTmAStages];
+    __shared__ __align__(8) uint64_t b_full[kTmBStages], b_empty[kTmBStages];
+    __shared__ __align__(8) uint64_t acc_full, acc_free, exp_full[kTmTables], tab_free[kTmTables];
     __shared__ uint32_t tmem_holder;
-    __shared__ int row_exp[2][128];          // largest E8M0 byte of every weight row of the tile (-1: none)
-    __shared__ int tok_exp[128];             // exponent removed from the token of every accumulator column
-    __shared__ int tok_row[128];             // activation row of every column (token index / slot)
-    __shared__ float tok_w[128];             // router weight of every column (down)
-    pdl_launch_dependents();
+    __shared__ int s_tiles[kMoeMaxExperts + 1], s_offsets[kMoeMaxExperts + 1];
+    // tables of a tile, by tile number mod 3: the aux warps fill tile N + 1 while tile N - 1 is being drained
+    __shared__ float tok_f0[kTmTables][kMoeTileTokens];       // up: 2^e_t;  down: w * 2^(half of the slot's exponent)
+    __shared__ float tok_f1[kTmTables][kMoeTileTokens];       // up: 2^-2q_t; down: 2^(the other half)
+    __shared__ int row_exp[kTmTables][2][kMoeTileRows];       // largest scale byte of every weight row
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    constexpr int kProducerWarps = kGemmProducers / 32;
-    const bool producer = warp < kProducerWarps;
-    const int n_kb = a.K / kGemmKBlock;
-    const int scale_row = a.K / 32;          // scale bytes per weight row
-    uint8_t* scale_cache = gemm_smem + L::kScaleCache;
+    const int n_kb = a.K / kTmKBlock, n_wb = a.K / kTmWBlock, row_s = a.K >> 5;
+    const uint32_t smem0 = smem_u32(gemm_smem);
 
-    if (warp == kProducerWarps) tc05_alloc(smem_u32(&tmem_holder), 256);
+    if (warp == kTmMmaWarp) tc05_alloc(smem_u32(&tmem_holder), 512);
     if (tid == 0) {
-        for (int s = 0; s < S; ++s) { mbar_init(smem_u32(&bar_full[s]), kProducerWarps); mbar_init(smem_u32(&bar_empty[s]), 1); }
-        mbar_init(smem_u32(&bar_accum), 1);
+        for (int s = 0; s < kTmWStages; ++s) { mbar_init(smem_u32(&w_full[s]), 1 + 32); mbar_init(smem_u32(&w_empty[s]), kTmDequantWarps); }
+        for (int s = 0; s < kTmAStages; ++s) { mbar_init(smem_u32(&a_full[s]), kTmDequantWarps / 2); mbar_init(smem_u32(&a_empty[s]), 1); }
+        for (int s = 0; s < kTmBStages; ++s) { mbar_init(smem_u32(&b_full[s]), 1); mbar_init(smem_u32(&b_empty[s]), 1); }
+        for (int s = 0; s < kTmTables; ++s) {
+            mbar_init(smem_u32(&exp_full[s]), 1);
+            mbar_init(smem_u32(&tab_free[s]), kTmDequantWarps);
+        }
+        mbar_init(smem_u32(&acc_full), 1);
+        mbar_init(smem_u32(&acc_free), kTmDequantWarps);
         mbar_init_fence();
     }
     pdl_wait();
+    pdl_launch_dependents();
+    for (int i = tid; i <= a.n_experts; i += kTmThreads) {
+        s_tiles[i] = __ldcg((MODE == 0 ? a.g.tiles_up : a.g.tiles_down) + i);
+        s_offsets[i] = __ldcg(a.g.offsets + i);
+    }
     tc05_fence_before_sync();
     __syncthreads();
     tc05_fence_after_sync();
     const uint32_t tmem = tmem_holder;
-
-    const int* tiles = MODE == 0 ? a.g.tiles_up : a.g.tiles_down;
-    const int n_tiles = tiles[a.n_experts];
-    const int m_tiles = a.rows / kMoeTileRows;
-    uint32_t it = 0;                          // stages produced / consumed so far (same count in both roles)
-    uint32_t tile_count = 0;
+    const int n_tiles = s_tiles[a.n_experts];
+    const int m_tiles = (a.rows + (MODE == 0 ? kMoeTileRows : 2 * kMoeTileRows) - 1) / (MODE == 0 ? kMoeTileRows : 2 * kMoeTileRows);
+    auto decode = [&](int tile) { return moe_tile_decode<MODE>(s_tiles, s_offsets, a.n_experts, m_tiles, a.rows, tile); };
     bool alive = true;
+    auto wait = [&](uint64_t& bar, uint32_t parity, int code) {
+        if (alive) alive = __all_sync(kFullMask, mbar_wait_bounded(smem_u32(&bar), parity & 1u, code));   // per warp
+    };
+    auto wait_one = [&](uint64_t& bar, uint32_t parity, int code) {        // roles of one thread
+        if (alive) alive = mbar_wait_bounded(smem_u32(&bar), parity & 1u, code);
+    };
+    uint32_t tc = 0;                                          // tiles begun by this CTA
 
-    for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++tile_count) {
-        // expert of this tile: last e with tiles[e] <= tile
-        int lo = 0, hi = a.n_experts;
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (tiles[mid] <= tile) lo = mid; else hi = mid;
-        }
-        const int e = lo;
-        const int local = tile - tiles[e];
-        const int nt = local / m_tiles, mt = local - nt * m_tiles;
-        const int slot0 = a.g.offsets[e] + nt * kMoeTileTokens;
-        const int n_valid = min(kMoeTileTokens, a.g.offsets[e + 1] - slot0);
-        const int n_mma = (n_valid + 15) & ~15;
-        const int m0 = mt * kMoeTileRows;
+    if (warp < kTmDequantWarps) {
+        const int group = warp >> 3, mat = (warp >> 2) & 1, quad = warp & 3, row = quad * 32 + lane;
 
-        if (producer) {
-            // ---- tile set-up: scale rows -> shared memory, row exponents, per-column token data
-            const uint8_t* sc_src[2] = {a.wa_s + e * a.stride_s + (long long)m0 * scale_row,
-                                        MODE == 0 ? a.wb_s + e * a.stride_s + (long long)m0 * scale_row : nullptr};
-            const int vec_per_mat = 128 * scale_row / 16;
-#pragma unroll
-            for (int m = 0; m < MATS; ++m)
-                for (int i = tid; i < vec_per_mat; i += kGemmProducers)
-                    reinterpret_cast<uint4*>(scale_cache + m * 128 * scale_row)[i] =
-                        ldg_stream_v4(sc_src[m] + (size_t)i * 16);
-            if (tid < n_valid) {
-                const int slot = slot0 + tid;
-                const int pair = a.g.slot_pair[slot];
-                const int token = pair / a.k_top;
-                tok_exp[tid] = a.xexp[token];
-                tok_row[tid] = MODE == 0 ? token : slot;
-                if (MODE == 1) tok_w[tid] = a.pair_w[pair];
-            }
-            asm volatile("bar.sync 1, %0;" ::"n"(kGemmProducers) : "memory");
-            if (tid < 128 * MATS) {
-                const int m = tid >> 7, r = tid & 127;
-                // scale rows are a multiple of 8 bytes (K is a multiple of 256)
-                const uint2* p = reinterpret_cast<const uint2*>(scale_cache + (m * 128 + r) * scale_row);
-                uint32_t best = 0;
-                bool any = false;
-                for (int i = 0; i < scale_row / 8; ++i) {
-                    const uint2 q = p[i];
-                    const uint32_t w[2] = {q.x, q.y};
-#pragma unroll
-                    for (int j = 0; j < 2; ++j) {
-                        const uint32_t is_ff = __vcmpeq4(w[j], 0xffffffffu);
-                        any = any || (is_ff != 0xffffffffu);
-                        best = __vmaxu4(best, w[j] & ~is_ff);
-                    }
-                }
-                const uint32_t b = max(max(best & 0xff, (best >> 8) & 0xff), max((best >> 16) & 0xff, best >> 24));
-                row_exp[m][r] = any ? (int)b : -1;
-            }
-            asm volatile("bar.sync 1, %0;" ::"n"(kGemmProducers) : "memory");
-
-            // ---- main loop: a thread owns one 32-value block (row, half) of ONE weight tile and 2 chunks of the
-            // token tile (with one weight matrix only half of the producers have a weight block)
-            const int mat = (tid >> 8) & 1;
-            const bool has_a = mat < MATS;
-            const int row = (tid & 255) >> 1, half = tid & 1;
-            const uint8_t* wbase = (mat == 0 || MODE != 0) ? a.wa_p : a.wb_p;
-            const uint8_t* wsrc = wbase + e * a.stride_p + (long long)(m0 + row) * (a.K >> 1) + half * 16;
-            const uint8_t* my_scale = scale_cache + ((has_a ? mat : 0) * 128 + row) * scale_row + half;
-            const int my_exp = row_exp[has_a ? mat : 0][row];
-            const __half* bsrc[2];
-            bool bok[2];
-#pragma unroll
-            for (int q = 0; q < 2; ++q) {
-                const int idx = tid + kGemmProducers * q;
-                const int n = idx >> 3, c = idx & 7;
-                bok[q] = n < n_valid;
-                bsrc[q] = a.act + (size_t)(bok[q] ? tok_row[n] : 0) * a.K + c * 8;
-            }
-            uint4 ring_a[4];
-            uint4 ring_b[2][2];
-            auto load_a = [&](int kb, uint4& dst) {
-                if (has_a) dst = ldg_stream_v4(wsrc + (size_t)kb * 32);
-            };
-            auto load_b = [&](int kb, uint4 (&dst)[2]) {
-#pragma unroll
-                for (int q = 0; q < 2; ++q)
-                    dst[q] = bok[q] ? __ldcg(reinterpret_cast<const uint4*>(bsrc[q] + (size_t)kb * kGemmKBlock))
-                                    : make_uint4(0, 0, 0, 0);
-            };
-#pragma unroll
-            for (int d = 0; d < 3; ++d)
-                if (d < n_kb) load_a(d, ring_a[d]);
-            load_b(0, ring_b[0]);
-            for (int kb0 = 0; kb0 < n_kb; kb0 += 4) {
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const int kb = kb0 + u;
-                    if (kb + 3 < n_kb) load_a(kb + 3, ring_a[(u + 3) & 3]);
-                    if (kb + 1 < n_kb) load_b(kb + 1, ring_b[(u + 1) & 1]);
-                    const uint32_t s = it % S;
-                    if (it >= (uint32_t)S && alive)
-                        alive = mbar_wait_bounded(smem_u32(&bar_empty[s]), ((it / S) - 1) & 1, 4);
-                    uint8_t* stage = gemm_smem + s * L::kStageBytes;
-                    if (has_a) {
-                        const int sb = my_scale[kb * 2];
-                        const uint32_t mult = (sb == 255 || my_exp < 0) ? 0u : half_pow2_bits(sb - my_exp);
-                        dequant_block_to_tile(ring_a[u & 3], mult, stage + mat * kGemmTileBytes, row, half);
-                    }
-#pragma unroll
-                    for (int q = 0; q < 2; ++q) {
-                        const int idx = tid + kGemmProducers * q;
-                        if ((idx >> 3) < n_mma)
-                            *reinterpret_cast<uint4*>(stage + MATS * kGemmTileBytes + tc05_sw128_offset(idx >> 3, idx & 7)) =
-                                ring_b[u & 1][q];
-                    }
-                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                    __syncwarp();
-                    if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&bar_full[s])) : "memory");
-                    ++it;
-                }
-            }
-        } else {
-            // ---- last warp: issue the MMAs of every stage; a stage is released when its MMAs have completed
-            const uint32_t idesc = tc05_idesc_f16(128, n_mma);
-            for (int kb = 0; kb < n_kb; ++kb, ++it) {
-                const uint32_t s = it % S;
-                if (alive) alive = mbar_wait_bounded(smem_u32(&bar_full[s]), (it / S) & 1, 5);
-                tc05_fence_after_sync();
-                if (lane == 0 && alive) {
-                    const uint32_t stage = smem_u32(gemm_smem) + s * L::kStageBytes;
-#pragma unroll
-                    for (int j = 0; j < kGemmKBlock / 16; ++j) {
-                        const uint64_t db = tc05_desc_k_sw128(stage + MATS * kGemmTileBytes + 32 * j);
-#pragma unroll
-                        for (int m = 0; m < MATS; ++m)
-                            tc05_mma_f16(tmem + m * 128, tc05_desc_k_sw128(stage + m * kGemmTileBytes + 32 * j), db, idesc,
-                                         (kb > 0 || j > 0) ? 1u : 0u);
-                    }
-                    tc05_commit(smem_u32(&bar_empty[s]));
-                    if (kb == n_kb - 1) tc05_commit(smem_u32(&bar_accum));
-                }
-                __syncwarp();
-            }
-        }
-
-        // ---- epilogue: warps 0..3 own accumulator rows 32 w .. 32 w + 31
-        if (warp < 4) {
-            if (alive) alive = mbar_wait_bounded(smem_u32(&bar_accum), tile_count & 1, 6);
+        // accumulators of tile number `count` -> global memory; warps q, q + 4, q + 8, q + 12 share lane quadrant q and take
+        // token chunks of 16 in turn
+        auto drain = [&](const MoeTile& t, uint32_t count) {
+            wait(acc_full, count, 6);
             tc05_fence_after_sync();
-            const int r = tid;                                   // accumulator row = weight row m0 + r
-            const uint32_t trow = tmem + ((uint32_t)(warp * 32) << 16);
-            const float sa = row_exp[0][r] < 0 ? 0.f : float_pow2(row_exp[0][r] - 127);
-            const float sb = (MODE == 0) ? (row_exp[1][r] < 0 ? 0.f : float_pow2(row_exp[1][r] - 127)) : 0.f;
-            for (int c0 = 0; c0 < n_mma && alive; c0 += 16) {
-                float g[16], u[16];
-                tc05_ld16(trow + c0, g);
-                if (MODE == 0) tc05_ld16(trow + 128 + c0, u);
+            const uint32_t trow = tmem + ((uint32_t)(quad * 32) << 16);
+            const uint32_t tab = count % kTmTables;
+            const int c0 = (warp >> 2) * 16;
+            const int m = t.m0 + row;
+            bool handed = false;
+            const int ea = row_exp[tab][0][row], eb = row_exp[tab][1][row];
+            float sa, sb, fa = 0.f, fb = 0.f;
+            sa = ea < 0 ? 0.f : float_pow2(ea - 127);
+            sb = eb < 0 ? 0.f : float_pow2(eb - 127);
+            int mid_base = 0;
+            if (MODE == 0) {
+                const int typ = __ldg(a.typical + t.e), c1 = typ & 255, c3 = typ >> 8;
+                fa = float_pow2(ea - c1);
+                fb = float_pow2(eb - c3 - a.mid_log);
+                mid_base = c1 + c3 - 254 + a.mid_log;
+            }
+            auto store = [&](const uint32_t (&g)[16], const uint32_t (&u)[16], int c) {
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
-                    const int n = c0 + i;
-                    if (n < n_valid) {
-                        const int ex = tok_exp[n];
-                        if (MODE == 0) {
-                            // g = gn * 2^ex, u = un * 2^ex; silu(g) * u / 2^(2 ex) = gn * sigmoid(g) * un: stored without
-                            // the token's scale (squared), bounded whatever the scale of x
-                            const float gn = g[i] * sa, un = u[i] * sb;
-                            const float stored = gn * (1.0f / (1.0f + __expf(-gn * float_pow2(ex)))) * un;
-                            a.mid[(size_t)(slot0 + n) * a.rows + m0 + r] =
-                                __float2half_rn(fminf(fmaxf(stored, -65504.f), 65504.f));
-                        } else {
-                            a.y[(size_t)(slot0 + n) * a.rows + m0 + r] =
-                                g[i] * sa * float_pow2(ex) * float_pow2(ex) * tok_w[n];
+                    const int n = c + i;
+                    if (n >= t.n_valid) break;
+                    const float f0 = tok_f0[tab][n], f1 = tok_f1[tab][n];
+                    const float gr = __uint_as_float(g[i]), ur = __uint_as_float(u[i]);
+                    if (MODE == 0) {
+                        const float gate = gr * sa * f0;                  // the true gate value, for the sigmoid
+                        const float v = __fdividef(gr * fa, 1.0f + __expf(-gate)) * (ur * fb) * f1;
+                        a.mid[(size_t)(t.slot0 + n) * a.rows + m] = __float2half_rn(fminf(fmaxf(v, -65504.f), 65504.f));
+                    } else {
+                        float* yrow = a.y + (size_t)(t.slot0 + n) * a.rows + m;
+                        yrow[0] = gr * sa * f0 * f1;
+                        if (t.mats == 2) yrow[kMoeTileRows] = ur * sb * f0 * f1;
+                    }
+                }
+            };
+#pragma unroll 1
+            for (int c = c0; c < kMoeTileTokens; c += 64) {
+                const bool has = c < t.n_valid && alive;
+                uint32_t g[16], u[16];
+                if (has) {
+                    tc05_ld16_issue(trow + c, g);
+                    tc05_ld16_issue(trow + kMoeTileTokens + c, u);
+                    tc05_wait_ld();
+                }
+                if (c + 64 >= t.n_valid && !handed) {                       // this warp has read all it wants of the accumulators
+                    handed = true;
+                    tc05_fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_one(smem_u32(&acc_free));
+                }
+                if (has) store(g, u, c);
+            }
+            if (MODE == 0 && t.m0 == 0 && warp == 0)
+                for (int n = lane; n < t.n_valid; n += 32) {
+                    const int2 x = __ldcg(a.xexp + t.slot0 + n);
+                    a.mid_exp[t.slot0 + n] = 2 * (x.x + x.y) + mid_base;
+                }
+            __syncwarp();
+            if (lane == 0) mbar_arrive_one(smem_u32(&tab_free[tab]));
+        };
+
+        MoeTile prev;
+        bool has_prev = false;
+        uint32_t kb_base = 0;                                 // K-blocks of the tiles before this one
+        for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++tc) {
+            const MoeTile t = decode(tile);
+            const uint32_t tab = tc % kTmTables;
+            wait(exp_full[tab], tc / kTmTables, 5);
+            const int c = row_exp[tab][mat][row];
+            for (int kb = group; kb < n_kb; kb += 2) {
+                const uint32_t it = kb_base + kb, wi = it >> 2, ws = wi % kTmWStages;
+                const int q = kb & 3;                         // K-block inside the weight stage
+                if (q < 2) wait(w_full[ws], wi / kTmWStages, 5);
+                const uint32_t wrow = smem0 + (ws * 2 + mat) * kTmWTile + row * 128;
+                const uint4 w0 = lds_v4(wrow + (((2 * q) ^ (row & 7)) << 4));
+                const uint4 w1 = lds_v4(wrow + (((2 * q + 1) ^ (row & 7)) << 4));
+                uint32_t sc;
+                asm volatile("ld.shared.u16 %0, [%1];" : "=r"(sc) : "r"(smem0 + kTmOffS + (ws * 2 + mat) * kTmWScale + row * 8 + q * 2));
+                const uint32_t as = it % kTmAStages;
+                const uint32_t acol = tmem + ((uint32_t)(quad * 32) << 16) + 256 + as * 64 + mat * 32;
+                if (it >= kTmAStages) wait(a_empty[as], it / kTmAStages - 1, 4);
+                tc05_fence_after_sync();
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    uint32_t r[16];
+                    dequant_block(h ? w1 : w0, c < 0 ? 0u : half2_pow2(h ? sc >> 8 : sc & 255, c), r);
+                    tc05_st16(acol + 16 * h, r);
+                }
+                if (q >= 2) {
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_one(smem_u32(&w_empty[ws]));
+                }
+                tc05_wait_st();
+                tc05_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_one(smem_u32(&a_full[as]));
+                // the first stages of this tile are in tensor memory: now drain the previous one
+                if (has_prev && kb == group + 2) drain(prev, tc - 1);
+            }
+            kb_base += n_kb;
+            prev = t;
+            has_prev = true;
+        }
+        if (has_prev) drain(prev, tc - 1);
+    } else if (warp == kTmTokenWarp) {
+        // ---- token rows
+        if (tc05_elect_one()) {
+            uint32_t it = 0;
+            for (int tile = blockIdx.x; tile < n_tiles && alive; tile += gridDim.x) {
+                const MoeTile t = decode(tile);
+                const uint32_t bytes = (uint32_t)moe_width(t.width, kMoeTileTokens) * 128u;
+                for (int kb = 0; kb < n_kb; ++kb, ++it) {
+                    const uint32_t s = it % kTmBStages;
+                    if (it >= kTmBStages) wait_one(b_empty[s], it / kTmBStages - 1, 4);
+                    if (!alive) break;
+                    mbar_arrive_expect_tx(smem_u32(&b_full[s]), bytes);
+                    tma_load_2d(smem0 + kTmOffB + s * kTmBStage, &maps.act[t.width], kb * kTmKBlock, t.slot0, smem_u32(&b_full[s]));
+                }
+            }
+            if (!alive)                         // gave up: let the copies in flight land before shared memory is released
+                for (uint32_t i = it > kTmBStages ? it - kTmBStages : 0; i < it; ++i)
+                    mbar_wait_limit(smem_u32(&b_full[i % kTmBStages]), (i / kTmBStages) & 1u, 0, 1u << 12);
+        }
+        __syncwarp();
+    } else if (warp == kTmWeightWarp) {
+        // ---- packed weights and their scale bytes (8 per row and stage)
+        uint32_t wi = 0;
+        for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+            const MoeTile t = decode(tile);
+            const long long first = (long long)t.e * a.rows + t.m0;
+            const uint8_t* s0 = a.wa_s + first * row_s;
+            const uint8_t* s1 = MODE == 0 ? a.wb_s + first * row_s : s0 + (long long)kMoeTileRows * row_s;
+            for (int wb = 0; wb < n_wb; ++wb, ++wi) {
+                const uint32_t ws = wi % kTmWStages;
+                if (wi >= kTmWStages) wait(w_empty[ws], wi / kTmWStages - 1, 4);
+                if (!alive) break;
+                const uint32_t bar = smem_u32(&w_full[ws]), dst = smem0 + ws * 2 * kTmWTile;
+                if (lane == 0) {
+                    mbar_arrive_expect_tx(bar, t.mats * kTmWTile);
+                    tma_load_2d(dst, &maps.wa, wb * 128, (int)first, bar);
+                    if (t.mats == 2) tma_load_2d(dst + kTmWTile, &maps.wb, wb * 128, (int)first + (MODE == 0 ? 0 : kMoeTileRows), bar);
+                }
+                const uint32_t sdst = smem0 + kTmOffS + ws * 2 * kTmWScale;
+#pragma unroll
+                for (int m = 0; m < 2; ++m)
+                    if (m < t.mats) {
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const int r = lane + 32 * i;
+                            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(sdst + m * kTmWScale + r * 8),
+                                         "l"((m == 0 ? s0 : s1) + (long long)r * row_s + wb * 8) : "memory");
                         }
                     }
+                asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
+            }
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        if (!alive)                             // gave up: let the copies in flight land before shared memory is released
+            for (uint32_t i = wi > kTmWStages ? wi - kTmWStages : 0; i < wi; ++i)
+                mbar_wait_limit(smem_u32(&w_full[i % kTmWStages]), (i / kTmWStages) & 1u, 0, 1u << 16);
+    } else if (warp == kTmMmaWarp) {
+        if (tc05_elect_one()) {
+            uint32_t it = 0;
+            for (int tile = blockIdx.x; tile < n_tiles && alive; tile += gridDim.x, ++tc) {
+                const MoeTile t = decode(tile);
+                const uint32_t idesc = tc05_idesc_f16(128, moe_width(t.width, kMoeTileTokens));
+                if (tc > 0) wait_one(acc_free, tc - 1, 7);
+                for (int kb = 0; kb < n_kb; ++kb, ++it) {
+                    const uint32_t as = it % kTmAStages, bs = it % kTmBStages;
+                    wait_one(b_full[bs], it / kTmBStages, 5);
+                    wait_one(a_full[as], it / kTmAStages, 5);
+                    if (!alive) break;
+                    tc05_fence_after_sync();
+                    const uint64_t db = tc05_desc_k_sw128(smem0 + kTmOffB + bs * kTmBStage);
+                    const uint32_t at = tmem + 256 + as * 64;
+                    if (t.mats == 2) {
+#pragma unroll
+                        for (int j = 0; j < kTmKBlock / 16; ++j) {
+                            const uint32_t acc = (kb > 0 || j > 0) ? 1u : 0u;
+                            tc05_mma_f16_ts(tmem, at + j * 8, db + 2 * j, idesc, acc);
+                            tc05_mma_f16_ts(tmem + kMoeTileTokens, at + 32 + j * 8, db + 2 * j, idesc, acc);
+                        }
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < kTmKBlock / 16; ++j)
+                            tc05_mma_f16_ts(tmem, at + j * 8, db + 2 * j, idesc, (kb > 0 || j > 0) ? 1u : 0u);
+                    }
+                    tc05_commit(smem_u32(&a_empty[as]));
+                    tc05_commit(smem_u32(&b_empty[bs]));
+                    if (kb == n_kb - 1) tc05_commit(smem_u32(&acc_full));
                 }
             }
         }
-        tc05_fence_before_sync();
-        __syncthreads();            // accumulators read, token tables free: the next tile may start
-        tc05_fence_after_sync();
+        __syncwarp();
+    } else {
+        // ---- a tile ahead of the others: the token tables, and the largest scale byte of every row
+        for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++tc) {
+            const MoeTile t = decode(tile);
+            const uint32_t tab = tc % kTmTables;
+            if (tc >= kTmTables) wait(tab_free[tab], tc / kTmTables - 1, 4);
+            for (int n = lane; n < t.n_valid; n += 32) {
+                const int slot = t.slot0 + n;
+                if (MODE == 0) {
+                    const int2 x = __ldcg(a.xexp + slot);
+                    tok_f0[tab][n] = float_pow2(x.x);
+                    tok_f1[tab][n] = float_pow2(-2 * x.y);
+                } else {
+                    const int me = __ldcg(a.mid_exp + slot), half = me >> 1;
+                    tok_f0[tab][n] = __ldcg(a.g.slot_w + slot) * float_pow2(half);
+                    tok_f1[tab][n] = float_pow2(me - half);
+                }
+            }
+            for (int m = 0; m < t.mats; ++m) {
+                const long long first = (long long)t.e * a.rows + t.m0 + (MODE == 1 ? m * kMoeTileRows : 0);
+                const uint8_t* base = (MODE == 0 && m == 1 ? a.wb_s : a.wa_s) + first * row_s;
+                const int n8 = row_s >> 3;
+                for (int i = 0; i < 4; i += 2) {              // two rows per lane at a time: 16 loads in flight
+                    const int r = lane + 32 * i;
+                    const uint2* p = reinterpret_cast<const uint2*>(base + (long long)r * row_s);
+                    uint32_t best[2] = {0, 0}, others[2] = {0, 0};      // `others`: bytes that are not 0xFF seen
+#pragma unroll 8
+                    for (int j = 0; j < n8; ++j)
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            const uint2 v = __ldg(p + j + h * 4 * row_s);      // 32 rows further down
+                            const uint32_t fx = __vcmpeq4(v.x, 0xffffffffu), fy = __vcmpeq4(v.y, 0xffffffffu);
+                            best[h] = __vmaxu4(best[h], __vmaxu4(v.x & ~fx, v.y & ~fy));
+                            others[h] |= ~fx | ~fy;
+                        }
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const uint32_t b = max(max(best[h] & 0xff, (best[h] >> 8) & 0xff), max((best[h] >> 16) & 0xff, best[h] >> 24));
+                        row_exp[tab][m][r + 32 * h] = others[h] ? (int)b : -1;
+                    }
+                }
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive_one(smem_u32(&exp_full[tab]));
+        }
     }
+    tc05_fence_before_sync();
     __syncthreads();
-    if (warp == kProducerWarps) tc05_dealloc(tmem, 256);
+    if (warp == kTmMmaWarp) tc05_dealloc(tmem, 512);
 }
 
 }  // namespace dsv4

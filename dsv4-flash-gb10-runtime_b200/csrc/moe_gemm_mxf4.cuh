@@ -1,26 +1,38 @@
 // Batched routed-expert GEMMs with BLOCK-SCALED tensor-core MMAs (tcgen05 kind::mxf4, UE8M0 scales in tensor
 // memory): the MXFP4 weights go from HBM to shared memory to the tensor cores exactly as the checkpoint stores them
 // (packed nibbles + E8M0 bytes) - no dequantisation instruction is executed, and a weight costs half a byte of
-// shared-memory traffic instead of the four bytes the fp16 path (moe_gemm_kernel.cuh) pays.
+// shared-memory traffic.
 //
 // The tensor cores multiply FP4 by FP4, so the activations are given as three MXFP4 terms (moe_prep.cuh):
 //   D = W * (q1 + q2 + q3) = W q1 + W q2 + W q3.
-// On B200 one tcgen05.mma of M = 128 occupies the tensor pipe for about the same ~190 clocks whether N is 32 or
-// 256 (measured), so the MMA count, not the flop count, decides the speed of this kernel.  The three terms are
-// therefore STACKED ALONG N: the B operand of a tile holds term 1 of its tokens in rows [0, n), term 2 in [n, 2n),
-// term 3 in [2n, 3n), and one MMA of N = 3n produces the three partial products in three column ranges of the
-// accumulator, which the epilogue adds.  When 3n > 256 (the MMA's largest N) the third term moves to row 256 and
-// gets an MMA of its own.
+// Tiles: two blocks of 256 weight rows (rows m0.. of W1 and of W3 for gate/up, rows m0.. and m0 + 256.. of W2 for down)
+// x up to 112 tokens, one tile per PAIR of CTAs (cta_group::2): each CTA holds 128 rows of both blocks and half of the
+// tokens.  A stage covers 256 K-elements (one 128-byte swizzled row per operand row = 4 MMAs of K = 64).
 //
-// Tiles: two blocks of 128 weight rows (two accumulators: rows m0.. of W1 and of W3 for gate/up, rows m0.. and
-// m0 + 128.. of W2 for down) x up to 64 tokens; a stage covers 256 K-elements (one 128-byte swizzled row per operand row = 4 MMAs of K = 64).  Per stage
-// the 16 producer warps copy with cp.async: the packed weight rows, the three packed activation terms of the
-// tile's tokens, and the scale bytes re-arranged into 512-byte scale atoms; one lane of the last warp copies the
-// atoms into tensor memory (tcgen05.cp) and issues the MMAs; tcgen05.commit releases the stage.  Persistent grid,
-// one CTA per SM.  Producers and the MMA warp run ahead across tile boundaries: the producers start filling the
-// stages of the next tile while the last MMAs of the current one are in flight, then (all 16 warps, four per lane
-// quadrant of tensor memory) drain the finished accumulator and hand it back to the MMA warp through an mbarrier.
-// Every wait is bounded.
+// How the terms are multiplied.  Each term is an MMA of its own into the SAME accumulator columns, with the weight tile
+// kept in the collector between the three: 3 x N / 2 clocks for N tokens (N >= 96), the full rate of the tensor pipe;
+// a stage's 24 MMAs and 10 scale copies take 1 170 clocks at N = 96 and 580 at N = 16.  Without the collector every MMA
+// reads its A tile again, 32 clocks at 128 bytes a clock.  Two accumulator sets of 2 x 112 columns fit into tensor memory,
+// so the MMAs of a tile run while the one before it is read out.
+//
+// What bounds it: the weights.  A CTA takes in 34 KB of weights and scales per stage, 1 400 clocks of its share of 7 TB/s,
+// so everything else has to keep out of the way of that stream, above all instruction issue: with six roles on a CTA an
+// instruction of a single-thread role takes tens of clocks, not four.  Hence few instructions per stage: ONE producer
+// thread with three copies (two weight boxes, one box with the three terms of the CTA's tokens - the rows of a tile are
+// neighbours in memory, in slot order), ONE full and ONE empty barrier.  Gathering token rows four at a time instead took
+// 36 copies per stage and held the stream at 4.6 TB/s.  Why pairs: they halve the activations a CTA takes in.
+//
+// CTA = 14 warps, persistent grid, one CTA per SM, tiles by static striding over the pairs:
+//   warps 0..7    epilogue: accumulators -> SwiGLU -> three MXFP4 terms (gate/up), or -> FP32 rows (down)
+//   warps 8..11   scale bytes of weights and activations -> 512-byte scale atoms in shared memory, two to four stages of
+//                 loads ahead
+//   warp 12       producer (one thread)
+//   warp 13       (CTA 0, one thread) scale atoms -> tensor memory, MMAs of the pair
+// The full barriers are CTA 0's: copies and scale warps of both CTAs arrive there.  The "empty" and "accumulator full"
+// barriers are signalled in both CTAs by the commits.
+// No operand passes through a register.
+// Every wait is bounded; a CTA that gives up has polled far longer than any copy takes, so nothing is in flight when it
+// leaves, and both CTAs meet at a cluster barrier before they exit.
 #pragma once
 
 #include "moe_gemm.cuh"
@@ -29,349 +41,407 @@ namespace dsv4 {
 
 constexpr int kQKBlock = 256;                        // K-elements per stage
 constexpr int kQTerms = 3;                           // activation terms
+constexpr int kQTok = 112;                           // tokens per tile at most
 constexpr uint32_t kQTile = 128 * 128;               // bytes of one packed weight tile (128 rows x 128 B)
-constexpr int kQTokUp = 64;                          // tokens per tile (3 x 64 = 192 accumulator columns x 2)
-constexpr int kQTokDown = 64;
-constexpr int kQRowsDown = 256;                      // W2 rows per down tile (two row blocks share the activation tile)
+constexpr uint32_t kQBStage = kQTerms * (kQTok / 2) * 128;           // activation rows of one stage and CTA
+constexpr uint32_t kQSfStage = 2 * 2 * 512 + 2 * kQTerms * 512;      // scale atoms: [mat][atom], then [atom][term]
+constexpr int kQStages = 3;
+constexpr int kQEpiWarps = 8, kQScaleWarps = 4;
+constexpr int kQScaleWarp = kQEpiWarps, kQProducerWarp = kQScaleWarp + kQScaleWarps, kQMmaWarp = kQProducerWarp + 1;
+constexpr int kQThreads = (kQMmaWarp + 1) * 32;
+constexpr uint32_t kQAccCols = 2 * kQTok;            // per accumulator set
+constexpr uint32_t kQSfCol = 2 * kQAccCols, kQSfCols = 16 + 8 * kQTerms;
+static_assert(kQSfCol + kQSfCols <= 512, "tensor memory overflow");
+constexpr uint32_t kQOffB = kQStages * 2 * kQTile, kQOffSf = kQOffB + kQStages * kQBStage;
+constexpr uint32_t kQOffTables = kQOffSf + kQStages * kQSfStage;
+// dynamic shared memory: stages, then the tile and offset tables of the experts
+__host__ __device__ __forceinline__ uint32_t moe_q_smem_bytes(int n_experts) { return kQOffTables + 8 * (uint32_t)(n_experts + 1) + 1024; }
+static_assert(kQOffTables + 8 * (kMoeMaxExperts + 1) + 1024 + 1024 <= 227 * 1024, "shared memory overflow");
 
 struct MoeQGemmArgs {
-    const uint8_t* wa_p; const uint8_t* wb_p;        // up: W1, W3 packed; down: W2
-    const uint8_t* wa_s; const uint8_t* wb_s;
-    long long stride_p, stride_s;                    // bytes per expert
-    int rows, K, n_experts, k_top;
-    const uint8_t* act_q;                            // [3][act_rows][K / 2]
-    const uint8_t* act_s;                            // [3][act_rows][K / 32]
-    long long act_rows;                              // rows of the activation matrix (tokens for up, pairs for down)
-    const float* pair_w;                             // [P] router weights (down)
+    const uint8_t* wa_s; const uint8_t* wb_s;        // E8M0 scales: up W1, W3; down W2 (wb unused)
+    int rows, K, n_experts;
+    const uint8_t* act_s;                            // [3][P][K / 32]
+    long long n_pairs;
     MoeGroups g;
-    float* mid;                                      // up output [P, rows] FP32
+    uint8_t* mid_q; uint8_t* mid_s;                  // up output [3][P][rows / 2], [3][P][rows / 32]
     float* y;                                        // down output [P, rows] FP32
 };
+// Weight boxes of 128 rows; activation boxes of 3 terms x half a tile's columns, one per column count.
+struct MoeQMaps { CUtensorMap wa, wb, act[kMoeWidths]; };
+
+// What a tile is: expert, tokens, and the first weight row of the pair's first block; the same in both CTAs.
+struct MoeQTile { int e, slot0, n_valid, width, m0, mats; };
+constexpr int kQRows = 2 * kMoeTileRows;             // weight rows of one block of a pair
+constexpr int kQTileRowsUp = kQRows, kQTileRowsDown = 2 * kQRows;
 
 template <int MODE>
-struct MoeQGemmLayout {
-    static constexpr int kMats = 2;
-    static constexpr int kTok = MODE == 0 ? kQTokUp : kQTokDown;
-    static constexpr int kStages = 3;
-    // rows of the stacked B operand: contiguous when the three terms fit one MMA, else term 3 at row 256
-    static constexpr int kBRows = 3 * kTok <= 256 ? 3 * kTok : 256 + kTok;
-    static constexpr int kRowGroups = (kBRows + 127) / 128;                  // scale atoms cover 128 rows
-    static constexpr uint32_t kOffB = kMats * kQTile;
-    static constexpr uint32_t kOffSfA = kOffB + kBRows * 128;
-    static constexpr uint32_t kOffSfB = kOffSfA + kMats * 1024;              // [mat][k-atom] x 512 B
-    static constexpr uint32_t kStageBytes = kOffSfB + 2 * kRowGroups * 512;  // [k-atom][row group] x 512 B
-    static constexpr uint32_t kBytes = kStages * kStageBytes + 1024;
-    // tensor memory: accumulators (one column per B row) first, then per stage the scale columns
-    static constexpr uint32_t kAccStride = kBRows;
-    static constexpr uint32_t kAccCols = kMats * kAccStride;
-    static constexpr uint32_t kSfBCol = kMats * 8;                           // B scales after the A scales
-    static constexpr uint32_t kSfColsPerStage = kMats * 8 + 2 * kRowGroups * 4;
-    static_assert(kStageBytes % 1024 == 0, "stage size must keep tiles 1024-byte aligned");
-    static_assert(kAccCols + kStages * kSfColsPerStage <= 512, "tensor memory overflow");
-    static_assert(kMats * 128 + kQTerms * kTok <= kGemmProducers, "one scale row per producer thread");
-    static_assert(kBytes <= 227 * 1024, "shared memory overflow");
-    static_assert(kTok <= 64, "the drain handles one 16-token chunk per warp");
-};
-
-// What a tile is: expert, rows, tokens; identical in every thread of the CTA.
-struct MoeQTile {
-    int e, slot0, n_valid, n_mma, m0, term_row2, mats;
-    bool split;
-};
-
-// tiles / offsets: the grouping kernel's prefix sums, staged in shared memory by the caller.
-template <int TOK>
 __device__ __forceinline__ MoeQTile moe_qtile_decode(const int* tiles, const int* offsets, int n_experts, int m_tiles,
-                                                     int tile_rows, int rows, int tile) {
-    int lo = 0, hi = n_experts;
+                                                     int rows, int tile) {
+    int lo = 0, hi = n_experts;                      // last expert with tiles[e] <= tile
     while (hi - lo > 1) {
         const int md = (lo + hi) >> 1;
         if (tiles[md] <= tile) lo = md; else hi = md;
     }
     MoeQTile t;
     t.e = lo;
-    const int local = tile - tiles[lo];
-    const int nt = local / m_tiles, mt = local - nt * m_tiles;
-    t.slot0 = offsets[lo] + nt * TOK;
-    t.n_valid = min(TOK, offsets[lo + 1] - t.slot0);
-    t.n_mma = (t.n_valid + 15) & ~15;
-    t.m0 = mt * tile_rows;
-    t.mats = (tile_rows == 2 * kMoeTileRows && t.m0 + kMoeTileRows >= rows) ? 1 : 2;   // a last, half down tile
-    t.split = 3 * t.n_mma > 256;                       // B rows (= accumulator columns) of the three terms
-    t.term_row2 = t.split ? 256 : 2 * t.n_mma;
+    const int local = tile - tiles[lo], nt = local / m_tiles;
+    const int per = moe_tokens_per_tile(offsets[lo + 1] - offsets[lo], kQTok);
+    t.slot0 = offsets[lo] + nt * per;
+    t.n_valid = min(per, offsets[lo + 1] - t.slot0);
+    t.width = moe_width_index(t.n_valid);
+    t.m0 = (local - nt * m_tiles) * (MODE == 0 ? kQTileRowsUp : kQTileRowsDown);
+    t.mats = (MODE == 1 && t.m0 + kQRows >= rows) ? 1 : 2;             // a last, half down tile
     return t;
 }
 
+// A position in a ring of stages: slot and the number of times it has been filled before.
+struct RingPos {
+    uint32_t slot = 0, round = 0;
+    __device__ __forceinline__ void next(uint32_t n) { if (++slot == n) { slot = 0; ++round; } }
+};
+
+// TMA loads of a CTA of a pair, into its own shared memory, counted on a barrier that may be the other CTA's (no
+// multicast).
+__device__ __forceinline__ void tma_pair_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%2, %3}], [%4];"
+                 ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void tma_pair_load_3d(uint32_t dst, const CUtensorMap* map, int x, int y, int z, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%2, %3, %4}], [%5];"
+                 ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar) : "memory");
+}
+
+// The MMAs of one stage, by one thread, as straight-line code: a branch or a descriptor put together between two of them
+// costs about 30 clocks, half of what the MMA itself takes.  The scale columns are the same in every stage: scale
+// copies and MMAs of one thread execute in the order they are issued.
+struct MoeQStage {
+    uint64_t w, b;                                   // descriptors of the first weight tile and of term 1
+    uint32_t sf, acc, sfa, b_term, idesc[2];
+    bool fresh;                                      // first stage of a tile: overwrite the accumulators
+};
+template <int MATS>
+__device__ __forceinline__ void moe_q_issue(const MoeQStage& q) {
+    const uint32_t sfb = q.sfa + 16;                 // columns: A [mat][atom] x 4, B [atom][term] x 4
+#pragma unroll
+    for (int at = 0; at < 2; ++at) {
+#pragma unroll
+        for (int m = 0; m < MATS; ++m) tc05_pair_copy_scale_atom(q.sfa + m * 8 + at * 4, q.sf + m * 1024 + at * 512);
+#pragma unroll
+        for (int i = 0; i < kQTerms; ++i)
+            tc05_pair_copy_scale_atom(sfb + (at * kQTerms + i) * 4, q.sf + 2048 + (at * kQTerms + i) * 512);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)                      // K-steps of 64 (32 bytes)
+#pragma unroll
+        for (int m = 0; m < MATS; ++m) {
+            const uint64_t da = q.w + m * (kQTile >> 4) + 2 * j;
+            const uint32_t d = q.acc + m * kQTok, sa = q.sfa + m * 8 + (j >> 1) * 4, sb = sfb + (j >> 1) * kQTerms * 4;
+            // the three terms multiply the same A: read once, kept in the collector
+            tc05_pair_mma_mxf4<kAFill>(d, da, q.b + 2 * j, q.idesc[j & 1], sa, sb, (j > 0 || !q.fresh) ? 1u : 0u);
+            tc05_pair_mma_mxf4<kAUse>(d, da, q.b + q.b_term + 2 * j, q.idesc[j & 1], sa, sb + 4, 1u);
+            tc05_pair_mma_mxf4<kALast>(d, da, q.b + 2 * q.b_term + 2 * j, q.idesc[j & 1], sa, sb + 8, 1u);
+        }
+}
+
+// Tokens and lanes trade places: on entry v[i] is token i of row `lane` of a 32-row block, on return v[j] is row
+// 16 (lane / 16) + j of token lane % 16 (a 16 x 16 transpose in each half of the warp, four exchange steps).
+__device__ __forceinline__ void moe_transpose16(float (&v)[16], int lane) {
+#pragma unroll
+    for (int bit = 8; bit > 0; bit >>= 1) {
+        const bool up = (lane & bit) != 0;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            if (i & bit) continue;
+            const float lo = v[i], hi = v[i + bit];
+            const float got = __shfl_xor_sync(kFullMask, up ? lo : hi, bit);
+            v[i] = up ? got : lo;
+            v[i + bit] = up ? hi : got;
+        }
+    }
+}
+
+// Half a 32-element block per lane (the other half in lane ^ 16) -> three MXFP4 terms: 8 packed bytes and the block's
+// scale byte each.  The rule of the terms is moe_quantize_mxfp4x3's; the residual is kept in units of the last scale, so that a
+// term needs no multiplication back.
+__device__ __forceinline__ void moe_quantize_half_block(float (&v)[16], uint2 (&packed)[kQTerms], uint32_t (&scale)[kQTerms]) {
+    int unit = 127;                                  // v is in units of 2^(unit - 127)
+#pragma unroll
+    for (int t = 0; t < kQTerms; ++t) {
+        uint32_t m = 0;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) m = max(m, __float_as_uint(v[i]) & 0x7fffffffu);
+        m = max(m, __shfl_xor_sync(kFullMask, m, 16));
+        int e = (int)((m + 0x003fffffu) >> 23) - 2 + (unit - 127);        // biased; smallest with amax <= 6 * 2^(e - 127)
+        e = min(max(e, 0), 254);
+        const float inv = __uint_as_float((uint32_t)min(max(127 + unit - e, 1), 254) << 23);
+        unit = e;
+        scale[t] = (uint32_t)e;
+        uint32_t r[2] = {0, 0};
+#pragma unroll
+        for (int i = 0; i < 16; i += 2) {
+            uint16_t q;
+            v[i] *= inv;
+            v[i + 1] *= inv;
+            asm("{\n .reg .b8 b;\n cvt.rn.satfinite.e2m1x2.f32 b, %2, %1;\n mov.b16 %0, {b, 0};\n}"
+                : "=h"(q) : "f"(v[i]), "f"(v[i + 1]));
+            if (t + 1 < kQTerms) {
+                const float2 back = e2m1x2_to_float2(q);
+                v[i] -= back.x;
+                v[i + 1] -= back.y;
+            }
+            r[i >> 3] |= (uint32_t)(q & 0xff) << (4 * (i & 7));
+        }
+        packed[t] = make_uint2(r[0], r[1]);
+    }
+}
+
 template <int MODE>
-__global__ void __launch_bounds__(kGemmThreads, 1) moe_gemm_mxf4_kernel(const MoeQGemmArgs a) {
-    using L = MoeQGemmLayout<MODE>;
-    constexpr int S = L::kStages;
-    constexpr int MATS = L::kMats;
-    constexpr int TOK = L::kTok;
-    constexpr int RG = L::kRowGroups;
-    constexpr int kProducerWarps = kGemmProducers / 32;
-    constexpr int kBChunks = (TOK * 8 + kGemmProducers - 1) / kGemmProducers;   // 16-byte chunks per thread and term
+__global__ void __launch_bounds__(kQThreads, 1) moe_gemm_mxf4_kernel(const __grid_constant__ MoeQMaps maps,
+                                                                                              const MoeQGemmArgs a) {
     extern __shared__ __align__(1024) uint8_t gemm_smem[];
-    __shared__ __align__(8) uint64_t bar_full[S], bar_empty[S], bar_accum, bar_acc_free;
+    __shared__ __align__(8) uint64_t full[kQStages], empty[kQStages], acc_full[2], acc_free[2];
     __shared__ uint32_t tmem_holder;
-    // Token tables, three deep: producers fill the table of tile N + 1 before its barrier while another warp may still
-    // be draining tile N - 1 (the drain runs inside tile N's loop), so two tables are not enough when a tile has
-    // few K steps (hidden <= 1536); a warp cannot get two tiles ahead of another warp's drain.
-    __shared__ int tok_row[3][128];          // activation row of every token of the tile (by tile number mod 3)
-    __shared__ float tok_w[3][128];          // router weight of every token (down)
-    __shared__ int s_tiles[kMoeMaxExperts + 1], s_offsets[kMoeMaxExperts + 1];
-    pdl_launch_dependents();
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const bool producer = warp < kProducerWarps;
-    const int n_kb = a.K / kQKBlock;
-    const int row_p = a.K >> 1, row_s = a.K >> 5;
+    const int n_st = a.K / kQKBlock, row_s = a.K >> 5;
+    const uint32_t smem_w = smem_u32(gemm_smem), smem_b = smem_w + kQOffB, smem_sf = smem_w + kQOffSf;
+    int* const s_tiles = reinterpret_cast<int*>(gemm_smem + kQOffTables);
+    int* const s_offsets = s_tiles + a.n_experts + 1;
 
-    if (warp == kProducerWarps) tc05_alloc(smem_u32(&tmem_holder), 512);
+    if (warp == kQMmaWarp) tc05_pair_alloc(smem_u32(&tmem_holder), 512);
     if (tid == 0) {
-        for (int s = 0; s < S; ++s) { mbar_init(smem_u32(&bar_full[s]), kGemmProducers); mbar_init(smem_u32(&bar_empty[s]), 1); }
-        mbar_init(smem_u32(&bar_accum), 1);
-        mbar_init(smem_u32(&bar_acc_free), kGemmProducers);
+        for (int s = 0; s < kQStages; ++s) { mbar_init(smem_u32(&full[s]), 2 * (1 + kQScaleWarps)); mbar_init(smem_u32(&empty[s]), 1); }
+        for (int s = 0; s < 2; ++s) { mbar_init(smem_u32(&acc_full[s]), 1); mbar_init(smem_u32(&acc_free[s]), 2 * kQEpiWarps); }
         mbar_init_fence();
     }
-    pdl_wait();
-    for (int i = tid; i <= a.n_experts; i += kGemmThreads) {
-        s_tiles[i] = (MODE == 0 ? a.g.tiles_up : a.g.tiles_down)[i];
-        s_offsets[i] = a.g.offsets[i];
+    // The tables come from the kernel before the one this launch depends on: a grid starts its dependents only after its own
+    // wait, so that kernel is complete; what the previous kernel wrote (the activations) is waited for by the roles that
+    // read it, and the first weights are requested before that.
+    for (int i = tid; i <= a.n_experts; i += kQThreads) {
+        s_tiles[i] = __ldcg((MODE == 0 ? a.g.tiles_up : a.g.tiles_down) + i);
+        s_offsets[i] = __ldcg(a.g.offsets + i);
     }
     tc05_fence_before_sync();
-    __syncthreads();
+    cluster_sync_all();                                       // barriers of both CTAs are initialised
     tc05_fence_after_sync();
     const uint32_t tmem = tmem_holder;
-
-    const int* tiles = s_tiles;
-    const int n_tiles = tiles[a.n_experts];
-    // gate/up: 128 rows of W1 and the same 128 rows of W3; down: 256 rows of W2 (the last tile may hold 128)
-    const int tile_rows = MODE == 0 ? kMoeTileRows : kQRowsDown;
-    const int m_tiles = (a.rows + tile_rows - 1) / tile_rows;
-    uint32_t it = 0, tile_count = 0;
+    const int rank = (int)cluster_rank(), pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
+    auto leader = [&](uint64_t& bar) { return cluster_map(smem_u32(&bar), 0); };
+    const int n_tiles = s_tiles[a.n_experts];
+    const int m_tiles = (a.rows + (MODE == 0 ? kQTileRowsUp : kQTileRowsDown) - 1) / (MODE == 0 ? kQTileRowsUp : kQTileRowsDown);
+    auto decode = [&](int tile) { return moe_qtile_decode<MODE>(s_tiles, s_offsets, a.n_experts, m_tiles, a.rows, tile); };
     bool alive = true;
+    auto wait = [&](uint64_t& bar, uint32_t parity, int code) {            // roles of whole warps
+        if (alive) alive = __all_sync(kFullMask, mbar_wait_bounded(smem_u32(&bar), parity & 1u, code));
+    };
+    auto wait_one = [&](uint64_t& bar, uint32_t parity, int code) {        // roles of one thread
+        if (alive) alive = mbar_wait_bounded(smem_u32(&bar), parity & 1u, code);
+    };
+    uint32_t tc = 0;                                          // tiles begun by this pair
 
-    if (producer) {
-        // ---- drain of a finished accumulator: warps q, q + 4, q + 8, q + 12 own lane quadrant q (rows 32 q ..)
-        // and share its token chunks of 16; a token's value is the sum of its three term columns (term order)
-        auto drain = [&](const MoeQTile& t, uint32_t count) {
-            if (alive) alive = mbar_wait_bounded(smem_u32(&bar_accum), count & 1, 6);
+    if (warp < kQEpiWarps) {
+        const int quad = warp & 3, r = quad * 32 + lane;
+        pdl_wait();
+        for (int tile = pair; tile < n_tiles; tile += n_pairs, ++tc) {
+            const MoeQTile t = decode(tile);
+            const uint32_t buf = tc & 1u;
+            const int m0 = t.m0 + rank * kMoeTileRows;        // first row of this CTA in block 0
+            // router weights (down): lane i holds those of tokens i and i + 16 of this warp's chunks, see below
+            float w[4];
+            if (MODE == 1)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int n = (warp >> 2) * 16 + 32 * i + (lane & 15);
+                    w[i] = n < t.n_valid ? __ldcg(a.g.slot_w + t.slot0 + n) : 0.f;
+                }
+            wait(acc_full[buf], tc >> 1, 6);
             tc05_fence_after_sync();
-            const int quad = warp & 3;
-            const int r = quad * 32 + lane;
-            const uint32_t trow = tmem + ((uint32_t)(quad * 32) << 16);
-            const float* w_of = tok_w[count % 3u];
-            auto hand_back = [&]() {
-                // this thread's last read of the accumulator and of the token tables is done
-                tc05_fence_before_sync();
-                asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&bar_acc_free)) : "memory");
-            };
-            // the three term columns of 16 tokens in flight together, one wait; summed in term order
-            auto load_sum = [&](uint32_t col, float (&v)[16]) {
-                uint32_t p0[16], p1[16], p2[16];
-                tc05_ld16_issue(trow + col, p0);
-                tc05_ld16_issue(trow + t.n_mma + col, p1);
-                tc05_ld16_issue(trow + t.term_row2 + col, p2);
+            const uint32_t trow = tmem + ((uint32_t)(quad * 32) << 16) + buf * kQAccCols;
+            // two warps per lane quadrant take chunks of 16 tokens in turn
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int c = (warp >> 2) * 16 + 32 * k;
+                if (c >= t.n_valid || !alive) break;
+                const int n = min(16, t.n_valid - c);
+                uint32_t p0[16], p1[16];
+                tc05_ld16_issue(trow + c, p0);
+                tc05_ld16_issue(trow + kQTok + c, p1);        // stale, and not used, in a half tile
                 tc05_wait_ld();
+                if (MODE == 0) {
+                    float g[16];
 #pragma unroll
-                for (int i = 0; i < 16; ++i)
-                    v[i] = (__uint_as_float(p0[i]) + __uint_as_float(p1[i])) + __uint_as_float(p2[i]);
+                    for (int i = 0; i < 16; ++i) {
+                        const float gate = __uint_as_float(p0[i]);
+                        g[i] = i < n ? __fdividef(gate, 1.0f + __expf(-gate)) * __uint_as_float(p1[i]) : 0.f;
+                    }
+                    moe_transpose16(g, lane);
+                    uint2 packed[kQTerms];
+                    uint32_t scale[kQTerms];
+                    moe_quantize_half_block(g, packed, scale);
+                    const int i = lane & 15;
+                    const long long slot = t.slot0 + c + i;
+                    if (i < n) {
+                        const int h0 = m0 + quad * 32;
+#pragma unroll
+                        for (int q = 0; q < kQTerms; ++q) {
+                            *reinterpret_cast<uint2*>(a.mid_q + (q * a.n_pairs + slot) * (a.rows >> 1) + (h0 >> 1) + (lane >> 4) * 8) = packed[q];
+                            if (lane < 16) a.mid_s[(q * a.n_pairs + slot) * (a.rows >> 5) + (h0 >> 5)] = (uint8_t)scale[q];
+                        }
+                    }
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) {
+                        const float wi = __shfl_sync(kFullMask, w[k], i);
+                        if (i < n) {
+                            float* yrow = a.y + (size_t)(t.slot0 + c + i) * a.rows + m0 + r;
+                            if (m0 < a.rows) yrow[0] = __uint_as_float(p0[i]) * wi;                  // (a.rows is a multiple of 128)
+                            if (m0 + kQRows < a.rows) yrow[kQRows] = __uint_as_float(p1[i]) * wi;
+                        }
+                    }
+                }
+            }
+            tc05_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(leader(acc_free[buf]));
+        }
+    } else if (warp < kQProducerWarp) {
+        // ---- scale bytes: 8 per row and stage.  Thread st holds weight row st of both matrices and up to three of the
+        // (term, token) rows; the loads of a stage are issued two to four stages before their bytes are stored.
+        const int st = tid - kQScaleWarp * 32;
+        RingPos pos;
+        pdl_wait();
+        for (int tile = pair; tile < n_tiles; tile += n_pairs) {
+            const MoeQTile t = decode(tile);
+            const uint8_t* src[2 + kQTerms];
+            uint32_t dst[2 + kQTerms];
+            const int m0 = t.m0 + rank * kMoeTileRows;
+            const long long first = (long long)t.e * a.rows + m0 + st;
+            src[0] = m0 < a.rows ? a.wa_s + first * row_s : nullptr;
+            src[1] = MODE == 0 ? a.wb_s + first * row_s : m0 + kQRows < a.rows ? a.wa_s + (first + kQRows) * row_s : nullptr;
+            dst[0] = tc05_scale_atom_offset(st, 0);
+            dst[1] = dst[0] + 1024;
+#pragma unroll
+            for (int i = 0; i < kQTerms; ++i) {               // thread st: token st of every term
+                dst[2 + i] = 2048 + i * 512 + dst[0];
+                src[2 + i] = st < t.n_valid ? a.act_s + (i * a.n_pairs + t.slot0 + st) * row_s : nullptr;
+            }
+            // two stages (16 bytes of a row) per load, one load where the rows are 16-byte aligned
+            uint4 v[2][2 + kQTerms];
+            auto fetch = [&](uint4 (&to)[2 + kQTerms], int s) {
+                if (s >= n_st) return;
+#pragma unroll
+                for (int i = 0; i < 2 + kQTerms; ++i) {
+                    if (!src[i]) continue;
+                    if ((row_s & 15) == 0) {
+                        to[i] = __ldcg(reinterpret_cast<const uint4*>(src[i] + 8 * s));
+                    } else {
+                        const uint2* p = reinterpret_cast<const uint2*>(src[i] + 8 * s);
+                        const uint2 lo = __ldcg(p), hi = s + 1 < n_st ? __ldcg(p + 1) : make_uint2(0, 0);
+                        to[i] = make_uint4(lo.x, lo.y, hi.x, hi.y);
+                    }
+                }
             };
-            const int ca = (warp >> 2) * 16;                      // this warp's 16 tokens (TOK <= 64: one chunk per warp)
-            const bool has_a = ca < t.n_mma && alive;
-            {
-                // both accumulators of this warp's 16 tokens: gate and up (SwiGLU), or two row blocks of W2
-                float g[16], u[16];
-                if (has_a) {
-                    load_sum(ca, g);
-                    if (t.mats == 2) load_sum(L::kAccStride + ca, u);
-                    if (MODE == 1) {
+            auto put = [&](const uint4 (&from)[2 + kQTerms], bool second) {
+                if (pos.round > 0) wait(empty[pos.slot], pos.round - 1, 4);
+                const uint32_t sf = smem_sf + pos.slot * kQSfStage;
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) {
-                            const float w = ca + i < t.n_valid ? w_of[ca + i] : 0.f;
-                            g[i] *= w;
-                            u[i] *= w;
-                        }
+                for (int i = 0; i < 2 + kQTerms; ++i)
+                    if (src[i]) {                             // scales 0..3 -> atom 0, 4..7 -> atom 1
+                        asm volatile("st.shared.u32 [%0], %1;" ::"r"(sf + dst[i]), "r"(second ? from[i].z : from[i].x) : "memory");
+                        asm volatile("st.shared.u32 [%0], %1;" ::"r"(sf + dst[i] + (i < 2 ? 512u : kQTerms * 512u)), "r"(second ? from[i].w : from[i].y) : "memory");
                     }
-                }
-                hand_back();
-                if (has_a) {
-#pragma unroll
-                    for (int i = 0; i < 16; ++i)
-                        if (ca + i < t.n_valid) {
-                            if (MODE == 0) {
-                                a.mid[(size_t)(t.slot0 + ca + i) * a.rows + t.m0 + r] = (g[i] / (1.0f + __expf(-g[i]))) * u[i];
-                            } else {
-                                float* yrow = a.y + (size_t)(t.slot0 + ca + i) * a.rows + t.m0 + r;
-                                yrow[0] = g[i];
-                                if (t.mats == 2) yrow[kMoeTileRows] = u[i];
-                            }
-                        }
-                }
-            }
-        };
-
-        MoeQTile prev;
-        bool has_prev = false;
-        const int drain_at = min(S, n_kb) - 1;        // the stage after whose issue the previous tile is drained
-        for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++tile_count) {
-            const MoeQTile t = moe_qtile_decode<TOK>(tiles, s_offsets, a.n_experts, m_tiles, tile_rows, a.rows, tile);
-            int* rows_of = tok_row[tile_count % 3u];
-            if (tid < t.n_valid) {
-                const int slot = t.slot0 + tid;
-                const int pair = a.g.slot_pair[slot];
-                rows_of[tid] = MODE == 0 ? pair / a.k_top : slot;
-                if (MODE == 1) tok_w[tile_count % 3u][tid] = a.pair_w[pair];
-            }
-            asm volatile("bar.sync 1, %0;" ::"n"(kGemmProducers) : "memory");
-
-            // what this thread copies in every stage
-            // weights: chunk (row, c) of each matrix; 128 rows x 8 chunks = 1024 per matrix, 2 per thread
-            const int wr[2] = {tid >> 3, (tid + kGemmProducers) >> 3};
-            const int wc = tid & 7;
-            const uint8_t* wsrc[MATS][2];
-#pragma unroll
-            for (int m = 0; m < MATS; ++m)
-#pragma unroll
-                for (int h = 0; h < 2; ++h)
-                    wsrc[m][h] = (MODE == 0 ? (m == 0 ? a.wa_p : a.wb_p) + t.e * a.stride_p + (long long)(t.m0 + wr[h]) * row_p
-                                            : a.wa_p + t.e * a.stride_p + (long long)(t.m0 + kMoeTileRows * m + wr[h]) * row_p) +
-                                 wc * 16;
-            // activations: chunk (token, c) of each term
-            const uint8_t* bsrc[kBChunks];
-            bool bok[kBChunks], bwrite[kBChunks];
-#pragma unroll
-            for (int h = 0; h < kBChunks; ++h) {
-                bok[h] = wr[h] < t.n_valid;
-                bwrite[h] = wr[h] < t.n_mma;
-                bsrc[h] = a.act_q + (long long)(bok[h] ? rows_of[wr[h]] : 0) * row_p + wc * 16;
-            }
-            // scales: one row of 8 bytes per thread; threads [0, 128 MATS) the weight rows, then TOK per term
-            const uint8_t* sfsrc = nullptr;
-            uint32_t sfdst = 0;
-            bool sfok = false;
-            if (tid < MATS * 128) {
-                const int m = tid >> 7, r = tid & 127;
-                sfsrc = MODE == 0 ? (m == 0 ? a.wa_s : a.wb_s) + t.e * a.stride_s + (long long)(t.m0 + r) * row_s
-                                  : a.wa_s + t.e * a.stride_s + (long long)(t.m0 + kMoeTileRows * m + r) * row_s;
-                sfdst = L::kOffSfA + m * 1024 + tc05_scale_atom_offset(r, 0);
-                sfok = m < t.mats;
-                if (!sfok) sfsrc = nullptr;
-            } else if (tid < MATS * 128 + kQTerms * TOK) {
-                const int idx = tid - MATS * 128;
-                const int term = idx / TOK, n = idx - term * TOK;
-                if (n < t.n_mma) {
-                    const int brow = (term == 2 ? t.term_row2 : term * t.n_mma) + n;
-                    sfok = true;
-                    sfdst = L::kOffSfB + (brow >> 7) * 512 + tc05_scale_atom_offset(brow & 127, 0);
-                    if (n < t.n_valid)                                // padding rows: scale 1, data 0
-                        sfsrc = a.act_s + (long long)term * a.act_rows * row_s + (long long)rows_of[n] * row_s;
-                }
-            }
-            const uint32_t sf_atom_stride = tid < MATS * 128 ? 512u : (uint32_t)RG * 512u;   // k-atom 0 -> 1
-
-            // Weights and activation terms go global -> shared memory with asynchronous 16-byte copies (no
-            // registers in between).  Every producer thread makes the stage's "full" barrier arrive when ITS copies
-            // have landed (cp.async.mbarrier.arrive), so a stage is published the moment its last byte arrives
-            // while the thread is already filling the next free stage.
-            for (int kb = 0; kb < n_kb; ++kb, ++it) {
-                uint2 sv = make_uint2(0x7f7f7f7fu, 0x7f7f7f7fu);
-                if (sfsrc) sv = __ldcg(reinterpret_cast<const uint2*>(sfsrc + (size_t)kb * 8));
-                const uint32_t s = it % S;
-                if (it >= (uint32_t)S && alive)
-                    alive = mbar_wait_bounded(smem_u32(&bar_empty[s]), ((it / S) - 1) & 1, 4);
-                const uint32_t stage = smem_u32(gemm_smem) + s * L::kStageBytes;
-#pragma unroll
-                for (int m = 0; m < MATS; ++m)
-                    if (m < t.mats) {
-#pragma unroll
-                        for (int h = 0; h < 2; ++h)
-                            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(stage + m * kQTile + tc05_sw128_offset(wr[h], wc)),
-                                         "l"(wsrc[m][h] + (size_t)kb * 128) : "memory");
-                    }
-#pragma unroll
-                for (int term = 0; term < kQTerms; ++term) {
-                    const int base_row = term == 2 ? t.term_row2 : term * t.n_mma;
-#pragma unroll
-                    for (int h = 0; h < kBChunks; ++h)
-                        if (bwrite[h])      // rows past the expert's tokens: source size 0 = zero fill
-                            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(stage + L::kOffB + tc05_sw128_offset(base_row + wr[h], wc)),
-                                         "l"(bsrc[h] + (long long)term * a.act_rows * row_p + (size_t)kb * 128), "r"(bok[h] ? 16 : 0) : "memory");
-                }
-                if (sfok) {
-                    // scales 0..3 -> k-atom 0, 4..7 -> k-atom 1; the four bytes of a row are one aligned word
-                    asm volatile("st.shared.u32 [%0], %1;" ::"r"(stage + sfdst), "r"(sv.x) : "memory");
-                    asm volatile("st.shared.u32 [%0], %1;" ::"r"(stage + sfdst + sf_atom_stride), "r"(sv.y) : "memory");
-                }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&bar_full[s])) : "memory");
-                // the first stages of this tile are on their way: now drain the previous tile's accumulator
-                if (kb == drain_at && has_prev) drain(prev, tile_count - 1);
-            }
-            prev = t;
-            has_prev = true;
-        }
-        if (has_prev) drain(prev, tile_count - 1);
-    } else {
-        // ---- last warp: scale atoms into tensor memory, then the MMAs of the stage
-        for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++tile_count) {
-            const MoeQTile t = moe_qtile_decode<TOK>(tiles, s_offsets, a.n_experts, m_tiles, tile_rows, a.rows, tile);
-            const int n_first = t.split ? 2 * t.n_mma : 3 * t.n_mma;     // N of the first MMA
-            const int groups = (t.term_row2 + t.n_mma + 127) >> 7;       // row groups of B scales in use
-            if (tile_count > 0 && alive)                                 // previous accumulator drained?
-                alive = mbar_wait_bounded(smem_u32(&bar_acc_free), (tile_count - 1) & 1, 7);
-            for (int kb = 0; kb < n_kb; ++kb, ++it) {
-                const uint32_t s = it % S;
-                if (alive) alive = mbar_wait_bounded(smem_u32(&bar_full[s]), (it / S) & 1, 5);
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // copies landed via the generic proxy
-                tc05_fence_after_sync();
-                if (lane == 0 && alive) {
-                    const uint32_t stage = smem_u32(gemm_smem) + s * L::kStageBytes;
-                    const uint32_t sfa_cols = tmem + L::kAccCols + s * L::kSfColsPerStage;  // [mat][k-atom] x 4 columns
-                    const uint32_t sfb_cols = sfa_cols + L::kSfBCol;                        // [k-atom][row group] x 4
-#pragma unroll
-                    for (int at = 0; at < 2; ++at) {
-#pragma unroll
-                        for (int m = 0; m < MATS; ++m)
-                            if (m < t.mats)
-                                tc05_copy_scale_atom(sfa_cols + m * 8 + at * 4, stage + L::kOffSfA + m * 1024 + at * 512);
-#pragma unroll
-                        for (int g = 0; g < RG; ++g)
-                            if (g < groups)
-                                tc05_copy_scale_atom(sfb_cols + (at * RG + g) * 4, stage + L::kOffSfB + (at * RG + g) * 512);
-                    }
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {                                           // K-steps of 64
-                        const uint32_t acc = (kb > 0 || j > 0) ? 1u : 0u;
-                        const uint32_t sfb = sfb_cols + (j >> 1) * RG * 4;
-                        const uint32_t idesc = tc05_idesc_mxf4(128, n_first, (j & 1) * 2, (j & 1) * 2);
-                        const uint64_t db = tc05_desc_k_sw128(stage + L::kOffB + 32 * j);
-#pragma unroll
-                        for (int m = 0; m < MATS; ++m)
-                            if (m < t.mats)
-                                tc05_mma_mxf4(tmem + m * L::kAccStride, tc05_desc_k_sw128(stage + m * kQTile + 32 * j), db,
-                                              idesc, sfa_cols + m * 8 + (j >> 1) * 4, sfb, acc);
-                        if (t.split) {
-                            const uint32_t idesc3 = tc05_idesc_mxf4(128, t.n_mma, (j & 1) * 2, (j & 1) * 2);
-                            const uint64_t db3 = tc05_desc_k_sw128(stage + L::kOffB + 256 * 128 + 32 * j);
-#pragma unroll
-                            for (int m = 0; m < MATS; ++m)
-                                if (m < t.mats) tc05_mma_mxf4(tmem + m * L::kAccStride + 256,
-                                              tc05_desc_k_sw128(stage + m * kQTile + 32 * j), db3, idesc3,
-                                              sfa_cols + m * 8 + (j >> 1) * 4, sfb + 8, acc);
-                        }
-                    }
-                    tc05_commit(smem_u32(&bar_empty[s]));
-                    if (kb == n_kb - 1) tc05_commit(smem_u32(&bar_accum));
-                }
                 __syncwarp();
+                if (lane == 0) mbar_arrive_cluster(leader(full[pos.slot]));
+                pos.next(kQStages);
+            };
+            fetch(v[0], 0);
+            fetch(v[1], 2);
+            for (int s = 0; s < n_st; s += 4) {
+                put(v[0], false);
+                if (s + 1 < n_st) put(v[0], true);
+                fetch(v[0], s + 4);
+                if (s + 2 < n_st) put(v[1], false);
+                if (s + 3 < n_st) put(v[1], true);
+                fetch(v[1], s + 6);
             }
         }
+    } else if (warp == kQProducerWarp) {
+        // ---- this role and the MMAs are one thread each: nothing in their loops is done by a warp, so no vote or
+        // reconvergence stands between a barrier and what follows it
+        if (tc05_elect_one()) {
+            RingPos pos;
+            bool waited = false;
+            for (int tile = pair; tile < n_tiles && alive; tile += n_pairs) {
+                const MoeQTile t = decode(tile);
+                const int first = t.e * a.rows + t.m0 + rank * kMoeTileRows;      // past the expert in a half tile: loaded, not used
+                const int half = moe_width(t.width, kQTok) >> 1, slot = t.slot0 + rank * half;
+                const CUtensorMap* act = &maps.act[t.width];
+                const uint32_t bytes = t.mats * kQTile + kQTerms * half * 128u;
+                auto weights = [&](int s, const RingPos& p) {
+                    const uint32_t bar = leader(full[p.slot]), dst = smem_w + p.slot * 2 * kQTile;
+                    mbar_arrive_expect_tx_cluster(bar, bytes);
+                    tma_pair_load_2d(dst, &maps.wa, s * 128, first, bar);
+                    if (t.mats == 2) tma_pair_load_2d(dst + kQTile, &maps.wb, s * 128, first + (MODE == 0 ? 0 : kQRows), bar);
+                };
+                auto tokens = [&](int s, const RingPos& p) {
+                    tma_pair_load_3d(smem_b + p.slot * kQBStage, act, s * 128, slot, 0, leader(full[p.slot]));
+                };
+                int s0 = 0;
+                if (!waited) {                                // the pair's first stages: weights before the wait
+                    s0 = min(n_st, kQStages);
+                    RingPos p;
+                    for (int s = 0; s < s0; ++s, p.next(kQStages)) weights(s, p);
+                    pdl_wait();
+                    pdl_launch_dependents();
+                    waited = true;
+                    for (int s = 0; s < s0; ++s, pos.next(kQStages)) tokens(s, pos);
+                }
+                for (int s = s0; s < n_st; ++s, pos.next(kQStages)) {
+                    if (pos.round > 0) wait_one(empty[pos.slot], pos.round - 1, 4);
+                    if (!alive) break;
+                    weights(s, pos);
+                    tokens(s, pos);
+                }
+            }
+            if (!waited) { pdl_wait(); pdl_launch_dependents(); }
+        }
+        __syncwarp();
+    } else {
+        if (rank == 0 && tc05_elect_one()) {
+            RingPos pos;
+            for (int tile = pair; tile < n_tiles && alive; tile += n_pairs, ++tc) {
+                const MoeQTile t = decode(tile);
+                const uint32_t buf = tc & 1u;
+                const int n = moe_width(t.width, kQTok);
+                MoeQStage q;
+                q.acc = tmem + buf * kQAccCols;
+                q.sfa = tmem + kQSfCol;
+                q.b_term = (uint32_t)n * 4;                   // 128 n / 2 bytes, in the descriptor's units
+                q.idesc[0] = tc05_idesc_mxf4(256, n, 0, 0);
+                q.idesc[1] = tc05_idesc_mxf4(256, n, 2, 2);
+                if (tc >= 2) wait_one(acc_free[buf], (tc >> 1) - 1, 7);
+                for (int s = 0; s < n_st; ++s, pos.next(kQStages)) {
+                    wait_one(full[pos.slot], pos.round, 5);
+                    if (!alive) break;
+                    tc05_fence_after_sync();
+                    q.w = tc05_desc_k_sw128(smem_w + pos.slot * 2 * kQTile);
+                    q.b = tc05_desc_k_sw128(smem_b + pos.slot * kQBStage);
+                    q.sf = smem_sf + pos.slot * kQSfStage;
+                    q.fresh = s == 0;
+                    if (t.mats == 2) moe_q_issue<2>(q); else moe_q_issue<1>(q);
+                    tc05_pair_commit(smem_u32(&empty[pos.slot]));
+                    if (s == n_st - 1) tc05_pair_commit(smem_u32(&acc_full[buf]));
+                }
+            }
+        }
+        __syncwarp();
     }
     tc05_fence_before_sync();
-    __syncthreads();
-    if (warp == kProducerWarps) tc05_dealloc(tmem, 512);
+    cluster_sync_all();                                       // no arrival for this CTA is still on its way
+    tc05_fence_after_sync();
+    if (warp == kQMmaWarp) tc05_pair_dealloc(tmem, 512);
 }
 
 }  // namespace dsv4

@@ -31,7 +31,7 @@ __global__ void __launch_bounds__(128) mxf4_mma_rate_kernel(int n_cols, int iter
     tc05_fence_after_sync();
     const uint32_t tmem = tmem_base;
     const long long t0 = clock64();
-    if (tid == 0) {
+    if (warp == 0 && tc05_elect_one()) {
         const uint32_t sa = smem_u32(rate_smem), sb = sa + 32768, sf = sa + kRateOperandBytes;
         for (int it = 0; it < iters; ++it) {
             for (int c = 0; c < copies; ++c) tc05_copy_scale_atom(tmem + 384 + 4 * c, sf + 512 * c);

@@ -32,6 +32,17 @@ __device__ __forceinline__ uint32_t tc05_idesc_f16(int m, int n) {
     return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
+// True in one lane of a converged warp.  The thread that issues MMAs, scale copies and commits is chosen with this and
+// not with a comparison of lane numbers: only then does the compiler know that one thread runs the branch and puts the
+// descriptors into uniform registers directly.  Issued under `lane == 0`, every MMA cost 94.5 clocks at any N up to 192
+// (the issue, not the tensor pipe); under elect.sync an fp16 MMA with A in tensor memory costs N / 2 + 10 (at least 40)
+// and a block-scaled one 40 at N = 16, 96 at N = 192.
+__device__ __forceinline__ bool tc05_elect_one() {
+    uint32_t p;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(p));
+    return p != 0;
+}
+
 __device__ __forceinline__ void tc05_alloc(uint32_t smem_result_addr, uint32_t n_cols) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_result_addr), "r"(n_cols)
                  : "memory");
@@ -45,18 +56,30 @@ __device__ __forceinline__ void tc05_dealloc(uint32_t tmem_addr, uint32_t n_cols
 __device__ __forceinline__ void tc05_fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc05_fence_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// D[tmem] (+)= A[smem] * B[smem]; issued by ONE thread.  accumulate == 0 overwrites D.
-__device__ __forceinline__ void tc05_mma_f16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
-                                             uint32_t accumulate) {
+// fp16 MMA: D[tmem] (+)= A[tmem] * B[smem]; issued by ONE thread.  accumulate == 0 overwrites D.  A: lane = row, every
+// 32-bit column holds two consecutive K values (the even one in the low half), so a K-step of 16 is 8 columns.
+__device__ __forceinline__ void tc05_mma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc,
+                                                uint32_t accumulate) {
     asm volatile(
         "{\n"
         " .reg .pred p;\n"
         " setp.ne.b32 p, %4, 0;\n"
-        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
+        " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
         "}\n" ::"r"(tmem_d),
-        "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+        "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
         : "memory");
 }
+
+// 16 consecutive columns of this thread's tensor-memory lane (lane quadrant = warp index % 4), registers -> tensor
+// memory; complete after tc05_wait_st().
+__device__ __forceinline__ void tc05_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr),
+        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+        "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+        : "memory");
+}
+__device__ __forceinline__ void tc05_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // Arrive (count 1) on an mbarrier of this CTA when all MMAs issued so far by this thread have completed.
 __device__ __forceinline__ void tc05_commit(uint32_t mbar_addr) {
@@ -64,20 +87,8 @@ __device__ __forceinline__ void tc05_commit(uint32_t mbar_addr) {
                  : "memory");
 }
 
-// 16 consecutive FP32 accumulator columns of this thread's row (lane quadrant = warp index % 4).
-__device__ __forceinline__ void tc05_ld16(uint32_t taddr, float (&v)[16]) {
-    uint32_t r[16];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
-}
-
-// The same without the wait: several loads can be in flight before one tc05_wait_ld().
+// 16 consecutive FP32 accumulator columns of this thread's row (lane quadrant = warp index % 4); several loads can be
+// in flight before one tc05_wait_ld().
 __device__ __forceinline__ void tc05_ld16_issue(uint32_t taddr, uint32_t (&r)[16]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
@@ -86,11 +97,6 @@ __device__ __forceinline__ void tc05_ld16_issue(uint32_t taddr, uint32_t (&r)[16
         : "r"(taddr));
 }
 __device__ __forceinline__ void tc05_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-
-// Byte offset of 16-byte chunk `chunk` (0..7) of row `row` inside a K-major 128-byte-swizzled tile.
-__device__ __forceinline__ uint32_t tc05_sw128_offset(int row, int chunk) {
-    return (uint32_t)row * 128u + (uint32_t)((chunk ^ (row & 7)) << 4);
-}
 
 // ---------------------------------------------------------------------------------------------------------------
 // Block-scaled MMA (kind::mxf4: E2M1 operands, one UE8M0 scale per 32 K-elements, scales in tensor memory)
@@ -138,6 +144,44 @@ __device__ __forceinline__ void tc05_mma_mxf4(uint32_t tmem_d, uint64_t desc_a, 
         "}\n" ::"r"(tmem_d),
         "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(tmem_sfa), "r"(tmem_sfb), "r"(accumulate)
         : "memory");
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// The same on a PAIR of CTAs (cta_group::2, a cluster of two): M = 256, CTA r of the pair holds rows 128 r .. of A and of the
+// accumulator and rows N/2 r .. of B, all at the same shared- and tensor-memory addresses in both; the A scales of its own
+// rows and the B scales of all N columns.  One thread of CTA 0 issues; commits arrive in both CTAs.
+// ---------------------------------------------------------------------------------------------------------------
+__device__ __forceinline__ void tc05_pair_alloc(uint32_t smem_result_addr, uint32_t n_cols) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_result_addr), "r"(n_cols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tc05_pair_dealloc(uint32_t tmem_addr, uint32_t n_cols) {
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_addr), "r"(n_cols) : "memory");
+}
+__device__ __forceinline__ void tc05_pair_copy_scale_atom(uint32_t tmem_col, uint32_t smem_atom_addr) {
+    asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(tmem_col), "l"(tc05_desc_scale_atom(smem_atom_addr)) : "memory");
+}
+__device__ __forceinline__ void tc05_pair_commit(uint32_t mbar_addr) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(mbar_addr),
+                 "h"((uint16_t)3) : "memory");
+}
+
+// A_USE says what happens to the A tile in the tensor core's collector buffer: kAFill (read and keep), kAUse (take the
+// kept one), kALast (take it and drop it).  MMAs that multiply the same A one after another read it from shared memory once
+// this way.
+enum { kAFill, kAUse, kALast };
+template <int A_USE>
+__device__ __forceinline__ void tc05_pair_mma_mxf4(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
+                                                   uint32_t tmem_sfa, uint32_t tmem_sfb, uint32_t accumulate) {
+#define DSV4_MMA_MXF4(COLLECTOR)                                                                                        \
+    asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %6, 0;\n"                                                          \
+                 " tcgen05.mma.cta_group::2.kind::mxf4.block_scale.scale_vec::2X" COLLECTOR                              \
+                 " [%0], %1, %2, %3, [%4], [%5], p;\n}\n" ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc),           \
+                 "r"(tmem_sfa), "r"(tmem_sfb), "r"(accumulate) : "memory")
+    if (A_USE == kAFill) DSV4_MMA_MXF4(".collector::a::fill");
+    else if (A_USE == kAUse) DSV4_MMA_MXF4(".collector::a::use");
+    else DSV4_MMA_MXF4(".collector::a::lastuse");
+#undef DSV4_MMA_MXF4
 }
 
 // Byte offset of scale (row r, scale j of 4) inside a scale atom.

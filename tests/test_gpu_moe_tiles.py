@@ -1,0 +1,51 @@
+"""GPU parity of the batched layer at the edges of its tiles: token counts on both sides of every column count (16, 32, 64,
+96, 112 / 128) and of a second tile, reduction lengths whose scale rows are not 16-byte aligned, output widths that leave
+half and quarter tiles, and pair counts grouped by one block and by a cluster."""
+import pytest
+import torch
+
+import oracle
+
+pytestmark = pytest.mark.gpu
+DEV = torch.device("cuda:0")
+
+
+def run_case(rt, qz, path, counts, K, H, O, seed):
+    """One expert per entry of `counts`, that many tokens on it (k = 1), tokens shuffled."""
+    g = torch.Generator().manual_seed(seed)
+    E, T = len(counts), sum(counts)
+    bank = qz.make_expert_bank(E, K, H, "cpu", seed=seed)
+    if O != K:
+        bank["w2p"], bank["w2s"] = qz.quantize_mxfp4((torch.randn(E, O, H, generator=g) * 0.02).to(torch.bfloat16))
+    ids = torch.repeat_interleave(torch.arange(E), torch.tensor(counts))[torch.randperm(T, generator=g)].to(torch.int32)[:, None]
+    w = torch.rand(T, 1, generator=g) + 0.5
+    x = torch.randn(T, K, generator=g).to(torch.bfloat16)
+    out = rt.moe_forward({n: v.to(DEV) for n, v in bank.items()}, x.to(DEV), ids.contiguous().to(DEV), w.to(DEV), path=path)
+    torch.cuda.synchronize()
+    assert rt.moe_device_status() == 0
+    ref = oracle.moe_layer_ref(x, bank, ids.numpy(), w.numpy())
+    got = out.float().cpu().numpy()
+    err, cos = oracle.max_abs_rel(got, ref), oracle.cosine(got, ref)
+    # the bounds the batched layer is held to elsewhere: bf16 output rounding (2^-9 of a value), and on the block-scaled
+    # path three MXFP4 terms for x and for the intermediate (1e-3 and 2e-3 of a row's norm)
+    tight = (5e-3, 0.99999) if path == "fp16" else (7e-3, 0.99997)
+    assert err <= tight[0] and cos >= tight[1], f"{path} {counts}: max-abs/inf {err:.3e} cosine {cos:.7f}"
+
+
+@pytest.mark.parametrize("path", ["mxf4", "fp16"])
+@pytest.mark.parametrize("counts", [[1, 0, 15, 16], [17, 31, 32, 33], [63, 64, 65], [95, 96, 97], [112, 113, 128, 129], [224, 225, 257]])
+def test_tile_widths(rt, qz, path, counts):
+    run_case(rt, qz, path, counts, K=256, H=256, O=256, seed=sum(counts))
+
+
+@pytest.mark.parametrize("path", ["mxf4", "fp16"])
+@pytest.mark.parametrize("K,H,O", [(768, 256, 128), (1280, 768, 384), (512, 1280, 640), (2304, 512, 1152)])
+def test_reduction_lengths_and_partial_row_tiles(rt, qz, path, K, H, O):
+    run_case(rt, qz, path, [3, 40, 100], K=K, H=H, O=O, seed=K + O)
+
+
+@pytest.mark.parametrize("path", ["mxf4", "fp16"])
+@pytest.mark.parametrize("n_pairs", [2048, 2049, 9001])
+def test_grouping_by_one_block_and_by_a_cluster(rt, qz, path, n_pairs):
+    counts = [n_pairs // 3, 0, n_pairs // 5, n_pairs - n_pairs // 3 - n_pairs // 5]
+    run_case(rt, qz, path, counts, K=256, H=256, O=128, seed=n_pairs)
