@@ -7,7 +7,8 @@ The directory name carries a hyphen, so it cannot be imported by name; load it w
 Layout
 ------
 csrc/      CUDA sources of the three shared libraries (Makefile in this directory builds them into lib/)
-lib/       built libraries: libmxfp4_grouped_gemv.so, libmxfp4_gemv.so, libfp8_e4m3_gemv.so, libmxfp4_moe.so
+lib/       built libraries: libmxfp4_grouped_gemv.so, libmxfp4_gemv.so, libfp8_e4m3_gemv.so, libmxfp4_moe.so,
+           and dsv4_host.so (the operators' call path)
 runtime/   host-side mirror of the reference's ctypes bindings (same function names and argument meaning),
            plus the routed-expert bank / router / expert-parallel helpers
 
@@ -27,6 +28,9 @@ LIB_FILES = {
     "fp8": "libfp8_e4m3_gemv.so",
     "moe": "libmxfp4_moe.so",
 }
+
+# Extension module with the operators' call path (csrc/host_calls.cpp).
+HOST_FILE = "dsv4_host.so"
 
 # Same override variables as the reference's bindings (runtime/mxfp4_grouped_gemv_binding.py:31-36,
 # runtime/mxfp4_gemv_binding.py:18-23, runtime/fp8_e4m3_gemv_binding.py:28-33).
@@ -53,6 +57,6 @@ def build(verbose: bool = False) -> None:
         raise RuntimeError("nvcc build failed:\n" + res.stdout + res.stderr)
     if verbose:
         print(res.stdout + res.stderr)
-    for key in LIB_FILES:
-        if not os.path.exists(os.path.join(LIB_DIR, LIB_FILES[key])):
-            raise RuntimeError(f"build did not produce {LIB_FILES[key]}")
+    for name in [*LIB_FILES.values(), HOST_FILE]:
+        if not os.path.exists(os.path.join(LIB_DIR, name)):
+            raise RuntimeError(f"build did not produce {name}")

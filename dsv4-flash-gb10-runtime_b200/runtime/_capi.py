@@ -5,7 +5,7 @@ import ctypes
 import os
 from ctypes import c_int, c_int64, c_longlong, c_size_t, c_void_p, c_float
 
-from .. import lib_path
+from .. import HOST_FILE, LIB_DIR, lib_path
 
 _P = c_void_p
 
@@ -52,6 +52,33 @@ SIGNATURES = {
 }
 
 _loaded: dict[str, ctypes.CDLL] = {}
+_host = None
+
+
+def host():
+    """The extension module with the operators' call path.  Its functions do the ordinary call and return None for
+    anything else, which then takes the checks in Python; it knows an entry point once that library has been loaded."""
+    global _host
+    if _host is None:
+        import importlib.util
+        import torch  # noqa: F401  (the module links against its libraries)
+        path = os.path.join(LIB_DIR, HOST_FILE)
+        if not os.path.exists(path):
+            raise FileNotFoundError(f"{HOST_FILE} not found at {path}: build it with `make` in the package directory")
+        spec = importlib.util.spec_from_file_location("dsv4_host", path)
+        mod = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(mod)
+        _host = mod
+        for lib in _loaded.values():
+            _bind(lib)
+    return _host
+
+
+def _bind(lib: ctypes.CDLL) -> None:
+    for table in SIGNATURES.values():
+        for name in table:
+            if hasattr(lib, name):
+                _host.bind(name, ctypes.cast(getattr(lib, name), c_void_p).value)
 
 
 def load(key: str) -> ctypes.CDLL:
@@ -71,6 +98,8 @@ def load(key: str) -> ctypes.CDLL:
         fn.restype = restype
         fn.argtypes = argtypes
     _loaded[key] = lib
+    if _host is not None:
+        _bind(lib)
     return lib
 
 

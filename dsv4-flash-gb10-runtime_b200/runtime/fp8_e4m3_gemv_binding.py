@@ -58,12 +58,18 @@ def _run(symbol: str, scale_dtype: torch.dtype, W_fp8, W_scale, x, out, stream):
 
 def fp8_e4m3_gemv(W_fp8: torch.Tensor, W_scale: torch.Tensor, x: torch.Tensor,
                   out: Optional[torch.Tensor] = None, stream: Optional[torch.cuda.Stream] = None) -> torch.Tensor:
+    done = (_capi._host or _capi.host()).fp8_gemv(W_fp8, W_scale, x, out, stream)
+    if done is not None:
+        return done
     return _run("fp8_e4m3_gemv_m1", torch.uint8, W_fp8, W_scale, x, out, stream)
 
 
 def fp8_e4m3_gemv_f32scale(W_fp8: torch.Tensor, W_scale: torch.Tensor, x: torch.Tensor,
                            out: Optional[torch.Tensor] = None,
                            stream: Optional[torch.cuda.Stream] = None) -> torch.Tensor:
+    done = (_capi._host or _capi.host()).fp8_gemv_f32scale(W_fp8, W_scale, x, out, stream)
+    if done is not None:
+        return done
     return _run("fp8_e4m3_gemv_m1_f32scale", torch.float32, W_fp8, W_scale, x, out, stream)
 
 
@@ -79,6 +85,9 @@ def fp8_e4m3_gemv_batched(W_fp8: torch.Tensor, W_scale: torch.Tensor, x: torch.T
     W_fp8 uint8 [n_groups*N, K], W_scale uint8 [n_groups*N/128, K/128], x bfloat16 [n_groups*K] or [S, n_groups*K];
     returns bfloat16 [n_groups*N] or [S, n_groups*N].  With one token the result equals the single-token operator's bit
     for bit; with several tokens it agrees with it to the last bfloat16 step (FP32 tensor-core sums)."""
+    done = (_capi._host or _capi.host()).fp8_gemv_batched(W_fp8, W_scale, x, n_groups, out, stream)
+    if done is not None:
+        return done
     _require(W_fp8.is_cuda and W_scale.is_cuda and x.is_cuda, "all tensors must be on CUDA device")
     _require(W_fp8.dtype == torch.uint8, f"W_fp8 must be uint8 (raw E4M3), got {W_fp8.dtype}")
     _require(W_scale.dtype == torch.uint8, f"W_scale must be uint8 (E8M0), got {W_scale.dtype}")
@@ -129,6 +138,9 @@ def fp8_shared_swiglu(shared: dict, x: torch.Tensor, limit_gate: float = 10.0, l
     `shared`: w1, w3 uint8 [hidden, K] and w2 uint8 [out_dim, hidden] raw E4M3, w1s / w3s / w2s uint8 E8M0 tile scales
     (what bank_loader.load_shared_expert_fp8 returns); x bfloat16 [K].  The defaults are the C++ engine's clamp (gate
     only, 10); the Python engine clamps both (10, 10)."""
+    done = (_capi._host or _capi.host()).fp8_shared_swiglu(shared, x, limit_gate, limit_up, out, workspace, stream)
+    if done is not None:
+        return done
     w1, w3, w2 = shared["w1"], shared["w3"], shared["w2"]
     K, hidden, out_dim = x.numel(), w1.shape[0], w2.shape[0]
     for name, t in (("w1", w1), ("w3", w3), ("w2", w2), ("w1s", shared["w1s"]), ("w3s", shared["w3s"]), ("w2s", shared["w2s"])):

@@ -17,6 +17,9 @@ import torch
 from . import _capi
 
 
+_PATHS = {"fp16": 0, "mxf4": 1}
+
+
 def forward_workspace_bytes(n_tokens: int, k: int, K_in: int, hidden: int, out_dim: int, n_experts: int) -> int:
     return int(_capi.load("moe").mxfp4_moe_forward_workspace_bytes(n_tokens, k, K_in, hidden, out_dim, n_experts))
 
@@ -27,6 +30,10 @@ def moe_forward(bank: Dict[str, torch.Tensor], x: torch.Tensor, ids: torch.Tenso
     """`path`: None = the library's default (block-scaled MXFP4 MMAs unless DSV4_B200_MOE_PATH=fp16), 'mxf4' =
     block-scaled MMAs fed with the packed weights (activations as three MXFP4 terms), 'fp16' = fp16 MMAs with
     in-kernel dequantisation (exact operands)."""
+    code = -1 if path is None else _PATHS[path]
+    done = (_capi._host or _capi.host()).moe_forward(bank, x, ids, weights, out, workspace, code)
+    if done is not None:
+        return done
     lib = _capi.load("moe")
     for name, t, dt in (("x", x, torch.bfloat16), ("ids", ids, torch.int32), ("weights", weights, torch.float32)):
         if not t.is_cuda or t.dtype != dt or not t.is_contiguous():
@@ -49,7 +56,7 @@ def moe_forward(bank: Dict[str, torch.Tensor], x: torch.Tensor, ids: torch.Tenso
     if path is None:
         rc = lib.mxfp4_moe_forward(*args)
     else:
-        rc = lib.mxfp4_moe_forward_path(c_int({"fp16": 0, "mxf4": 1}[path]), *args)
+        rc = lib.mxfp4_moe_forward_path(c_int(code), *args)
     if rc != 0:
         raise RuntimeError(f"mxfp4_moe_forward returned {rc}")
     return out
@@ -73,7 +80,7 @@ STAGES = ("group", "quantise_x", "gemm_gate_up", "quantise_intermediate", "gemm_
 
 
 def stage_timing(enable: bool) -> bool:
-    """Switch the stage timing of the block-scaled batched path on or off (diagnostic: a timed call loses the overlap
+    """Switch the stage timing of the batched layer on or off (diagnostic: a timed call loses the overlap
     of programmatic dependent launch); returns the previous setting."""
     return bool(_capi.load("moe").mxfp4_moe_stage_timing(c_int(1 if enable else 0)))
 

@@ -22,6 +22,9 @@ def _require(cond: bool, msg: str) -> None:
 
 def mxfp4_gemv(W_packed: torch.Tensor, W_scale: torch.Tensor, x: torch.Tensor,
                out: Optional[torch.Tensor] = None, stream: Optional[torch.cuda.Stream] = None) -> torch.Tensor:
+    done = (_capi._host or _capi.host()).mxfp4_gemv(W_packed, W_scale, x, out, stream)
+    if done is not None:
+        return done
     _require(W_packed.is_cuda and W_scale.is_cuda and x.is_cuda, "all tensors must be on CUDA device")
     _require(W_packed.dtype == torch.uint8, f"W_packed must be uint8, got {W_packed.dtype}")
     _require(W_scale.dtype == torch.uint8, f"W_scale must be uint8, got {W_scale.dtype}")

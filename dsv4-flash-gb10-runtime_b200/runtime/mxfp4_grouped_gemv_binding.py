@@ -60,6 +60,9 @@ def mxfp4_grouped_gemv(W1: Dict[str, torch.Tensor], W3: Dict[str, torch.Tensor],
                        scales: Any, x: torch.Tensor, r: torch.Tensor, out: Optional[torch.Tensor] = None,
                        workspace: Optional[torch.Tensor] = None) -> torch.Tensor:
     del scales
+    done = (_capi._host or _capi.host()).grouped_gemv(W1, W3, W2, x, r, out, workspace)
+    if done is not None:
+        return done
     lib = _capi.load("grouped")
     _check(x, "x", torch.bfloat16)
     _check(r, "r", torch.float32)
@@ -116,6 +119,9 @@ def mxfp4_grouped_gemv_ids(bank: Dict[str, torch.Tensor], ids: torch.Tensor, x: 
     """Same FFN, experts `ids` (int32 CUDA [n_exp]) picked from a resident bank
     {'w1p','w3p','w2p','w1s','w3s','w2s'} stacked over ALL experts.  `stage_mask` 1 / 2 runs only the gate-up /
     the down kernel (profiling); `check=False` skips the Python-side shape checks for callers that made them once."""
+    done = (_capi._host or _capi.host()).grouped_gemv_ids(bank, ids, x, r, out, workspace, stage_mask)
+    if done is not None:
+        return done
     lib = _capi.load("grouped")
     K_in = x.numel()
     n_exp = ids.numel()
@@ -152,6 +158,9 @@ def moe_route_topk(logits: torch.Tensor, k: int = 6, score_func: str = "sqrt_sof
     score_func 'sqrt_softplus' is the engine's rule (kernel/cpp-engine-mxfp4/routed.cu:156-208, Python twin
     runtime/dsv4_engine_mxfp4.py:363-370); 'softmax' renormalises softmax probabilities over the k picks.
     """
+    done = (_capi._host or _capi.host()).route_topk(logits, k, score_func, eps, scaling, ids_out, w_out)
+    if done is not None:
+        return done
     lib = _capi.load("grouped")
     _check(logits, "logits", torch.float32)
     if logits.dim() == 1:
@@ -175,6 +184,9 @@ def moe_decode_layer(bank: Dict[str, torch.Tensor], logits: torch.Tensor, x: tor
 
     logits float32 [n_experts], x bfloat16 [K_in]; returns bfloat16 [out_dim].  Pass `workspace` (uint8,
     `decode_workspace_bytes`) to read the picks afterwards with `decode_picks`."""
+    done = (_capi._host or _capi.host()).decode_layer(bank, logits, x, k, score_func, eps, scaling, out, workspace)
+    if done is not None:
+        return done
     lib = _capi.load("grouped")
     K_in, n_experts = x.numel(), logits.numel()
     hidden, out_dim = bank["w1p"].shape[1], bank["w2p"].shape[1]
