@@ -1,11 +1,9 @@
 // Dense M=1 GEMV over a quantized weight matrix, shared by the MXFP4 and FP8-E4M3 libraries.
 //   y[n] = bf16( sum_k W[n,k] * x[k] ),  FP32 accumulation across blocks.
-// A CTA owns a contiguous range of output rows; a warp owns one 32-block slice of the reduction axis
-// (1024 MXFP4 elements / 512 FP8 elements) and walks down the CTA's rows with 8 row loads in flight
-// per lane and the next 8 already requested.  Per-slice partial sums meet in shared memory.
+// The rows stream through shared memory (row_stream.cuh); per-slice partial sums meet there as well.
 #pragma once
 
-#include "gemv_engine.cuh"
+#include "row_stream.cuh"
 
 #include <cstdio>
 #include <cstdlib>
@@ -13,10 +11,7 @@
 
 namespace dsv4 {
 
-constexpr int kDenseThreads = 256;
-constexpr int kDenseRows = 8;          // rows per warp batch
-constexpr int kDenseCap = 64;          // rows per CTA
-constexpr int kDenseMaxSlices = 32;    // FP8 K <= 16384 -> 1024 blocks -> 32 slices
+constexpr uint32_t kDenseParts = 12 * 1024;            // partial sums of a CTA at most
 
 struct DenseArgs {
     const __nv_bfloat16* x;
@@ -27,67 +22,18 @@ struct DenseArgs {
     __nv_bfloat16* y;
 };
 
-// Where the scale of (row, block) lives, how it is fetched (raw 32 bits) and what it is worth.
-struct Fp4Scale {   // E8M0 [N, K/32]: one byte per row per block
-    __device__ static __forceinline__ uint32_t fetch(const uint8_t* s, int row, int blk, long long s_stride) {
-        return ldg_stream_u8(s + (long long)row * s_stride + blk);
-    }
-    __device__ static __forceinline__ float value(uint32_t raw) { return e8m0_to_float(raw); }
-};
-struct Fp8Scale {   // E8M0 [N/128, K/128]: one byte per 128x128 tile; a block is 16 elements
-    __device__ static __forceinline__ uint32_t fetch(const uint8_t* s, int row, int blk, long long s_stride) {
-        return ldg_stream_u8(s + (long long)(row >> 7) * s_stride + (blk >> 3));
-    }
-    __device__ static __forceinline__ float value(uint32_t raw) { return e8m0_to_float(raw); }
-};
-struct Fp8ScaleF32 {   // FP32 [N/128, K/128], row stride in bytes
-    __device__ static __forceinline__ uint32_t fetch(const uint8_t* s, int row, int blk, long long s_stride) {
-        return __ldg(reinterpret_cast<const uint32_t*>(s + (long long)(row >> 7) * s_stride) + (blk >> 3));
-    }
-    __device__ static __forceinline__ float value(uint32_t raw) { return __uint_as_float(raw); }
-};
-
-struct DenseBatch {
-    uint4 w[kDenseRows];
-    uint32_t s[kDenseRows];
-};
-
-template <class Sc>
-__device__ __forceinline__ void dense_issue(const DenseArgs& a, int row, int step, int row_end, int blk,
-                                            bool lane_ok, DenseBatch& b) {
-#pragma unroll
-    for (int i = 0; i < kDenseRows; ++i) {
-        const int n = row + i * step;
-        b.w[i] = make_uint4(0, 0, 0, 0);
-        b.s[i] = 0;
-        if (n < row_end && lane_ok) {
-            b.w[i] = ldg_stream_v4(a.w + (long long)n * a.w_stride + (long long)blk * 16);
-            b.s[i] = Sc::fetch(a.s, n, blk, a.s_stride);
-        }
-    }
-}
-
-template <class Fmt, class Sc>
-__device__ __forceinline__ void dense_consume(const DenseBatch& b, const ActBlock<Fmt>& xb, int lane, int local0,
-                                              int step, int n_local, int ks, float (*part)[kDenseMaxSlices]) {
-    float v[kDenseRows];
-#pragma unroll
-    for (int i = 0; i < kDenseRows; ++i) {
-        v[i] = 0.f;
-        if (local0 + i * step < n_local) v[i] = Fmt::dot(b.w[i], xb.h) * (Sc::value(b.s[i]) * xb.scale);
-    }
-    multi_reduce<kDenseRows>(v, lane);
-    if (multi_reduce_owner<kDenseRows>(lane)) {
-        const int local = local0 + multi_reduce_index<kDenseRows>(lane) * step;
-        if (local < n_local) part[local][ks] = v[0];
-    }
-}
-
+// MATS = 1: y = W x.
+// MATS = 2: the gate / up pair of a gated FFN, act[n] = bf16( silu(clamp(g[n])) * clamp(u[n]) ), g = Wg x, u = Wu x, both
+//   rounded to bf16 first (as two separate GEMV calls would leave them); rows n of both matrices travel in one stage.
+//   limit_g / limit_u <= 0 switch the clamp of that operand off.
 // GROUPED: blockIdx.y picks one of several independent problems stacked along the rows of W (FP8 tile scales):
-// group g multiplies rows [g N, (g+1) N) with x[g K, (g+1) K) into y[g N, (g+1) N).
-template <class Fmt, class Sc, bool GROUPED = false>
-__global__ void __launch_bounds__(kDenseThreads, 2) dense_gemv_kernel(const DenseArgs a_in) {
-    __shared__ float part[kDenseCap][kDenseMaxSlices];
+//   group g multiplies rows [g N, (g+1) N) with x[g K, (g+1) K) into y[g N, (g+1) N).
+// RPW rows per warp and stage, SPW slices of the reduction axis per warp.
+template <class Fmt, class Sc, int MATS, int RPW, int SPW, bool GROUPED>
+__global__ void __launch_bounds__(kRowThreads, 2) dense_stream_kernel(const DenseArgs a_in, const uint8_t* w2, const uint8_t* s2,
+                                                                     const RowPlan p, float limit_g, float limit_u) {
+    extern __shared__ __align__(128) uint8_t row_smem[];
+    __shared__ RowRing ring;
     pdl_launch_dependents();
     DenseArgs a = a_in;
     if (GROUPED) {
@@ -97,118 +43,123 @@ __global__ void __launch_bounds__(kDenseThreads, 2) dense_gemv_kernel(const Dens
         a.s += grp * (a.N >> 7) * a.s_stride;
         a.y += grp * a.N;
     }
-
-    const int lane = threadIdx.x & 31;
-    const int warp = threadIdx.x >> 5;
-    const int n_warps = blockDim.x >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int r_begin = (int)((long long)a.N * blockIdx.x / gridDim.x), r_end = (int)((long long)a.N * (blockIdx.x + 1) / gridDim.x);
+    const int n_local = r_end - r_begin, n_stages = (n_local + p.rows - 1) / p.rows;
     const int n_blk = a.K / Fmt::kElems;
-    const int n_slices = (n_blk + 31) >> 5;
-    const int n_groups = max(1, n_warps / n_slices);
-    const int n_tasks = n_slices * n_groups;
+    float* const part = reinterpret_cast<float*>(row_smem + p.off_part);                   // [MATS][n_local][n_slices]
+    const uint32_t smem = smem_u32(row_smem);
 
-    const int r_begin = (int)((long long)a.N * blockIdx.x / gridDim.x);
-    const int r_end = (int)((long long)a.N * (blockIdx.x + 1) / gridDim.x);
-    const int n_local = r_end - r_begin;
-    const int span = kDenseRows * n_groups;
-
-    bool waited = false;
-    for (int task = warp; task < n_tasks; task += n_warps) {
-        const int ks = task % n_slices;
-        const int rg = task / n_slices;
-        const int blk = ks * 32 + lane;
-        const bool lane_ok = blk < n_blk;
-
-        DenseBatch b0, b1;
-        // weights never depend on the previous kernel in the stream: request them before waiting for it
-        dense_issue<Sc>(a, r_begin + rg, n_groups, r_end, blk, lane_ok, b0);
-        if (!waited) { pdl_wait(); waited = true; }
-
-        ActBlock<Fmt> xb;
-        act_block_load_bf16<Fmt>(a.x + (size_t)blk * Fmt::kElems, lane_ok, xb);
-
-        for (int local0 = rg; local0 < n_local; local0 += 2 * span) {
-            dense_issue<Sc>(a, r_begin + local0 + span, n_groups, r_end, blk, lane_ok, b1);
-            dense_consume<Fmt, Sc>(b0, xb, lane, local0, n_groups, n_local, ks, part);
-            dense_issue<Sc>(a, r_begin + local0 + 2 * span, n_groups, r_end, blk, lane_ok, b0);
-            dense_consume<Fmt, Sc>(b1, xb, lane, local0 + span, n_groups, n_local, ks, part);
-        }
-    }
-    if (!waited) pdl_wait();
-    __syncthreads();
-
-    for (int t = threadIdx.x; t < n_local; t += blockDim.x) {
-        float acc = 0.f;
-        for (int s = 0; s < n_slices; ++s) acc += part[t][s];
-        a.y[r_begin + t] = __float2bfloat16(acc);
-    }
-}
-
-// Gate / up pair of a gated FFN with one token: act[n] = bf16( silu(clamp(g[n])) * clamp(u[n]) ), g = Wg x, u = Wu x,
-// both rounded to bf16 first (as two separate GEMV calls would leave them).  Same streaming scheme as
-// dense_gemv_kernel; a CTA owns a range of n and walks it once per matrix, so g[n] and u[n] meet in its shared memory.
-// limit_g / limit_u <= 0 switch the clamp of that operand off.
-constexpr int kDualCap = kDenseCap / 2;      // n per CTA
-
-template <class Fmt, class Sc>
-__global__ void __launch_bounds__(kDenseThreads, 2) dense_dual_swiglu_kernel(const DenseArgs ag, const DenseArgs au,
-                                                                             float limit_g, float limit_u) {
-    __shared__ float part[kDenseCap][kDenseMaxSlices];      // rows [0, kDualCap): gate, [kDualCap, 2 kDualCap): up
-    pdl_launch_dependents();
-
-    const int lane = threadIdx.x & 31;
-    const int warp = threadIdx.x >> 5;
-    const int n_warps = blockDim.x >> 5;
-    const int n_blk = ag.K / Fmt::kElems;
-    const int n_slices = (n_blk + 31) >> 5;
-    const int n_groups = max(1, n_warps / n_slices);
-    const int n_tasks = n_slices * n_groups;
-
-    const int r_begin = (int)((long long)ag.N * blockIdx.x / gridDim.x);
-    const int r_end = (int)((long long)ag.N * (blockIdx.x + 1) / gridDim.x);
-    const int n_local = r_end - r_begin;
-    const int span = kDenseRows * n_groups;
-
-    bool waited = false;
-    for (int task = warp; task < n_tasks; task += n_warps) {
-        const int ks = task % n_slices;
-        const int rg = task / n_slices;
-        const int blk = ks * 32 + lane;
-        const bool lane_ok = blk < n_blk;
-        ActBlock<Fmt> xb;
+    if (tid == kRowWarps * 32) row_ring_init(ring, p);
+    auto produce = [&](int st0, int st1, RowPos& pos) {
+        for (int st = st0; st < st1; ++st, pos.next(p.slots)) {
+            if (pos.round > 0 && !mbar_wait_bounded(smem_u32(&ring.empty[pos.slot]), (pos.round - 1) & 1u, 1)) break;
+            const int row = st * p.rows, rows = min(p.rows, n_local - row);
+            const uint32_t bar = smem_u32(&ring.full[pos.slot]), dst = smem + pos.slot * p.stage_bytes;
+            const long long first = r_begin + row;
+            uint32_t bytes = MATS * rows * p.row_bytes;
+            if (Sc::kPerRow)
 #pragma unroll
-        for (int m = 0; m < 2; ++m) {
-            const DenseArgs& a = m == 0 ? ag : au;
-            float (*pm)[kDenseMaxSlices] = part + m * kDualCap;
-            DenseBatch b0, b1;
-            dense_issue<Sc>(a, r_begin + rg, n_groups, r_end, blk, lane_ok, b0);
-            if (!waited) { pdl_wait(); waited = true; }
-            if (m == 0) act_block_load_bf16<Fmt>(a.x + (size_t)blk * Fmt::kElems, lane_ok, xb);
-            for (int local0 = rg; local0 < n_local; local0 += 2 * span) {
-                dense_issue<Sc>(a, r_begin + local0 + span, n_groups, r_end, blk, lane_ok, b1);
-                dense_consume<Fmt, Sc>(b0, xb, lane, local0, n_groups, n_local, ks, pm);
-                dense_issue<Sc>(a, r_begin + local0 + 2 * span, n_groups, r_end, blk, lane_ok, b0);
-                dense_consume<Fmt, Sc>(b1, xb, lane, local0 + span, n_groups, n_local, ks, pm);
+                for (int m = 0; m < MATS; ++m) bytes += row_scale_bytes(p, (m == 0 ? a.s : s2) + first * a.s_stride, n_blk, rows);
+            mbar_arrive_expect_tx(bar, bytes);
+#pragma unroll
+            for (int m = 0; m < MATS; ++m) {
+                row_copy(dst + m * p.rows * p.row_bytes, (m == 0 ? a.w : w2) + first * a.w_stride, a.w_stride, p.row_bytes, rows, bar);
+                if (Sc::kPerRow)
+                    row_scale_copy(p, dst + MATS * p.rows * p.row_bytes + m * p.s_area, (m == 0 ? a.s : s2) + first * a.s_stride, a.s_stride,
+                                   n_blk, rows, bar);
             }
         }
+    };
+    RowPos made;                             // the producer's position
+    const int first_stages = min(p.slots, n_stages);
+    // weights never depend on the previous kernel in the stream: the ring is filled without waiting for it
+    if (tid == kRowWarps * 32) produce(0, first_stages, made);
+    __syncwarp();
+    // tile scales of this CTA's rows as floats: [MATS][tile rows][n_blk / 8]
+    const int tiles_k = n_blk >> 3, tile0 = r_begin >> 7, n_tr = ((r_end - 1) >> 7) - tile0 + 1;
+    float* const table = reinterpret_cast<float*>(row_smem + p.off_table);
+    if (!Sc::kPerRow)
+        for (int i = tid; i < MATS * n_tr * tiles_k; i += kRowThreads) {
+            const int m = i / (n_tr * tiles_k), j = i - m * n_tr * tiles_k, tr = j / tiles_k;
+            table[i] = Sc::value(Sc::fetch(m == 0 ? a.s : s2, (tile0 + tr) << 7, (j - tr * tiles_k) << 3, a.s_stride));
+        }
+    __syncthreads();                         // barriers, tile scales
+    pdl_wait();                              // every thread: the outputs below may still be read by the kernel before
+    if (warp < p.warps) {
+        const int w_slices = p.warps / p.n_groups, ks0 = warp % w_slices, rg = warp / w_slices;
+        int blk[SPW];
+        bool ok[SPW];
+#pragma unroll
+        for (int q = 0; q < SPW; ++q) { blk[q] = (ks0 + q * w_slices) * 32 + lane; ok[q] = blk[q] < n_blk; }
+        if (tid == 0) row_x_request(ring, smem + p.off_x, a.x, a.K * 2);
+        bool alive = __all_sync(kFullMask, mbar_wait_bounded(smem_u32(&ring.x), 0, 2));
+        ActBlock<Fmt> xb[SPW];
+#pragma unroll
+        for (int q = 0; q < SPW; ++q) {
+            row_act_block<Fmt>(smem + p.off_x, blk[q], ok[q], xb[q]);
+            if (!ok[q]) blk[q] = 0;
+        }
+        RowPos pos;
+        for (int st = 0; st < n_stages; ++st) {
+            if (alive) alive = __all_sync(kFullMask, mbar_wait_bounded(smem_u32(&ring.full[pos.slot]), pos.round & 1u, 2));
+            const uint32_t stage = smem + pos.slot * p.stage_bytes;
+            const int row = st * p.rows + rg, left = n_local - row;
+            const uint32_t s_row = (uint32_t)(r_begin + st * p.rows) * (uint32_t)a.s_stride;
+#pragma unroll
+            for (int q = 0; q < SPW; ++q) {
+                if (q > 0 && ks0 + w_slices >= p.n_slices) continue;
+                // All loads first, without conditions (a branch around a row keeps the next row's loads behind its sums):
+                // rows past the CTA's last hold stale bytes and their sums are dropped, lanes past the row's end read
+                // block 0 against activations of zero.
+                uint4 w[MATS * RPW];
+                float sc[MATS * RPW];
+#pragma unroll
+                for (int m = 0; m < MATS; ++m)
+#pragma unroll
+                    for (int i = 0; i < RPW; ++i) {
+                        const int r = rg + i * p.n_groups, k = m * RPW + i;
+                        w[k] = lds_v4(stage + (m * p.rows + r) * p.row_bytes + blk[q] * 16);
+                        if (Sc::kPerRow) {
+                            const uint32_t s_addr = (uint32_t)reinterpret_cast<uintptr_t>(m == 0 ? a.s : s2) + s_row;
+                            sc[k] = Sc::value(lds_u8(stage + MATS * p.rows * p.row_bytes + m * p.s_area + row_scale_offset(p, s_addr, r) + blk[q]));
+                        } else {
+                            sc[k] = table[(m * n_tr + ((r_begin + st * p.rows + r) >> 7) - tile0) * tiles_k + (blk[q] >> 3)];
+                        }
+                    }
+                float v[MATS * RPW];
+#pragma unroll
+                for (int k = 0; k < MATS * RPW; ++k) v[k] = Fmt::dot(w[k], xb[q].h) * (sc[k] * xb[q].scale);
+                row_store<RPW>(v, left, p.n_groups, lane, part + row * p.n_slices + ks0 + q * w_slices, p.n_slices, n_local * p.n_slices);
+            }
+            row_release(ring, p, pos, lane);
+        }
+    } else if (tid == kRowWarps * 32) {
+        produce(first_stages, n_stages, made);
     }
-    if (!waited) pdl_wait();
     __syncthreads();
 
-    for (int t = threadIdx.x; t < n_local; t += blockDim.x) {
-        float g = 0.f, u = 0.f;
-        for (int s = 0; s < n_slices; ++s) { g += part[t][s]; u += part[kDualCap + t][s]; }
-        g = __bfloat162float(__float2bfloat16(g));
-        u = __bfloat162float(__float2bfloat16(u));
-        if (limit_g > 0.f) g = fminf(fmaxf(g, -limit_g), limit_g);
-        if (limit_u > 0.f) u = fminf(fmaxf(u, -limit_u), limit_u);
-        ag.y[r_begin + t] = __float2bfloat16((g / (1.0f + expf(-g))) * u);
+    for (int t = tid; t < n_local; t += kRowThreads) {
+        float g = 0.f;
+        for (int s = 0; s < p.n_slices; ++s) g += part[t * p.n_slices + s];
+        if (MATS == 1) {
+            a.y[r_begin + t] = __float2bfloat16(g);
+        } else {
+            float u = 0.f;
+            for (int s = 0; s < p.n_slices; ++s) u += part[(n_local + t) * p.n_slices + s];
+            g = __bfloat162float(__float2bfloat16(g));
+            u = __bfloat162float(__float2bfloat16(u));
+            if (limit_g > 0.f) g = fminf(fmaxf(g, -limit_g), limit_g);
+            if (limit_u > 0.f) u = fminf(fmaxf(u, -limit_u), limit_u);
+            a.y[r_begin + t] = __float2bfloat16((g / (1.0f + expf(-g))) * u);
+        }
     }
 }
 
 // Several tokens and several independent groups in one launch (FP8 only: the attention projections):
 //   y[t, g*N + n] = bf16( sum_k W[g*N + n, k] * x[t, g*K + k] ),   W [G*N, K], scales [G*N/128, K/128].
 // G = 1 is a plain batched GEMV; G > 1 is the block-diagonal shape of the grouped output projection (one launch
-// instead of G).  One token runs the grouped form of dense_gemv_kernel (bit-identical to the M = 1 entry); several
+// instead of G).  One token runs the grouped form of dense_stream_kernel (bit-identical to the M = 1 entry); several
 // tokens run dense_mma_gemv_kernel (dense_mma_gemv.cuh), which reads every weight byte once per 8 tokens.
 struct DenseMultiArgs {
     DenseArgs a;                   // group 0, token 0; a.N = rows per group
@@ -268,23 +219,54 @@ inline bool dense_pdl_enabled() {
     return v == 1;
 }
 
-// CTAs per SM that one launch asks for.  Two fill the machine (126 registers x 256 threads) and are what a large
-// matrix wants.  A matrix small enough that one CTA per SM requests all of its rows up front (two batches of
-// kDenseRows per warp) is bound by the launch chain instead: with one CTA per SM the next launch of the chain
-// becomes resident beside this one and has its weights on the way while this one finishes (2048 x 4096 MXFP4:
-// 4.3 us per call against 5.6).  DSV4_B200_DENSE_WAVES = 1 .. 4 overrides the choice.
-inline int dense_waves(int n_rows, int n_blk) {
-    static int forced = -1;
-    if (forced < 0) {
-        const char* e = std::getenv("DSV4_B200_DENSE_WAVES");
-        const int w = e ? std::atoi(e) : 0;
-        forced = (w >= 1 && w <= 4) ? w : 0;
+// One CTA per SM over all groups (two successive launches share each SM), more where a CTA's partial sums would not fit.
+// Needs 16-byte aligned x, weights and row strides.
+template <class Fmt, class Sc, int MATS, int RPW, int SPW, bool GROUPED>
+inline cudaError_t dense_stream_launch_as(const DenseArgs& a, const uint8_t* w2, const uint8_t* s2, float limit_g, float limit_u,
+                                          int n_groups, cudaStream_t stream) {
+    auto kernel = dense_stream_kernel<Fmt, Sc, MATS, RPW, SPW, GROUPED>;
+    const int n_blk = a.K / Fmt::kElems;
+    RowPlan p = row_plan(n_blk, MATS, RPW, SPW);
+    const long long cap = kDenseParts / (4 * MATS * p.n_slices);          // rows per CTA
+    long long grid = (dense_sm_count() + n_groups - 1) / n_groups;
+    const long long need = ((long long)a.N + cap - 1) / cap;
+    if (grid < need) grid = need;
+    if (grid > a.N) grid = a.N;
+    const int most = (int)((a.N + grid - 1) / grid);
+    if (Sc::kPerRow) row_plan_scales(p, MATS, n_blk, a.s_stride, 1);
+    row_plan_finish(p, a.K * 2, 4 * MATS * most * p.n_slices, Sc::kPerRow ? 0 : 4 * MATS * (most / 128 + 3) * (n_blk / 8));
+    static bool done[64] = {false};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return cudaErrorInvalidDevice;
+    if (dev < 0 || dev >= 64 || !done[dev]) {
+        const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowSmemMost);
+        if (err != cudaSuccess) return err;
+        if (dev >= 0 && dev < 64) done[dev] = true;
     }
-    if (forced > 0) return forced;
-    const int n_slices = (n_blk + 31) >> 5;
-    const int n_groups = (kDenseThreads / 32) / n_slices > 0 ? (kDenseThreads / 32) / n_slices : 1;
-    const long long up_front = 2LL * kDenseRows * n_groups * dense_sm_count();
-    return n_rows <= up_front ? 1 : 2;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid, (unsigned)n_groups);
+    cfg.blockDim = dim3(kRowThreads);
+    cfg.dynamicSmemBytes = p.smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = dense_pdl_enabled() ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, a, w2, s2, p, limit_g, limit_u);
+}
+// Four rows per warp and stage where a stage of that stays within kRowStage, else two; FP8 rows longer than 8192 have more
+// slices than there are warps: two per warp.
+template <class Fmt, class Sc, int MATS, bool GROUPED>
+inline cudaError_t dense_stream_launch(const DenseArgs& a, const uint8_t* w2, const uint8_t* s2, float limit_g, float limit_u,
+                                       int n_groups, cudaStream_t stream) {
+    const int n_blk = a.K / Fmt::kElems;
+    if constexpr (Fmt::kElems == 16) {
+        if (n_blk > 32 * kRowWarps) return dense_stream_launch_as<Fmt, Sc, MATS, 2, 2, GROUPED>(a, w2, s2, limit_g, limit_u, n_groups, stream);
+    }
+    if (row_plan(n_blk, MATS, 4, 1).stage_bytes <= kRowStage)
+        return dense_stream_launch_as<Fmt, Sc, MATS, 4, 1, GROUPED>(a, w2, s2, limit_g, limit_u, n_groups, stream);
+    return dense_stream_launch_as<Fmt, Sc, MATS, 2, 1, GROUPED>(a, w2, s2, limit_g, limit_u, n_groups, stream);
 }
 
 // Launches the aligned streaming kernel when it can, the byte-wise one otherwise.
@@ -296,47 +278,21 @@ inline cudaError_t dense_launch(const DenseArgs& a, cudaStream_t stream) {
         dense_gemv_unaligned_kernel<Fmt, Sc><<<(a.N + warps - 1) / warps, warps * 32, 0, stream>>>(a);
         return cudaGetLastError();
     }
-    long long grid = (long long)dense_waves(a.N, a.K / Fmt::kElems) * dense_sm_count();
-    const long long need = ((long long)a.N + kDenseCap - 1) / kDenseCap;
-    if (grid < need) grid = need;
-    if (grid > a.N) grid = a.N;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(kDenseThreads);
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = dense_pdl_enabled() ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, dense_gemv_kernel<Fmt, Sc>, a);
+    return dense_stream_launch<Fmt, Sc, 1, false>(a, nullptr, nullptr, 0.f, 0.f, 1, stream);
 }
 
 template <class Sc>
 inline cudaError_t dense_mma_launch(const DenseMultiArgs& m, cudaStream_t stream);      // dense_mma_gemv.cuh
 
 // Several tokens / groups: needs 16-byte aligned x, weights, row strides and token strides (cudaErrorInvalidValue
-// otherwise).  One token: grid.y = groups, at most kDenseCap rows per CTA.
+// otherwise).
 template <class Sc>
 inline cudaError_t dense_multi_launch(const DenseMultiArgs& m, cudaStream_t stream) {
     const DenseArgs& a = m.a;
     auto mis = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) != 0; };
     if (mis(a.x) || mis(a.w) || (a.w_stride & 15) != 0 || (m.x_tok & 7) != 0 || m.n_groups > 65535)
         return cudaErrorInvalidValue;
-    const long long need = ((long long)a.N + kDenseCap - 1) / kDenseCap;
-    long long per_group = (2LL * dense_sm_count() + m.n_groups - 1) / m.n_groups;
-    if (per_group < need) per_group = need;
-    if (per_group > a.N) per_group = a.N;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)per_group, (unsigned)m.n_groups);
-    cfg.blockDim = dim3(kDenseThreads);
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = dense_pdl_enabled() ? 1 : 0;
-    if (m.n_tok == 1) return cudaLaunchKernelEx(&cfg, dense_gemv_kernel<Fp8Format, Sc, true>, a);
+    if (m.n_tok == 1) return dense_stream_launch<Fp8Format, Sc, 1, true>(a, nullptr, nullptr, 0.f, 0.f, m.n_groups, stream);
     return dense_mma_launch<Sc>(m, stream);
 }
 
@@ -348,20 +304,7 @@ inline cudaError_t dense_dual_launch(const DenseArgs& ag, const DenseArgs& au, f
     auto mis = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) != 0; };
     if (mis(ag.x) || mis(ag.w) || mis(au.w) || (ag.w_stride & 15) != 0 || (au.w_stride & 15) != 0)
         return cudaErrorInvalidValue;
-    long long grid = 2LL * dense_sm_count();
-    const long long need = ((long long)ag.N + kDualCap - 1) / kDualCap;
-    if (grid < need) grid = need;
-    if (grid > ag.N) grid = ag.N;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(kDenseThreads);
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = dense_pdl_enabled() ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, dense_dual_swiglu_kernel<Fmt, Sc>, ag, au, limit_g, limit_u);
+    return dense_stream_launch<Fmt, Sc, 2, false>(ag, au.w, au.s, limit_g, limit_u, 1, stream);
 }
 
 }  // namespace dsv4

@@ -1,6 +1,6 @@
 // FP8 GEMV for 2..8 tokens per pass over the weights (several passes for more) and several independent groups:
 //   y[t, g*N + n] = bf16( sum_k e4m3(W[g*N + n, k]) * scale[(g*N + n)/128, k/128] * x[t, g*K + k] ).
-// With a handful of tokens the per-lane fp16 dot products of dense_gemv_kernel become instruction bound (decode
+// With a handful of tokens the per-lane fp16 dot products of dense_stream_kernel become instruction bound (decode
 // once, multiply T times, widen, reduce across lanes).  Here a warp owns a tile of 16 weight rows and feeds it to
 // mma.sync.m16n8k16 (fp16 x fp16 -> fp32): the 8 columns are the tokens, so the whole token batch costs one MMA
 // per 16 x 16 weights and there is no cross-lane reduction.  The products E4M3 x fp16 are exact in FP32; the

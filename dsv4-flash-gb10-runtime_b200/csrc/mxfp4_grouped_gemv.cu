@@ -7,242 +7,24 @@
 // order, return codes and ownership rules (caller owns all buffers, work is enqueued on the caller's
 // stream, no allocation, no synchronisation).
 //
-// At the DSv4 shapes one persistent kernel does the whole call (decode_stream.cuh).  Elsewhere, and on request,
-// two kernels chained by programmatic dependent launch, so that the second one can request its first weight rows
-// while the first one drains:
-//   gate/up kernel : a warp owns a contiguous run of (expert, hidden-row) pairs and streams the W1 and W3
-//                    row of a pair whole (a lane owns up to 4 blocks of the row, the activation vector
-//                    lives in its registers), reduces across lanes and writes silu(g)*u as FP32 into the
-//                    workspace; no shared memory, no block barrier.
-//   down kernel    : a CTA owns a contiguous range of output rows for ALL experts, a warp owns one expert;
-//                    the router-weighted sum over experts is taken inside the CTA in a fixed order
-//                    (deterministic, no float atomics) and rounded once to bf16.
+// At the DSv4 shapes one persistent kernel does the whole call (decode_stream.cuh).  Elsewhere two kernels chained by
+// programmatic dependent launch (grouped_stream.cuh), so that the second one has its first weight rows on the way while the
+// first one drains; on request, at the DSv4 shapes, the two kernels of grouped_ring.cuh.
 #include "gemv_engine.cuh"
 #include "stream_ring.cuh"
 #include "grouped_args.cuh"
 #include "router.cuh"
 #include "grouped_ring.cuh"
 #include "decode_stream.cuh"
+#include "grouped_stream.cuh"
 
 #include <cstdio>
 #include <cstdlib>
 
 namespace dsv4 {
 
-constexpr int kMaxBlocksPerLane = 4;   // reduction axis <= 4096 elements = 128 blocks = 4 per lane
+constexpr int kMaxReduction = 4096;    // K_in and hidden at most
 constexpr int kMaxExperts = 8;         // experts per call (the reference fixes 6)
-
-constexpr int kGateThreads = 384;      // 12 warps, one (W1,W3) row pair in flight per warp
-constexpr int kDownThreads = 384;      // 12 warps = 6 experts x 2 row groups at the DSv4 shape
-constexpr int kDownCap = 64;           // output rows per CTA held in shared memory
-constexpr int kDownLoads = 8;          // 16-byte loads per lane per batch
-
-
-// One weight row as seen by a lane: BPL 16-byte blocks and their scale bytes.
-template <int BPL>
-struct RowRegs {
-    uint4 w[BPL];
-    uint32_t s[BPL];
-};
-
-template <int BPL>
-__device__ __forceinline__ void row_clear(RowRegs<BPL>& r) {
-#pragma unroll
-    for (int j = 0; j < BPL; ++j) { r.w[j] = make_uint4(0, 0, 0, 0); r.s[j] = 0; }
-}
-
-// wp / sp already point at this lane's first block / scale byte of the row.
-template <int BPL>
-__device__ __forceinline__ void row_issue(const uint8_t* wp, const uint8_t* sp, const bool (&ok)[BPL],
-                                          RowRegs<BPL>& r) {
-#pragma unroll
-    for (int j = 0; j < BPL; ++j)
-        if (ok[j]) {
-            r.w[j] = ldg_stream_v4(wp + 512 * j);
-            r.s[j] = ldg_stream_u8(sp + 32 * j);
-        }
-}
-
-// Dot product of the lane's part of a row with the activations; each block's registers are refilled with the
-// same block of a later row (at nwp / nsp) as soon as they have been consumed, so the lane always has its
-// full set of loads in flight without a second register buffer.
-template <int BPL>
-__device__ __forceinline__ float row_dot_refill(RowRegs<BPL>& r, const LaneAct<Fp4Format, BPL>& a,
-                                                const uint8_t* nwp, const uint8_t* nsp, bool more,
-                                                const bool (&ok)[BPL]) {
-    float acc = 0.f;
-#pragma unroll
-    for (int j = 0; j < BPL; ++j) {
-        const float d = Fp4Format::dot(r.w[j], a.h[j]);
-        const float sc = e8m0_to_float_fast(r.s[j]);
-        if (more && ok[j]) {
-            r.w[j] = ldg_stream_v4(nwp + 512 * j);
-            r.s[j] = ldg_stream_u8(nsp + 32 * j);
-        }
-        acc = fmaf(d, sc, acc);
-    }
-    return acc * a.scale;
-}
-
-// ------------------------------------------------------------------------------------------------
-// gate/up + SwiGLU: a warp owns a contiguous run of (expert slot, hidden row) pairs and streams the W1 and
-// W3 row of a pair together (2 x BPL loads of 512 contiguous bytes per warp)
-// ------------------------------------------------------------------------------------------------
-
-struct GateCursor {
-    const uint8_t* w1; const uint8_t* w3; const uint8_t* s1; const uint8_t* s3;   // this lane's position in pair q
-    int q, h, e;
-};
-
-__device__ __forceinline__ void gate_seek(const GroupedArgs& a, GateCursor& c, int lane) {
-    const long long eid = a.ids ? (long long)a.ids[c.e] : (long long)c.e;
-    const long long po = eid * a.strideAp + (long long)c.h * (a.K >> 1) + lane * 16;
-    const long long so = eid * a.strideAs + (long long)c.h * (a.K >> 5) + lane;
-    c.w1 = a.w1p + po; c.w3 = a.w3p + po; c.s1 = a.w1s + so; c.s3 = a.w3s + so;
-}
-
-__device__ __forceinline__ void gate_advance(const GroupedArgs& a, GateCursor& c, int q_end, int lane) {
-    const int row_p = a.K >> 1, row_s = a.K >> 5;
-    c.q += 1;
-    c.h += 1;
-    c.w1 += row_p; c.w3 += row_p; c.s1 += row_s; c.s3 += row_s;
-    if (c.h == a.H) {          // next expert slot: stacked experts are contiguous, a bank needs a new base
-        c.h = 0;
-        c.e += 1;
-        if (a.ids != nullptr && c.q < q_end) gate_seek(a, c, lane);
-    }
-}
-
-template <int BPL>
-__global__ void __launch_bounds__(kGateThreads, 1) grouped_gate_up_kernel(const GroupedArgs a) {
-    pdl_launch_dependents();
-    const int lane = threadIdx.x & 31;
-    const int gw = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    const int n_gw = gridDim.x * (blockDim.x >> 5);
-    const int n_blk = a.K >> 5;
-    bool ok[BPL];
-#pragma unroll
-    for (int j = 0; j < BPL; ++j) ok[j] = lane + 32 * j < n_blk;
-
-    const long long total = (long long)a.E * a.H;
-    const int q_begin = (int)(total * gw / n_gw);
-    const int q_end = (int)(total * (gw + 1) / n_gw);
-
-    GateCursor cur;
-    cur.q = q_begin;
-    cur.e = q_begin / a.H;
-    cur.h = q_begin - cur.e * a.H;
-    cur.w1 = cur.w3 = cur.s1 = cur.s3 = nullptr;
-
-    RowRegs<BPL> g, u;
-    row_clear(g);
-    row_clear(u);
-    const bool any = q_begin < q_end;
-    // stacked weights do not depend on the previous kernel in the stream: request them before waiting for it
-    if (a.ids == nullptr && any) {
-        gate_seek(a, cur, lane);
-        row_issue<BPL>(cur.w1, cur.s1, ok, g);
-        row_issue<BPL>(cur.w3, cur.s3, ok, u);
-    }
-    pdl_wait();
-    if (a.ids != nullptr && any) {
-        gate_seek(a, cur, lane);
-        row_issue<BPL>(cur.w1, cur.s1, ok, g);
-        row_issue<BPL>(cur.w3, cur.s3, ok, u);
-    }
-    LaneAct<Fp4Format, BPL> x;
-    lane_act_load<Fp4Format, BPL>(a.x, lane, n_blk, x);
-
-    for (int q = q_begin; q < q_end; ++q) {
-        gate_advance(a, cur, q_end, lane);                       // cur now describes pair q + 1
-        const bool more = q + 1 < q_end;
-        float v[2];
-        v[0] = row_dot_refill<BPL>(g, x, cur.w1, cur.s1, more, ok);
-        v[1] = row_dot_refill<BPL>(u, x, cur.w3, cur.s3, more, ok);
-        multi_reduce<2>(v, lane);                                // lane 0: gate sum, lane 16: up sum
-        const float up = __shfl_sync(kFullMask, v[0], 16);
-        if (lane == 0) a.mid[q] = swiglu_f32(v[0], up);
-    }
-}
-
-// ------------------------------------------------------------------------------------------------
-// down projection + router-weighted combine: a CTA owns a contiguous range of output rows for ALL experts,
-// a warp owns (expert slot, row group); the sum over experts is taken in a fixed order inside the CTA
-// ------------------------------------------------------------------------------------------------
-
-template <int BPL>
-__global__ void __launch_bounds__(kDownThreads, 1) grouped_down_kernel(const GroupedArgs a) {
-    constexpr int RB = kDownLoads / BPL;          // rows in flight per warp
-    __shared__ float part[kDownCap][kMaxExperts];
-    pdl_launch_dependents();
-
-    const int lane = threadIdx.x & 31;
-    const int warp = threadIdx.x >> 5;
-    const int n_warps = blockDim.x >> 5;
-    const int n_blk = a.H >> 5;
-    bool ok[BPL];
-#pragma unroll
-    for (int j = 0; j < BPL; ++j) ok[j] = lane + 32 * j < n_blk;
-
-    const int n_groups = n_warps / a.E;                       // host guarantees E <= n_warps
-    const int e = warp % a.E;
-    const int rg = warp / a.E;
-    const int o_begin = (int)((long long)a.O * blockIdx.x / gridDim.x);
-    const int o_end = (int)((long long)a.O * (blockIdx.x + 1) / gridDim.x);
-    const int n_local = o_end - o_begin;
-    // this warp's rows: a contiguous share of the CTA's range
-    const int l_begin = (int)((long long)n_local * rg / n_groups);
-    const int l_end = (rg < n_groups) ? (int)((long long)n_local * (rg + 1) / n_groups) : l_begin;
-    const int row_p = a.H >> 1, row_s = a.H >> 5;
-    const bool any = l_begin < l_end;
-
-    RowRegs<BPL> b[RB];
-#pragma unroll
-    for (int i = 0; i < RB; ++i) row_clear(b[i]);
-
-    const uint8_t* wp = nullptr;     // this lane's position in row l0 of the loop below
-    const uint8_t* sp = nullptr;
-    auto first_issue = [&]() {
-        const long long eid = a.ids ? (long long)a.ids[e] : (long long)e;
-        wp = a.w2p + eid * a.strideBp + (long long)(o_begin + l_begin) * row_p + lane * 16;
-        sp = a.w2s + eid * a.strideBs + (long long)(o_begin + l_begin) * row_s + lane;
-#pragma unroll
-        for (int i = 0; i < RB; ++i)
-            if (l_begin + i < l_end) row_issue<BPL>(wp + (long long)i * row_p, sp + i * row_s, ok, b[i]);
-    };
-    if (a.ids == nullptr && any) first_issue();
-    pdl_wait();
-    if (a.ids != nullptr && any) first_issue();
-
-    if (any) {
-        LaneAct<Fp4Format, BPL> m;
-        lane_act_load<Fp4Format, BPL>(a.mid + (size_t)e * a.H, lane, n_blk, m);
-        for (int l0 = l_begin; l0 < l_end; l0 += RB) {
-            float v[RB];
-#pragma unroll
-            for (int i = 0; i < RB; ++i) {
-                v[i] = 0.f;
-                if (l0 + i < l_end)
-                    v[i] = row_dot_refill<BPL>(b[i], m, wp + (long long)(RB + i) * row_p, sp + (RB + i) * row_s,
-                                               l0 + RB + i < l_end, ok);
-            }
-            multi_reduce<RB>(v, lane);
-            if (multi_reduce_owner<RB>(lane)) {
-                const int l = l0 + multi_reduce_index<RB>(lane);
-                if (l < l_end) part[l][e] = v[0];
-            }
-            wp += (long long)RB * row_p;
-            sp += RB * row_s;
-        }
-    }
-    __syncthreads();
-
-    for (int t = threadIdx.x; t < n_local; t += blockDim.x) {
-        float acc = 0.f;
-        for (int k = 0; k < a.E; ++k) acc = fmaf(__ldcg(a.r + k), part[t][k], acc);
-        a.out[o_begin + t] = __float2bfloat16(acc);
-    }
-}
 
 // ------------------------------------------------------------------------------------------------
 // router: scores, top-k, normalised weights — on the device, no host round trip
@@ -513,28 +295,37 @@ static int grouped_try_ring(const GroupedArgs& a, cudaStream_t stream, const cha
     return 1;
 }
 
-template <int BPL_A, int BPL_B>
+// Any other shape: the two row-streaming kernels.
 static int grouped_launch(const GroupedArgs& a, cudaStream_t stream, const char* who, int stages) {
+    static int gate_done[64] = {0}, down_done[64] = {0};
     const int sms = sm_count();
     const bool pdl = pdl_enabled();
     if (stages & 1) {
+        RowPlan p = row_plan(a.K >> 5, 2, kGateRpw, 1);
         const long long pairs = (long long)a.E * a.H;
-        long long grid = sms;
-        const long long max_grid = (pairs + (kGateThreads / 32) - 1) / (kGateThreads / 32);
-        if (grid > max_grid) grid = max_grid;
-        cudaError_t err = launch(grouped_gate_up_kernel<BPL_A>, dim3((unsigned)grid), dim3(kGateThreads), stream,
-                                 pdl, a);
+        const long long grid = sms < pairs ? sms : pairs;
+        row_plan_scales(p, 2, a.K >> 5, a.K >> 5, 2);
+        row_plan_finish(p, a.K * 2, (uint32_t)(2 * 4 * ((pairs + grid - 1) / grid) * p.n_slices), 0);
+        cudaError_t err = allow_smem(grouped_gate_stream_kernel, p.smem, gate_done);
+        if (err == cudaSuccess)
+            err = launch_smem(grouped_gate_stream_kernel, dim3((unsigned)grid), dim3(kRowThreads), p.smem, stream, pdl, a, p);
         if (err != cudaSuccess) {
             std::fprintf(stderr, "%s: gate/up launch failed: %s\n", who, cudaGetErrorString(err));
             return -5;
         }
     }
     if (stages & 2) {
+        RowPlan p = row_plan(a.H >> 5, 1, kDownRpw, 1);
+        const long long cap = kDownParts / (4 * a.E * p.n_slices);           // output rows whose partial sums a CTA holds
         long long grid = sms;
-        const long long need = ((long long)a.O + kDownCap - 1) / kDownCap;
-        if (grid < need) grid = need;
+        if (grid < (a.O + cap - 1) / cap) grid = (a.O + cap - 1) / cap;
         if (grid > a.O) grid = a.O;
-        cudaError_t err = launch(grouped_down_kernel<BPL_B>, dim3((unsigned)grid), dim3(kDownThreads), stream, pdl, a);
+        row_plan_scales(p, 1, a.H >> 5, a.H >> 5, 1);
+        row_plan_finish(p, (uint32_t)a.E * (a.H >> 5) * 68, (uint32_t)(4 * ((a.O + grid - 1) / grid) * a.E * p.n_slices), 0);
+        cudaError_t err = allow_smem(grouped_down_stream_kernel, p.smem, down_done);
+        if (err == cudaSuccess)
+            err = launch_smem(grouped_down_stream_kernel, dim3((unsigned)grid), dim3(kRowThreads), p.smem, stream, pdl, a, p,
+                              stages == 3 ? 1 : 0);
         if (err != cudaSuccess) {
             std::fprintf(stderr, "%s: down launch failed: %s\n", who, cudaGetErrorString(err));
             return -6;
@@ -544,17 +335,8 @@ static int grouped_launch(const GroupedArgs& a, cudaStream_t stream, const char*
 }
 
 static int grouped_forward(const GroupedArgs& a, cudaStream_t stream, const char* who, int stages = 3) {
-    const int ba = ((a.K >> 5) + 31) >> 5;    // 16-byte blocks per lane on the K_in axis: 1..4
-    const int bb = ((a.H >> 5) + 31) >> 5;    // and on the hidden axis
-    const int bpl_a = ba <= 1 ? 1 : (ba <= 2 ? 2 : 4);
-    const int bpl_b = bb <= 1 ? 1 : (bb <= 2 ? 2 : 4);
     if (int rc = grouped_try_ring(a, stream, who, stages); rc != 1) return rc;
-#define DSV4_CASE(A, B) if (bpl_a == A && bpl_b == B) return grouped_launch<A, B>(a, stream, who, stages);
-    DSV4_CASE(1, 1) DSV4_CASE(1, 2) DSV4_CASE(1, 4)
-    DSV4_CASE(2, 1) DSV4_CASE(2, 2) DSV4_CASE(2, 4)
-    DSV4_CASE(4, 1) DSV4_CASE(4, 2) DSV4_CASE(4, 4)
-#undef DSV4_CASE
-    return -3;
+    return grouped_launch(a, stream, who, stages);
 }
 
 static int check_shape(const char* who, int K_in, int hidden, int out_dim) {
@@ -566,8 +348,8 @@ static int check_shape(const char* who, int K_in, int hidden, int out_dim) {
         std::fprintf(stderr, "%s: hidden=%d not a positive multiple of 32\n", who, hidden);
         return -2;
     }
-    if (K_in > 1024 * kMaxBlocksPerLane || hidden > 1024 * kMaxBlocksPerLane) {
-        std::fprintf(stderr, "%s: K_in/hidden > %d\n", who, 1024 * kMaxBlocksPerLane);
+    if (K_in > kMaxReduction || hidden > kMaxReduction) {
+        std::fprintf(stderr, "%s: K_in/hidden > %d\n", who, kMaxReduction);
         return -3;
     }
     if (out_dim <= 0) {

@@ -1,0 +1,190 @@
+// Row streaming through shared memory, shared by the dense GEMVs and the routed-expert FFN of one token.
+//
+// A CTA owns a contiguous range of weight rows.  One producer thread brings them in with bulk copies (cp.async.bulk, a
+// stage of whole rows and their scale bytes), up to kRowSlots stages ahead; sixteen consumer warps take a stage together: a
+// warp owns one slice of 32 16-byte blocks of the reduction axis (a lane one block of it) and every n_groups-th row, so its
+// activations stay in 8 or 16 registers.
+//
+// What bounds it: HBM, and the chain of one launch after another.  The products need x, so they all come after the wait
+// for the previous kernel; what can come before is the loading.  Loads into registers (the form before this one: 256
+// threads x 126 registers) filled the register file, so the next launch of a chain could not become resident and every
+// launch paid the whole ramp.  A CTA takes less than half of the SM's registers and shared memory here: under programmatic
+// dependent launch the next kernel's CTAs sit beside these and have their first ~90 KB per SM (13 MB) on the way while
+// these finish.  Nothing is loaded by the consumers inside the loop: a load queues behind the SM's own weight copies, one to
+// four microseconds (scale bytes fetched that way, two stages ahead, made 33.6 MB of FP8 take 11.1 us).
+#pragma once
+
+#include "gemv_engine.cuh"
+#include "stream_ring.cuh"
+
+namespace dsv4 {
+
+constexpr int kRowWarps = 16;                          // consumer warps
+constexpr int kRowThreads = (kRowWarps + 1) * 32;
+constexpr int kRowSlots = 8;                           // stages at most
+constexpr uint32_t kRowStage = 32 * 1024;              // weight bytes of one stage, where four rows per warp fit that
+constexpr uint32_t kRowSmem = 111 * 1024;              // dynamic shared memory of a CTA: two fit an SM
+constexpr uint32_t kRowSmemMost = 220 * 1024;          // taken where two stages would not fit otherwise
+
+__host__ __device__ __forceinline__ uint32_t round16(uint32_t v) { return (v + 15u) & ~15u; }
+
+// How a matrix of n_blk 16-byte blocks per row is cut up.  Slices beyond the 16 warps (FP8 rows longer than 8192) are taken
+// two per warp.
+struct RowPlan {
+    int n_slices, n_groups, warps;                     // warps that take part
+    int rows;                                          // rows per stage (of each matrix)
+    int slots;
+    uint32_t row_bytes, stage_bytes;
+    // scale bytes of the rows (MXFP4), behind the stage's weights: s_area bytes per matrix, see row_scale_offset
+    uint32_t s_area, s_pitch, s_adv;
+    uint32_t off_x, off_part, off_table;               // behind the ring
+    uint32_t smem;
+};
+// The bytes of a stage's scale rows are copied with the 16-byte chunks they lie in (such a chunk never leaves the memory page
+// of its bytes).  Rows dense in memory: one copy, row i at i * s_pitch behind the first; otherwise a copy per row, each with
+// its own misalignment.
+__device__ __forceinline__ uint32_t row_scale_offset(const RowPlan& p, uint32_t addr0, int i) {
+    return (uint32_t)i * p.s_pitch + ((addr0 + (uint32_t)i * p.s_adv) & 15u);
+}
+// rpw: rows per warp and stage, spw: slices per warp, mats: matrices streamed side by side
+inline RowPlan row_plan(int n_blk, int mats, int rpw, int spw) {
+    RowPlan p = {};
+    p.n_slices = (n_blk + 31) / 32;
+    const int w = (p.n_slices + spw - 1) / spw;
+    p.n_groups = kRowWarps / w;
+    p.warps = w * p.n_groups;
+    p.row_bytes = (uint32_t)n_blk * 16u;
+    p.rows = rpw * p.n_groups;
+    p.stage_bytes = (uint32_t)mats * p.rows * p.row_bytes;
+    return p;
+}
+// row_s scale bytes per row, stride bytes from row to row; `pieces` runs of rows that are apart in memory
+inline void row_plan_scales(RowPlan& p, int mats, uint32_t row_s, long long stride, int pieces) {
+    const bool dense = stride == (long long)row_s;
+    p.s_pitch = dense ? row_s : round16(row_s) + 16;
+    p.s_adv = dense ? 0u : (uint32_t)(stride & 15);
+    p.s_area = (dense ? round16(p.rows * row_s) : p.rows * p.s_pitch) + 32u * pieces;
+    p.stage_bytes += mats * p.s_area;
+}
+// Ring depth and offsets: x_bytes of activations, part_bytes of partial sums, table_bytes of tile scales behind the ring.
+inline void row_plan_finish(RowPlan& p, uint32_t x_bytes, uint32_t part_bytes, uint32_t table_bytes) {
+    const uint32_t rest = round16(x_bytes) + round16(part_bytes) + round16(table_bytes);
+    uint32_t most = kRowSmem;
+    if (rest + 2 * p.stage_bytes > most) most = kRowSmemMost;
+    const int fit = (int)((most - rest) / p.stage_bytes);
+    p.slots = fit < kRowSlots ? fit : kRowSlots;
+    p.off_x = p.slots * p.stage_bytes;
+    p.off_part = p.off_x + round16(x_bytes);
+    p.off_table = p.off_part + round16(part_bytes);
+    p.smem = p.off_table + round16(table_bytes);
+}
+
+// Scales.  Per row and block (MXFP4): they travel with the rows.  Per 128 x 128 tile (FP8): a table in shared memory.
+struct Fp4Scale {   // E8M0 [N, K/32]: one byte per row per block
+    static constexpr bool kPerRow = true;
+    __device__ static __forceinline__ uint32_t fetch(const uint8_t* s, int row, int blk, long long s_stride) {
+        return ldg_stream_u8(s + (long long)row * s_stride + blk);
+    }
+    __device__ static __forceinline__ float value(uint32_t raw) { return e8m0_to_float(raw); }
+};
+struct Fp8Scale {   // E8M0 [N/128, K/128]: one byte per 128x128 tile; a block is 16 elements
+    static constexpr bool kPerRow = false;
+    __device__ static __forceinline__ uint32_t fetch(const uint8_t* s, int row, int blk, long long s_stride) {
+        return ldg_stream_u8(s + (long long)(row >> 7) * s_stride + (blk >> 3));
+    }
+    __device__ static __forceinline__ float value(uint32_t raw) { return e8m0_to_float(raw); }
+};
+struct Fp8ScaleF32 {   // FP32 [N/128, K/128], row stride in bytes
+    static constexpr bool kPerRow = false;
+    __device__ static __forceinline__ uint32_t fetch(const uint8_t* s, int row, int blk, long long s_stride) {
+        return __ldg(reinterpret_cast<const uint32_t*>(s + (long long)(row >> 7) * s_stride) + (blk >> 3));
+    }
+    __device__ static __forceinline__ float value(uint32_t raw) { return __uint_as_float(raw); }
+};
+
+// The barriers of a CTA: the ring's, and one for x.
+struct RowRing {
+    uint64_t full[kRowSlots], empty[kRowSlots], x;
+};
+__device__ __forceinline__ void row_ring_init(RowRing& r, const RowPlan& p) {
+    for (int s = 0; s < p.slots; ++s) { mbar_init(smem_u32(&r.full[s]), 1); mbar_init(smem_u32(&r.empty[s]), p.warps); }
+    mbar_init(smem_u32(&r.x), 1);
+    mbar_init_fence();
+}
+struct RowPos {
+    int slot = 0;
+    uint32_t round = 0;
+    __device__ __forceinline__ void next(int n) { if (++slot == n) { slot = 0; ++round; } }
+};
+__device__ __forceinline__ void row_release(RowRing& r, const RowPlan& p, RowPos& pos, int lane) {
+    __syncwarp();
+    if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&r.empty[pos.slot])) : "memory");
+    pos.next(p.slots);
+}
+
+// `rows` weight rows from `src` to shared memory, dense there: one copy where they are dense in memory.  Returns the bytes.
+__device__ __forceinline__ void row_copy(uint32_t dst, const uint8_t* src, long long stride, uint32_t row_bytes, int rows, uint32_t bar) {
+    if (stride == (long long)row_bytes) {
+        bulk_copy_g2s(dst, src, rows * row_bytes, bar);
+    } else {
+        for (int i = 0; i < rows; ++i) bulk_copy_g2s(dst + i * row_bytes, src + i * stride, row_bytes, bar);
+    }
+}
+// Bytes that the copies of `rows` scale rows at `src` bring in, and the copies.
+__device__ __forceinline__ uint32_t row_scale_bytes(const RowPlan& p, const uint8_t* src, uint32_t row_s, int rows) {
+    const uint32_t a = (uint32_t)reinterpret_cast<uintptr_t>(src);
+    if (p.s_pitch == row_s) return round16((a & 15u) + rows * row_s);
+    uint32_t sum = 0;
+    for (int i = 0; i < rows; ++i) sum += round16(((a + i * p.s_adv) & 15u) + row_s);
+    return sum;
+}
+__device__ __forceinline__ void row_scale_copy(const RowPlan& p, uint32_t dst, const uint8_t* src, long long stride, uint32_t row_s, int rows,
+                                               uint32_t bar) {
+    if (p.s_pitch == row_s) {
+        const uint32_t mis = (uint32_t)reinterpret_cast<uintptr_t>(src) & 15u;
+        bulk_copy_g2s(dst, src - mis, round16(mis + rows * row_s), bar);
+    } else {
+        for (int i = 0; i < rows; ++i) {
+            const uint8_t* at = src + i * stride;
+            const uint32_t mis = (uint32_t)reinterpret_cast<uintptr_t>(at) & 15u;
+            bulk_copy_g2s(dst + i * p.s_pitch, at - mis, round16(mis + row_s), bar);
+        }
+    }
+}
+
+// This lane's activation block from a bf16 vector in shared memory.
+template <class Fmt>
+__device__ __forceinline__ void row_act_block(uint32_t x_smem, int blk, bool valid, ActBlock<Fmt>& a) {
+    float v[Fmt::kElems];
+#pragma unroll
+    for (int i = 0; i < Fmt::kElems / 8; ++i) {
+        uint4 q = make_uint4(0, 0, 0, 0);
+        if (valid) q = lds_v4(x_smem + (uint32_t)blk * (Fmt::kElems * 2) + 16 * i);
+        const uint32_t u[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            v[8 * i + 2 * j + 0] = __uint_as_float(u[j] << 16);
+            v[8 * i + 2 * j + 1] = __uint_as_float(u[j] & 0xffff0000u);
+        }
+    }
+    act_block_finish<Fmt>(v, a);
+}
+// x (bf16, 16-byte aligned, a multiple of 16 bytes) -> shared memory, once per CTA, by one thread after its pdl_wait: every
+// warp reading its slice from global memory put 600 readers on each line of x, half a microsecond of L2 time.
+__device__ __forceinline__ void row_x_request(RowRing& r, uint32_t x_smem, const __nv_bfloat16* x, uint32_t bytes) {
+    mbar_arrive_expect_tx(smem_u32(&r.x), bytes);
+    bulk_copy_g2s(x_smem, x, bytes, smem_u32(&r.x));
+}
+
+// Sums over the lanes of a warp's rows of one stage: v[m * RPW + i] is row i * n_groups of matrix m, and goes to
+// part[m * mat_stride + i * n_groups * part_stride] (one writer per row).
+template <int RPW, int V>
+__device__ __forceinline__ void row_store(float (&v)[V], int rows_left, int n_groups, int lane, float* part, int part_stride, int mat_stride) {
+    multi_reduce<V>(v, lane);
+    if (multi_reduce_owner<V>(lane)) {
+        const int k = multi_reduce_index<V>(lane), i = k % RPW;
+        if (i * n_groups < rows_left) part[(V > RPW ? k / RPW * mat_stride : 0) + i * n_groups * part_stride] = v[0];
+    }
+}
+
+}  // namespace dsv4
