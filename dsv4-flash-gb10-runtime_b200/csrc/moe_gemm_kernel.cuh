@@ -11,14 +11,17 @@
 //
 // A tile: 128 rows of two matrices (gate/up: the same rows of W1 and W3; down: two row blocks of W2) x up to 128 tokens.
 // CTA = 20 warps (five per scheduler: 96 registers a thread), persistent grid, one CTA per SM, tiles by static striding:
-//   warps 0..15  dequantise: warp = (K-block parity, matrix, lane quadrant); a thread owns one weight row, takes 32
+//   warp 0       issues the MMAs (one thread)
+//   warp 1       token rows -> shared memory (one TMA box per K-block, the rows of a tile being neighbours)
+//   warp 2       packed weights -> shared memory (TMA, 256 K-elements = 16 KB per matrix and stage) and their scales
+//   warp 3       a tile ahead: token tables, and the largest scale byte of every row
+//   warps 4..19  dequantise: warp = (K-block parity, matrix, lane quadrant); a thread owns one weight row, takes 32
 //                bytes and two scale bytes of it per K-block of 64 and writes 32 tensor-memory columns.  They also drain the
 //                finished accumulators, after the first stages of the NEXT tile are in tensor memory, so that the MMAs
 //                continue as soon as the accumulators have been read.
-//   warp 16      token rows -> shared memory (one TMA box per K-block, the rows of a tile being neighbours), six ahead
-//   warp 17      packed weights -> shared memory (TMA, 256 K-elements = 16 KB per matrix and stage) and their scales
-//   warp 18      issues the MMAs
-//   warp 19      a tile ahead: token tables, and the largest scale byte of every row
+// A K-block's weights (in tensor memory) and tokens (in shared memory) share one full and one empty barrier: for tiles of a
+// few tokens the issuing thread sets the pace, not the MMAs (320 clocks), and with a barrier pair for each operand
+// it took 1 070 clocks per K-block.
 // Tensor memory: columns 0..255 two accumulators of 128, 256..511 four stages of two 128 x 64 fp16 tiles.
 // Every wait is bounded (stream_ring.cuh).
 #pragma once
@@ -27,19 +30,17 @@
 
 namespace dsv4 {
 
-constexpr int kTmDequantWarps = 16;
-constexpr int kTmTokenWarp = kTmDequantWarps, kTmWeightWarp = kTmTokenWarp + 1;
-constexpr int kTmMmaWarp = kTmWeightWarp + 1, kTmAuxWarp = kTmMmaWarp + 1;
-constexpr int kTmThreads = (kTmAuxWarp + 1) * 32;
+constexpr int kTmMmaWarp = 0, kTmTokenWarp = 1, kTmWeightWarp = 2, kTmAuxWarp = 3, kTmDequantWarp = 4, kTmDequantWarps = 16;
+constexpr int kTmThreads = (kTmDequantWarp + kTmDequantWarps) * 32;
 constexpr int kTmKBlock = 64;                         // K-elements per tensor-memory / token stage
 constexpr int kTmWBlock = 256;                        // K-elements per packed-weight stage (128 bytes per row)
-constexpr int kTmWStages = 3, kTmAStages = 4, kTmBStages = 6, kTmTables = 3;
+constexpr int kTmWStages = 4, kTmStages = 4, kTmTables = 3;
 constexpr uint32_t kTmWTile = 128 * 128;              // packed weights of one matrix and stage
 constexpr uint32_t kTmWScale = 128 * 8;               // scale bytes of one matrix and stage
 constexpr uint32_t kTmWStage = 2 * kTmWTile + 2 * kTmWScale;
 constexpr uint32_t kTmBStage = kMoeTileTokens * 128;
 constexpr uint32_t kTmOffB = kTmWStages * 2 * kTmWTile;                       // every tile 1024-byte aligned
-constexpr uint32_t kTmOffS = kTmOffB + kTmBStages * kTmBStage;
+constexpr uint32_t kTmOffS = kTmOffB + kTmStages * kTmBStage;
 constexpr uint32_t kTmSmem = kTmOffS + kTmWStages * 2 * kTmWScale + 1024;
 
 struct MoeGemmArgs {
@@ -107,8 +108,7 @@ __device__ __forceinline__ void dequant_block(const uint4& w, uint32_t mult, uin
 template <int MODE>
 __global__ void __launch_bounds__(kTmThreads, 1) moe_gemm_kernel(const __grid_constant__ MoeMaps maps, const MoeGemmArgs a) {
     extern __shared__ __align__(1024) uint8_t gemm_smem[];
-    __shared__ __align__(8) uint64_t w_full[kTmWStages], w_empty[kTmWStages], a_full[kTmAStages], a_empty[kTmAStages];
-    __shared__ __align__(8) uint64_t b_full[kTmBStages], b_empty[kTmBStages];
+    __shared__ __align__(8) uint64_t w_full[kTmWStages], w_empty[kTmWStages], full[kTmStages], empty[kTmStages];
     __shared__ __align__(8) uint64_t acc_full, acc_free, exp_full[kTmTables], tab_free[kTmTables];
     __shared__ uint32_t tmem_holder;
     __shared__ int s_tiles[kMoeMaxExperts + 1], s_offsets[kMoeMaxExperts + 1];
@@ -124,8 +124,7 @@ __global__ void __launch_bounds__(kTmThreads, 1) moe_gemm_kernel(const __grid_co
     if (warp == kTmMmaWarp) tc05_alloc(smem_u32(&tmem_holder), 512);
     if (tid == 0) {
         for (int s = 0; s < kTmWStages; ++s) { mbar_init(smem_u32(&w_full[s]), 1 + 32); mbar_init(smem_u32(&w_empty[s]), kTmDequantWarps); }
-        for (int s = 0; s < kTmAStages; ++s) { mbar_init(smem_u32(&a_full[s]), kTmDequantWarps / 2); mbar_init(smem_u32(&a_empty[s]), 1); }
-        for (int s = 0; s < kTmBStages; ++s) { mbar_init(smem_u32(&b_full[s]), 1); mbar_init(smem_u32(&b_empty[s]), 1); }
+        for (int s = 0; s < kTmStages; ++s) { mbar_init(smem_u32(&full[s]), kTmDequantWarps / 2 + 1); mbar_init(smem_u32(&empty[s]), 1); }
         for (int s = 0; s < kTmTables; ++s) {
             mbar_init(smem_u32(&exp_full[s]), 1);
             mbar_init(smem_u32(&tab_free[s]), kTmDequantWarps);
@@ -156,8 +155,8 @@ __global__ void __launch_bounds__(kTmThreads, 1) moe_gemm_kernel(const __grid_co
     };
     uint32_t tc = 0;                                          // tiles begun by this CTA
 
-    if (warp < kTmDequantWarps) {
-        const int group = warp >> 3, mat = (warp >> 2) & 1, quad = warp & 3, row = quad * 32 + lane;
+    if (warp >= kTmDequantWarp) {
+        const int dw = warp - kTmDequantWarp, group = dw >> 3, mat = (dw >> 2) & 1, quad = warp & 3, row = quad * 32 + lane;
 
         // accumulators of tile number `count` -> global memory; warps q, q + 4, q + 8, q + 12 share lane quadrant q and take
         // token chunks of 16 in turn
@@ -166,7 +165,7 @@ __global__ void __launch_bounds__(kTmThreads, 1) moe_gemm_kernel(const __grid_co
             tc05_fence_after_sync();
             const uint32_t trow = tmem + ((uint32_t)(quad * 32) << 16);
             const uint32_t tab = count % kTmTables;
-            const int c0 = (warp >> 2) * 16;
+            const int c0 = (dw >> 2) * 16;
             const int m = t.m0 + row;
             bool handed = false;
             const int ea = row_exp[tab][0][row], eb = row_exp[tab][1][row];
@@ -215,7 +214,7 @@ __global__ void __launch_bounds__(kTmThreads, 1) moe_gemm_kernel(const __grid_co
                 }
                 if (has) store(g, u, c);
             }
-            if (MODE == 0 && t.m0 == 0 && warp == 0)
+            if (MODE == 0 && t.m0 == 0 && dw == 0)
                 for (int n = lane; n < t.n_valid; n += 32) {
                     const int2 x = __ldcg(a.xexp + t.slot0 + n);
                     a.mid_exp[t.slot0 + n] = 2 * (x.x + x.y) + mid_base;
@@ -241,9 +240,9 @@ __global__ void __launch_bounds__(kTmThreads, 1) moe_gemm_kernel(const __grid_co
                 const uint4 w1 = lds_v4(wrow + (((2 * q + 1) ^ (row & 7)) << 4));
                 uint32_t sc;
                 asm volatile("ld.shared.u16 %0, [%1];" : "=r"(sc) : "r"(smem0 + kTmOffS + (ws * 2 + mat) * kTmWScale + row * 8 + q * 2));
-                const uint32_t as = it % kTmAStages;
+                const uint32_t as = it % kTmStages;
                 const uint32_t acol = tmem + ((uint32_t)(quad * 32) << 16) + 256 + as * 64 + mat * 32;
-                if (it >= kTmAStages) wait(a_empty[as], it / kTmAStages - 1, 4);
+                if (it >= kTmStages) wait(empty[as], it / kTmStages - 1, 4);
                 tc05_fence_after_sync();
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
@@ -258,7 +257,7 @@ __global__ void __launch_bounds__(kTmThreads, 1) moe_gemm_kernel(const __grid_co
                 tc05_wait_st();
                 tc05_fence_before_sync();
                 __syncwarp();
-                if (lane == 0) mbar_arrive_one(smem_u32(&a_full[as]));
+                if (lane == 0) mbar_arrive_one(smem_u32(&full[as]));
                 // the first stages of this tile are in tensor memory: now drain the previous one
                 if (has_prev && kb == group + 2) drain(prev, tc - 1);
             }
@@ -275,16 +274,13 @@ __global__ void __launch_bounds__(kTmThreads, 1) moe_gemm_kernel(const __grid_co
                 const MoeTile t = decode(tile);
                 const uint32_t bytes = (uint32_t)moe_width(t.width, kMoeTileTokens) * 128u;
                 for (int kb = 0; kb < n_kb; ++kb, ++it) {
-                    const uint32_t s = it % kTmBStages;
-                    if (it >= kTmBStages) wait_one(b_empty[s], it / kTmBStages - 1, 4);
+                    const uint32_t s = it % kTmStages;
+                    if (it >= kTmStages) wait_one(empty[s], it / kTmStages - 1, 4);
                     if (!alive) break;
-                    mbar_arrive_expect_tx(smem_u32(&b_full[s]), bytes);
-                    tma_load_2d(smem0 + kTmOffB + s * kTmBStage, &maps.act[t.width], kb * kTmKBlock, t.slot0, smem_u32(&b_full[s]));
+                    mbar_arrive_expect_tx(smem_u32(&full[s]), bytes);
+                    tma_load_2d(smem0 + kTmOffB + s * kTmBStage, &maps.act[t.width], kb * kTmKBlock, t.slot0, smem_u32(&full[s]));
                 }
             }
-            if (!alive)                         // gave up: let the copies in flight land before shared memory is released
-                for (uint32_t i = it > kTmBStages ? it - kTmBStages : 0; i < it; ++i)
-                    mbar_wait_limit(smem_u32(&b_full[i % kTmBStages]), (i / kTmBStages) & 1u, 0, 1u << 12);
         }
         __syncwarp();
     } else if (warp == kTmWeightWarp) {
@@ -331,12 +327,11 @@ __global__ void __launch_bounds__(kTmThreads, 1) moe_gemm_kernel(const __grid_co
                 const uint32_t idesc = tc05_idesc_f16(128, moe_width(t.width, kMoeTileTokens));
                 if (tc > 0) wait_one(acc_free, tc - 1, 7);
                 for (int kb = 0; kb < n_kb; ++kb, ++it) {
-                    const uint32_t as = it % kTmAStages, bs = it % kTmBStages;
-                    wait_one(b_full[bs], it / kTmBStages, 5);
-                    wait_one(a_full[as], it / kTmAStages, 5);
+                    const uint32_t as = it % kTmStages;
+                    wait_one(full[as], it / kTmStages, 5);
                     if (!alive) break;
                     tc05_fence_after_sync();
-                    const uint64_t db = tc05_desc_k_sw128(smem0 + kTmOffB + bs * kTmBStage);
+                    const uint64_t db = tc05_desc_k_sw128(smem0 + kTmOffB + as * kTmBStage);
                     const uint32_t at = tmem + 256 + as * 64;
                     if (t.mats == 2) {
 #pragma unroll
@@ -350,8 +345,7 @@ __global__ void __launch_bounds__(kTmThreads, 1) moe_gemm_kernel(const __grid_co
                         for (int j = 0; j < kTmKBlock / 16; ++j)
                             tc05_mma_f16_ts(tmem, at + j * 8, db + 2 * j, idesc, (kb > 0 || j > 0) ? 1u : 0u);
                     }
-                    tc05_commit(smem_u32(&a_empty[as]));
-                    tc05_commit(smem_u32(&b_empty[bs]));
+                    tc05_commit(smem_u32(&empty[as]));
                     if (kb == n_kb - 1) tc05_commit(smem_u32(&acc_full));
                 }
             }

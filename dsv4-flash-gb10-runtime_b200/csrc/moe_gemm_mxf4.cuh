@@ -22,12 +22,14 @@
 // neighbours in memory, in slot order), ONE full and ONE empty barrier.  Gathering token rows four at a time instead took
 // 36 copies per stage and held the stream at 4.6 TB/s.  Why pairs: they halve the activations a CTA takes in.
 //
-// CTA = 14 warps, persistent grid, one CTA per SM, tiles by static striding over the pairs:
-//   warps 0..7    epilogue: accumulators -> SwiGLU -> three MXFP4 terms (gate/up), or -> FP32 rows (down)
-//   warps 8..11   scale bytes of weights and activations -> 512-byte scale atoms in shared memory, two to four stages of
-//                 loads ahead
-//   warp 12       producer (one thread)
-//   warp 13       (CTA 0, one thread) scale atoms -> tensor memory, MMAs of the pair
+// CTA = 24 warps, persistent grid, one CTA per SM, tiles by static striding over the pairs:
+//   warp 0        (CTA 0, one thread) scale atoms -> tensor memory, MMAs of the pair
+//   warp 1        producer (one thread)
+//   warps 4..15   epilogue: accumulators -> SwiGLU -> three MXFP4 terms (gate/up), or -> FP32 rows (down)
+//   warps 16..23  scale bytes of weights and activations -> 512-byte scale atoms in shared memory; two groups of four warps
+//                 take pairs of stages in turn, their loads a pair ahead, across tiles
+// With one group of scale warps (busy 1 200 clocks per stage) and eight epilogue warps (1 100) the two of them, not the MMAs,
+// set the pace: 1 700 clocks per stage of gate/up and 2 170 of down, whose tiles are half as long.
 // The full barriers are CTA 0's: copies and scale warps of both CTAs arrive there.  The "empty" and "accumulator full"
 // barriers are signalled in both CTAs by the commits.
 // No operand passes through a register.
@@ -46,9 +48,11 @@ constexpr uint32_t kQTile = 128 * 128;               // bytes of one packed weig
 constexpr uint32_t kQBStage = kQTerms * (kQTok / 2) * 128;           // activation rows of one stage and CTA
 constexpr uint32_t kQSfStage = 2 * 2 * 512 + 2 * kQTerms * 512;      // scale atoms: [mat][atom], then [atom][term]
 constexpr int kQStages = 3;
-constexpr int kQEpiWarps = 8, kQScaleWarps = 4;
-constexpr int kQScaleWarp = kQEpiWarps, kQProducerWarp = kQScaleWarp + kQScaleWarps, kQMmaWarp = kQProducerWarp + 1;
-constexpr int kQThreads = (kQMmaWarp + 1) * 32;
+constexpr int kQEpiWarps = 12, kQScaleWarps = 8;
+constexpr int kQEpiGroups = kQEpiWarps / 4;          // warps per lane quadrant of tensor memory
+constexpr int kQEpiRounds = (kQTok + 16 * kQEpiGroups - 1) / (16 * kQEpiGroups);
+constexpr int kQMmaWarp = 0, kQProducerWarp = 1, kQEpiWarp = 4, kQScaleWarp = kQEpiWarp + kQEpiWarps;    // warps 2, 3: idle
+constexpr int kQThreads = (kQScaleWarp + kQScaleWarps) * 32;
 constexpr uint32_t kQAccCols = 2 * kQTok;            // per accumulator set
 constexpr uint32_t kQSfCol = 2 * kQAccCols, kQSfCols = 16 + 8 * kQTerms;
 static_assert(kQSfCol + kQSfCols <= 512, "tensor memory overflow");
@@ -211,7 +215,7 @@ __global__ void __launch_bounds__(kQThreads, 1) moe_gemm_mxf4_kernel(const __gri
 
     if (warp == kQMmaWarp) tc05_pair_alloc(smem_u32(&tmem_holder), 512);
     if (tid == 0) {
-        for (int s = 0; s < kQStages; ++s) { mbar_init(smem_u32(&full[s]), 2 * (1 + kQScaleWarps)); mbar_init(smem_u32(&empty[s]), 1); }
+        for (int s = 0; s < kQStages; ++s) { mbar_init(smem_u32(&full[s]), 2 * (1 + kQScaleWarps / 2)); mbar_init(smem_u32(&empty[s]), 1); }
         for (int s = 0; s < 2; ++s) { mbar_init(smem_u32(&acc_full[s]), 1); mbar_init(smem_u32(&acc_free[s]), 2 * kQEpiWarps); }
         mbar_init_fence();
     }
@@ -240,28 +244,28 @@ __global__ void __launch_bounds__(kQThreads, 1) moe_gemm_mxf4_kernel(const __gri
     };
     uint32_t tc = 0;                                          // tiles begun by this pair
 
-    if (warp < kQEpiWarps) {
+    if (warp >= kQEpiWarp && warp < kQScaleWarp) {
         const int quad = warp & 3, r = quad * 32 + lane;
         pdl_wait();
         for (int tile = pair; tile < n_tiles; tile += n_pairs, ++tc) {
             const MoeQTile t = decode(tile);
             const uint32_t buf = tc & 1u;
             const int m0 = t.m0 + rank * kMoeTileRows;        // first row of this CTA in block 0
-            // router weights (down): lane i holds those of tokens i and i + 16 of this warp's chunks, see below
-            float w[4];
+            // router weights (down): lanes i and i + 16 hold that of token i of each of this warp's chunks
+            float w[kQEpiRounds];
             if (MODE == 1)
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int n = (warp >> 2) * 16 + 32 * i + (lane & 15);
+                for (int i = 0; i < kQEpiRounds; ++i) {
+                    const int n = (((warp - kQEpiWarp) >> 2) + kQEpiGroups * i) * 16 + (lane & 15);
                     w[i] = n < t.n_valid ? __ldcg(a.g.slot_w + t.slot0 + n) : 0.f;
                 }
             wait(acc_full[buf], tc >> 1, 6);
             tc05_fence_after_sync();
             const uint32_t trow = tmem + ((uint32_t)(quad * 32) << 16) + buf * kQAccCols;
-            // two warps per lane quadrant take chunks of 16 tokens in turn
+            // the warps of a lane quadrant take chunks of 16 tokens in turn
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const int c = (warp >> 2) * 16 + 32 * k;
+            for (int k = 0; k < kQEpiRounds; ++k) {
+                const int c = (((warp - kQEpiWarp) >> 2) + kQEpiGroups * k) * 16;
                 if (c >= t.n_valid || !alive) break;
                 const int n = min(16, t.n_valid - c);
                 uint32_t p0[16], p1[16];
@@ -305,67 +309,77 @@ __global__ void __launch_bounds__(kQThreads, 1) moe_gemm_mxf4_kernel(const __gri
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(leader(acc_free[buf]));
         }
-    } else if (warp < kQProducerWarp) {
-        // ---- scale bytes: 8 per row and stage.  Thread st holds weight row st of both matrices and up to three of the
-        // (term, token) rows; the loads of a stage are issued two to four stages before their bytes are stored.
-        const int st = tid - kQScaleWarp * 32;
-        RingPos pos;
-        pdl_wait();
-        for (int tile = pair; tile < n_tiles; tile += n_pairs) {
-            const MoeQTile t = decode(tile);
-            const uint8_t* src[2 + kQTerms];
-            uint32_t dst[2 + kQTerms];
-            const int m0 = t.m0 + rank * kMoeTileRows;
-            const long long first = (long long)t.e * a.rows + m0 + st;
-            src[0] = m0 < a.rows ? a.wa_s + first * row_s : nullptr;
-            src[1] = MODE == 0 ? a.wb_s + first * row_s : m0 + kQRows < a.rows ? a.wa_s + (first + kQRows) * row_s : nullptr;
-            dst[0] = tc05_scale_atom_offset(st, 0);
-            dst[1] = dst[0] + 1024;
+    } else if (warp >= kQScaleWarp) {
+        // ---- scale bytes: 8 per row and stage.  Thread st of a group holds weight row st of both matrices and token st of
+        // every term.  A group takes every second pair of stages (16 bytes of a row per load); its next pair is loaded
+        // before the current one is stored, whichever tile it belongs to.
+        const int st = (tid - kQScaleWarp * 32) & 127, group = (warp - kQScaleWarp) >> 2;
+        const int n_prs = (n_st + 1) >> 1;
+        int tile = pair, count = 0, pr = group;               // next pair to load: pr of tile number `count`
+        const uint8_t* src[2 + kQTerms] = {};
+        bool fresh = true;
+        struct Loaded { uint4 v[2 + kQTerms]; uint32_t has; uint32_t it; bool two; };
+        auto load = [&](Loaded& l) -> bool {
+            while (pr >= n_prs) { pr -= n_prs; tile += n_pairs; ++count; fresh = true; }
+            if (tile >= n_tiles) return false;
+            if (fresh) {
+                const MoeQTile t = decode(tile);
+                const int m0 = t.m0 + rank * kMoeTileRows;
+                const long long first = (long long)t.e * a.rows + m0 + st;
+                src[0] = m0 < a.rows ? a.wa_s + first * row_s : nullptr;
+                src[1] = MODE == 0 ? a.wb_s + first * row_s : m0 + kQRows < a.rows ? a.wa_s + (first + kQRows) * row_s : nullptr;
 #pragma unroll
-            for (int i = 0; i < kQTerms; ++i) {               // thread st: token st of every term
-                dst[2 + i] = 2048 + i * 512 + dst[0];
-                src[2 + i] = st < t.n_valid ? a.act_s + (i * a.n_pairs + t.slot0 + st) * row_s : nullptr;
+                for (int i = 0; i < kQTerms; ++i)
+                    src[2 + i] = st < t.n_valid ? a.act_s + (i * a.n_pairs + t.slot0 + st) * row_s : nullptr;
+                fresh = false;
             }
-            // two stages (16 bytes of a row) per load, one load where the rows are 16-byte aligned
-            uint4 v[2][2 + kQTerms];
-            auto fetch = [&](uint4 (&to)[2 + kQTerms], int s) {
-                if (s >= n_st) return;
+            l.has = 0;
+            l.it = (uint32_t)count * n_st + 2 * pr;
+            l.two = 2 * pr + 1 < n_st;
 #pragma unroll
-                for (int i = 0; i < 2 + kQTerms; ++i) {
-                    if (!src[i]) continue;
-                    if ((row_s & 15) == 0) {
-                        to[i] = __ldcg(reinterpret_cast<const uint4*>(src[i] + 8 * s));
-                    } else {
-                        const uint2* p = reinterpret_cast<const uint2*>(src[i] + 8 * s);
-                        const uint2 lo = __ldcg(p), hi = s + 1 < n_st ? __ldcg(p + 1) : make_uint2(0, 0);
-                        to[i] = make_uint4(lo.x, lo.y, hi.x, hi.y);
-                    }
+            for (int i = 0; i < 2 + kQTerms; ++i) {
+                if (!src[i]) continue;
+                l.has |= 1u << i;
+                if ((row_s & 15) == 0) {                       // otherwise the rows are 8-byte aligned
+                    l.v[i] = __ldcg(reinterpret_cast<const uint4*>(src[i]) + pr);
+                } else {
+                    const uint2* p = reinterpret_cast<const uint2*>(src[i]) + 2 * pr;
+                    const uint2 lo = __ldcg(p), hi = l.two ? __ldcg(p + 1) : make_uint2(0, 0);
+                    l.v[i] = make_uint4(lo.x, lo.y, hi.x, hi.y);
                 }
-            };
-            auto put = [&](const uint4 (&from)[2 + kQTerms], bool second) {
-                if (pos.round > 0) wait(empty[pos.slot], pos.round - 1, 4);
-                const uint32_t sf = smem_sf + pos.slot * kQSfStage;
-#pragma unroll
-                for (int i = 0; i < 2 + kQTerms; ++i)
-                    if (src[i]) {                             // scales 0..3 -> atom 0, 4..7 -> atom 1
-                        asm volatile("st.shared.u32 [%0], %1;" ::"r"(sf + dst[i]), "r"(second ? from[i].z : from[i].x) : "memory");
-                        asm volatile("st.shared.u32 [%0], %1;" ::"r"(sf + dst[i] + (i < 2 ? 512u : kQTerms * 512u)), "r"(second ? from[i].w : from[i].y) : "memory");
-                    }
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                __syncwarp();
-                if (lane == 0) mbar_arrive_cluster(leader(full[pos.slot]));
-                pos.next(kQStages);
-            };
-            fetch(v[0], 0);
-            fetch(v[1], 2);
-            for (int s = 0; s < n_st; s += 4) {
-                put(v[0], false);
-                if (s + 1 < n_st) put(v[0], true);
-                fetch(v[0], s + 4);
-                if (s + 2 < n_st) put(v[1], false);
-                if (s + 3 < n_st) put(v[1], true);
-                fetch(v[1], s + 6);
             }
+            pr += 2;
+            return true;
+        };
+        const uint32_t atom = tc05_scale_atom_offset(st, 0);
+        auto put_stage = [&](const Loaded& l, uint32_t it, bool second) {
+            const uint32_t slot = it % kQStages, round = it / kQStages;
+            if (round > 0) wait(empty[slot], round - 1, 4);
+            const uint32_t sf = smem_sf + slot * kQSfStage + atom;
+#pragma unroll
+            for (int i = 0; i < 2 + kQTerms; ++i)
+                if (l.has & (1u << i)) {                       // scales 0..3 -> atom 0, 4..7 -> atom 1
+                    const uint32_t at = sf + (i < 2 ? i * 1024u : 2048u + (i - 2) * 512u);
+                    asm volatile("st.shared.u32 [%0], %1;" ::"r"(at), "r"(second ? l.v[i].z : l.v[i].x) : "memory");
+                    asm volatile("st.shared.u32 [%0], %1;" ::"r"(at + (i < 2 ? 512u : kQTerms * 512u)), "r"(second ? l.v[i].w : l.v[i].y) : "memory");
+                }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(leader(full[slot]));
+        };
+        auto put = [&](const Loaded& l) {
+            put_stage(l, l.it, false);
+            if (l.two) put_stage(l, l.it + 1, true);
+        };
+        pdl_wait();
+        Loaded l0, l1;
+        bool more = load(l0);
+        while (more) {
+            more = load(l1);
+            put(l0);
+            if (!more) break;
+            more = load(l0);
+            put(l1);
         }
     } else if (warp == kQProducerWarp) {
         // ---- this role and the MMAs are one thread each: nothing in their loops is done by a warp, so no vote or
@@ -373,8 +387,9 @@ __global__ void __launch_bounds__(kQThreads, 1) moe_gemm_mxf4_kernel(const __gri
         if (tc05_elect_one()) {
             RingPos pos;
             bool waited = false;
-            for (int tile = pair; tile < n_tiles && alive; tile += n_pairs) {
-                const MoeQTile t = decode(tile);
+            MoeQTile t = {}, next = {};                       // the next tile is looked up while this one's stages are on their way
+            if (pair < n_tiles) t = decode(pair);
+            for (int tile = pair; tile < n_tiles && alive; tile += n_pairs, t = next) {
                 const int first = t.e * a.rows + t.m0 + rank * kMoeTileRows;      // past the expert in a half tile: loaded, not used
                 const int half = moe_width(t.width, kQTok) >> 1, slot = t.slot0 + rank * half;
                 const CUtensorMap* act = &maps.act[t.width];
@@ -403,16 +418,19 @@ __global__ void __launch_bounds__(kQThreads, 1) moe_gemm_mxf4_kernel(const __gri
                     if (!alive) break;
                     weights(s, pos);
                     tokens(s, pos);
+                    if (s == n_st >> 1 && tile + n_pairs < n_tiles) next = decode(tile + n_pairs);
                 }
+                if (s0 > n_st >> 1 && tile + n_pairs < n_tiles) next = decode(tile + n_pairs);
             }
             if (!waited) { pdl_wait(); pdl_launch_dependents(); }
         }
         __syncwarp();
-    } else {
+    } else if (warp == kQMmaWarp) {
         if (rank == 0 && tc05_elect_one()) {
             RingPos pos;
-            for (int tile = pair; tile < n_tiles && alive; tile += n_pairs, ++tc) {
-                const MoeQTile t = decode(tile);
+            MoeQTile t = {}, next = {};
+            if (pair < n_tiles) t = decode(pair);
+            for (int tile = pair; tile < n_tiles && alive; tile += n_pairs, ++tc, t = next) {
                 const uint32_t buf = tc & 1u;
                 const int n = moe_width(t.width, kQTok);
                 MoeQStage q;
@@ -432,6 +450,7 @@ __global__ void __launch_bounds__(kQThreads, 1) moe_gemm_mxf4_kernel(const __gri
                     q.fresh = s == 0;
                     if (t.mats == 2) moe_q_issue<2>(q); else moe_q_issue<1>(q);
                     tc05_pair_commit(smem_u32(&empty[pos.slot]));
+                    if (s == n_st >> 1 && tile + n_pairs < n_tiles) next = decode(tile + n_pairs);
                     if (s == n_st - 1) tc05_pair_commit(smem_u32(&acc_full[buf]));
                 }
             }
