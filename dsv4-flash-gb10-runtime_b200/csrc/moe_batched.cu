@@ -160,11 +160,11 @@ cudaError_t term_maps(CUtensorMap (&map)[kMoeWidths], const uint8_t* base, long 
     return err;
 }
 // fp16 activations [P, K]: a tile's columns
-cudaError_t half_maps(CUtensorMap (&map)[kMoeWidths], const __half* base, long long P, int K) {
+cudaError_t half_maps(CUtensorMap (&map)[kMoeWidths], const __half* base, long long P, int K, int cap) {
     cudaError_t err = cudaSuccess;
     for (int i = 0; i < kMoeWidths && err == cudaSuccess; ++i) {
         const cuuint64_t dim[2] = {(cuuint64_t)K, (cuuint64_t)P};
-        const cuuint32_t box[2] = {kTmKBlock, (cuuint32_t)moe_width(i, kMoeTileTokens)};
+        const cuuint32_t box[2] = {64, (cuuint32_t)moe_width(i, cap)};
         err = box_map(&map[i], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, base, 2, dim, box);
     }
     return err;
@@ -264,7 +264,8 @@ static int moe_forward_impl(int path, const __nv_bfloat16* x, const uint8_t* ban
     ga.ids = ids; ga.weights = weights; ga.n_pairs = P; ga.n_experts = n_experts; ga.g = g; ga.status = status;
     const int rows_up = path == 1 ? kQTileRowsUp : kMoeTileRows, rows_down = path == 1 ? kQTileRowsDown : 2 * kMoeTileRows;
     ga.m_tiles_up = hidden / rows_up; ga.m_tiles_down = (out_dim + rows_down - 1) / rows_down;
-    ga.tile_tokens = path == 1 ? kQTok : kMoeTileTokens;
+    const int cap16 = P <= (long long)kTmFewTokens * n_experts ? 64 : kMoeTileTokens;      // tokens per tile, fp16 path
+    ga.tile_tokens = path == 1 ? kQTok : cap16;
     launch_k(moe_group_kernel, dim3(P > kGroupOneBlockPairs ? kGroupCluster : 1), dim3(kPrepThreads), 0, stream, P > kGroupOneBlockPairs ? kGroupCluster : 1, ga);
     stage_mark(stream, 1);
 
@@ -306,7 +307,6 @@ static int moe_forward_impl(int path, const __nv_bfloat16* x, const uint8_t* ban
         }
     } else {
         // ---- fp16 tensor-core path: weights dequantised into tensor memory
-        static int up_done[64] = {0}, down_done[64] = {0};
         const int blocks = (n_tokens + kActRows - 1) / kActRows;
         const dim3 agrid((n_experts + 31) / 32 + (blocks < 2 * grid ? blocks : 2 * grid)), ablock(kPrepThreads);
         launch_k(peer_in ? moe_act_fp16_kernel<true> : moe_act_fp16_kernel<false>, agrid, ablock, 0, stream, 1, aa, pin);
@@ -315,10 +315,10 @@ static int moe_forward_impl(int path, const __nv_bfloat16* x, const uint8_t* ban
         MoeMaps up_maps, down_maps;
         err = weight_map(&up_maps.wa, bank_W1_packed, (long long)n_experts * hidden, K_in);
         if (err == cudaSuccess) err = weight_map(&up_maps.wb, bank_W3_packed, (long long)n_experts * hidden, K_in);
-        if (err == cudaSuccess) err = half_maps(up_maps.act, aa.xh, P, K_in);
+        if (err == cudaSuccess) err = half_maps(up_maps.act, aa.xh, P, K_in, cap16);
         if (err == cudaSuccess) err = weight_map(&down_maps.wa, bank_W2_packed, (long long)n_experts * out_dim, hidden);
         down_maps.wb = down_maps.wa;
-        if (err == cudaSuccess) err = half_maps(down_maps.act, mid, P, hidden);
+        if (err == cudaSuccess) err = half_maps(down_maps.act, mid, P, hidden, cap16);
         MoeGemmArgs up;
         up.wa_s = bank_W1_scale; up.wb_s = bank_W3_scale; up.rows = hidden; up.K = K_in; up.n_experts = n_experts;
         up.xexp = aa.xexp; up.typical = aa.typical; up.g = g;
@@ -327,14 +327,18 @@ static int moe_forward_impl(int path, const __nv_bfloat16* x, const uint8_t* ban
         up.mid = mid; up.mid_exp = reinterpret_cast<int*>(ws + m.mid_exp); up.y = y;
         MoeGemmArgs down = up;
         down.wa_s = bank_W2_scale; down.wb_s = nullptr; down.rows = out_dim; down.K = hidden;
-        if (err == cudaSuccess) err = allow_smem(moe_gemm_kernel<0>, kTmSmem, up_done);
-        if (err == cudaSuccess) err = allow_smem(moe_gemm_kernel<1>, kTmSmem, down_done);
-        if (err == cudaSuccess) {
-            launch_k(moe_gemm_kernel<0>, dim3(grid), dim3(kTmThreads), kTmSmem, stream, 1, up_maps, up);
+        auto gemms = [&](auto up_kernel, auto down_kernel, uint32_t smem, int (&up_done)[64], int (&down_done)[64]) {
+            if (err == cudaSuccess) err = allow_smem(up_kernel, smem, up_done);
+            if (err == cudaSuccess) err = allow_smem(down_kernel, smem, down_done);
+            if (err != cudaSuccess) return;
+            launch_k(up_kernel, dim3(grid), dim3(kTmThreads), smem, stream, 1, up_maps, up);
             stage_mark(stream, 3);
             stage_mark(stream, 4);
-            launch_k(moe_gemm_kernel<1>, dim3(grid), dim3(kTmThreads), kTmSmem, stream, 1, down_maps, down);
-        }
+            launch_k(down_kernel, dim3(grid), dim3(kTmThreads), smem, stream, 1, down_maps, down);
+        };
+        static int up64[64] = {0}, down64[64] = {0}, up128[64] = {0}, down128[64] = {0};
+        if (cap16 == 64) gemms(moe_gemm_kernel<0, 64>, moe_gemm_kernel<1, 64>, MoeTmShape<64>::kSmem, up64, down64);
+        else gemms(moe_gemm_kernel<0, 128>, moe_gemm_kernel<1, 128>, MoeTmShape<128>::kSmem, up128, down128);
     }
     if (err == cudaSuccess) {
         stage_mark(stream, 5);

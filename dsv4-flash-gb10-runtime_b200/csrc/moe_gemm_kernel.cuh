@@ -1,13 +1,13 @@
 // Grouped GEMMs of the fp16 path: fp16 tcgen05 MMAs whose A operand, the dequantised weight tile, lives in TENSOR
 // MEMORY (number formats: moe_gemm.cuh).
 //
-// What bounds it.  A weight tile of 128 rows x 64 K-elements is 4 KB in HBM.  Written to shared memory as fp16 it is
-// 16 KB, written and read through the port the MMAs also fetch the tokens from; a kernel that did so was bound there
-// (348 TFLOP/s at 4096 tokens).  Here the tile goes registers -> tensor memory (tcgen05.st, 128 lanes x 32 columns), which
-// costs shared memory nothing, and the MMA (A from tensor memory, B = tokens from shared memory) runs at N / 2 clocks
-// per 128 x N x 16: 4 N clocks for the two matrices and 64 K-elements of a stage.  Dequantisation takes about 280 clocks
-// of each scheduler for the same stage (E2M1 conversion + one half-rate multiply per two weights), so tiles of
-// 80 .. 128 tokens are bound by the tensor pipe and tiles of a few tokens by HBM (8.7 KB per stage and SM).
+// What bounds it.  A weight tile of 128 rows x 128 K-elements (a K-block) is 8 KB in HBM.  Written to shared memory as fp16
+// it is 32 KB, written and read through the port the MMAs also fetch the tokens from; a kernel that did so was bound there
+// (348 TFLOP/s at 4096 tokens).  Here the tile goes registers -> tensor memory (tcgen05.st, 128 lanes x 64 columns), which
+// costs shared memory nothing, and the MMA (A from tensor memory, B = tokens from shared memory) takes N / 2 + 10 clocks
+// per 128 x N x 16, at least 40: 640 clocks and up for the two matrices of a K-block.  Dequantisation takes about 470
+// issue slots of each scheduler (E2M1 conversion + one half-rate multiply per two weights), HBM 730 clocks of the SM's
+// share.  Measured: 1 370 clocks per K-block with 24 tokens per expert, 1 550 in handshakes of 64 K-elements.
 //
 // A tile: 128 rows of two matrices (gate/up: the same rows of W1 and W3; down: two row blocks of W2) x up to 128 tokens.
 // CTA = 20 warps (five per scheduler: 96 registers a thread), persistent grid, one CTA per SM, tiles by static striding:
@@ -16,13 +16,11 @@
 //   warp 2       packed weights -> shared memory (TMA, 256 K-elements = 16 KB per matrix and stage) and their scales
 //   warp 3       a tile ahead: token tables, and the largest scale byte of every row
 //   warps 4..19  dequantise: warp = (K-block parity, matrix, lane quadrant); a thread owns one weight row, takes 32
-//                bytes and two scale bytes of it per K-block of 64 and writes 32 tensor-memory columns.  They also drain the
-//                finished accumulators, after the first stages of the NEXT tile are in tensor memory, so that the MMAs
+//                bytes x 2 and four scale bytes of it per K-block and writes 64 tensor-memory columns.  They also drain the
+//                finished accumulators, after the first K-blocks of the NEXT tile are in tensor memory, so that the MMAs
 //                continue as soon as the accumulators have been read.
-// A K-block's weights (in tensor memory) and tokens (in shared memory) share one full and one empty barrier: for tiles of a
-// few tokens the issuing thread sets the pace, not the MMAs (320 clocks), and with a barrier pair for each operand
-// it took 1 070 clocks per K-block.
-// Tensor memory: columns 0..255 two accumulators of 128, 256..511 four stages of two 128 x 64 fp16 tiles.
+// A K-block's weights (in tensor memory) and tokens (in shared memory) share one full and one empty barrier.
+// Tensor memory: two accumulators, then the stages of two 128 x 128 fp16 tiles (128 columns) each.
 // Every wait is bounded (stream_ring.cuh).
 #pragma once
 
@@ -32,16 +30,26 @@ namespace dsv4 {
 
 constexpr int kTmMmaWarp = 0, kTmTokenWarp = 1, kTmWeightWarp = 2, kTmAuxWarp = 3, kTmDequantWarp = 4, kTmDequantWarps = 16;
 constexpr int kTmThreads = (kTmDequantWarp + kTmDequantWarps) * 32;
-constexpr int kTmKBlock = 64;                         // K-elements per tensor-memory / token stage
+constexpr int kTmKBlock = 128;                        // K-elements per tensor-memory / token stage (a K-block)
 constexpr int kTmWBlock = 256;                        // K-elements per packed-weight stage (128 bytes per row)
-constexpr int kTmWStages = 4, kTmStages = 4, kTmTables = 3;
+constexpr int kTmWStages = 4, kTmTables = 3;
 constexpr uint32_t kTmWTile = 128 * 128;              // packed weights of one matrix and stage
 constexpr uint32_t kTmWScale = 128 * 8;               // scale bytes of one matrix and stage
 constexpr uint32_t kTmWStage = 2 * kTmWTile + 2 * kTmWScale;
-constexpr uint32_t kTmBStage = kMoeTileTokens * 128;
 constexpr uint32_t kTmOffB = kTmWStages * 2 * kTmWTile;                       // every tile 1024-byte aligned
-constexpr uint32_t kTmOffS = kTmOffB + kTmStages * kTmBStage;
-constexpr uint32_t kTmSmem = kTmOffS + kTmWStages * 2 * kTmWScale + 1024;
+// Two shapes of the kernel: tiles of up to 128 tokens with two stages, or of up to 64 with three (the columns that the
+// accumulators leave).  The host takes the second where experts have kTmFewTokens or fewer tokens on average, so that second
+// passes over a weight tile are rare.
+template <int CAP>
+struct MoeTmShape {
+    static constexpr int kStages = CAP <= 64 ? 3 : 2;
+    static constexpr uint32_t kACol = 2 * CAP;                                  // accumulators in [0, 2 CAP)
+    static constexpr uint32_t kBHalf = CAP * 128, kBStage = 2 * kBHalf;         // 64 fp16 values of every token, twice
+    static constexpr uint32_t kOffS = kTmOffB + kStages * kBStage;
+    static constexpr uint32_t kSmem = kOffS + kTmWStages * 2 * kTmWScale + 1024;
+    static_assert(kACol + kStages * 128 <= 512, "tensor memory overflow");
+};
+constexpr int kTmFewTokens = 40;
 
 struct MoeGemmArgs {
     const uint8_t* wa_s; const uint8_t* wb_s;   // E8M0 scales: up W1, W3; down W2 (wb unused)
@@ -61,7 +69,7 @@ struct MoeMaps { CUtensorMap wa, wb, act[kMoeWidths]; };
 
 struct MoeTile { int e, slot0, n_valid, width, m0, mats; };
 
-template <int MODE>
+template <int MODE, int CAP>
 __device__ __forceinline__ MoeTile moe_tile_decode(const int* tiles, const int* offsets, int n_experts, int m_tiles, int rows,
                                                    int tile) {
     int lo = 0, hi = n_experts;                 // last expert with tiles[e] <= tile
@@ -72,7 +80,7 @@ __device__ __forceinline__ MoeTile moe_tile_decode(const int* tiles, const int* 
     MoeTile t;
     t.e = lo;
     const int local = tile - tiles[lo], nt = local / m_tiles, n = offsets[lo + 1] - offsets[lo];
-    const int per = moe_tokens_per_tile(n, kMoeTileTokens);
+    const int per = moe_tokens_per_tile(n, CAP);
     t.slot0 = offsets[lo] + nt * per;
     t.n_valid = min(per, offsets[lo + 1] - t.slot0);
     t.width = moe_width_index(t.n_valid);
@@ -105,16 +113,18 @@ __device__ __forceinline__ void dequant_block(const uint4& w, uint32_t mult, uin
     }
 }
 
-template <int MODE>
+template <int MODE, int CAP>
 __global__ void __launch_bounds__(kTmThreads, 1) moe_gemm_kernel(const __grid_constant__ MoeMaps maps, const MoeGemmArgs a) {
+    using L = MoeTmShape<CAP>;
+    constexpr int kTmStages = L::kStages;
     extern __shared__ __align__(1024) uint8_t gemm_smem[];
     __shared__ __align__(8) uint64_t w_full[kTmWStages], w_empty[kTmWStages], full[kTmStages], empty[kTmStages];
     __shared__ __align__(8) uint64_t acc_full, acc_free, exp_full[kTmTables], tab_free[kTmTables];
     __shared__ uint32_t tmem_holder;
     __shared__ int s_tiles[kMoeMaxExperts + 1], s_offsets[kMoeMaxExperts + 1];
     // tables of a tile, by tile number mod 3: the aux warps fill tile N + 1 while tile N - 1 is being drained
-    __shared__ float tok_f0[kTmTables][kMoeTileTokens];       // up: 2^e_t;  down: w * 2^(half of the slot's exponent)
-    __shared__ float tok_f1[kTmTables][kMoeTileTokens];       // up: 2^-2q_t; down: 2^(the other half)
+    __shared__ float tok_f0[kTmTables][CAP];       // up: 2^e_t;  down: w * 2^(half of the slot's exponent)
+    __shared__ float tok_f1[kTmTables][CAP];       // up: 2^-2q_t; down: 2^(the other half)
     __shared__ int row_exp[kTmTables][2][kMoeTileRows];       // largest scale byte of every weight row
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -145,7 +155,7 @@ __global__ void __launch_bounds__(kTmThreads, 1) moe_gemm_kernel(const __grid_co
     const uint32_t tmem = tmem_holder;
     const int n_tiles = s_tiles[a.n_experts];
     const int m_tiles = (a.rows + (MODE == 0 ? kMoeTileRows : 2 * kMoeTileRows) - 1) / (MODE == 0 ? kMoeTileRows : 2 * kMoeTileRows);
-    auto decode = [&](int tile) { return moe_tile_decode<MODE>(s_tiles, s_offsets, a.n_experts, m_tiles, a.rows, tile); };
+    auto decode = [&](int tile) { return moe_tile_decode<MODE, CAP>(s_tiles, s_offsets, a.n_experts, m_tiles, a.rows, tile); };
     bool alive = true;
     auto wait = [&](uint64_t& bar, uint32_t parity, int code) {
         if (alive) alive = __all_sync(kFullMask, mbar_wait_bounded(smem_u32(&bar), parity & 1u, code));   // per warp
@@ -198,12 +208,12 @@ __global__ void __launch_bounds__(kTmThreads, 1) moe_gemm_kernel(const __grid_co
                 }
             };
 #pragma unroll 1
-            for (int c = c0; c < kMoeTileTokens; c += 64) {
+            for (int c = c0; c < CAP; c += 64) {
                 const bool has = c < t.n_valid && alive;
                 uint32_t g[16], u[16];
                 if (has) {
                     tc05_ld16_issue(trow + c, g);
-                    tc05_ld16_issue(trow + kMoeTileTokens + c, u);
+                    tc05_ld16_issue(trow + CAP + c, u);
                     tc05_wait_ld();
                 }
                 if (c + 64 >= t.n_valid && !handed) {                       // this warp has read all it wants of the accumulators
@@ -232,34 +242,31 @@ __global__ void __launch_bounds__(kTmThreads, 1) moe_gemm_kernel(const __grid_co
             wait(exp_full[tab], tc / kTmTables, 5);
             const int c = row_exp[tab][mat][row];
             for (int kb = group; kb < n_kb; kb += 2) {
-                const uint32_t it = kb_base + kb, wi = it >> 2, ws = wi % kTmWStages;
-                const int q = kb & 3;                         // K-block inside the weight stage
-                if (q < 2) wait(w_full[ws], wi / kTmWStages, 5);
+                const uint32_t it = kb_base + kb, wi = it >> 1, ws = wi % kTmWStages, as = it % kTmStages;
+                wait(w_full[ws], wi / kTmWStages, 5);
                 const uint32_t wrow = smem0 + (ws * 2 + mat) * kTmWTile + row * 128;
-                const uint4 w0 = lds_v4(wrow + (((2 * q) ^ (row & 7)) << 4));
-                const uint4 w1 = lds_v4(wrow + (((2 * q + 1) ^ (row & 7)) << 4));
+                uint4 w[4];
+#pragma unroll
+                for (int h = 0; h < 4; ++h) w[h] = lds_v4(wrow + (((4 * group + h) ^ (row & 7)) << 4));
                 uint32_t sc;
-                asm volatile("ld.shared.u16 %0, [%1];" : "=r"(sc) : "r"(smem0 + kTmOffS + (ws * 2 + mat) * kTmWScale + row * 8 + q * 2));
-                const uint32_t as = it % kTmStages;
-                const uint32_t acol = tmem + ((uint32_t)(quad * 32) << 16) + 256 + as * 64 + mat * 32;
+                asm volatile("ld.shared.u32 %0, [%1];" : "=r"(sc) : "r"(smem0 + L::kOffS + (ws * 2 + mat) * kTmWScale + row * 8 + group * 4));
+                const uint32_t acol = tmem + ((uint32_t)(quad * 32) << 16) + L::kACol + as * 128 + mat * 64;
                 if (it >= kTmStages) wait(empty[as], it / kTmStages - 1, 4);
                 tc05_fence_after_sync();
 #pragma unroll
-                for (int h = 0; h < 2; ++h) {
+                for (int h = 0; h < 4; ++h) {
                     uint32_t r[16];
-                    dequant_block(h ? w1 : w0, c < 0 ? 0u : half2_pow2(h ? sc >> 8 : sc & 255, c), r);
+                    dequant_block(w[h], c < 0 ? 0u : half2_pow2((sc >> (8 * h)) & 255, c), r);
                     tc05_st16(acol + 16 * h, r);
                 }
-                if (q >= 2) {
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive_one(smem_u32(&w_empty[ws]));
-                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive_one(smem_u32(&w_empty[ws]));
                 tc05_wait_st();
                 tc05_fence_before_sync();
                 __syncwarp();
                 if (lane == 0) mbar_arrive_one(smem_u32(&full[as]));
                 // the first stages of this tile are in tensor memory: now drain the previous one
-                if (has_prev && kb == group + 2) drain(prev, tc - 1);
+                if (has_prev && kb == group) drain(prev, tc - 1);
             }
             kb_base += n_kb;
             prev = t;
@@ -272,13 +279,15 @@ __global__ void __launch_bounds__(kTmThreads, 1) moe_gemm_kernel(const __grid_co
             uint32_t it = 0;
             for (int tile = blockIdx.x; tile < n_tiles && alive; tile += gridDim.x) {
                 const MoeTile t = decode(tile);
-                const uint32_t bytes = (uint32_t)moe_width(t.width, kMoeTileTokens) * 128u;
+                const uint32_t bytes = (uint32_t)moe_width(t.width, CAP) * 256u;
                 for (int kb = 0; kb < n_kb; ++kb, ++it) {
                     const uint32_t s = it % kTmStages;
                     if (it >= kTmStages) wait_one(empty[s], it / kTmStages - 1, 4);
                     if (!alive) break;
                     mbar_arrive_expect_tx(smem_u32(&full[s]), bytes);
-                    tma_load_2d(smem0 + kTmOffB + s * kTmBStage, &maps.act[t.width], kb * kTmKBlock, t.slot0, smem_u32(&full[s]));
+                    const uint32_t dst = smem0 + kTmOffB + s * L::kBStage;
+                    tma_load_2d(dst, &maps.act[t.width], kb * kTmKBlock, t.slot0, smem_u32(&full[s]));
+                    tma_load_2d(dst + L::kBHalf, &maps.act[t.width], kb * kTmKBlock + 64, t.slot0, smem_u32(&full[s]));
                 }
             }
         }
@@ -301,7 +310,7 @@ __global__ void __launch_bounds__(kTmThreads, 1) moe_gemm_kernel(const __grid_co
                     tma_load_2d(dst, &maps.wa, wb * 128, (int)first, bar);
                     if (t.mats == 2) tma_load_2d(dst + kTmWTile, &maps.wb, wb * 128, (int)first + (MODE == 0 ? 0 : kMoeTileRows), bar);
                 }
-                const uint32_t sdst = smem0 + kTmOffS + ws * 2 * kTmWScale;
+                const uint32_t sdst = smem0 + L::kOffS + ws * 2 * kTmWScale;
 #pragma unroll
                 for (int m = 0; m < 2; ++m)
                     if (m < t.mats) {
@@ -324,26 +333,27 @@ __global__ void __launch_bounds__(kTmThreads, 1) moe_gemm_kernel(const __grid_co
             uint32_t it = 0;
             for (int tile = blockIdx.x; tile < n_tiles && alive; tile += gridDim.x, ++tc) {
                 const MoeTile t = decode(tile);
-                const uint32_t idesc = tc05_idesc_f16(128, moe_width(t.width, kMoeTileTokens));
+                const uint32_t idesc = tc05_idesc_f16(128, moe_width(t.width, CAP));
                 if (tc > 0) wait_one(acc_free, tc - 1, 7);
                 for (int kb = 0; kb < n_kb; ++kb, ++it) {
                     const uint32_t as = it % kTmStages;
                     wait_one(full[as], it / kTmStages, 5);
                     if (!alive) break;
                     tc05_fence_after_sync();
-                    const uint64_t db = tc05_desc_k_sw128(smem0 + kTmOffB + as * kTmBStage);
-                    const uint32_t at = tmem + 256 + as * 64;
+                    const uint64_t db = tc05_desc_k_sw128(smem0 + kTmOffB + as * L::kBStage);
+                    const uint32_t at = tmem + L::kACol + as * 128;
+                    auto b_of = [&](int j) { return db + (j >> 2) * (L::kBHalf >> 4) + 2 * (j & 3); };      // K-step j of 16
                     if (t.mats == 2) {
 #pragma unroll
                         for (int j = 0; j < kTmKBlock / 16; ++j) {
                             const uint32_t acc = (kb > 0 || j > 0) ? 1u : 0u;
-                            tc05_mma_f16_ts(tmem, at + j * 8, db + 2 * j, idesc, acc);
-                            tc05_mma_f16_ts(tmem + kMoeTileTokens, at + 32 + j * 8, db + 2 * j, idesc, acc);
+                            tc05_mma_f16_ts(tmem, at + j * 8, b_of(j), idesc, acc);
+                            tc05_mma_f16_ts(tmem + CAP, at + 64 + j * 8, b_of(j), idesc, acc);
                         }
                     } else {
 #pragma unroll
                         for (int j = 0; j < kTmKBlock / 16; ++j)
-                            tc05_mma_f16_ts(tmem, at + j * 8, db + 2 * j, idesc, (kb > 0 || j > 0) ? 1u : 0u);
+                            tc05_mma_f16_ts(tmem, at + j * 8, b_of(j), idesc, (kb > 0 || j > 0) ? 1u : 0u);
                     }
                     tc05_commit(smem_u32(&empty[as]));
                     if (kb == n_kb - 1) tc05_commit(smem_u32(&acc_full));
