@@ -65,3 +65,26 @@ def test_grouped_experts_across_stage_ends(rt, qz, E, K, H, O):
     sub = {k: v[ids] for k, v in bank.items()}
     close(out, oracle.grouped_gemv_ref(x, sub["w1p"], sub["w3p"], sub["w2p"], sub["w1s"], sub["w3s"], sub["w2s"], r), f"E={E} K={K} H={H}")
     assert rt.device_status() == 0
+
+
+@pytest.mark.parametrize("K,N,G,S,gap", [
+    (128, 128, 2, 2, 0),               # one K step: one warp per row tile
+    (896, 2048, 8, 40, 0),             # 7 K steps over warps that do not divide them, several items per CTA, a last pass of 8 of 16 tokens
+    (1152, 128, 200, 3, 16),           # 9 K steps, items of different groups, rows apart in memory
+    (16384, 512, 1, 16, 0),            # activations in ranges
+    (4224, 2176, 1, 9, 128),           # 33 K steps, tiles that do not fill the last item
+    (1024, 4736, 1, 8, 0),
+])
+def test_fp8_several_tokens(rt, qz, K, N, G, S, gap):
+    g = torch.Generator().manual_seed(K + N)
+    w, s = qz.quantize_fp8_block128(torch.randn(G * N, K, generator=g) * 0.02, "e8m0")
+    s = (s.int() + torch.arange(s.numel()).view(s.shape) % 3).to(torch.uint8)
+    x = torch.randn(S, G * K, generator=g).to(torch.bfloat16)
+    wide = torch.zeros(G * N, K + gap, dtype=w.dtype, device=DEV)
+    wide[:, :K].copy_(w.to(DEV))
+    y = rt.fp8_e4m3_gemv_batched(wide[:, :K], s.to(DEV), x.to(DEV), n_groups=G)
+    scale = torch.ldexp(torch.ones(s.shape), s.int() - 127)
+    for grp in {0, G // 2, G - 1}:
+        r, b = slice(grp * N, (grp + 1) * N), slice(grp * N // 128, (grp + 1) * N // 128)
+        full = w[r].view(torch.float8_e4m3fn).float() * torch.repeat_interleave(torch.repeat_interleave(scale[b], 128, 0), 128, 1)
+        close(y[:, r], (x[:, grp * K:(grp + 1) * K].float() @ full.T).numpy(), f"group {grp} of {G}x{N}x{K}, {S} tokens")
