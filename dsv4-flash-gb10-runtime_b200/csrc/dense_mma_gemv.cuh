@@ -5,13 +5,13 @@
 // mma.sync.m16n8k16 (fp16 x fp16 -> fp32): the 8 columns are the tokens, so 8 tokens cost one MMA
 // per 16 x 16 weights and there is no cross-lane reduction.  The products E4M3 x fp16 are exact in FP32; the
 // accumulation is FP32 in a fixed order.
-//   * A lane (g = lane / 4, t = lane % 4) loads 32 consecutive bytes of rows g and g + 8 per 128-element K step;
-//     the K index inside an MMA is a permutation of the true one, the same for the weights and the activations.
+//   * A lane (g = lane / 4, t = lane % 4) loads the 16-byte chunks t and t + 4 of rows g and g + 8 per 128-element K step
+//     (four lanes 64 consecutive bytes: with 32 consecutive bytes per lane every sector was asked for twice); the K index inside an MMA is a permutation of the true one, the same for the weights and the activations.
 //   * The activations of a pass's tokens are staged in shared memory as fp16, 4096 K-elements at a time (once per
 //     CTA when K <= 4096 and there is one group), each (token, 2048-element half) scaled by a power of two so that
 //     its largest magnitude lies in [2^14, 2^15).
 //   * One CTA of 16 warps per SM walks a list of work items (pass, group, 16 / ks row tiles); the weight loads run
-//     kMmaDepth K steps ahead, across item boundaries.
+//     kDepth K steps ahead, across item boundaries.
 //   * A 128 x 128 scale tile covers one K step of a row tile: acc (one K step) is folded into the running sum
 //     with scale * activation scale.
 //   * ks in {1, 2, 4, 8, 16} warps share a row tile (interleaved K steps) when there are few row tiles; their partial
@@ -26,7 +26,6 @@ constexpr int kMmaPanel = 2048;                       // K elements one warp con
 constexpr int kMmaStage = 2 * kMmaPanel;               // K elements of activations resident in shared memory
 constexpr int kMmaRowBytes = kMmaStage * 2 + 16;      // fp16 row of one token; +16: tokens g and g+1 in odd banks
 constexpr int kMmaThreads = 512;
-constexpr int kMmaDepth = 3;                          // K steps of weights in flight per warp
 
 __device__ __forceinline__ void mma_f16_m16n8k16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
                                                  uint32_t b0, uint32_t b1) {
@@ -36,14 +35,9 @@ __device__ __forceinline__ void mma_f16_m16n8k16(float (&c)[4], uint32_t a0, uin
 }
 
 struct MmaWeights {
-    uint4 w[4];        // row g: bytes [0,16), [16,32) of the lane's 32; row g + 8: the same
+    uint4 w[4];        // row g: chunks t, t + 4; row g + 8: the same
     uint32_t s;        // raw scale of the (row tile, K step)
 };
-
-// 16-byte chunk `idx` of a token's fp16 panel row sits at chunk position idx ^ (bit 3 of idx << 1): the four lanes
-// t of a quarter-warp read chunks 4 t + c, which would otherwise meet in two bank groups.
-__device__ __forceinline__ int mma_x_chunk(int idx) { return idx ^ (((idx >> 3) & 1) << 1); }
-
 
 // Work items: item = (pass * n_groups + group) * n_tg + tg; a tile group tg is 16 >> ks_shift row tiles, each shared
 // by 1 << ks_shift warps (interleaved K steps).  CTA b takes items b, b + gridDim.x, ...
@@ -52,6 +46,7 @@ template <class Sc, int NT, bool RAGGED>
 __global__ void __launch_bounds__(kMmaThreads, 1) dense_mma_gemv_kernel(const DenseMultiArgs m, const int ks_shift,
                                                                        const int n_tg, const int n_items) {
     constexpr int kMmaTokens = 8 * NT;
+    constexpr int kDepth = NT == 2 && RAGGED ? 2 : 3;             // K steps of weights in flight per warp (a third one spilled there)
     extern __shared__ __align__(16) uint8_t x_stage[];              // kMmaTokens rows of kMmaRowBytes
     __shared__ __align__(8) float x_scale[2][kMmaTokens];           // per 2048-element half of the staged K range
     __shared__ __align__(16) float red[2][kMmaThreads / 32][128 * NT];              // partial sums of the warps sharing a tile
@@ -72,9 +67,9 @@ __global__ void __launch_bounds__(kMmaThreads, 1) dense_mma_gemv_kernel(const De
     const int my_items = n_items > (int)blockIdx.x ? (n_items - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
     const int total = my_items * nq;
 
-    // ---- the load stream: kMmaDepth steps ahead of the consumer, across items
+    // ---- the load stream: kDepth steps ahead of the consumer, across items
     int i_item = blockIdx.x, i_q = 0;
-    const uint8_t* i_w = nullptr;        // row r0 + g of the item's tile, byte t * 32; nullptr: no tile
+    const uint8_t* i_w = nullptr;        // row r0 + g of the item's tile, byte t * 16; nullptr: no tile
     const uint8_t* i_s = nullptr;        // scale tensor of the item's group
     int i_r0 = 0;
     auto load_item = [&]() {
@@ -85,7 +80,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1) dense_mma_gemv_kernel(const De
             const int tile = tg * tiles_per_tg + tile_local;
             if (tile < tiles) {
                 i_r0 = tile << 4;
-                i_w = a.w + ((long long)grp * a.N + i_r0 + g) * a.w_stride + t * 32;
+                i_w = a.w + ((long long)grp * a.N + i_r0 + g) * a.w_stride + t * 16;
                 i_s = a.s + (long long)grp * (a.N >> 7) * a.s_stride;
             }
         }
@@ -98,9 +93,9 @@ __global__ void __launch_bounds__(kMmaThreads, 1) dense_mma_gemv_kernel(const De
         if (i_w != nullptr && (!RAGGED || k0 < a.K)) {
             const uint8_t* w1 = i_w + 8 * a.w_stride;
             b.w[0] = ldg_stream_v4(i_w + k0);
-            b.w[1] = ldg_stream_v4(i_w + k0 + 16);
+            b.w[1] = ldg_stream_v4(i_w + k0 + 64);
             b.w[2] = ldg_stream_v4(w1 + k0);
-            b.w[3] = ldg_stream_v4(w1 + k0 + 16);
+            b.w[3] = ldg_stream_v4(w1 + k0 + 64);
             b.s = Sc::fetch(i_s, i_r0, k0 >> 4, a.s_stride);
         }
         if (++i_q == nq) {
@@ -146,7 +141,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1) dense_mma_gemv_kernel(const De
                                                     __uint_as_float(u[j] & 0xffff0000u) * inv);
                 h[j] = *reinterpret_cast<const uint32_t*>(&p);
             }
-            *reinterpret_cast<uint4*>(row + mma_x_chunk(half * (kMmaPanel / 8) + idx) * 16) = make_uint4(h[0], h[1], h[2], h[3]);
+            *reinterpret_cast<uint4*>(row + (half * (kMmaPanel / 8) + idx) * 16) = make_uint4(h[0], h[1], h[2], h[3]);
         }
         if (lane == 0) x_scale[half][token] = __uint_as_float((uint32_t)(e - 14) << 23);
     };
@@ -196,7 +191,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1) dense_mma_gemv_kernel(const De
                 uint4 xv[NT];
 #pragma unroll
                 for (int n = 0; n < NT; ++n)
-                    xv[n] = *reinterpret_cast<const uint4*>(xrow + n * 8 * kMmaRowBytes + mma_x_chunk(it_local * 16 + t * 4 + c) * 16);
+                    xv[n] = *reinterpret_cast<const uint4*>(xrow + n * 8 * kMmaRowBytes + (it_local * 16 + (c >> 1) * 8 + 2 * t + (c & 1)) * 16);
                 const uint4& wg = b.w[c >> 1];
                 const uint4& wh = b.w[2 + (c >> 1)];
                 const uint32_t word_g[2] = {(c & 1) ? wg.z : wg.x, (c & 1) ? wg.w : wg.y};
@@ -260,16 +255,16 @@ __global__ void __launch_bounds__(kMmaThreads, 1) dense_mma_gemv_kernel(const De
         }
     };
 
-    MmaWeights buf[kMmaDepth];
+    MmaWeights buf[kDepth];
     load_item();
 #pragma unroll
-    for (int d = 0; d < kMmaDepth; ++d) issue(buf[d]);          // weights never depend on the previous kernel
+    for (int d = 0; d < kDepth; ++d) issue(buf[d]);          // weights never depend on the previous kernel
     pdl_wait();
 
 #pragma unroll 1
-    for (int s0 = 0; s0 < total; s0 += kMmaDepth) {
+    for (int s0 = 0; s0 < total; s0 += kDepth) {
 #pragma unroll
-        for (int d = 0; d < kMmaDepth; ++d) {
+        for (int d = 0; d < kDepth; ++d) {
             if (s0 + d < total) {                               // uniform over the CTA
                 consume(buf[d]);
                 issue(buf[d]);
