@@ -34,6 +34,7 @@ __global__ void __launch_bounds__(kRowThreads, 2) dense_stream_kernel(const Dens
                                                                      const RowPlan p, float limit_g, float limit_u) {
     extern __shared__ __align__(128) uint8_t row_smem[];
     __shared__ RowRing ring;
+    __shared__ volatile int x_asked;
     pdl_launch_dependents();
     DenseArgs a = a_in;
     if (GROUPED) {
@@ -51,8 +52,9 @@ __global__ void __launch_bounds__(kRowThreads, 2) dense_stream_kernel(const Dens
     const uint32_t smem = smem_u32(row_smem);
 
     if (tid == kRowWarps * 32) row_ring_init(ring, p);
-    auto produce = [&](int st0, int st1, RowPos& pos) {
-        for (int st = st0; st < st1; ++st, pos.next(p.slots)) {
+    auto produce = [&]() {
+        RowPos pos;
+        for (int st = 0; st < n_stages; ++st, pos.next(p.slots)) {
             if (pos.round > 0 && !mbar_wait_bounded(smem_u32(&ring.empty[pos.slot]), (pos.round - 1) & 1u, 1)) break;
             const int row = st * p.rows, rows = min(p.rows, n_local - row);
             const uint32_t bar = smem_u32(&ring.full[pos.slot]), dst = smem + pos.slot * p.stage_bytes;
@@ -71,28 +73,42 @@ __global__ void __launch_bounds__(kRowThreads, 2) dense_stream_kernel(const Dens
             }
         }
     };
-    RowPos made;                             // the producer's position
-    const int first_stages = min(p.slots, n_stages);
-    // weights never depend on the previous kernel in the stream: the ring is filled without waiting for it
-    if (tid == kRowWarps * 32) produce(0, first_stages, made);
-    __syncwarp();
-    // tile scales of this CTA's rows as floats: [MATS][tile rows][n_blk / 8]
-    const int tiles_k = n_blk >> 3, tile0 = r_begin >> 7, n_tr = ((r_end - 1) >> 7) - tile0 + 1;
+    // tile scales of this CTA's rows as floats: [MATS][tile rows][n_blk / 8].  Requested before the first copies: a load queues
+    // behind those.
+    const int tiles_k = n_blk >> 3, tile0 = r_begin >> 7, n_tr = ((r_end - 1) >> 7) - tile0 + 1, n_table = Sc::kPerRow ? 0 : MATS * n_tr * tiles_k;
     float* const table = reinterpret_cast<float*>(row_smem + p.off_table);
-    if (!Sc::kPerRow)
-        for (int i = tid; i < MATS * n_tr * tiles_k; i += kRowThreads) {
-            const int m = i / (n_tr * tiles_k), j = i - m * n_tr * tiles_k, tr = j / tiles_k;
-            table[i] = Sc::value(Sc::fetch(m == 0 ? a.s : s2, (tile0 + tr) << 7, (j - tr * tiles_k) << 3, a.s_stride));
+    auto tile_scale = [&](int i) {
+        const int m = i / (n_tr * tiles_k), j = i - m * n_tr * tiles_k, tr = j / tiles_k;
+        return Sc::fetch(m == 0 ? a.s : s2, (tile0 + tr) << 7, (j - tr * tiles_k) << 3, a.s_stride);
+    };
+    uint32_t raw = 0;
+    if (tid < n_table) raw = tile_scale(tid);
+    if (tid == 0) x_asked = 0;
+    __syncthreads();                         // barriers
+    // The consumers go on without the producer: when it filled the ring before the barrier above, asking for x and the tile
+    // scales waited for that (eight launches of 4096 x 4096 MXFP4 35.1 us then, 31.0 now; of 2048 x 4096 FP8 28.1, 23.8).
+    if (warp == kRowWarps) {
+        // weights never depend on the previous kernel in the stream: they are requested without waiting for it
+        if (lane == 0) {
+            if (n_local * p.row_bytes * MATS > kRowSmall) row_pause(&x_asked);
+            produce();
         }
-    __syncthreads();                         // barriers, tile scales
-    pdl_wait();                              // every thread: the outputs below may still be read by the kernel before
+    } else {
+        if (tid < n_table) table[tid] = Sc::value(raw);
+        for (int i = tid + kRowWarps * 32; i < n_table; i += kRowWarps * 32) table[i] = Sc::value(tile_scale(i));
+        if (!Sc::kPerRow) asm volatile("bar.sync 1, %0;" ::"n"(kRowWarps * 32) : "memory");
+        pdl_wait();                          // x, and the outputs below may still be read by the kernel before
+        if (tid == 0) {
+            row_x_request(ring, smem + p.off_x, a.x, a.K * 2);
+            x_asked = 1;
+        }
+    }
     if (warp < p.warps) {
         const int w_slices = p.warps / p.n_groups, ks0 = warp % w_slices, rg = warp / w_slices;
         int blk[SPW];
         bool ok[SPW];
 #pragma unroll
         for (int q = 0; q < SPW; ++q) { blk[q] = (ks0 + q * w_slices) * 32 + lane; ok[q] = blk[q] < n_blk; }
-        if (tid == 0) row_x_request(ring, smem + p.off_x, a.x, a.K * 2);
         bool alive = __all_sync(kFullMask, mbar_wait_bounded(smem_u32(&ring.x), 0, 2));
         ActBlock<Fmt> xb[SPW];
 #pragma unroll
@@ -134,8 +150,6 @@ __global__ void __launch_bounds__(kRowThreads, 2) dense_stream_kernel(const Dens
             }
             row_release(ring, p, pos, lane);
         }
-    } else if (tid == kRowWarps * 32) {
-        produce(first_stages, n_stages, made);
     }
     __syncthreads();
 

@@ -176,6 +176,17 @@ __device__ __forceinline__ void row_x_request(RowRing& r, uint32_t x_smem, const
     bulk_copy_g2s(x_smem, x, bytes, smem_u32(&r.x));
 }
 
+// Before the first copies of a CTA: the previous launch's CTA on this SM asks for its activations about when this one starts (a
+// third CTA has just made room for it), and behind a full ring they come a microsecond late.  So a ring of more than kRowSmall
+// bytes waits kRowPause clocks, unless this CTA's own activations have been asked for (nothing runs before it).  Eight launches of
+// 10007 x 2912 MXFP4 50.2 -> 48.5 us, eight of 8192 x 4096 FP8 65.5 -> 63.7 us; smaller rings lose by waiting (6000 x 1600: 30.8 -> 32.8).
+constexpr uint32_t kRowSmall = 40 * 1024;
+constexpr int kRowPause = 800;
+__device__ __forceinline__ void row_pause(const volatile int* x_asked) {
+    const long long t0 = clock64();
+    while (clock64() - t0 < kRowPause && !*x_asked) { }
+}
+
 // Sums over the lanes of a warp's rows of one stage: v[m * RPW + i] is row i * n_groups of matrix m, and goes to
 // part[m * mat_stride + i * n_groups * part_stride] (one writer per row).
 template <int RPW, int V>
