@@ -143,9 +143,11 @@ __global__ void __launch_bounds__(kRowThreads, 2) dense_stream_kernel(const Dens
                             sc[k] = table[(m * n_tr + ((r_begin + st * p.rows + r) >> 7) - tile0) * tiles_k + (blk[q] >> 3)];
                         }
                     }
-                float v[MATS * RPW];
+                float v[MATS * row_pow2(RPW)] = {};
 #pragma unroll
-                for (int k = 0; k < MATS * RPW; ++k) v[k] = Fmt::dot(w[k], xb[q].h) * (sc[k] * xb[q].scale);
+                for (int m = 0; m < MATS; ++m)
+#pragma unroll
+                    for (int i = 0; i < RPW; ++i) v[m * row_pow2(RPW) + i] = Fmt::dot(w[m * RPW + i], xb[q].h) * (sc[m * RPW + i] * xb[q].scale);
                 row_store<RPW>(v, left, p.n_groups, lane, part + row * p.n_slices + ks0 + q * w_slices, p.n_slices, n_local * p.n_slices);
             }
             row_release(ring, p, pos, lane);

@@ -14,7 +14,7 @@
 
 namespace dsv4 {
 
-constexpr int kGateRpw = 2, kDownRpw = 4;
+constexpr int kGateRpw = 2, kDownRpw = 4;             // rows per warp and stage (down: at most)
 constexpr uint32_t kDownParts = 12 * 1024;             // partial sums of a CTA at most
 
 __global__ void __launch_bounds__(kRowThreads, 2) grouped_gate_stream_kernel(const GroupedArgs a, const RowPlan p) {
@@ -138,10 +138,13 @@ __global__ void __launch_bounds__(kRowThreads, 2) grouped_gate_stream_kernel(con
 }
 
 // early_ids: the launch before this one is the gate/up kernel of the same call, so the picks may be read before waiting.
+// RPW: rows per warp and stage (row_spread).
+template <int RPW>
 __global__ void __launch_bounds__(kRowThreads, 2) grouped_down_stream_kernel(const GroupedArgs a, const RowPlan p, int early_ids) {
     extern __shared__ __align__(128) uint8_t row_smem[];
     __shared__ RowRing ring;
     __shared__ int expert[8];
+    __shared__ float weight[8];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int o_begin = (int)((long long)a.O * blockIdx.x / gridDim.x), o_end = (int)((long long)a.O * (blockIdx.x + 1) / gridDim.x);
     const int n_local = o_end - o_begin, per_e = (n_local + p.rows - 1) / p.rows, n_stages = a.E * per_e;
@@ -173,6 +176,7 @@ __global__ void __launch_bounds__(kRowThreads, 2) grouped_down_stream_kernel(con
         pdl_wait();
     } else {
         pdl_wait();
+        if (tid < a.E) weight[tid] = __ldcg(a.r + tid);
         // The intermediate of every expert -> fp16 blocks with a power of two each; chunk c of block b at (c + (b >> 1)) & 3,
         // so that lanes reading the same chunk of neighbouring blocks meet in no bank.  Eight lanes share a block (four
         // values each) and a thread has four pieces in flight: with a block per thread the loads were 128 bytes apart, and
@@ -230,17 +234,17 @@ __global__ void __launch_bounds__(kRowThreads, 2) grouped_down_stream_kernel(con
                     const uint32_t stage = smem + pos.slot * p.stage_bytes, sbase = stage + p.rows * p.row_bytes + blk_r;
                     const uint32_t s_addr = s_first + row0 * n_blk;
                     const int row = row0 + rg;
-                    uint4 w[kDownRpw];
-                    float sc[kDownRpw], v[kDownRpw];
+                    uint4 w[RPW];
+                    float sc[RPW], v[row_pow2(RPW)] = {};
 #pragma unroll
-                    for (int j = 0; j < kDownRpw; ++j) {
+                    for (int j = 0; j < RPW; ++j) {
                         const int i = rg + j * p.n_groups;
                         w[j] = lds_v4(stage + i * p.row_bytes + blk_r * 16);
                         sc[j] = e8m0_to_float_fast(lds_u8(sbase + row_scale_offset(p, s_addr, i)));
                     }
 #pragma unroll
-                    for (int j = 0; j < kDownRpw; ++j) v[j] = Fp4Format::dot(w[j], xb.h) * (sc[j] * xb.scale);
-                    row_store<kDownRpw>(v, n_local - row, p.n_groups, lane, part + (row * a.E + e) * p.n_slices + ks, a.E * p.n_slices, 0);
+                    for (int j = 0; j < RPW; ++j) v[j] = Fp4Format::dot(w[j], xb.h) * (sc[j] * xb.scale);
+                    row_store<RPW>(v, n_local - row, p.n_groups, lane, part + (row * a.E + e) * p.n_slices + ks, a.E * p.n_slices, 0);
                     row_release(ring, p, pos, lane);
                 }
             }
@@ -252,7 +256,7 @@ __global__ void __launch_bounds__(kRowThreads, 2) grouped_down_stream_kernel(con
         for (int k = 0; k < a.E; ++k) {
             float v = 0.f;
             for (int s = 0; s < p.n_slices; ++s) v += part[(t * a.E + k) * p.n_slices + s];
-            acc = fmaf(__ldcg(a.r + k), v, acc);
+            acc = fmaf(weight[k], v, acc);
         }
         a.out[o_begin + t] = __float2bfloat16(acc);
     }

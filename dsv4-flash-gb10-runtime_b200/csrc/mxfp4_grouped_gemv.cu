@@ -297,7 +297,7 @@ static int grouped_try_ring(const GroupedArgs& a, cudaStream_t stream, const cha
 
 // Any other shape: the two row-streaming kernels.
 static int grouped_launch(const GroupedArgs& a, cudaStream_t stream, const char* who, int stages) {
-    static int gate_done[64] = {0}, down_done[64] = {0};
+    static int gate_done[64] = {0}, down_done[kDownRpw][64] = {};
     const int sms = sm_count();
     const bool pdl = pdl_enabled();
     if (stages & 1) {
@@ -320,11 +320,15 @@ static int grouped_launch(const GroupedArgs& a, cudaStream_t stream, const char*
         long long grid = sms;
         if (grid < (a.O + cap - 1) / cap) grid = (a.O + cap - 1) / cap;
         if (grid > a.O) grid = a.O;
+        const int rpw = row_spread((int)((a.O + grid - 1) / grid), p.n_groups, kDownRpw);
+        p = row_plan(a.H >> 5, 1, rpw, 1);
         row_plan_scales(p, 1, a.H >> 5, a.H >> 5, 1);
         row_plan_finish(p, (uint32_t)a.E * (a.H >> 5) * 68, (uint32_t)(4 * ((a.O + grid - 1) / grid) * a.E * p.n_slices), 0);
-        cudaError_t err = allow_smem(grouped_down_stream_kernel, p.smem, down_done);
+        auto kernel = rpw == 1 ? grouped_down_stream_kernel<1> : rpw == 2 ? grouped_down_stream_kernel<2>
+                      : rpw == 3 ? grouped_down_stream_kernel<3> : grouped_down_stream_kernel<4>;
+        cudaError_t err = allow_smem(kernel, p.smem, down_done[rpw - 1]);
         if (err == cudaSuccess)
-            err = launch_smem(grouped_down_stream_kernel, dim3((unsigned)grid), dim3(kRowThreads), p.smem, stream, pdl, a, p,
+            err = launch_smem(kernel, dim3((unsigned)grid), dim3(kRowThreads), p.smem, stream, pdl, a, p,
                               stages == 3 ? 1 : 0);
         if (err != cudaSuccess) {
             std::fprintf(stderr, "%s: down launch failed: %s\n", who, cudaGetErrorString(err));
