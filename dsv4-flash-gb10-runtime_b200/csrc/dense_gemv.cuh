@@ -235,7 +235,14 @@ inline bool dense_pdl_enabled() {
     return v == 1;
 }
 
-// One CTA per SM over all groups (two successive launches share each SM), more where a CTA's partial sums would not fit.
+// CTAs per group: one CTA per SM over all groups (two successive launches share each SM), more where a CTA's partial sums would
+// not fit.
+inline long long dense_grid(const DenseArgs& a, int mats, const RowPlan& p, int n_groups) {
+    const long long cap = kDenseParts / (4 * mats * p.n_slices);          // rows per CTA
+    const long long sms = (dense_sm_count() + n_groups - 1) / n_groups, need = ((long long)a.N + cap - 1) / cap;
+    const long long grid = sms < need ? need : sms;
+    return grid < a.N ? grid : a.N;
+}
 // Needs 16-byte aligned x, weights and row strides.
 template <class Fmt, class Sc, int MATS, int RPW, int SPW, bool GROUPED>
 inline cudaError_t dense_stream_launch_as(const DenseArgs& a, const uint8_t* w2, const uint8_t* s2, float limit_g, float limit_u,
@@ -243,11 +250,7 @@ inline cudaError_t dense_stream_launch_as(const DenseArgs& a, const uint8_t* w2,
     auto kernel = dense_stream_kernel<Fmt, Sc, MATS, RPW, SPW, GROUPED>;
     const int n_blk = a.K / Fmt::kElems;
     RowPlan p = row_plan(n_blk, MATS, RPW, SPW);
-    const long long cap = kDenseParts / (4 * MATS * p.n_slices);          // rows per CTA
-    long long grid = (dense_sm_count() + n_groups - 1) / n_groups;
-    const long long need = ((long long)a.N + cap - 1) / cap;
-    if (grid < need) grid = need;
-    if (grid > a.N) grid = a.N;
+    const long long grid = dense_grid(a, MATS, p, n_groups);
     const int most = (int)((a.N + grid - 1) / grid);
     if (Sc::kPerRow) row_plan_scales(p, MATS, n_blk, a.s_stride, 1);
     row_plan_finish(p, a.K * 2, 4 * MATS * most * p.n_slices, Sc::kPerRow ? 0 : 4 * MATS * (most / 128 + 3) * (n_blk / 8));
@@ -255,7 +258,7 @@ inline cudaError_t dense_stream_launch_as(const DenseArgs& a, const uint8_t* w2,
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return cudaErrorInvalidDevice;
     if (dev < 0 || dev >= 64 || !done[dev]) {
-        const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowSmemMost);
+        const cudaError_t err = allow_shared(kernel, kRowSmemMost);
         if (err != cudaSuccess) return err;
         if (dev >= 0 && dev < 64) done[dev] = true;
     }
@@ -271,8 +274,8 @@ inline cudaError_t dense_stream_launch_as(const DenseArgs& a, const uint8_t* w2,
     cfg.numAttrs = dense_pdl_enabled() ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, a, w2, s2, p, limit_g, limit_u);
 }
-// Four rows per warp and stage where a stage of that stays within kRowStage, else two; FP8 rows longer than 8192 have more
-// slices than there are warps: two per warp.
+// At most four rows per warp and stage where a stage of that stays within kRowStage, else two (as many as the rows of a CTA
+// need: row_spread); FP8 rows longer than 8192 have more slices than there are warps: two per warp.
 template <class Fmt, class Sc, int MATS, bool GROUPED>
 inline cudaError_t dense_stream_launch(const DenseArgs& a, const uint8_t* w2, const uint8_t* s2, float limit_g, float limit_u,
                                        int n_groups, cudaStream_t stream) {
@@ -280,9 +283,14 @@ inline cudaError_t dense_stream_launch(const DenseArgs& a, const uint8_t* w2, co
     if constexpr (Fmt::kElems == 16) {
         if (n_blk > 32 * kRowWarps) return dense_stream_launch_as<Fmt, Sc, MATS, 2, 2, GROUPED>(a, w2, s2, limit_g, limit_u, n_groups, stream);
     }
-    if (row_plan(n_blk, MATS, 4, 1).stage_bytes <= kRowStage)
-        return dense_stream_launch_as<Fmt, Sc, MATS, 4, 1, GROUPED>(a, w2, s2, limit_g, limit_u, n_groups, stream);
-    return dense_stream_launch_as<Fmt, Sc, MATS, 2, 1, GROUPED>(a, w2, s2, limit_g, limit_u, n_groups, stream);
+    const RowPlan p = row_plan(n_blk, MATS, 4, 1);
+    const long long grid = dense_grid(a, MATS, p, n_groups);
+    switch (row_spread((int)((a.N + grid - 1) / grid), p.n_groups, p.stage_bytes <= kRowStage ? 4 : 2)) {
+        case 1: return dense_stream_launch_as<Fmt, Sc, MATS, 1, 1, GROUPED>(a, w2, s2, limit_g, limit_u, n_groups, stream);
+        case 2: return dense_stream_launch_as<Fmt, Sc, MATS, 2, 1, GROUPED>(a, w2, s2, limit_g, limit_u, n_groups, stream);
+        case 3: return dense_stream_launch_as<Fmt, Sc, MATS, 3, 1, GROUPED>(a, w2, s2, limit_g, limit_u, n_groups, stream);
+        default: return dense_stream_launch_as<Fmt, Sc, MATS, 4, 1, GROUPED>(a, w2, s2, limit_g, limit_u, n_groups, stream);
+    }
 }
 
 // Launches the aligned streaming kernel when it can, the byte-wise one otherwise.

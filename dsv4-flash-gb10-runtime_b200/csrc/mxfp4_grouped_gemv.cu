@@ -130,7 +130,7 @@ static cudaError_t allow_smem(Kernel kernel, size_t bytes, int (&done)[64]) {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
     if (done[dev] >= (int)bytes) return cudaSuccess;
-    cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    cudaError_t err = allow_shared(kernel, bytes);
     if (err == cudaSuccess) done[dev] = (int)bytes;
     return err;
 }

@@ -110,6 +110,16 @@ inline int row_spread(int rows, int n_groups, int most) {
     return (rows + stages * n_groups - 1) / (stages * n_groups);
 }
 
+// Dynamic shared memory of a kernel, and the SM's memory split for the most shared memory.  The split follows a kernel's own
+// needs otherwise, and an SM changes it only when it is empty: launches with different needs then do not overlap
+// (eight shared experts of 1536, 1152: 48.4 -> 38.5 us).
+template <class Kernel>
+inline cudaError_t allow_shared(Kernel kernel, size_t bytes) {
+    const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (err != cudaSuccess) return err;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+}
+
 // The barriers of a CTA: the ring's, and one for x.
 struct RowRing {
     uint64_t full[kRowSlots], empty[kRowSlots], x;
