@@ -98,7 +98,11 @@ __global__ void __launch_bounds__(kRowThreads, 2) dense_stream_kernel(const Dens
         for (int i = tid + kRowWarps * 32; i < n_table; i += kRowWarps * 32) table[i] = Sc::value(tile_scale(i));
         if (!Sc::kPerRow) asm volatile("bar.sync 1, %0;" ::"n"(kRowWarps * 32) : "memory");
         pdl_wait();                          // x, and the outputs below may still be read by the kernel before
-        if (tid == 0) {
+        if constexpr (Sc::kPerRow) {
+            if (tid == 0) x_asked = 1;
+            row_x_convert(smem + p.off_x, a.x, n_blk, tid);
+            asm volatile("bar.sync 1, %0;" ::"n"(kRowWarps * 32) : "memory");
+        } else if (tid == 0) {
             row_x_request(ring, smem + p.off_x, a.x, a.K * 2);
             x_asked = 1;
         }
@@ -109,11 +113,12 @@ __global__ void __launch_bounds__(kRowThreads, 2) dense_stream_kernel(const Dens
         bool ok[SPW];
 #pragma unroll
         for (int q = 0; q < SPW; ++q) { blk[q] = (ks0 + q * w_slices) * 32 + lane; ok[q] = blk[q] < n_blk; }
-        bool alive = __all_sync(kFullMask, mbar_wait_bounded(smem_u32(&ring.x), 0, 2));
+        bool alive = Sc::kPerRow || __all_sync(kFullMask, mbar_wait_bounded(smem_u32(&ring.x), 0, 2));
         ActBlock<Fmt> xb[SPW];
 #pragma unroll
         for (int q = 0; q < SPW; ++q) {
-            row_act_block<Fmt>(smem + p.off_x, blk[q], ok[q], xb[q]);
+            if constexpr (Sc::kPerRow) row_act_block(smem + p.off_x, n_blk, blk[q], ok[q], xb[q]);
+            else row_act_block_bf16<Fmt>(smem + p.off_x, blk[q], ok[q], xb[q]);
             if (!ok[q]) blk[q] = 0;
         }
         RowPos pos;
@@ -253,7 +258,7 @@ inline cudaError_t dense_stream_launch_as(const DenseArgs& a, const uint8_t* w2,
     const long long grid = dense_grid(a, MATS, p, n_groups);
     const int most = (int)((a.N + grid - 1) / grid);
     if (Sc::kPerRow) row_plan_scales(p, MATS, n_blk, a.s_stride, 1);
-    row_plan_finish(p, a.K * 2, 4 * MATS * most * p.n_slices, Sc::kPerRow ? 0 : 4 * MATS * (most / 128 + 3) * (n_blk / 8));
+    row_plan_finish(p, Sc::kPerRow ? row_x_bytes(n_blk) : a.K * 2, 4 * MATS * most * p.n_slices, Sc::kPerRow ? 0 : 4 * MATS * (most / 128 + 3) * (n_blk / 8));
     static bool done[64] = {false};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return cudaErrorInvalidDevice;

@@ -93,13 +93,14 @@ __global__ void __launch_bounds__(kRowThreads, 2) grouped_gate_stream_kernel(con
         pdl_wait();
     } else {
         pdl_wait();
-        if (tid == 0) row_x_request(ring, smem + p.off_x, a.x, a.K * 2);
+        row_x_convert(smem + p.off_x, a.x, row_s, tid);
+        asm volatile("bar.sync 1, %0;" ::"n"(kRowWarps * 32) : "memory");
         if (warp < p.warps) {
             const int ks = warp % p.n_slices, rg = warp / p.n_slices, blk = ks * 32 + lane;
             const bool ok = blk < row_s;
-            bool alive = __all_sync(kFullMask, mbar_wait_bounded(smem_u32(&ring.x), 0, 1));
+            bool alive = true;
             ActBlock<Fp4Format> xb;
-            row_act_block<Fp4Format>(smem + p.off_x, blk, ok, xb);
+            row_act_block(smem + p.off_x, row_s, blk, ok, xb);
             const uint32_t blk_r = ok ? blk : 0;               // lanes past the row's end: block 0 against zeros
             RowPos pos;
             Walk c = walk_start();

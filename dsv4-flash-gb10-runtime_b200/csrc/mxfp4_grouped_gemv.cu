@@ -305,7 +305,7 @@ static int grouped_launch(const GroupedArgs& a, cudaStream_t stream, const char*
         const long long pairs = (long long)a.E * a.H;
         const long long grid = sms < pairs ? sms : pairs;
         row_plan_scales(p, 2, a.K >> 5, a.K >> 5, 2);
-        row_plan_finish(p, a.K * 2, (uint32_t)(2 * 4 * ((pairs + grid - 1) / grid) * p.n_slices), 0);
+        row_plan_finish(p, row_x_bytes(a.K >> 5), (uint32_t)(2 * 4 * ((pairs + grid - 1) / grid) * p.n_slices), 0);
         cudaError_t err = allow_smem(grouped_gate_stream_kernel, p.smem, gate_done);
         if (err == cudaSuccess)
             err = launch_smem(grouped_gate_stream_kernel, dim3((unsigned)grid), dim3(kRowThreads), p.smem, stream, pdl, a, p);

@@ -170,9 +170,9 @@ __device__ __forceinline__ void row_scale_copy(const RowPlan& p, uint32_t dst, c
     }
 }
 
-// This lane's activation block from a bf16 vector in shared memory.
+// Activations, FP8: a bulk copy of x, and a lane converts its block.
 template <class Fmt>
-__device__ __forceinline__ void row_act_block(uint32_t x_smem, int blk, bool valid, ActBlock<Fmt>& a) {
+__device__ __forceinline__ void row_act_block_bf16(uint32_t x_smem, int blk, bool valid, ActBlock<Fmt>& a) {
     float v[Fmt::kElems];
 #pragma unroll
     for (int i = 0; i < Fmt::kElems / 8; ++i) {
@@ -192,6 +192,59 @@ __device__ __forceinline__ void row_act_block(uint32_t x_smem, int blk, bool val
 __device__ __forceinline__ void row_x_request(RowRing& r, uint32_t x_smem, const __nv_bfloat16* x, uint32_t bytes) {
     mbar_arrive_expect_tx(smem_u32(&r.x), bytes);
     bulk_copy_g2s(x_smem, x, bytes, smem_u32(&r.x));
+}
+// Activations, MXFP4: x (bf16, 16-byte aligned) -> shared memory as fp16 blocks with a power of two each, once per CTA, by the
+// consumers after their pdl_wait; four lanes share a block.  A block is 32 values here, and every warp converting its own cost half
+// a microsecond of a launch: eight launches of 10007 x 2912 46.7 -> 43.0 us, of 1000 x 1024 19.1 -> 16.7.  (FP8 blocks are 16
+// values: eight launches of 2048 x 4096 took 23.8 us with the copy and 24.6 this way.)  A barrier of the consumers must follow.  Chunks of a block are placed so that lanes reading the same chunk of neighbouring blocks meet in no bank.
+__device__ __forceinline__ uint32_t row_x_chunk(int blk, int c) { return (uint32_t)blk * 4 + ((c + (blk >> 1)) & 3); }
+__host__ __device__ __forceinline__ uint32_t row_x_bytes(int n_blk) { return (uint32_t)n_blk * 68; }
+__device__ __forceinline__ void row_x_convert(uint32_t x_smem, const __nv_bfloat16* x, int n_blk, int tid) {
+    constexpr int kPieces = 2;
+    const int n = n_blk * 4;
+    for (int base = 0; base < n; base += kPieces * kRowWarps * 32) {          // the same trips for every thread: lanes exchange
+        uint4 q[kPieces];
+#pragma unroll
+        for (int u = 0; u < kPieces; ++u) {
+            const int i = base + u * kRowWarps * 32 + tid;
+            q[u] = i < n ? __ldcg(reinterpret_cast<const uint4*>(x) + i) : make_uint4(0, 0, 0, 0);
+        }
+#pragma unroll
+        for (int u = 0; u < kPieces; ++u) {
+            const int i = base + u * kRowWarps * 32 + tid, b = i >> 2, c = i & 3;
+            if (base + u * kRowWarps * 32 >= n) break;
+            const uint32_t w[4] = {q[u].x, q[u].y, q[u].z, q[u].w};
+            uint32_t m = 0, h[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) m = max(m, max(w[j] & 0x7fffu, (w[j] >> 16) & 0x7fffu));
+#pragma unroll
+            for (int off = 1; off < 4; off <<= 1) m = max(m, __shfl_xor_sync(kFullMask, m, off));
+            const int e = min(max((int)(m >> 7) - Fp4Format::kActExp, 1), 253);     // biased exponent of the scale
+            const float inv = __uint_as_float((uint32_t)(254 - e) << 23);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const __half2 p = __floats2half2_rn(__uint_as_float(w[j] << 16) * inv, __uint_as_float(w[j] & 0xffff0000u) * inv);
+                h[j] = *reinterpret_cast<const uint32_t*>(&p);
+            }
+            if (i < n) {
+                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(x_smem + row_x_chunk(b, c) * 16),
+                             "r"(h[0]), "r"(h[1]), "r"(h[2]), "r"(h[3]) : "memory");
+                if (c == 0) asm volatile("st.shared.b32 [%0], %1;" ::"r"(x_smem + (uint32_t)n * 16 + b * 4), "r"((uint32_t)e << 23) : "memory");
+            }
+        }
+    }
+}
+__device__ __forceinline__ void row_act_block(uint32_t x_smem, int n_blk, int blk, bool valid, ActBlock<Fp4Format>& a) {
+    const int b = valid ? blk : 0;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        uint4 q = lds_v4(x_smem + row_x_chunk(b, c) * 16);
+        if (!valid) q = make_uint4(0, 0, 0, 0);
+        *reinterpret_cast<uint4*>(&a.h[4 * c]) = q;
+    }
+    uint32_t s;
+    asm volatile("ld.shared.b32 %0, [%1];" : "=r"(s) : "r"(x_smem + (uint32_t)n_blk * 64 + b * 4));
+    a.scale = __uint_as_float(s);
 }
 
 // Before the first copies of a CTA: the previous launch's CTA on this SM asks for its activations about when this one starts (a
