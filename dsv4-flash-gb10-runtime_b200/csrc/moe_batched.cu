@@ -150,11 +150,11 @@ cudaError_t weight_map(CUtensorMap* map, const uint8_t* base, long long rows, in
     return box_map(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, base, 2, dim, box);
 }
 // three MXFP4 terms [3][P][K / 2]: half a tile's columns of every term
-cudaError_t term_maps(CUtensorMap (&map)[kMoeWidths], const uint8_t* base, long long P, int K) {
+cudaError_t term_maps(CUtensorMap (&map)[kMoeWidths], const uint8_t* base, long long P, int K, int cap) {
     cudaError_t err = cudaSuccess;
     for (int i = 0; i < kMoeWidths && err == cudaSuccess; ++i) {
         const cuuint64_t dim[3] = {(cuuint64_t)(K / 2), (cuuint64_t)P, kQTerms};
-        const cuuint32_t box[3] = {128, (cuuint32_t)moe_width(i, kQTok) / 2, kQTerms};
+        const cuuint32_t box[3] = {128, (cuuint32_t)moe_width(i, cap) / 2, kQTerms};
         err = box_map(&map[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, base, 3, dim, box);
     }
     return err;
@@ -265,7 +265,9 @@ static int moe_forward_impl(int path, const __nv_bfloat16* x, const uint8_t* ban
     const int rows_up = path == 1 ? kQTileRowsUp : kMoeTileRows, rows_down = path == 1 ? kQTileRowsDown : 2 * kMoeTileRows;
     ga.m_tiles_up = hidden / rows_up; ga.m_tiles_down = (out_dim + rows_down - 1) / rows_down;
     const int cap16 = P <= (long long)kTmFewTokens * n_experts ? 64 : kMoeTileTokens;      // tokens per tile, fp16 path
-    ga.tile_tokens = path == 1 ? kQTok : cap16;
+    const bool few = P <= (long long)kQFewTokens * n_experts;
+    const int cap_q = few ? 32 : kQTok;                                                    // tokens per tile, block-scaled path
+    ga.tile_tokens = path == 1 ? cap_q : cap16;
     launch_k(moe_group_kernel, dim3(P > kGroupOneBlockPairs ? kGroupCluster : 1), dim3(kPrepThreads), 0, stream, P > kGroupOneBlockPairs ? kGroupCluster : 1, ga);
     stage_mark(stream, 1);
 
@@ -279,7 +281,6 @@ static int moe_forward_impl(int path, const __nv_bfloat16* x, const uint8_t* ban
     cudaError_t err = cudaSuccess;
     if (path == 1) {
         // ---- block-scaled MXFP4 tensor-core path; a warp per 256 elements, at most eight blocks of eight warps per SM
-        static int qup_done[64] = {0}, qdown_done[64] = {0};
         const long long blocks = ((long long)n_tokens * (K_in / 256) + 7) / 8;
         const dim3 agrid((unsigned)(blocks < 8LL * grid ? blocks : 8LL * grid)), ablock(256);
         launch_k(peer_in ? moe_act_mxf4_kernel<true> : moe_act_mxf4_kernel<false>, agrid, ablock, 0, stream, 1, aa, pin);
@@ -287,24 +288,27 @@ static int moe_forward_impl(int path, const __nv_bfloat16* x, const uint8_t* ban
         MoeQMaps up_maps, down_maps;
         err = weight_map(&up_maps.wa, bank_W1_packed, (long long)n_experts * hidden, K_in);
         if (err == cudaSuccess) err = weight_map(&up_maps.wb, bank_W3_packed, (long long)n_experts * hidden, K_in);
-        if (err == cudaSuccess) err = term_maps(up_maps.act, aa.q, P, K_in);
+        if (err == cudaSuccess) err = term_maps(up_maps.act, aa.q, P, K_in, cap_q);
         if (err == cudaSuccess) err = weight_map(&down_maps.wa, bank_W2_packed, (long long)n_experts * out_dim, hidden);
         down_maps.wb = down_maps.wa;
-        if (err == cudaSuccess) err = term_maps(down_maps.act, ws + m.mq, P, hidden);
+        if (err == cudaSuccess) err = term_maps(down_maps.act, ws + m.mq, P, hidden, cap_q);
         MoeQGemmArgs qu;
         qu.wa_s = bank_W1_scale; qu.wb_s = bank_W3_scale; qu.rows = hidden; qu.K = K_in; qu.n_experts = n_experts;
         qu.act_s = aa.s; qu.n_pairs = P; qu.g = g; qu.mid_q = ws + m.mq; qu.mid_s = ws + m.ms; qu.y = nullptr;
         MoeQGemmArgs qd = qu;
         qd.wa_s = bank_W2_scale; qd.wb_s = nullptr; qd.rows = out_dim; qd.K = hidden; qd.act_s = ws + m.ms; qd.y = y;
-        const uint32_t smem = moe_q_smem_bytes(n_experts);
-        if (err == cudaSuccess) err = allow_smem(moe_gemm_mxf4_kernel<0>, smem, qup_done);
-        if (err == cudaSuccess) err = allow_smem(moe_gemm_mxf4_kernel<1>, smem, qdown_done);
-        if (err == cudaSuccess) {
-            launch_k(moe_gemm_mxf4_kernel<0>, dim3(grid & ~1), dim3(kQThreads), smem, stream, 2, up_maps, qu);
+        auto gemms = [&](auto up_kernel, auto down_kernel, uint32_t smem, int (&up_done)[64], int (&down_done)[64]) {
+            if (err == cudaSuccess) err = allow_smem(up_kernel, smem, up_done);
+            if (err == cudaSuccess) err = allow_smem(down_kernel, smem, down_done);
+            if (err != cudaSuccess) return;
+            launch_k(up_kernel, dim3(grid & ~1), dim3(kQThreads), smem, stream, 2, up_maps, qu);
             stage_mark(stream, 3);
             stage_mark(stream, 4);
-            launch_k(moe_gemm_mxf4_kernel<1>, dim3(grid & ~1), dim3(kQThreads), smem, stream, 2, down_maps, qd);
-        }
+            launch_k(down_kernel, dim3(grid & ~1), dim3(kQThreads), smem, stream, 2, down_maps, qd);
+        };
+        static int up_few[64] = {0}, down_few[64] = {0}, up_most[64] = {0}, down_most[64] = {0};
+        if (few) gemms(moe_gemm_mxf4_kernel<0, 32>, moe_gemm_mxf4_kernel<1, 32>, MoeQShape<32>::smem(n_experts), up_few, down_few);
+        else gemms(moe_gemm_mxf4_kernel<0, kQTok>, moe_gemm_mxf4_kernel<1, kQTok>, MoeQShape<kQTok>::smem(n_experts), up_most, down_most);
     } else {
         // ---- fp16 tensor-core path: weights dequantised into tensor memory
         const int blocks = (n_tokens + kActRows - 1) / kActRows;

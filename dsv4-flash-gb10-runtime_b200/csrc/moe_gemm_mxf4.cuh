@@ -45,9 +45,21 @@ constexpr int kQKBlock = 256;                        // K-elements per stage
 constexpr int kQTerms = 3;                           // activation terms
 constexpr int kQTok = 112;                           // tokens per tile at most
 constexpr uint32_t kQTile = 128 * 128;               // bytes of one packed weight tile (128 rows x 128 B)
-constexpr uint32_t kQBStage = kQTerms * (kQTok / 2) * 128;           // activation rows of one stage and CTA
 constexpr uint32_t kQSfStage = 2 * 2 * 512 + 2 * kQTerms * 512;      // scale atoms: [mat][atom], then [atom][term]
-constexpr int kQStages = 3;
+// Tiles of up to CAP tokens.  Where experts have few tokens the weights' way from HBM is what a tile waits for: five stages of 32
+// tokens instead of three of 112 keep more of them on it (256 experts of 4096, 2048, top 6: 17 tokens 216 -> 209.5 us, 64 zipf 278 ->
+// 270, 300 579 -> 567; below ten tokens no difference).  Taken up to kQFewTokens pairs per expert, where next to no expert has more
+// than 32.
+constexpr int kQFewTokens = 16;
+template <int CAP>
+struct MoeQShape {
+    static constexpr int kStages = CAP <= 32 ? 5 : 3;
+    static constexpr uint32_t kBStage = kQTerms * (CAP / 2) * 128;           // activation rows of one stage and CTA
+    static constexpr uint32_t kOffB = kStages * 2 * kQTile, kOffSf = kOffB + kStages * kBStage, kOffTables = kOffSf + kStages * kQSfStage;
+    // dynamic shared memory: stages, then the tile and offset tables of the experts
+    static __host__ __device__ __forceinline__ uint32_t smem(int n_experts) { return kOffTables + 8 * (uint32_t)(n_experts + 1) + 1024; }
+    static_assert(kOffTables + 8 * (kMoeMaxExperts + 1) + 1024 + 1024 <= 227 * 1024, "shared memory overflow");
+};
 constexpr int kQEpiWarps = 12, kQScaleWarps = 8;
 constexpr int kQEpiGroups = kQEpiWarps / 4;          // warps per lane quadrant of tensor memory
 constexpr int kQEpiRounds = (kQTok + 16 * kQEpiGroups - 1) / (16 * kQEpiGroups);
@@ -56,11 +68,6 @@ constexpr int kQThreads = (kQScaleWarp + kQScaleWarps) * 32;
 constexpr uint32_t kQAccCols = 2 * kQTok;            // per accumulator set
 constexpr uint32_t kQSfCol = 2 * kQAccCols, kQSfCols = 16 + 8 * kQTerms;
 static_assert(kQSfCol + kQSfCols <= 512, "tensor memory overflow");
-constexpr uint32_t kQOffB = kQStages * 2 * kQTile, kQOffSf = kQOffB + kQStages * kQBStage;
-constexpr uint32_t kQOffTables = kQOffSf + kQStages * kQSfStage;
-// dynamic shared memory: stages, then the tile and offset tables of the experts
-__host__ __device__ __forceinline__ uint32_t moe_q_smem_bytes(int n_experts) { return kQOffTables + 8 * (uint32_t)(n_experts + 1) + 1024; }
-static_assert(kQOffTables + 8 * (kMoeMaxExperts + 1) + 1024 + 1024 <= 227 * 1024, "shared memory overflow");
 
 struct MoeQGemmArgs {
     const uint8_t* wa_s; const uint8_t* wb_s;        // E8M0 scales: up W1, W3; down W2 (wb unused)
@@ -79,7 +86,7 @@ struct MoeQTile { int e, slot0, n_valid, width, m0, mats; };
 constexpr int kQRows = 2 * kMoeTileRows;             // weight rows of one block of a pair
 constexpr int kQTileRowsUp = kQRows, kQTileRowsDown = 2 * kQRows;
 
-template <int MODE>
+template <int MODE, int CAP>
 __device__ __forceinline__ MoeQTile moe_qtile_decode(const int* tiles, const int* offsets, int n_experts, int m_tiles,
                                                      int rows, int tile) {
     int lo = 0, hi = n_experts;                      // last expert with tiles[e] <= tile
@@ -90,7 +97,7 @@ __device__ __forceinline__ MoeQTile moe_qtile_decode(const int* tiles, const int
     MoeQTile t;
     t.e = lo;
     const int local = tile - tiles[lo], nt = local / m_tiles;
-    const int per = moe_tokens_per_tile(offsets[lo + 1] - offsets[lo], kQTok);
+    const int per = moe_tokens_per_tile(offsets[lo + 1] - offsets[lo], CAP);
     t.slot0 = offsets[lo] + nt * per;
     t.n_valid = min(per, offsets[lo + 1] - t.slot0);
     t.width = moe_width_index(t.n_valid);
@@ -200,17 +207,19 @@ __device__ __forceinline__ void moe_quantize_half_block(float (&v)[16], uint2 (&
     }
 }
 
-template <int MODE>
+template <int MODE, int CAP>
 __global__ void __launch_bounds__(kQThreads, 1) moe_gemm_mxf4_kernel(const __grid_constant__ MoeQMaps maps,
                                                                                               const MoeQGemmArgs a) {
+    using Q = MoeQShape<CAP>;
+    constexpr int kQStages = Q::kStages;
     extern __shared__ __align__(1024) uint8_t gemm_smem[];
     __shared__ __align__(8) uint64_t full[kQStages], empty[kQStages], acc_full[2], acc_free[2];
     __shared__ uint32_t tmem_holder;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int n_st = a.K / kQKBlock, row_s = a.K >> 5;
-    const uint32_t smem_w = smem_u32(gemm_smem), smem_b = smem_w + kQOffB, smem_sf = smem_w + kQOffSf;
-    int* const s_tiles = reinterpret_cast<int*>(gemm_smem + kQOffTables);
+    const uint32_t smem_w = smem_u32(gemm_smem), smem_b = smem_w + Q::kOffB, smem_sf = smem_w + Q::kOffSf;
+    int* const s_tiles = reinterpret_cast<int*>(gemm_smem + Q::kOffTables);
     int* const s_offsets = s_tiles + a.n_experts + 1;
 
     if (warp == kQMmaWarp) tc05_pair_alloc(smem_u32(&tmem_holder), 512);
@@ -234,7 +243,7 @@ __global__ void __launch_bounds__(kQThreads, 1) moe_gemm_mxf4_kernel(const __gri
     auto leader = [&](uint64_t& bar) { return cluster_map(smem_u32(&bar), 0); };
     const int n_tiles = s_tiles[a.n_experts];
     const int m_tiles = (a.rows + (MODE == 0 ? kQTileRowsUp : kQTileRowsDown) - 1) / (MODE == 0 ? kQTileRowsUp : kQTileRowsDown);
-    auto decode = [&](int tile) { return moe_qtile_decode<MODE>(s_tiles, s_offsets, a.n_experts, m_tiles, a.rows, tile); };
+    auto decode = [&](int tile) { return moe_qtile_decode<MODE, CAP>(s_tiles, s_offsets, a.n_experts, m_tiles, a.rows, tile); };
     bool alive = true;
     auto wait = [&](uint64_t& bar, uint32_t parity, int code) {            // roles of whole warps
         if (alive) alive = __all_sync(kFullMask, mbar_wait_bounded(smem_u32(&bar), parity & 1u, code));
@@ -391,7 +400,7 @@ __global__ void __launch_bounds__(kQThreads, 1) moe_gemm_mxf4_kernel(const __gri
             if (pair < n_tiles) t = decode(pair);
             for (int tile = pair; tile < n_tiles && alive; tile += n_pairs, t = next) {
                 const int first = t.e * a.rows + t.m0 + rank * kMoeTileRows;      // past the expert in a half tile: loaded, not used
-                const int half = moe_width(t.width, kQTok) >> 1, slot = t.slot0 + rank * half;
+                const int half = moe_width(t.width, CAP) >> 1, slot = t.slot0 + rank * half;
                 const CUtensorMap* act = &maps.act[t.width];
                 const uint32_t bytes = t.mats * kQTile + kQTerms * half * 128u;
                 auto weights = [&](int s, const RingPos& p) {
@@ -401,7 +410,7 @@ __global__ void __launch_bounds__(kQThreads, 1) moe_gemm_mxf4_kernel(const __gri
                     if (t.mats == 2) tma_pair_load_2d(dst + kQTile, &maps.wb, s * 128, first + (MODE == 0 ? 0 : kQRows), bar);
                 };
                 auto tokens = [&](int s, const RingPos& p) {
-                    tma_pair_load_3d(smem_b + p.slot * kQBStage, act, s * 128, slot, 0, leader(full[p.slot]));
+                    tma_pair_load_3d(smem_b + p.slot * Q::kBStage, act, s * 128, slot, 0, leader(full[p.slot]));
                 };
                 int s0 = 0;
                 if (!waited) {                                // the pair's first stages: weights before the wait
@@ -432,7 +441,7 @@ __global__ void __launch_bounds__(kQThreads, 1) moe_gemm_mxf4_kernel(const __gri
             if (pair < n_tiles) t = decode(pair);
             for (int tile = pair; tile < n_tiles && alive; tile += n_pairs, ++tc, t = next) {
                 const uint32_t buf = tc & 1u;
-                const int n = moe_width(t.width, kQTok);
+                const int n = moe_width(t.width, CAP);
                 MoeQStage q;
                 q.acc = tmem + buf * kQAccCols;
                 q.sfa = tmem + kQSfCol;
@@ -445,7 +454,7 @@ __global__ void __launch_bounds__(kQThreads, 1) moe_gemm_mxf4_kernel(const __gri
                     if (!alive) break;
                     tc05_fence_after_sync();
                     q.w = tc05_desc_k_sw128(smem_w + pos.slot * 2 * kQTile);
-                    q.b = tc05_desc_k_sw128(smem_b + pos.slot * kQBStage);
+                    q.b = tc05_desc_k_sw128(smem_b + pos.slot * Q::kBStage);
                     q.sf = smem_sf + pos.slot * kQSfStage;
                     q.fresh = s == 0;
                     if (t.mats == 2) moe_q_issue<2>(q); else moe_q_issue<1>(q);

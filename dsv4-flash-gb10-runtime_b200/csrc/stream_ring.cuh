@@ -117,20 +117,4 @@ __device__ __forceinline__ uint32_t lds_u8(uint32_t addr) {
     return v;
 }
 
-// Lane's part of one MXFP4 row held in a ring slot: weights at `w` (row start), scale bytes at `s`.
-template <int BPL>
-__device__ __forceinline__ float ring_row_dot(uint32_t w, uint32_t s, int lane, const bool (&ok)[BPL],
-                                              const LaneAct<Fp4Format, BPL>& a) {
-    float acc = 0.f;
-#pragma unroll
-    for (int j = 0; j < BPL; ++j) {
-        if (ok[j]) {
-            const uint4 q = lds_v4(w + (lane + 32 * j) * 16);
-            const float sc = e8m0_to_float_fast(lds_u8(s + lane + 32 * j));
-            acc = fmaf(Fp4Format::dot(q, a.h[j]), sc, acc);
-        }
-    }
-    return acc * a.scale;
-}
-
 }  // namespace dsv4

@@ -49,3 +49,10 @@ def test_reduction_lengths_and_partial_row_tiles(rt, qz, path, K, H, O):
 def test_grouping_by_one_block_and_by_a_cluster(rt, qz, path, n_pairs):
     counts = [n_pairs // 3, 0, n_pairs // 5, n_pairs - n_pairs // 3 - n_pairs // 5]
     run_case(rt, qz, path, counts, K=256, H=256, O=128, seed=n_pairs)
+
+
+@pytest.mark.parametrize("K,H", [(256, 256), (1280, 512), (1536, 256)])
+@pytest.mark.parametrize("counts", [[33, 0, 0], [64, 31, 1] + [0] * 5, [0] * 7 + [112], [32] * 2 + [0] * 2])
+def test_tiles_of_few_tokens(rt, qz, counts, K, H):
+    """At most 16 pairs per expert on average: tiles of up to 32 tokens, five stages, more tiles than one for a busy expert."""
+    run_case(rt, qz, "mxf4", counts, K=K, H=H, O=K, seed=sum(counts) + K)
