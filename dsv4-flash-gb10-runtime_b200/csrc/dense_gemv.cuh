@@ -35,6 +35,7 @@ __global__ void __launch_bounds__(kRowThreads, 2) dense_stream_kernel(const Dens
     extern __shared__ __align__(128) uint8_t row_smem[];
     __shared__ RowRing ring;
     __shared__ volatile int x_asked;
+    __shared__ int failed;                   // MATS = 2: a wait ran out (the clamp would turn NaN into a number)
     pdl_launch_dependents();
     DenseArgs a = a_in;
     if (GROUPED) {
@@ -54,8 +55,8 @@ __global__ void __launch_bounds__(kRowThreads, 2) dense_stream_kernel(const Dens
     if (tid == kRowWarps * 32) row_ring_init(ring, p);
     auto produce = [&]() {
         RowPos pos;
-        for (int st = 0; st < n_stages; ++st, pos.next(p.slots)) {
-            if (pos.round > 0 && !mbar_wait_bounded(smem_u32(&ring.empty[pos.slot]), (pos.round - 1) & 1u, 1)) break;
+        for (int st = 0; st < n_stages - p.withheld; ++st, pos.next(p.slots)) {
+            if (!row_wait_free(ring, p, pos, 1)) break;
             const int row = st * p.rows, rows = min(p.rows, n_local - row);
             const uint32_t bar = smem_u32(&ring.full[pos.slot]), dst = smem + pos.slot * p.stage_bytes;
             const long long first = r_begin + row;
@@ -83,7 +84,10 @@ __global__ void __launch_bounds__(kRowThreads, 2) dense_stream_kernel(const Dens
     };
     uint32_t raw = 0;
     if (tid < n_table) raw = tile_scale(tid);
-    if (tid == 0) x_asked = 0;
+    if (tid == 0) {
+        x_asked = 0;
+        if (MATS == 2) failed = 0;
+    }
     __syncthreads();                         // barriers
     // The consumers go on without the producer: when it filled the ring before the barrier above, asking for x and the tile
     // scales waited for that (eight launches of 4096 x 4096 MXFP4 35.1 us then, 31.0 now; of 2048 x 4096 FP8 28.1, 23.8).
@@ -113,17 +117,23 @@ __global__ void __launch_bounds__(kRowThreads, 2) dense_stream_kernel(const Dens
         bool ok[SPW];
 #pragma unroll
         for (int q = 0; q < SPW; ++q) { blk[q] = (ks0 + q * w_slices) * 32 + lane; ok[q] = blk[q] < n_blk; }
-        bool alive = Sc::kPerRow || __all_sync(kFullMask, mbar_wait_bounded(smem_u32(&ring.x), 0, 2));
+        bool alive = Sc::kPerRow || __all_sync(kFullMask, row_wait(p, ring.x, 0, 2));
+        if (MATS == 2 && !alive) failed = 1;
         ActBlock<Fmt> xb[SPW];
 #pragma unroll
         for (int q = 0; q < SPW; ++q) {
             if constexpr (Sc::kPerRow) row_act_block(smem + p.off_x, n_blk, blk[q], ok[q], xb[q]);
             else row_act_block_bf16<Fmt>(smem + p.off_x, blk[q], ok[q], xb[q]);
             if (!ok[q]) blk[q] = 0;
+            if (!Sc::kPerRow && !alive) xb[q].scale = row_nan();
         }
         RowPos pos;
         for (int st = 0; st < n_stages; ++st) {
-            if (alive) alive = __all_sync(kFullMask, mbar_wait_bounded(smem_u32(&ring.full[pos.slot]), pos.round & 1u, 2));
+            if (alive && !__all_sync(kFullMask, row_wait(p, ring.full[pos.slot], pos.round, 2))) {
+                alive = false;
+                for (int q = 0; q < SPW; ++q) xb[q].scale = row_nan();
+                if (MATS == 2) failed = 1;
+            }
             const uint32_t stage = smem + pos.slot * p.stage_bytes;
             const int row = st * p.rows + rg, left = n_local - row;
             const uint32_t s_row = (uint32_t)(r_begin + st * p.rows) * (uint32_t)a.s_stride;
@@ -155,7 +165,7 @@ __global__ void __launch_bounds__(kRowThreads, 2) dense_stream_kernel(const Dens
                     for (int i = 0; i < RPW; ++i) v[m * row_pow2(RPW) + i] = Fmt::dot(w[m * RPW + i], xb[q].h) * (sc[m * RPW + i] * xb[q].scale);
                 row_store<RPW>(v, left, p.n_groups, lane, part + row * p.n_slices + ks0 + q * w_slices, p.n_slices, n_local * p.n_slices);
             }
-            row_release(ring, p, pos, lane);
+            row_release(ring, p, pos, lane, alive);
         }
     }
     __syncthreads();
@@ -172,7 +182,7 @@ __global__ void __launch_bounds__(kRowThreads, 2) dense_stream_kernel(const Dens
             u = __bfloat162float(__float2bfloat16(u));
             if (limit_g > 0.f) g = fminf(fmaxf(g, -limit_g), limit_g);
             if (limit_u > 0.f) u = fminf(fmaxf(u, -limit_u), limit_u);
-            a.y[r_begin + t] = __float2bfloat16((g / (1.0f + expf(-g))) * u);
+            a.y[r_begin + t] = __float2bfloat16(failed ? row_nan() : (g / (1.0f + expf(-g))) * u);
         }
     }
 }

@@ -60,8 +60,8 @@ __global__ void __launch_bounds__(kRowThreads, 2) grouped_gate_stream_kernel(con
         if (lane == 0) {
             RowPos pos;
             Walk c = walk_start();
-            for (int st = 0; st < n_stages; ++st, pos.next(p.slots), walk_next(c)) {
-                if (pos.round > 0 && !mbar_wait_bounded(smem_u32(&ring.empty[pos.slot]), (pos.round - 1) & 1u, 1)) break;
+            for (int st = 0; st < n_stages - p.withheld; ++st, pos.next(p.slots), walk_next(c)) {
+                if (!row_wait_free(ring, p, pos, 1)) break;
                 walk_stage(c, st);
                 const uint32_t bar = smem_u32(&ring.full[pos.slot]), dst = smem + pos.slot * p.stage_bytes;
                 uint32_t s0[2], b0[2], s1[2], b1[2], bytes = 2 * (c.n0 + c.n1) * p.row_bytes;
@@ -105,7 +105,10 @@ __global__ void __launch_bounds__(kRowThreads, 2) grouped_gate_stream_kernel(con
             RowPos pos;
             Walk c = walk_start();
             for (int st = 0; st < n_stages; ++st, walk_next(c)) {
-                if (alive) alive = __all_sync(kFullMask, mbar_wait_bounded(smem_u32(&ring.full[pos.slot]), pos.round & 1u, 1));
+                if (alive && !__all_sync(kFullMask, row_wait(p, ring.full[pos.slot], pos.round, 1))) {
+                    alive = false;
+                    xb.scale = row_nan();
+                }
                 walk_stage(c, st);
                 const uint32_t stage = smem + pos.slot * p.stage_bytes;
                 const int row = st * p.rows + rg;
@@ -126,7 +129,7 @@ __global__ void __launch_bounds__(kRowThreads, 2) grouped_gate_stream_kernel(con
 #pragma unroll
                 for (int k = 0; k < 2 * kGateRpw; ++k) v[k] = Fp4Format::dot(w[k], xb.h) * (sc[k] * xb.scale);
                 row_store<kGateRpw>(v, n_local - row, p.n_groups, lane, part + row * p.n_slices + ks, p.n_slices, n_local * p.n_slices);
-                row_release(ring, p, pos, lane);
+                row_release(ring, p, pos, lane, alive);
             }
         }
     }
@@ -163,8 +166,8 @@ __global__ void __launch_bounds__(kRowThreads, 2) grouped_down_stream_kernel(con
     if (warp == kRowWarps) {
         if (lane == 0) {
             RowPos pos;
-            for (int st = 0; st < n_stages; ++st, pos.next(p.slots)) {
-                if (pos.round > 0 && !mbar_wait_bounded(smem_u32(&ring.empty[pos.slot]), (pos.round - 1) & 1u, 2)) break;
+            for (int st = 0; st < n_stages - p.withheld; ++st, pos.next(p.slots)) {
+                if (!row_wait_free(ring, p, pos, 2)) break;
                 const int e = st / per_e, row = (st - e * per_e) * p.rows, rows = min(p.rows, n_local - row);
                 const uint32_t bar = smem_u32(&ring.full[pos.slot]), dst = smem + pos.slot * p.stage_bytes;
                 const uint8_t* s = scales_of(e, row);
@@ -227,11 +230,14 @@ __global__ void __launch_bounds__(kRowThreads, 2) grouped_down_stream_kernel(con
                         if (!ok) q = make_uint4(0, 0, 0, 0);
                         *reinterpret_cast<uint4*>(&xb.h[4 * c]) = q;
                     }
-                    xb.scale = mid_scale[b];
+                    xb.scale = alive ? mid_scale[b] : row_nan();
                 }
                 const uint32_t s_first = (uint32_t)reinterpret_cast<uintptr_t>(scales_of(e, 0));
                 for (int row0 = 0; row0 < n_local; row0 += p.rows) {
-                    if (alive) alive = __all_sync(kFullMask, mbar_wait_bounded(smem_u32(&ring.full[pos.slot]), pos.round & 1u, 2));
+                    if (alive && !__all_sync(kFullMask, row_wait(p, ring.full[pos.slot], pos.round, 2))) {
+                        alive = false;
+                        xb.scale = row_nan();
+                    }
                     const uint32_t stage = smem + pos.slot * p.stage_bytes, sbase = stage + p.rows * p.row_bytes + blk_r;
                     const uint32_t s_addr = s_first + row0 * n_blk;
                     const int row = row0 + rg;
@@ -246,7 +252,7 @@ __global__ void __launch_bounds__(kRowThreads, 2) grouped_down_stream_kernel(con
 #pragma unroll
                     for (int j = 0; j < RPW; ++j) v[j] = Fp4Format::dot(w[j], xb.h) * (sc[j] * xb.scale);
                     row_store<RPW>(v, n_local - row, p.n_groups, lane, part + (row * a.E + e) * p.n_slices + ks, a.E * p.n_slices, 0);
-                    row_release(ring, p, pos, lane);
+                    row_release(ring, p, pos, lane, alive);
                 }
             }
         }

@@ -35,3 +35,18 @@ DSV4_API int mxfp4_gemv_m1(const __nv_bfloat16* x, const uint8_t* W_packed, cons
     }
     return 0;
 }
+
+// Added (diagnostic): 0 unless a kernel of this library gave up on a bounded wait since the last call (1 = a slot of a
+// CTA's ring never became free, 2 = weight rows or activations never landed); the output rows that depend on what did
+// not arrive are NaN.  Clears the status.  Synchronises the device.
+DSV4_API int mxfp4_gemv_device_status(void) {
+    int v = 0, zero = 0;
+    if (cudaMemcpyFromSymbol(&v, g_device_status, sizeof(int)) != cudaSuccess) return -1;
+    if (v != 0) cudaMemcpyToSymbol(g_device_status, &zero, sizeof(int));
+    return v;
+}
+
+// Added (test hook): poll budget of the device-side waits, and the stages at the end of every CTA's rows that are not
+// requested, so that the waits for them run out - without a fault, a trap or an unbounded loop.  (0, 0) restores the
+// defaults.  Returns -1 for negative arguments.
+DSV4_API int mxfp4_gemv_test_wait_limits(long long polls, int withheld_stages) { return row_wait_limits(polls, withheld_stages); }

@@ -580,7 +580,7 @@ DSV4_API int mxfp4_dequant_bf16(const uint8_t* packed, const uint8_t* scale, lon
 }
 
 // Added (diagnostic): 0 unless a kernel of this library gave up on a bounded wait since the last call
-// (1 = a gate/up row or its scales never landed, 2 = a down row or its scales, 3 = an expert's intermediate never
+// (1 = a gate/up row or its scales never landed or their slot never became free, 2 = a down row or its scales, 3 = an expert's intermediate never
 // became complete); the status is cleared by the call.  Synchronises the device.
 DSV4_API int dsv4_b200_device_status(void) {
     int v = 0, zero = 0;
@@ -602,15 +602,17 @@ DSV4_API int dsv4_b200_set_launch_mode(int mode) {
     return before;
 }
 
-// Added (test hook, no counterpart): poll budget of the device-side waits of the single-kernel path, and a number of
-// producers that never arrive.  With phantom_ctas > 0 the next calls wait for readiness flags nobody publishes, give
-// up after `polls` polls (microseconds for a few thousand), record status 3 and write NaN - without a fault, a
-// trap or an unbounded loop.  (0, 0) restores the defaults.  Returns -1 for negative arguments.
+// Added (test hook, no counterpart): poll budget of the device-side waits of the single-kernel path and of the
+// row-streaming kernels, and a number of producers that never arrive.  With phantom_ctas > 0 the next calls wait for
+// what nobody delivers - the single kernel for readiness flags (status 3), the row-streaming kernels for the last
+// phantom_ctas stages of every CTA (status 1 or 2) -, give up after `polls` polls (microseconds for a few thousand) and
+// write NaN, without a fault, a trap or an unbounded loop.  (0, 0) restores the defaults.  Returns -1 for negative
+// arguments.
 DSV4_API int dsv4_b200_test_wait_limits(long long polls, int phantom_ctas) {
     if (polls < 0 || phantom_ctas < 0 || phantom_ctas > 64) return -1;
     g_spin_limit = polls == 0 ? kSpinLimit : (unsigned)(polls > 0xffffffffLL ? 0xffffffffLL : polls);
     g_phantom = phantom_ctas;
-    return 0;
+    return row_wait_limits(polls, phantom_ctas);
 }
 
 // ------------------------------------------------------------------------------------------------

@@ -12,6 +12,11 @@
 // dependent launch the next kernel's CTAs sit beside these and have their first ~90 KB per SM (13 MB) on the way while
 // these finish.  Nothing is loaded by the consumers inside the loop: a load queues behind the SM's own weight copies, one to
 // four microseconds (scale bytes fetched that way, two stages ahead, made 33.6 MB of FP8 take 11.1 us).
+//
+// Every wait has a poll budget.  A consumer warp whose wait runs out records a status, takes NaN for its activations' scale - so
+// that the rows it did not get come out as NaN - and goes through its remaining stages without waiting and without freeing a slot.
+// Nothing is requested past the ring then, and what was requested landed long before the last role has given up: no copy is on
+// its way when the CTA leaves.  (A flag for the whole CTA, looked at behind the last stage, made every launch 0.05 to 0.1 us longer.)
 #pragma once
 
 #include "gemv_engine.cuh"
@@ -39,7 +44,19 @@ struct RowPlan {
     uint32_t s_area, s_pitch, s_adv;
     uint32_t off_x, off_part, off_table;               // behind the ring
     uint32_t smem;
+    uint32_t polls;                                    // budget of a wait
+    int withheld;                                      // stages at a CTA's end that its producer does not request (0; see row_wait_limits)
 };
+// What the next launches of this library take: the poll budget of their waits, and the stages a test withholds so that waits run
+// out without a fault.
+static uint32_t g_row_polls = kSpinLimit;
+static int g_row_withheld = 0;
+inline int row_wait_limits(long long polls, int withheld) {
+    if (polls < 0 || withheld < 0) return -1;
+    g_row_polls = polls == 0 || polls > (long long)kSpinLimit ? kSpinLimit : (uint32_t)polls;
+    g_row_withheld = withheld;
+    return 0;
+}
 // The bytes of a stage's scale rows are copied with the 16-byte chunks they lie in (such a chunk never leaves the memory page
 // of its bytes).  Rows dense in memory: one copy, row i at i * s_pitch behind the first; otherwise a copy per row, each with
 // its own misalignment.
@@ -49,6 +66,8 @@ __device__ __forceinline__ uint32_t row_scale_offset(const RowPlan& p, uint32_t 
 // rpw: rows per warp and stage, spw: slices per warp, mats: matrices streamed side by side
 inline RowPlan row_plan(int n_blk, int mats, int rpw, int spw) {
     RowPlan p = {};
+    p.polls = g_row_polls;
+    p.withheld = g_row_withheld;
     p.n_slices = (n_blk + 31) / 32;
     const int w = (p.n_slices + spw - 1) / spw;
     p.n_groups = kRowWarps / w;
@@ -134,9 +153,29 @@ struct RowPos {
     uint32_t round = 0;
     __device__ __forceinline__ void next(int n) { if (++slot == n) { slot = 0; ++round; } }
 };
-__device__ __forceinline__ void row_release(RowRing& r, const RowPlan& p, RowPos& pos, int lane) {
+// Waits for a phase; the budget is looked at only where a wait is a long one.
+__device__ __forceinline__ bool row_wait(const RowPlan& p, uint64_t& bar, uint32_t parity, int code) {
+    for (uint32_t it = 0;; ++it) {
+        if (mbar_try_wait(smem_u32(&bar), parity & 1u)) return true;
+        if (it > 64) {
+            __nanosleep(64);
+            if (it >= p.polls) break;
+        }
+    }
+    atomicExch(&g_device_status, code);
+    return false;
+}
+// The producer's wait for a free slot.  The consumers free nothing before the previous kernel's end, which may be any time away:
+// that wait comes first and is not part of the budget.
+__device__ __forceinline__ bool row_wait_free(RowRing& r, const RowPlan& p, const RowPos& pos, int code) {
+    if (pos.round == 0) return true;
+    if (pos.round == 1 && pos.slot == 0) pdl_wait();
+    return row_wait(p, r.empty[pos.slot], pos.round - 1, code);
+}
+__device__ __forceinline__ float row_nan() { return __uint_as_float(0x7fffffffu); }
+__device__ __forceinline__ void row_release(RowRing& r, const RowPlan& p, RowPos& pos, int lane, bool alive) {
     __syncwarp();
-    if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&r.empty[pos.slot])) : "memory");
+    if (lane == 0 && alive) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&r.empty[pos.slot])) : "memory");
     pos.next(p.slots);
 }
 

@@ -18,7 +18,8 @@ namespace dsv4 {
 
 constexpr uint32_t kSpinLimit = 1u << 22;
 
-// Set to a non-zero code by a kernel whose bounded wait ran out; read by dsv4_b200_device_status().
+// Set to a non-zero code by a kernel whose bounded wait ran out; every library has its own and an entry that reads it
+// (dsv4_b200_device_status, mxfp4_gemv_device_status, fp8_e4m3_gemv_device_status, mxfp4_moe_device_status).
 __device__ int g_device_status = 0;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {

@@ -27,6 +27,8 @@ SIGNATURES = {
     },
     "mxfp4": {
         "mxfp4_gemv_m1": (c_int, [_P, _P, _P, c_int, c_int, c_int64, c_int64, _P, _P]),
+        "mxfp4_gemv_device_status": (c_int, []),
+        "mxfp4_gemv_test_wait_limits": (c_int, [c_longlong, c_int]),
     },
     "moe": {
         "mxfp4_moe_forward": (c_int, [_P] * 9 + [c_int] * 6 + [_P, _P, _P]),
@@ -48,6 +50,8 @@ SIGNATURES = {
                                           _P, _P]),
         "fp8_e4m3_shared_swiglu_workspace_bytes": (c_size_t, [c_int]),
         "fp8_e4m3_shared_swiglu_m1": (c_int, [_P] * 7 + [c_int] * 3 + [c_float] * 2 + [_P] * 3),
+        "fp8_e4m3_gemv_device_status": (c_int, []),
+        "fp8_e4m3_gemv_test_wait_limits": (c_int, [c_longlong, c_int]),
     },
 }
 

@@ -168,4 +168,10 @@ def fp8_shared_swiglu(shared: dict, x: torch.Tensor, limit_gate: float = 10.0, l
     return out
 
 
-__all__ = ["fp8_e4m3_gemv", "fp8_e4m3_gemv_f32scale", "fp8_e4m3_gemv_batched", "fp8_shared_swiglu", "FP8_BLOCK_TILE"]
+def device_status() -> int:
+    """0 unless a kernel of this library gave up on one of its bounded waits since the last call; the output rows
+    that it could not compute are NaN (synchronises the device)."""
+    return int(_capi.load("fp8").fp8_e4m3_gemv_device_status())
+
+
+__all__ = ["fp8_e4m3_gemv", "fp8_e4m3_gemv_f32scale", "fp8_e4m3_gemv_batched", "fp8_shared_swiglu", "device_status", "FP8_BLOCK_TILE"]

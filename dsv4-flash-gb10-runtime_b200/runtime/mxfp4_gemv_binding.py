@@ -56,4 +56,10 @@ def mxfp4_gemv(W_packed: torch.Tensor, W_scale: torch.Tensor, x: torch.Tensor,
     return out
 
 
-__all__ = ["mxfp4_gemv"]
+def device_status() -> int:
+    """0 unless a kernel of this library gave up on one of its bounded waits since the last call; the output rows
+    that it could not compute are NaN (synchronises the device)."""
+    return int(_capi.load("mxfp4").mxfp4_gemv_device_status())
+
+
+__all__ = ["mxfp4_gemv", "device_status"]

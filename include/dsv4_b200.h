@@ -104,10 +104,12 @@ int mxfp4_dequant_bf16(const uint8_t* packed, const uint8_t* scale, long long ro
                        void* stream);
 
 /* Added (diagnostic, no counterpart): 0 unless a kernel of this library gave up on one of its bounded waits since
- * the last call (1 = a gate/up row never landed, 2 = a down row, 3 = an expert's intermediate never became complete),
+ * the last call (1 = a gate/up row never landed or its slot never became free, 2 = a down row, 3 = an expert's
+ * intermediate never became complete),
  * or the router of mxfp4_moe_decode_layer found fewer than k pickable experts (4: NaN or -inf logits; the missing
  * picks run with weight 0, where the reference's host router aborts with -2, routed.cu:186-199);
- * clears the status.  A kernel that gives up writes NaN to its output rows, so the damage is also visible downstream.
+ * clears the status.  A kernel that gives up writes NaN to the output rows it could not compute, so the damage is also
+ * visible downstream (not so the two ring kernels of launch mode 0: their output is undefined then).
  * Synchronises the device. */
 int dsv4_b200_device_status(void);
 
@@ -117,14 +119,16 @@ int dsv4_b200_device_status(void);
  *     layer's CTAs are scheduled while this layer's exit), every other stream a cooperative launch (co-residency
  *     guaranteed by the runtime) - any mix of streams makes progress;
  *   1 cooperative for every stream;  3 programmatic for every stream (only for callers with ONE stream per device);
- *   0 two chained kernels that wait for nothing.
+ *   0 two chained kernels whose CTAs do not wait for one another.
  * The environment variable DSV4_B200_FUSED (auto | coop | pdl | 0) sets the initial mode.  Returns the previous mode,
  * -1 for another value. */
 int dsv4_b200_set_launch_mode(int mode);
 
-/* Added (test hook, no counterpart): poll budget of the device-side waits of the single-kernel path, and a number of
- * producers that never arrive (> 0: the next calls wait for data nobody writes, give up after `polls` polls, record
- * status 3 and write NaN - nothing faults or spins without a limit).  (0, 0) restores the defaults. */
+/* Added (test hook, no counterpart): poll budget of the device-side waits of the single-kernel path and of the kernels of
+ * the other shapes, and a number of producers that never arrive (> 0: the next calls wait for data nobody delivers - the
+ * single kernel for intermediates, the others for the last phantom_ctas stages of every CTA's rows -, give up after
+ * `polls` polls, record status 3, or 1 and 2, and write NaN - nothing faults or spins without a limit).  (0, 0) restores
+ * the defaults. */
 int dsv4_b200_test_wait_limits(long long polls, int phantom_ctas);
 
 /* ---- libmxfp4_gemv.so --------------------------------------------------------------------------------- */
@@ -134,6 +138,15 @@ int dsv4_b200_test_wait_limits(long long polls, int phantom_ctas);
  * -8 null pointer or N < 0. */
 int mxfp4_gemv_m1(const uint16_t* x, const uint8_t* W_packed, const uint8_t* W_scale, int K, int N,
                   int64_t packed_row_stride_bytes, int64_t scale_row_stride_bytes, uint16_t* y, void* stream);
+
+/* Added (diagnostic, no counterpart): 0 unless a kernel of this library gave up on one of its bounded waits since the
+ * last call (1 = a slot of a CTA's ring never became free, 2 = weight rows or activations never landed): the output rows
+ * that depend on what did not arrive are NaN.  Clears the status.  Synchronises the device. */
+int mxfp4_gemv_device_status(void);
+/* Added (test hook): poll budget of those waits, and how many stages at the end of every CTA's rows are not requested, so
+ * that the waits for them run out - nothing faults or spins without a limit.  (0, 0) restores the defaults.  Returns -1
+ * for negative arguments. */
+int mxfp4_gemv_test_wait_limits(long long polls, int withheld_stages);
 
 /* ---- libfp8_e4m3_gemv.so ------------------------------------------------------------------------------ */
 
@@ -175,6 +188,10 @@ int fp8_e4m3_shared_swiglu_m1(const uint16_t* x, const uint8_t* W1_fp8, const ui
                               const uint8_t* W3_scale, const uint8_t* W2_fp8, const uint8_t* W2_scale, int K_in,
                               int hidden, int out_dim, float limit_gate, float limit_up, uint16_t* out, void* workspace,
                               void* stream);
+
+/* As mxfp4_gemv_device_status and mxfp4_gemv_test_wait_limits, for this library. */
+int fp8_e4m3_gemv_device_status(void);
+int fp8_e4m3_gemv_test_wait_limits(long long polls, int withheld_stages);
 
 /* ---- libmxfp4_moe.so (added; no counterpart: the reference runs one token at a time) ---------------------- */
 

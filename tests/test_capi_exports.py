@@ -94,3 +94,12 @@ def test_bindings_reject_cpu_tensors(rt):
     w = {"packed": torch.zeros(6, 32, 32, dtype=torch.uint8), "scale": torch.zeros(6, 32, 2, dtype=torch.uint8)}
     with pytest.raises(ValueError):
         rt.mxfp4_grouped_gemv(w, w, w, None, x, torch.zeros(6))
+
+
+def test_wait_limit_hooks_check_their_arguments(pkg):
+    import importlib
+    capi = importlib.import_module("dsv4_b200.runtime._capi")
+    for limits in (capi.load("mxfp4").mxfp4_gemv_test_wait_limits, capi.load("fp8").fp8_e4m3_gemv_test_wait_limits,
+                   capi.load("grouped").dsv4_b200_test_wait_limits):
+        assert limits(-1, 0) == -1 and limits(0, -1) == -1
+        assert limits(0, 0) == 0

@@ -82,3 +82,56 @@ def test_bounded_wait_gives_up_reports_and_recovers(rt, case):
     got = again.float().cpu().numpy()
     assert oracle.max_abs_rel(got, ref) <= 1e-2 and oracle.cosine(got, ref) >= 0.9999
     assert gb.device_status() == 0
+
+
+def test_row_streaming_gives_up_with_nan_rows(rt, qz):
+    """The dense GEMVs and the routed FFN of the other shapes (csrc/row_stream.cuh): the last stage of every CTA is not
+    requested, so the wait for it runs out; the status is reported, the rows that depend on it are NaN, the others right, and
+    the next call is bit-exact."""
+    capi = importlib.import_module("dsv4_b200.runtime._capi")
+    dev = torch.device("cuda:0")
+    g = torch.Generator(device=dev).manual_seed(5)
+
+    def act(n):
+        return torch.randn(n, generator=g, device=dev).to(torch.bfloat16)
+
+    x4, p4 = act(2912), qz.quantize_mxfp4((torch.randn(3000, 2912, generator=g, device=dev) * 0.02).to(torch.bfloat16))
+    x8, p8 = act(4096), qz.quantize_fp8_block128(torch.randn(2048, 4096, generator=g, device=dev) * 0.02)
+    shared = {}
+    for name, n, k_ in (("w1", 1024, 2048), ("w3", 1024, 2048), ("w2", 2048, 1024)):
+        shared[name], shared[name + "s"] = qz.quantize_fp8_block128(torch.randn(n, k_, generator=g, device=dev) * 0.02)
+    xs, bank, xg = act(2048), qz.make_expert_bank(6, 2880, 1440, dev, seed=3), act(2880)
+    stacked = [{"packed": bank[n + "p"], "scale": bank[n + "s"]} for n in ("w1", "w3", "w2")]
+    r = torch.rand(6, generator=g, device=dev) + 0.1
+    mxfp4, fp8, grouped = capi.load("mxfp4"), capi.load("fp8"), capi.load("grouped")
+    cases = [
+        ("mxfp4", lambda: rt.mxfp4_gemv(*p4, x4), mxfp4.mxfp4_gemv_test_wait_limits, mxfp4.mxfp4_gemv_device_status, (2,)),
+        ("fp8", lambda: rt.fp8_e4m3_gemv(*p8, x8), fp8.fp8_e4m3_gemv_test_wait_limits, fp8.fp8_e4m3_gemv_device_status, (2,)),
+        ("fp8 groups", lambda: rt.fp8_e4m3_gemv_batched(*p8, torch.cat((x8, x8)).view(1, -1), n_groups=2),
+         fp8.fp8_e4m3_gemv_test_wait_limits, fp8.fp8_e4m3_gemv_device_status, (2,)),
+        ("shared expert", lambda: rt.fp8_shared_swiglu(shared, xs), fp8.fp8_e4m3_gemv_test_wait_limits,
+         fp8.fp8_e4m3_gemv_device_status, (2,)),
+        ("stacked experts", lambda: rt.mxfp4_grouped_gemv(*stacked, None, xg, r), grouped.dsv4_b200_test_wait_limits,
+         grouped.dsv4_b200_device_status, (1, 2)),
+    ]
+    for what, call, limits, status, codes in cases:
+        good = call().clone()
+        torch.cuda.synchronize()
+        assert status() == 0, what
+        try:
+            assert limits(-1, 0) == -1 and limits(0, -1) == -1
+            assert limits(2000, 1) == 0
+            bad = call().clone()
+            assert status() in codes, what      # (synchronises: the kernel has returned)
+            assert status() == 0, what
+            nan = torch.isnan(bad.float())      # the last stage's rows, or all where they feed a second product; no row is silently wrong
+            assert nan.any() and torch.equal(bad[~nan].view(torch.int16), good[~nan].view(torch.int16)), what
+            assert limits(2000, 64) == 0        # every stage
+            bad = call().clone()
+            assert status() in codes, what
+            assert torch.isnan(bad.float()).all(), what
+        finally:
+            limits(0, 0)
+        again = call()
+        torch.cuda.synchronize()
+        assert torch.equal(again.view(torch.int16), good.view(torch.int16)) and status() == 0, what
