@@ -71,6 +71,8 @@ int sm_count() {
     return cached[dev];
 }
 
+// Per function and device, once: `bytes` is the most that any shape needs.  (With the bytes of the call, two threads with
+// different numbers of experts could leave the smaller of the two set.)
 template <class Kernel>
 cudaError_t allow_smem(Kernel kernel, size_t bytes, int (&done)[64]) {
     int dev = 0;
@@ -297,9 +299,9 @@ static int moe_forward_impl(int path, const __nv_bfloat16* x, const uint8_t* ban
         qu.act_s = aa.s; qu.n_pairs = P; qu.g = g; qu.mid_q = ws + m.mq; qu.mid_s = ws + m.ms; qu.y = nullptr;
         MoeQGemmArgs qd = qu;
         qd.wa_s = bank_W2_scale; qd.wb_s = nullptr; qd.rows = out_dim; qd.K = hidden; qd.act_s = ws + m.ms; qd.y = y;
-        auto gemms = [&](auto up_kernel, auto down_kernel, uint32_t smem, int (&up_done)[64], int (&down_done)[64]) {
-            if (err == cudaSuccess) err = allow_smem(up_kernel, smem, up_done);
-            if (err == cudaSuccess) err = allow_smem(down_kernel, smem, down_done);
+        auto gemms = [&](auto up_kernel, auto down_kernel, uint32_t smem, uint32_t most, int (&up_done)[64], int (&down_done)[64]) {
+            if (err == cudaSuccess) err = allow_smem(up_kernel, most, up_done);
+            if (err == cudaSuccess) err = allow_smem(down_kernel, most, down_done);
             if (err != cudaSuccess) return;
             launch_k(up_kernel, dim3(grid & ~1), dim3(kQThreads), smem, stream, 2, up_maps, qu);
             stage_mark(stream, 3);
@@ -307,8 +309,10 @@ static int moe_forward_impl(int path, const __nv_bfloat16* x, const uint8_t* ban
             launch_k(down_kernel, dim3(grid & ~1), dim3(kQThreads), smem, stream, 2, down_maps, qd);
         };
         static int up_few[64] = {0}, down_few[64] = {0}, up_most[64] = {0}, down_most[64] = {0};
-        if (few) gemms(moe_gemm_mxf4_kernel<0, 32>, moe_gemm_mxf4_kernel<1, 32>, MoeQShape<32>::smem(n_experts), up_few, down_few);
-        else gemms(moe_gemm_mxf4_kernel<0, kQTok>, moe_gemm_mxf4_kernel<1, kQTok>, MoeQShape<kQTok>::smem(n_experts), up_most, down_most);
+        if (few) gemms(moe_gemm_mxf4_kernel<0, 32>, moe_gemm_mxf4_kernel<1, 32>, MoeQShape<32>::smem(n_experts),
+                       MoeQShape<32>::smem(kMoeMaxExperts), up_few, down_few);
+        else gemms(moe_gemm_mxf4_kernel<0, kQTok>, moe_gemm_mxf4_kernel<1, kQTok>, MoeQShape<kQTok>::smem(n_experts),
+                   MoeQShape<kQTok>::smem(kMoeMaxExperts), up_most, down_most);
     } else {
         // ---- fp16 tensor-core path: weights dequantised into tensor memory
         const int blocks = (n_tokens + kActRows - 1) / kActRows;

@@ -124,7 +124,8 @@ static bool ring_enabled() {
     return v == 1;
 }
 
-// Shared-memory opt-in above 48 KB is a per-function, per-device attribute: set it once per device.
+// Shared-memory opt-in above 48 KB is a per-function, per-device attribute: set it once per device, to the most that any
+// shape needs.  (With the bytes of the call, two threads with different shapes could leave the smaller of the two set.)
 template <class Kernel>
 static cudaError_t allow_smem(Kernel kernel, size_t bytes, int (&done)[64]) {
     int dev = 0;
@@ -306,7 +307,7 @@ static int grouped_launch(const GroupedArgs& a, cudaStream_t stream, const char*
         const long long grid = sms < pairs ? sms : pairs;
         row_plan_scales(p, 2, a.K >> 5, a.K >> 5, 2);
         row_plan_finish(p, row_x_bytes(a.K >> 5), (uint32_t)(2 * 4 * ((pairs + grid - 1) / grid) * p.n_slices), 0);
-        cudaError_t err = allow_smem(grouped_gate_stream_kernel, p.smem, gate_done);
+        cudaError_t err = allow_smem(grouped_gate_stream_kernel, kRowSmemMost, gate_done);
         if (err == cudaSuccess)
             err = launch_smem(grouped_gate_stream_kernel, dim3((unsigned)grid), dim3(kRowThreads), p.smem, stream, pdl, a, p);
         if (err != cudaSuccess) {
@@ -326,7 +327,7 @@ static int grouped_launch(const GroupedArgs& a, cudaStream_t stream, const char*
         row_plan_finish(p, (uint32_t)a.E * (a.H >> 5) * 68, (uint32_t)(4 * ((a.O + grid - 1) / grid) * a.E * p.n_slices), 0);
         auto kernel = rpw == 1 ? grouped_down_stream_kernel<1> : rpw == 2 ? grouped_down_stream_kernel<2>
                       : rpw == 3 ? grouped_down_stream_kernel<3> : grouped_down_stream_kernel<4>;
-        cudaError_t err = allow_smem(kernel, p.smem, down_done[rpw - 1]);
+        cudaError_t err = allow_smem(kernel, kRowSmemMost, down_done[rpw - 1]);
         if (err == cudaSuccess)
             err = launch_smem(kernel, dim3((unsigned)grid), dim3(kRowThreads), p.smem, stream, pdl, a, p,
                               stages == 3 ? 1 : 0);
