@@ -40,6 +40,17 @@ const struct { const char* name; void** slot; } kEntries[] = {
 };
 template <class F>
 F fn(void* p) { return reinterpret_cast<F>(p); }
+// The C entry, called as ctypes calls it: other Python threads go on meanwhile (a launch blocks while its queue is full).  The
+// arguments are evaluated before the lock is given up.
+struct Unlocked {
+    PyThreadState* const state = PyEval_SaveThread();
+    ~Unlocked() { PyEval_RestoreThread(state); }
+};
+template <class... Params, class... Args>
+int call(int (*f)(Params...), Args... args) {
+    Unlocked unlocked;
+    return f(args...);
+}
 
 // A CUDA tensor of the given type, or nullptr.
 const Tensor* cuda(PyObject* o, ScalarType type) {
@@ -106,7 +117,7 @@ PyObject* dense_gemv(void* f, const char* what, PyObject* const* a, Py_ssize_t n
     void* y;
     if (a[3] == Py_None) { made = empty({N}, kBf16, x); y = made.mutable_data_ptr(); }
     else y = THPVariable_Unpack(a[3]).mutable_data_ptr();
-    const int rc = fn<int (*)(P, P, P, int, int, int64_t, int64_t, void*, void*)>(f)(
+    const int rc = call(fn<int (*)(P, P, P, int, int, int64_t, int64_t, void*, void*)>(f),
         ptr(x), ptr(w), ptr(s), (int)K, (int)N, w->stride(0), s->stride(0) * (int64_t)s->element_size(), y, stream_of(x));
     if (rc != 0) return failed(what, rc);
     return result(a[3], std::move(made));
@@ -126,7 +137,7 @@ FAST(fp8_gemv_batched) { GUARD(
     ORDINARY(G >= 1 && row == G * K && rows % G == 0 && K % 128 == 0 && (rows / G) % 128 == 0 && s->size(0) == rows / 128 &&
              s->size(1) == K / 128 && w->stride(1) == 1 && s->stride(1) == 1 && x->stride(-1) == 1 && a[4] == Py_None);
     Tensor y = single ? empty({rows}, kBf16, x) : empty({S, rows}, kBf16, x);
-    const int rc = fn<int (*)(P, P, P, int, int, int64_t, int64_t, int, int, int64_t, int64_t, void*, void*)>(entry.fp8_e4m3_gemv_batched)(
+    const int rc = call(fn<int (*)(P, P, P, int, int, int64_t, int64_t, int, int, int64_t, int64_t, void*, void*)>(entry.fp8_e4m3_gemv_batched),
         ptr(x), ptr(w), ptr(s), (int)K, (int)(rows / G), w->stride(0), s->stride(0), (int)G, (int)S,
         S > 1 ? x->stride(0) : G * K, rows, y.mutable_data_ptr(), stream_of(x));
     if (rc != 0) return failed("fp8_e4m3_gemv_batched", rc);
@@ -157,7 +168,7 @@ FAST(fp8_shared_swiglu) { GUARD(
     void* y;
     if (a[4] == Py_None) { made = empty({O}, kBf16, x); y = made.mutable_data_ptr(); }
     else y = THPVariable_Unpack(a[4]).mutable_data_ptr();
-    const int rc = fn<int (*)(P, P, P, P, P, P, P, int, int, int, float, float, void*, void*, void*)>(entry.fp8_e4m3_shared_swiglu_m1)(
+    const int rc = call(fn<int (*)(P, P, P, P, P, P, P, int, int, int, float, float, void*, void*, void*)>(entry.fp8_e4m3_shared_swiglu_m1),
         ptr(x), ptr(w1), ptr(s1), ptr(w3), ptr(s3), ptr(w2), ptr(s2), (int)K, (int)H, (int)O, (float)lg, (float)lu, y,
         ws.mutable_data_ptr(), stream_of(x));
     if (rc != 0) return failed("fp8_e4m3_shared_swiglu_m1", rc);
@@ -202,7 +213,7 @@ FAST(grouped_gemv) { GUARD(
     void *y, *w;
     ORDINARY(take(a[5], e.O, kBf16, x, out, y));
     ORDINARY(take(a[6], (int64_t)fn<size_t (*)(int, int, int)>(entry.mxfp4_grouped_workspace_bytes)((int)e.E, (int)e.H, (int)e.O), kByte, x, ws, w));
-    const int rc = fn<int (*)(P, P, P, P, P, P, P, P, int, int, int, int, void*, void*, void*)>(entry.mxfp4_grouped_gemv_topk)(
+    const int rc = call(fn<int (*)(P, P, P, P, P, P, P, P, int, int, int, int, void*, void*, void*)>(entry.mxfp4_grouped_gemv_topk),
         ptr(x), ptr(e.p1), ptr(e.p3), ptr(e.p2), ptr(e.s1), ptr(e.s3), ptr(e.s2), ptr(r), (int)x->numel(), (int)e.H, (int)e.O,
         (int)e.E, y, w, stream_of(x));
     if (rc != 0) return failed("mxfp4_grouped_gemv_topk", rc);
@@ -220,7 +231,7 @@ FAST(grouped_gemv_ids) { GUARD(
     const int k = (int)ids->numel();
     ORDINARY(take(a[4], e.O, kBf16, x, out, y));
     ORDINARY(take(a[5], (int64_t)fn<size_t (*)(int, int, int)>(entry.mxfp4_grouped_workspace_bytes)(k, (int)e.H, (int)e.O), kByte, x, ws, w));
-    const int rc = fn<int (*)(P, P, P, P, P, P, P, P, P, int, int, int, int, void*, void*, int, void*)>(entry.mxfp4_grouped_gemv_topk_ids_stages)(
+    const int rc = call(fn<int (*)(P, P, P, P, P, P, P, P, P, int, int, int, int, void*, void*, int, void*)>(entry.mxfp4_grouped_gemv_topk_ids_stages),
         ptr(x), ptr(e.p1), ptr(e.p3), ptr(e.p2), ptr(e.s1), ptr(e.s3), ptr(e.s2), ptr(ids), ptr(r), (int)x->numel(), (int)e.H,
         (int)e.O, k, y, w, (int)PyLong_AsLong(a[6]), stream_of(x));
     if (rc != 0) return failed("mxfp4_grouped_gemv_topk_ids", rc);
@@ -241,7 +252,7 @@ FAST(route_topk) { GUARD(
     ORDINARY((a[5] == Py_None || THPVariable_Check(a[5])) && (a[6] == Py_None || THPVariable_Check(a[6])));
     ids = a[5] == Py_None ? empty({T, k}, kI32, l) : THPVariable_Unpack(a[5]);
     w = a[6] == Py_None ? empty({T, k}, kF32, l) : THPVariable_Unpack(a[6]);
-    const int rc = fn<int (*)(P, int, int, int, int, float, float, void*, void*, void*)>(entry.mxfp4_moe_route_topk)(
+    const int rc = call(fn<int (*)(P, int, int, int, int, float, float, void*, void*, void*)>(entry.mxfp4_moe_route_topk),
         ptr(l), (int)T, (int)E, (int)k, func, (float)eps, (float)scaling, ids.mutable_data_ptr(), w.mutable_data_ptr(), stream_of(l));
     if (rc != 0) return failed("mxfp4_moe_route_topk", rc);
     PyObject* pair = PyTuple_New(2);
@@ -264,7 +275,7 @@ FAST(decode_layer) { GUARD(
     void *y, *w;
     ORDINARY(k > 0 && take(a[7], e.O, kBf16, x, out, y));
     ORDINARY(take(a[8], (int64_t)fn<size_t (*)(int, int, int)>(entry.mxfp4_moe_decode_workspace_bytes)(k, (int)e.H, (int)e.O), kByte, x, ws, w));
-    const int rc = fn<int (*)(P, P, P, P, P, P, P, P, int, int, float, float, int, int, int, int, void*, void*, void*)>(entry.mxfp4_moe_decode_layer)(
+    const int rc = call(fn<int (*)(P, P, P, P, P, P, P, P, int, int, float, float, int, int, int, int, void*, void*, void*)>(entry.mxfp4_moe_decode_layer),
         ptr(x), ptr(e.p1), ptr(e.p3), ptr(e.p2), ptr(e.s1), ptr(e.s3), ptr(e.s2), ptr(l), (int)e.E, func, (float)eps, (float)scaling,
         (int)x->numel(), (int)e.H, (int)e.O, k, y, w, stream_of(x));
     if (rc != 0) return failed("mxfp4_moe_decode_layer", rc);
@@ -294,11 +305,11 @@ FAST(moe_forward) { GUARD(
     const int path = (int)PyLong_AsLong(a[6]);
     int rc;
     if (path < 0)
-        rc = fn<int (*)(P, P, P, P, P, P, P, P, P, int, int, int, int, int, int, void*, void*, void*)>(entry.mxfp4_moe_forward)(
+        rc = call(fn<int (*)(P, P, P, P, P, P, P, P, P, int, int, int, int, int, int, void*, void*, void*)>(entry.mxfp4_moe_forward),
             ptr(x), ptr(e.p1), ptr(e.p3), ptr(e.p2), ptr(e.s1), ptr(e.s3), ptr(e.s2), ptr(ids), ptr(w), (int)T, (int)e.E, (int)K,
             (int)e.H, (int)e.O, (int)k, y, wp, stream_of(x));
     else
-        rc = fn<int (*)(int, P, P, P, P, P, P, P, P, P, int, int, int, int, int, int, void*, void*, void*)>(entry.mxfp4_moe_forward_path)(
+        rc = call(fn<int (*)(int, P, P, P, P, P, P, P, P, P, int, int, int, int, int, int, void*, void*, void*)>(entry.mxfp4_moe_forward_path),
             path, ptr(x), ptr(e.p1), ptr(e.p3), ptr(e.p2), ptr(e.s1), ptr(e.s3), ptr(e.s2), ptr(ids), ptr(w), (int)T, (int)e.E,
             (int)K, (int)e.H, (int)e.O, (int)k, y, wp, stream_of(x));
     if (rc != 0) return failed("mxfp4_moe_forward", rc);
