@@ -2,14 +2,15 @@
 // entry, for the common case of well-formed CUDA tensors on the current stream.
 //
 // A call through ctypes with its checks in Python took 17 us of host time, more than the kernel of every dense operator;
-// this takes about 3 (most of it the launch itself).  A function returns None when anything is out of the ordinary (another
-// device, a stride, a shape that does not fit, an explicit stream): the caller then goes through the checks in Python, which
-// name what is wrong, or copy what may be copied.  Entry addresses come from the ctypes-loaded libraries (bind), so the
+// this takes about 3 (most of it the launch itself).  A function returns None when anything is out of the ordinary (tensors of
+// several devices, a stride, a shape that does not fit, an explicit stream): the caller then goes through the checks in Python,
+// which name what is wrong, or copy what may be copied.  Entry addresses come from the ctypes-loaded libraries (bind), so the
 // environment overrides of the library paths hold here too.
 #include <Python.h>
 
 #include <ATen/ATen.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
@@ -65,6 +66,25 @@ const Tensor* dense(PyObject* o, ScalarType type) {
 bool shape(const Tensor& t, std::initializer_list<int64_t> want) {
     return t.sizes() == at::IntArrayRef(want);
 }
+// All on the device of the first one.
+bool together(std::initializer_list<const Tensor*> tensors) {
+    const auto device = (*tensors.begin())->device();
+    for (const Tensor* t : tensors)
+        if (t->device() != device) return false;
+    return true;
+}
+// An optional output or workspace: on that device, or not on a GPU at all (mapped host memory, where an operator takes it).
+bool reachable(PyObject* given, const Tensor* like) {
+    if (given == Py_None) return true;
+    if (!THPVariable_Check(given)) return false;
+    const Tensor& t = THPVariable_Unpack(given);
+    return !t.is_cuda() || t.device() == like->device();
+}
+// Allocation, stream and launch on the device of the tensors, whichever is current.
+struct OnDevice {
+    c10::cuda::CUDAGuard guard;
+    explicit OnDevice(const Tensor* t) : guard(t->device()) {}
+};
 P ptr(const Tensor* t) { return t->const_data_ptr(); }
 void* stream_of(const Tensor* t) { return c10::cuda::getCurrentCUDAStream(t->device().index()).stream(); }
 Tensor empty(at::IntArrayRef size, ScalarType type, const Tensor* like) {
@@ -99,10 +119,10 @@ FAST(bind) {
 }
 
 // A caller's optional output vector of `rows` bf16 values: None, or one that fits.
-bool good_out(PyObject* o, std::initializer_list<int64_t> want) {
+bool good_out(PyObject* o, std::initializer_list<int64_t> want, const Tensor* like) {
     if (o == Py_None) return true;
     const Tensor* t = dense(o, kBf16);
-    return t && shape(*t, want);
+    return t && shape(*t, want) && t->device() == like->device();
 }
 
 PyObject* dense_gemv(void* f, const char* what, PyObject* const* a, Py_ssize_t n, int64_t per_block_k, int64_t tile, ScalarType scale_type) {
@@ -112,7 +132,8 @@ PyObject* dense_gemv(void* f, const char* what, PyObject* const* a, Py_ssize_t n
     const int64_t K = x->size(0), N = w->size(0);
     const bool fp4 = tile == 1;
     ORDINARY(K % per_block_k == 0 && N % tile == 0 && w->size(1) == (fp4 ? K / 2 : K) && s->size(0) == N / tile &&
-             s->size(1) == K / per_block_k && w->stride(1) == 1 && s->stride(1) == 1 && good_out(a[3], {N}));
+             s->size(1) == K / per_block_k && w->stride(1) == 1 && s->stride(1) == 1 && together({x, w, s}) && good_out(a[3], {N}, x));
+    OnDevice here(x);
     Tensor made;
     void* y;
     if (a[3] == Py_None) { made = empty({N}, kBf16, x); y = made.mutable_data_ptr(); }
@@ -135,7 +156,8 @@ FAST(fp8_gemv_batched) { GUARD(
     const bool single = x->dim() == 1;
     const int64_t S = single ? 1 : x->size(0), row = single ? x->size(0) : x->size(1);
     ORDINARY(G >= 1 && row == G * K && rows % G == 0 && K % 128 == 0 && (rows / G) % 128 == 0 && s->size(0) == rows / 128 &&
-             s->size(1) == K / 128 && w->stride(1) == 1 && s->stride(1) == 1 && x->stride(-1) == 1 && a[4] == Py_None);
+             s->size(1) == K / 128 && w->stride(1) == 1 && s->stride(1) == 1 && x->stride(-1) == 1 && a[4] == Py_None && together({x, w, s}));
+    OnDevice here(x);
     Tensor y = single ? empty({rows}, kBf16, x) : empty({S, rows}, kBf16, x);
     const int rc = call(fn<int (*)(P, P, P, int, int, int64_t, int64_t, int, int, int64_t, int64_t, void*, void*)>(entry.fp8_e4m3_gemv_batched),
         ptr(x), ptr(w), ptr(s), (int)K, (int)(rows / G), w->stride(0), s->stride(0), (int)G, (int)S,
@@ -153,7 +175,8 @@ FAST(fp8_shared_swiglu) { GUARD(
     ORDINARY(w1 && w3 && w2 && s1 && s3 && s2 && x && x->dim() == 1 && w1->dim() == 2 && w2->dim() == 2);
     const int64_t K = x->size(0), H = w1->size(0), O = w2->size(0);
     ORDINARY(shape(*w1, {H, K}) && shape(*w3, {H, K}) && shape(*w2, {O, H}) && shape(*s1, {H / 128, K / 128}) &&
-             shape(*s3, {H / 128, K / 128}) && shape(*s2, {O / 128, H / 128}) && good_out(a[4], {O}));
+             shape(*s3, {H / 128, K / 128}) && shape(*s2, {O / 128, H / 128}) && together({x, w1, w3, w2, s1, s3, s2}) && good_out(a[4], {O}, x) && reachable(a[5], x));
+    OnDevice here(x);
     const double lg = PyFloat_AsDouble(a[2]), lu = PyFloat_AsDouble(a[3]);
     if (PyErr_Occurred()) return nullptr;
     const size_t need = fn<size_t (*)(int)>(entry.fp8_e4m3_shared_swiglu_workspace_bytes)((int)H);
@@ -161,7 +184,6 @@ FAST(fp8_shared_swiglu) { GUARD(
     if (a[5] == Py_None) {
         ws = empty({(int64_t)need}, kByte, x);
     } else {
-        ORDINARY(THPVariable_Check(a[5]));
         ws = THPVariable_Unpack(a[5]);
         ORDINARY(ws.is_cuda() && ws.nbytes() >= need);
     }
@@ -178,8 +200,8 @@ FAST(fp8_shared_swiglu) { GUARD(
 struct Experts {
     const Tensor *p1, *p3, *p2, *s1, *s3, *s2;
     int64_t E, H, O;
-    bool ok(int64_t K) {
-        if (!p1 || !p3 || !p2 || !s1 || !s3 || !s2 || p1->dim() != 3 || p2->dim() != 3) return false;
+    bool ok(const Tensor* x, int64_t K) {
+        if (!p1 || !p3 || !p2 || !s1 || !s3 || !s2 || p1->dim() != 3 || p2->dim() != 3 || !together({x, p1, p3, p2, s1, s3, s2})) return false;
         E = p1->size(0); H = p1->size(1); O = p2->size(1);
         return shape(*p1, {E, H, K / 2}) && shape(*p3, {E, H, K / 2}) && shape(*s1, {E, H, K / 32}) && shape(*s3, {E, H, K / 32}) &&
                shape(*p2, {E, O, H / 2}) && shape(*s2, {E, O, H / 32});
@@ -189,13 +211,10 @@ Experts bank_of(PyObject* d) {
     return {dense(get(d, kW1p), kByte), dense(get(d, kW3p), kByte), dense(get(d, kW2p), kByte), dense(get(d, kW1s), kByte),
             dense(get(d, kW3s), kByte), dense(get(d, kW2s), kByte), 0, 0, 0};
 }
-// Output and workspace as the operators take them: None = allocate; a given tensor is used as it is.
-bool take(PyObject* o, int64_t n, ScalarType type, const Tensor* like, Tensor& keep, void*& p) {
-    if (o == Py_None) keep = empty({n}, type, like);
-    else if (THPVariable_Check(o)) keep = THPVariable_Unpack(o);
-    else return false;
-    p = keep.mutable_data_ptr();
-    return true;
+// Output and workspace as the operators take them: None = allocate; a given (reachable) tensor is used as it is.
+void* take(PyObject* o, int64_t n, ScalarType type, const Tensor* like, Tensor& keep) {
+    keep = o == Py_None ? empty({n}, type, like) : THPVariable_Unpack(o);
+    return keep.mutable_data_ptr();
 }
 int score_of(PyObject* o) {
     if (!PyUnicode_Check(o)) return -1;
@@ -208,11 +227,11 @@ FAST(grouped_gemv) { GUARD(
     Experts e = {dense(get(a[0], kPacked), kByte), dense(get(a[1], kPacked), kByte), dense(get(a[2], kPacked), kByte),
                  dense(get(a[0], kScale), kByte), dense(get(a[1], kScale), kByte), dense(get(a[2], kScale), kByte), 0, 0, 0};
     const Tensor *x = dense(a[3], kBf16), *r = dense(a[4], kF32);
-    ORDINARY(x && r && e.ok(x->numel()) && shape(*r, {e.E}));
+    ORDINARY(x && r && e.ok(x, x->numel()) && shape(*r, {e.E}) && together({x, r}) && reachable(a[5], x) && reachable(a[6], x));
+    OnDevice here(x);
     Tensor out, ws;
-    void *y, *w;
-    ORDINARY(take(a[5], e.O, kBf16, x, out, y));
-    ORDINARY(take(a[6], (int64_t)fn<size_t (*)(int, int, int)>(entry.mxfp4_grouped_workspace_bytes)((int)e.E, (int)e.H, (int)e.O), kByte, x, ws, w));
+    void* y = take(a[5], e.O, kBf16, x, out);
+    void* w = take(a[6], (int64_t)fn<size_t (*)(int, int, int)>(entry.mxfp4_grouped_workspace_bytes)((int)e.E, (int)e.H, (int)e.O), kByte, x, ws);
     const int rc = call(fn<int (*)(P, P, P, P, P, P, P, P, int, int, int, int, void*, void*, void*)>(entry.mxfp4_grouped_gemv_topk),
         ptr(x), ptr(e.p1), ptr(e.p3), ptr(e.p2), ptr(e.s1), ptr(e.s3), ptr(e.s2), ptr(r), (int)x->numel(), (int)e.H, (int)e.O,
         (int)e.E, y, w, stream_of(x));
@@ -225,12 +244,12 @@ FAST(grouped_gemv_ids) { GUARD(
     ORDINARY(n == 7 && entry.mxfp4_grouped_gemv_topk_ids_stages && entry.mxfp4_grouped_workspace_bytes && PyLong_Check(a[6]));
     Experts e = bank_of(a[0]);
     const Tensor *ids = dense(a[1], kI32), *x = dense(a[2], kBf16), *r = dense(a[3], kF32);
-    ORDINARY(ids && x && r && e.ok(x->numel()) && shape(*r, {ids->numel()}));
+    ORDINARY(ids && x && r && e.ok(x, x->numel()) && shape(*r, {ids->numel()}) && together({x, ids, r}) && reachable(a[4], x) && reachable(a[5], x));
+    OnDevice here(x);
     Tensor out, ws;
-    void *y, *w;
     const int k = (int)ids->numel();
-    ORDINARY(take(a[4], e.O, kBf16, x, out, y));
-    ORDINARY(take(a[5], (int64_t)fn<size_t (*)(int, int, int)>(entry.mxfp4_grouped_workspace_bytes)(k, (int)e.H, (int)e.O), kByte, x, ws, w));
+    void* y = take(a[4], e.O, kBf16, x, out);
+    void* w = take(a[5], (int64_t)fn<size_t (*)(int, int, int)>(entry.mxfp4_grouped_workspace_bytes)(k, (int)e.H, (int)e.O), kByte, x, ws);
     const int rc = call(fn<int (*)(P, P, P, P, P, P, P, P, P, int, int, int, int, void*, void*, int, void*)>(entry.mxfp4_grouped_gemv_topk_ids_stages),
         ptr(x), ptr(e.p1), ptr(e.p3), ptr(e.p2), ptr(e.s1), ptr(e.s3), ptr(e.s2), ptr(ids), ptr(r), (int)x->numel(), (int)e.H,
         (int)e.O, k, y, w, (int)PyLong_AsLong(a[6]), stream_of(x));
@@ -249,7 +268,8 @@ FAST(route_topk) { GUARD(
     const double eps = PyFloat_AsDouble(a[3]), scaling = PyFloat_AsDouble(a[4]);
     if (PyErr_Occurred()) return nullptr;
     Tensor ids; Tensor w;
-    ORDINARY((a[5] == Py_None || THPVariable_Check(a[5])) && (a[6] == Py_None || THPVariable_Check(a[6])));
+    ORDINARY(reachable(a[5], l) && reachable(a[6], l));
+    OnDevice here(l);
     ids = a[5] == Py_None ? empty({T, k}, kI32, l) : THPVariable_Unpack(a[5]);
     w = a[6] == Py_None ? empty({T, k}, kF32, l) : THPVariable_Unpack(a[6]);
     const int rc = call(fn<int (*)(P, int, int, int, int, float, float, void*, void*, void*)>(entry.mxfp4_moe_route_topk),
@@ -267,14 +287,15 @@ FAST(decode_layer) { GUARD(
     Experts e = bank_of(a[0]);
     const Tensor *l = dense(a[1], kF32), *x = dense(a[2], kBf16);
     const int func = score_of(a[4]);
-    ORDINARY(l && x && func >= 0 && e.ok(x->numel()) && l->numel() == e.E);
+    ORDINARY(l && x && func >= 0 && e.ok(x, x->numel()) && l->numel() == e.E && together({x, l}) && reachable(a[7], x) && reachable(a[8], x));
     const int k = (int)PyLong_AsLong(a[3]);
     const double eps = PyFloat_AsDouble(a[5]), scaling = PyFloat_AsDouble(a[6]);
     if (PyErr_Occurred()) return nullptr;
+    ORDINARY(k > 0);
+    OnDevice here(x);
     Tensor out, ws;
-    void *y, *w;
-    ORDINARY(k > 0 && take(a[7], e.O, kBf16, x, out, y));
-    ORDINARY(take(a[8], (int64_t)fn<size_t (*)(int, int, int)>(entry.mxfp4_moe_decode_workspace_bytes)(k, (int)e.H, (int)e.O), kByte, x, ws, w));
+    void* y = take(a[7], e.O, kBf16, x, out);
+    void* w = take(a[8], (int64_t)fn<size_t (*)(int, int, int)>(entry.mxfp4_moe_decode_workspace_bytes)(k, (int)e.H, (int)e.O), kByte, x, ws);
     const int rc = call(fn<int (*)(P, P, P, P, P, P, P, P, int, int, float, float, int, int, int, int, void*, void*, void*)>(entry.mxfp4_moe_decode_layer),
         ptr(x), ptr(e.p1), ptr(e.p3), ptr(e.p2), ptr(e.s1), ptr(e.s3), ptr(e.s2), ptr(l), (int)e.E, func, (float)eps, (float)scaling,
         (int)x->numel(), (int)e.H, (int)e.O, k, y, w, stream_of(x));
@@ -287,18 +308,18 @@ FAST(moe_forward) { GUARD(
     ORDINARY(n == 7 && entry.mxfp4_moe_forward && entry.mxfp4_moe_forward_path && entry.mxfp4_moe_forward_workspace_bytes && PyLong_Check(a[6]));
     Experts e = bank_of(a[0]);
     const Tensor *x = dense(a[1], kBf16), *ids = dense(a[2], kI32), *w = dense(a[3], kF32);
-    ORDINARY(x && ids && w && x->dim() == 2 && ids->dim() == 2 && e.ok(x->size(1)));
+    ORDINARY(x && ids && w && x->dim() == 2 && ids->dim() == 2 && e.ok(x, x->size(1)) && together({x, ids, w}) && reachable(a[4], x) && reachable(a[5], x));
+    OnDevice here(x);
     const int64_t T = x->size(0), K = x->size(1), k = ids->size(1);
     ORDINARY(shape(*ids, {T, k}) && shape(*w, {T, k}));
     Tensor out, ws;
     void *y, *wp;
     if (a[4] == Py_None) { out = empty({T, e.O}, kBf16, x); y = out.mutable_data_ptr(); }
-    else { ORDINARY(THPVariable_Check(a[4])); y = THPVariable_Unpack(a[4]).mutable_data_ptr(); }
+    else y = THPVariable_Unpack(a[4]).mutable_data_ptr();
     if (a[5] == Py_None) {
         const size_t need = fn<size_t (*)(int, int, int, int, int, int)>(entry.mxfp4_moe_forward_workspace_bytes)((int)T, (int)k, (int)K, (int)e.H, (int)e.O, (int)e.E);
         ws = empty({(int64_t)need}, kByte, x);
     } else {
-        ORDINARY(THPVariable_Check(a[5]));
         ws = THPVariable_Unpack(a[5]);
     }
     wp = ws.mutable_data_ptr();

@@ -111,6 +111,23 @@ def ptr(t) -> c_void_p:
     return c_void_p(t.data_ptr())
 
 
+BANK = ("w1p", "w3p", "w2p", "w1s", "w3s", "w2s")
+
+
+def elsewhere(x, **tensors):
+    """Name of the first tensor that lives on another GPU than x, or None (None and host tensors are passed over)."""
+    for name, t in tensors.items():
+        if t is not None and t.is_cuda and t.device != x.device:
+            return name
+    return None
+
+
+def on_device(x):
+    """Context in which the GPU of x is the current one: a launch goes to the current device, whatever its stream."""
+    import torch
+    return torch.cuda.device(x.device)
+
+
 def stream_ptr(device, stream=None) -> c_void_p:
     import torch
     s = stream if stream is not None else torch.cuda.current_stream(device)

@@ -24,6 +24,7 @@ def _require(cond: bool, msg: str) -> None:
 
 def _run(symbol: str, scale_dtype: torch.dtype, W_fp8, W_scale, x, out, stream):
     _require(W_fp8.is_cuda and W_scale.is_cuda and x.is_cuda, "all tensors must be on CUDA device")
+    _require(_capi.elsewhere(x, W_fp8=W_fp8, W_scale=W_scale, out=out) is None, "all tensors must be on one CUDA device")
     _require(W_fp8.dtype == torch.uint8, f"W_fp8 must be uint8 (raw E4M3), got {W_fp8.dtype}")
     _require(W_scale.dtype == scale_dtype, f"W_scale must be {scale_dtype}, got {W_scale.dtype}")
     _require(x.dtype == torch.bfloat16, f"x must be bfloat16, got {x.dtype}")
@@ -47,10 +48,11 @@ def _run(symbol: str, scale_dtype: torch.dtype, W_fp8, W_scale, x, out, stream):
         _require(tuple(out.shape) == (N,) and out.dtype == torch.bfloat16 and out.is_cuda and out.is_contiguous(),
                  f"out must be a contiguous cuda bfloat16 [{N}]")
     lib = _capi.load("fp8")
-    rc = getattr(lib, symbol)(_capi.ptr(x), _capi.ptr(W_fp8), _capi.ptr(W_scale), c_int(K), c_int(N),
-                              c_int64(W_fp8.stride(0) * W_fp8.element_size()),
-                              c_int64(W_scale.stride(0) * W_scale.element_size()), _capi.ptr(out),
-                              _capi.stream_ptr(x.device, stream))
+    with _capi.on_device(x):
+        rc = getattr(lib, symbol)(_capi.ptr(x), _capi.ptr(W_fp8), _capi.ptr(W_scale), c_int(K), c_int(N),
+                                  c_int64(W_fp8.stride(0) * W_fp8.element_size()),
+                                  c_int64(W_scale.stride(0) * W_scale.element_size()), _capi.ptr(out),
+                                  _capi.stream_ptr(x.device, stream))
     if rc != 0:
         raise RuntimeError(f"{symbol} returned {rc}")
     return out
@@ -89,6 +91,7 @@ def fp8_e4m3_gemv_batched(W_fp8: torch.Tensor, W_scale: torch.Tensor, x: torch.T
     if done is not None:
         return done
     _require(W_fp8.is_cuda and W_scale.is_cuda and x.is_cuda, "all tensors must be on CUDA device")
+    _require(_capi.elsewhere(x, W_fp8=W_fp8, W_scale=W_scale, out=out) is None, "all tensors must be on one CUDA device")
     _require(W_fp8.dtype == torch.uint8, f"W_fp8 must be uint8 (raw E4M3), got {W_fp8.dtype}")
     _require(W_scale.dtype == torch.uint8, f"W_scale must be uint8 (E8M0), got {W_scale.dtype}")
     _require(x.dtype == torch.bfloat16, f"x must be bfloat16, got {x.dtype}")
@@ -119,11 +122,12 @@ def fp8_e4m3_gemv_batched(W_fp8: torch.Tensor, W_scale: torch.Tensor, x: torch.T
                  f"out must be a cuda bfloat16 {list(shape)} with unit inner stride")
         out2 = out.unsqueeze(0) if single else out
     lib = _capi.load("fp8")
-    rc = lib.fp8_e4m3_gemv_batched(_capi.ptr(xs), _capi.ptr(W_fp8), _capi.ptr(W_scale), c_int(K), c_int(N),
-                                   c_int64(W_fp8.stride(0)), c_int64(W_scale.stride(0)), c_int(n_groups), c_int(S),
-                                   c_int64(xs.stride(0) if S > 1 else n_groups * K),
-                                   c_int64(out2.stride(0) if S > 1 else n_groups * N), _capi.ptr(out2),
-                                   _capi.stream_ptr(x.device, stream))
+    with _capi.on_device(x):
+        rc = lib.fp8_e4m3_gemv_batched(_capi.ptr(xs), _capi.ptr(W_fp8), _capi.ptr(W_scale), c_int(K), c_int(N),
+                                       c_int64(W_fp8.stride(0)), c_int64(W_scale.stride(0)), c_int(n_groups), c_int(S),
+                                       c_int64(xs.stride(0) if S > 1 else n_groups * K),
+                                       c_int64(out2.stride(0) if S > 1 else n_groups * N), _capi.ptr(out2),
+                                       _capi.stream_ptr(x.device, stream))
     if rc != 0:
         raise RuntimeError(f"fp8_e4m3_gemv_batched returned {rc}")
     return out2[0] if single else out2
@@ -146,6 +150,8 @@ def fp8_shared_swiglu(shared: dict, x: torch.Tensor, limit_gate: float = 10.0, l
     for name, t in (("w1", w1), ("w3", w3), ("w2", w2), ("w1s", shared["w1s"]), ("w3s", shared["w3s"]), ("w2s", shared["w2s"])):
         _require(t.is_cuda and t.dtype == torch.uint8 and t.is_contiguous(), f"{name} must be a contiguous cuda uint8 tensor")
     _require(x.is_cuda and x.dtype == torch.bfloat16 and x.dim() == 1 and x.is_contiguous(), "x must be a contiguous cuda bfloat16 [K]")
+    _require(_capi.elsewhere(x, out=out, workspace=workspace, w1=w1, w3=w3, w2=w2, w1s=shared["w1s"], w3s=shared["w3s"],
+                             w2s=shared["w2s"]) is None, "all tensors must be on one CUDA device")
     _require(tuple(w1.shape) == (hidden, K) and tuple(w3.shape) == (hidden, K) and tuple(w2.shape) == (out_dim, hidden),
              "w1 / w3 must be [hidden, K] and w2 [out_dim, hidden]")
     for name, t, rows, cols in (("w1s", shared["w1s"], hidden, K), ("w3s", shared["w3s"], hidden, K), ("w2s", shared["w2s"], out_dim, hidden)):
@@ -159,10 +165,11 @@ def fp8_shared_swiglu(shared: dict, x: torch.Tensor, limit_gate: float = 10.0, l
         out = torch.empty(out_dim, dtype=torch.bfloat16, device=x.device)
     _require(tuple(out.shape) == (out_dim,) and out.dtype == torch.bfloat16 and out.is_cuda and out.is_contiguous(),
              f"out must be a contiguous cuda bfloat16 [{out_dim}]")
-    rc = lib.fp8_e4m3_shared_swiglu_m1(_capi.ptr(x), _capi.ptr(w1), _capi.ptr(shared["w1s"]), _capi.ptr(w3),
-                                       _capi.ptr(shared["w3s"]), _capi.ptr(w2), _capi.ptr(shared["w2s"]), c_int(K),
-                                       c_int(hidden), c_int(out_dim), c_float(limit_gate), c_float(limit_up),
-                                       _capi.ptr(out), _capi.ptr(workspace), _capi.stream_ptr(x.device, stream))
+    with _capi.on_device(x):
+        rc = lib.fp8_e4m3_shared_swiglu_m1(_capi.ptr(x), _capi.ptr(w1), _capi.ptr(shared["w1s"]), _capi.ptr(w3),
+                                           _capi.ptr(shared["w3s"]), _capi.ptr(w2), _capi.ptr(shared["w2s"]), c_int(K),
+                                           c_int(hidden), c_int(out_dim), c_float(limit_gate), c_float(limit_up),
+                                           _capi.ptr(out), _capi.ptr(workspace), _capi.stream_ptr(x.device, stream))
     if rc != 0:
         raise RuntimeError(f"fp8_e4m3_shared_swiglu_m1 returned {rc}")
     return out

@@ -45,6 +45,9 @@ def moe_forward(bank: Dict[str, torch.Tensor], x: torch.Tensor, ids: torch.Tenso
         raise ValueError("ids / weights must be [T, k]")
     if bank["w1p"].shape[2] != K // 2 or bank["w2p"].shape[2] != hidden // 2:
         raise ValueError("bank shapes do not match x")
+    name = _capi.elsewhere(x, ids=ids, weights=weights, out=out, workspace=workspace, **{n: bank[n] for n in _capi.BANK})
+    if name is not None:
+        raise ValueError(f"{name}: on another CUDA device than {x.device}")
     if out is None:
         out = torch.empty(T, out_dim, dtype=torch.bfloat16, device=x.device)
     if workspace is None:
@@ -53,10 +56,8 @@ def moe_forward(bank: Dict[str, torch.Tensor], x: torch.Tensor, ids: torch.Tenso
                                _capi.ptr(bank["w1s"]), _capi.ptr(bank["w3s"]), _capi.ptr(bank["w2s"]), _capi.ptr(ids),
                                _capi.ptr(weights), c_int(T), c_int(E), c_int(K), c_int(hidden), c_int(out_dim), c_int(k),
                                _capi.ptr(out), _capi.ptr(workspace), _capi.stream_ptr(x.device))
-    if path is None:
-        rc = lib.mxfp4_moe_forward(*args)
-    else:
-        rc = lib.mxfp4_moe_forward_path(c_int(code), *args)
+    with _capi.on_device(x):
+        rc = lib.mxfp4_moe_forward(*args) if path is None else lib.mxfp4_moe_forward_path(c_int(code), *args)
     if rc != 0:
         raise RuntimeError(f"mxfp4_moe_forward returned {rc}")
     return out
@@ -69,8 +70,9 @@ def mma_clocks(n_cols: int = 256, scale_copies: int = 0, iters: int = 2000, devi
     device = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
     scratch = torch.zeros(1, dtype=torch.int64, device=device)
     out = ctypes.c_double(0.0)
-    rc = _capi.load("moe").mxfp4_moe_mma_rate(c_int(n_cols), c_int(scale_copies), c_int(iters), _capi.ptr(scratch),
-                                              ctypes.cast(ctypes.byref(out), ctypes.c_void_p), _capi.stream_ptr(device))
+    with _capi.on_device(scratch):
+        rc = _capi.load("moe").mxfp4_moe_mma_rate(c_int(n_cols), c_int(scale_copies), c_int(iters), _capi.ptr(scratch),
+                                                  ctypes.cast(ctypes.byref(out), ctypes.c_void_p), _capi.stream_ptr(device))
     if rc != 0:
         raise RuntimeError(f"mxfp4_moe_mma_rate returned {rc}")
     return float(out.value)

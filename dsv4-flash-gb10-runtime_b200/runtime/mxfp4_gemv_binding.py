@@ -26,6 +26,7 @@ def mxfp4_gemv(W_packed: torch.Tensor, W_scale: torch.Tensor, x: torch.Tensor,
     if done is not None:
         return done
     _require(W_packed.is_cuda and W_scale.is_cuda and x.is_cuda, "all tensors must be on CUDA device")
+    _require(_capi.elsewhere(x, W_packed=W_packed, W_scale=W_scale, out=out) is None, "all tensors must be on one CUDA device")
     _require(W_packed.dtype == torch.uint8, f"W_packed must be uint8, got {W_packed.dtype}")
     _require(W_scale.dtype == torch.uint8, f"W_scale must be uint8, got {W_scale.dtype}")
     _require(x.dtype == torch.bfloat16, f"x must be bfloat16, got {x.dtype}")
@@ -48,9 +49,10 @@ def mxfp4_gemv(W_packed: torch.Tensor, W_scale: torch.Tensor, x: torch.Tensor,
         _require(tuple(out.shape) == (N,) and out.dtype == torch.bfloat16 and out.is_cuda and out.is_contiguous(),
                  f"out must be a contiguous cuda bfloat16 [{N}]")
     lib = _capi.load("mxfp4")
-    rc = lib.mxfp4_gemv_m1(_capi.ptr(x), _capi.ptr(W_packed), _capi.ptr(W_scale), c_int(K), c_int(N),
-                           c_int64(W_packed.stride(0)), c_int64(W_scale.stride(0)), _capi.ptr(out),
-                           _capi.stream_ptr(x.device, stream))
+    with _capi.on_device(x):
+        rc = lib.mxfp4_gemv_m1(_capi.ptr(x), _capi.ptr(W_packed), _capi.ptr(W_scale), c_int(K), c_int(N),
+                               c_int64(W_packed.stride(0)), c_int64(W_scale.stride(0)), _capi.ptr(out),
+                               _capi.stream_ptr(x.device, stream))
     if rc != 0:
         raise RuntimeError(f"mxfp4_gemv_m1 returned {rc}")
     return out

@@ -32,6 +32,12 @@ def _check(t: torch.Tensor, name: str, dtype: torch.dtype) -> None:
         raise ValueError(f"{name}: tensor must be contiguous")
 
 
+def _check_device(x: torch.Tensor, **tensors) -> None:
+    name = _capi.elsewhere(x, **tensors)
+    if name is not None:
+        raise ValueError(f"{name}: on another CUDA device than {x.device}")
+
+
 def _check_expert_set(W1, W3, W2, K_in):
     for name, w in (("W1", W1), ("W3", W3), ("W2", W2)):
         if "packed" not in w or "scale" not in w:
@@ -70,15 +76,18 @@ def mxfp4_grouped_gemv(W1: Dict[str, torch.Tensor], W3: Dict[str, torch.Tensor],
     n_exp, hidden, out_dim = _check_expert_set(W1, W3, W2, K_in)
     if tuple(r.shape) != (n_exp,):
         raise ValueError(f"r shape {tuple(r.shape)} != ({n_exp},)")
+    _check_device(x, r=r, out=out, workspace=workspace, W1_scale=W1["scale"], W3_scale=W3["scale"], W2_scale=W2["scale"],
+                  W1_packed=W1["packed"], W3_packed=W3["packed"], W2_packed=W2["packed"])
     if out is None:
         out = torch.empty(out_dim, dtype=torch.bfloat16, device=x.device)
     if workspace is None:
         workspace = torch.empty(workspace_bytes(n_exp, hidden, out_dim), dtype=torch.uint8, device=x.device)
-    rc = lib.mxfp4_grouped_gemv_topk(
-        _capi.ptr(x), _capi.ptr(W1["packed"]), _capi.ptr(W3["packed"]), _capi.ptr(W2["packed"]),
-        _capi.ptr(W1["scale"]), _capi.ptr(W3["scale"]), _capi.ptr(W2["scale"]), _capi.ptr(r),
-        c_int(K_in), c_int(hidden), c_int(out_dim), c_int(n_exp), _capi.ptr(out), _capi.ptr(workspace),
-        _capi.stream_ptr(x.device))
+    with _capi.on_device(x):
+        rc = lib.mxfp4_grouped_gemv_topk(
+            _capi.ptr(x), _capi.ptr(W1["packed"]), _capi.ptr(W3["packed"]), _capi.ptr(W2["packed"]),
+            _capi.ptr(W1["scale"]), _capi.ptr(W3["scale"]), _capi.ptr(W2["scale"]), _capi.ptr(r),
+            c_int(K_in), c_int(hidden), c_int(out_dim), c_int(n_exp), _capi.ptr(out), _capi.ptr(workspace),
+            _capi.stream_ptr(x.device))
     if rc != 0:
         raise RuntimeError(f"mxfp4_grouped_gemv_topk returned {rc}")
     return out
@@ -101,12 +110,15 @@ def mxfp4_grouped_gemv_static(W1: Dict[str, torch.Tensor], W3: Dict[str, torch.T
     if tuple(r.shape) != (n_exp,):
         raise ValueError(f"r shape {tuple(r.shape)} != ({n_exp},)")
     _check(out, "out", torch.bfloat16)
+    _check_device(x, r=r, out=out, W1_scale=W1["scale"], W3_scale=W3["scale"], W2_scale=W2["scale"],
+                  W1_packed=W1["packed"], W3_packed=W3["packed"], W2_packed=W2["packed"])
     if tuple(out.shape) != (out_dim,):
         raise ValueError(f"out shape {tuple(out.shape)} != ({out_dim},)")
-    rc = lib.mxfp4_grouped_gemv_topk_static(
-        _capi.ptr(x), _capi.ptr(W1["packed"]), _capi.ptr(W3["packed"]), _capi.ptr(W2["packed"]),
-        _capi.ptr(W1["scale"]), _capi.ptr(W3["scale"]), _capi.ptr(W2["scale"]), _capi.ptr(r),
-        c_int(K_in), c_int(hidden), c_int(out_dim), c_int(n_exp), _capi.ptr(out), _capi.stream_ptr(x.device))
+    with _capi.on_device(x):
+        rc = lib.mxfp4_grouped_gemv_topk_static(
+            _capi.ptr(x), _capi.ptr(W1["packed"]), _capi.ptr(W3["packed"]), _capi.ptr(W2["packed"]),
+            _capi.ptr(W1["scale"]), _capi.ptr(W3["scale"]), _capi.ptr(W2["scale"]), _capi.ptr(r),
+            c_int(K_in), c_int(hidden), c_int(out_dim), c_int(n_exp), _capi.ptr(out), _capi.stream_ptr(x.device))
     if rc != 0:
         raise RuntimeError(f"mxfp4_grouped_gemv_topk_static returned {rc}")
     return out
@@ -136,15 +148,17 @@ def mxfp4_grouped_gemv_ids(bank: Dict[str, torch.Tensor], ids: torch.Tensor, x: 
             raise ValueError(f"r shape {tuple(r.shape)} != ({n_exp},)")
     else:
         hidden, out_dim = bank["w1p"].shape[1], bank["w2p"].shape[1]
+    _check_device(x, ids=ids, r=r, out=out, workspace=workspace, **{n: bank[n] for n in _capi.BANK})
     if out is None:
         out = torch.empty(out_dim, dtype=torch.bfloat16, device=x.device)
     if workspace is None:
         workspace = torch.empty(workspace_bytes(n_exp, hidden, out_dim), dtype=torch.uint8, device=x.device)
-    rc = lib.mxfp4_grouped_gemv_topk_ids_stages(
-        _capi.ptr(x), _capi.ptr(bank["w1p"]), _capi.ptr(bank["w3p"]), _capi.ptr(bank["w2p"]),
-        _capi.ptr(bank["w1s"]), _capi.ptr(bank["w3s"]), _capi.ptr(bank["w2s"]), _capi.ptr(ids), _capi.ptr(r),
-        c_int(K_in), c_int(hidden), c_int(out_dim), c_int(n_exp), _capi.ptr(out), _capi.ptr(workspace),
-        c_int(stage_mask), _capi.stream_ptr(x.device))
+    with _capi.on_device(x):
+        rc = lib.mxfp4_grouped_gemv_topk_ids_stages(
+            _capi.ptr(x), _capi.ptr(bank["w1p"]), _capi.ptr(bank["w3p"]), _capi.ptr(bank["w2p"]),
+            _capi.ptr(bank["w1s"]), _capi.ptr(bank["w3s"]), _capi.ptr(bank["w2s"]), _capi.ptr(ids), _capi.ptr(r),
+            c_int(K_in), c_int(hidden), c_int(out_dim), c_int(n_exp), _capi.ptr(out), _capi.ptr(workspace),
+            c_int(stage_mask), _capi.stream_ptr(x.device))
     if rc != 0:
         raise RuntimeError(f"mxfp4_grouped_gemv_topk_ids returned {rc}")
     return out
@@ -163,14 +177,16 @@ def moe_route_topk(logits: torch.Tensor, k: int = 6, score_func: str = "sqrt_sof
         return done
     lib = _capi.load("grouped")
     _check(logits, "logits", torch.float32)
+    _check_device(logits, ids_out=ids_out, w_out=w_out)
     if logits.dim() == 1:
         logits = logits.unsqueeze(0)
     T, E = logits.shape
     func = {"softmax": 0, "sqrt_softplus": 1}[score_func]
     ids = ids_out if ids_out is not None else torch.empty(T, k, dtype=torch.int32, device=logits.device)
     w = w_out if w_out is not None else torch.empty(T, k, dtype=torch.float32, device=logits.device)
-    rc = lib.mxfp4_moe_route_topk(_capi.ptr(logits), c_int(T), c_int(E), c_int(k), c_int(func), c_float(eps),
-                                  c_float(scaling), _capi.ptr(ids), _capi.ptr(w), _capi.stream_ptr(logits.device))
+    with _capi.on_device(logits):
+        rc = lib.mxfp4_moe_route_topk(_capi.ptr(logits), c_int(T), c_int(E), c_int(k), c_int(func), c_float(eps),
+                                      c_float(scaling), _capi.ptr(ids), _capi.ptr(w), _capi.stream_ptr(logits.device))
     if rc != 0:
         raise RuntimeError(f"mxfp4_moe_route_topk returned {rc}")
     return ids, w
@@ -197,16 +213,18 @@ def moe_decode_layer(bank: Dict[str, torch.Tensor], logits: torch.Tensor, x: tor
                           {"packed": bank["w2p"], "scale": bank["w2s"]}, K_in)
         if bank["w1p"].shape[0] != n_experts:
             raise ValueError(f"bank holds {bank['w1p'].shape[0]} experts, logits {n_experts}")
+    _check_device(x, logits=logits, out=out, workspace=workspace, **{n: bank[n] for n in _capi.BANK})
     if out is None:
         out = torch.empty(out_dim, dtype=torch.bfloat16, device=x.device)
     if workspace is None:
         workspace = torch.empty(decode_workspace_bytes(k, hidden, out_dim), dtype=torch.uint8, device=x.device)
     func = {"softmax": 0, "sqrt_softplus": 1}[score_func]
-    rc = lib.mxfp4_moe_decode_layer(
-        _capi.ptr(x), _capi.ptr(bank["w1p"]), _capi.ptr(bank["w3p"]), _capi.ptr(bank["w2p"]), _capi.ptr(bank["w1s"]),
-        _capi.ptr(bank["w3s"]), _capi.ptr(bank["w2s"]), _capi.ptr(logits), c_int(n_experts), c_int(func),
-        c_float(eps), c_float(scaling), c_int(K_in), c_int(hidden), c_int(out_dim), c_int(k), _capi.ptr(out),
-        _capi.ptr(workspace), _capi.stream_ptr(x.device))
+    with _capi.on_device(x):
+        rc = lib.mxfp4_moe_decode_layer(
+            _capi.ptr(x), _capi.ptr(bank["w1p"]), _capi.ptr(bank["w3p"]), _capi.ptr(bank["w2p"]), _capi.ptr(bank["w1s"]),
+            _capi.ptr(bank["w3s"]), _capi.ptr(bank["w2s"]), _capi.ptr(logits), c_int(n_experts), c_int(func),
+            c_float(eps), c_float(scaling), c_int(K_in), c_int(hidden), c_int(out_dim), c_int(k), _capi.ptr(out),
+            _capi.ptr(workspace), _capi.stream_ptr(x.device))
     if rc != 0:
         raise RuntimeError(f"mxfp4_moe_decode_layer returned {rc}")
     return out
@@ -228,12 +246,14 @@ def mxfp4_dequant_bf16(packed: torch.Tensor, scale: torch.Tensor) -> torch.Tenso
     lib = _capi.load("grouped")
     _check(packed, "packed", torch.uint8)
     _check(scale, "scale", torch.uint8)
+    _check_device(packed, scale=scale)
     rows, cols = packed.shape[0], packed.shape[1] * 2
     if tuple(scale.shape) != (rows, cols // 32):
         raise ValueError(f"scale shape {tuple(scale.shape)} != ({rows}, {cols // 32})")
     out = torch.empty(rows, cols, dtype=torch.bfloat16, device=packed.device)
-    rc = lib.mxfp4_dequant_bf16(_capi.ptr(packed), _capi.ptr(scale), c_longlong(rows), c_int(cols), _capi.ptr(out),
-                                _capi.stream_ptr(packed.device))
+    with _capi.on_device(packed):
+        rc = lib.mxfp4_dequant_bf16(_capi.ptr(packed), _capi.ptr(scale), c_longlong(rows), c_int(cols), _capi.ptr(out),
+                                    _capi.stream_ptr(packed.device))
     if rc != 0:
         raise RuntimeError(f"mxfp4_dequant_bf16 returned {rc}")
     return out

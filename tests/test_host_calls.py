@@ -1,0 +1,65 @@
+"""Tensors of several GPUs: the native call path hands them to the checks in Python, and those refuse them (fake tensors: no GPU
+needed, nothing is launched)."""
+import importlib
+
+import pytest
+import torch
+from torch._subclasses.fake_tensor import FakeTensorMode
+
+K, H, E, T = 256, 256, 8, 3
+
+
+def cases(rt):
+    """name -> (native arguments in order, index of the argument or of (argument, key) to move, operator call)."""
+    def u8(*shape):
+        return lambda dev: torch.empty(*shape, dtype=torch.uint8, device=dev)
+
+    def of(dtype, *shape):
+        return lambda dev: torch.empty(*shape, dtype=dtype, device=dev)
+
+    bf, f32, i32 = torch.bfloat16, torch.float32, torch.int32
+    bank = {"w1p": u8(E, H, K // 2), "w3p": u8(E, H, K // 2), "w2p": u8(E, K, H // 2), "w1s": u8(E, H, K // 32), "w3s": u8(E, H, K // 32),
+            "w2s": u8(E, K, H // 32)}
+    shared = {"w1": u8(H, K), "w3": u8(H, K), "w2": u8(K, H), "w1s": u8(2, 2), "w3s": u8(2, 2), "w2s": u8(2, 2)}
+    stack = [{"packed": bank[n + "p"], "scale": bank[n + "s"]} for n in ("w1", "w3", "w2")]
+    x, out = of(bf, K), of(bf, K)
+    return {
+        "mxfp4_gemv": ([u8(64, K // 2), u8(64, K // 32), x, of(bf, 64), None], lambda a: rt.mxfp4_gemv(*a)),
+        "fp8_gemv": ([u8(128, K), u8(1, 2), x, of(bf, 128), None], lambda a: rt.fp8_e4m3_gemv(*a)),
+        "fp8_gemv_f32scale": ([u8(128, K), of(f32, 1, 2), x, of(bf, 128), None], lambda a: rt.fp8_e4m3_gemv_f32scale(*a)),
+        "fp8_gemv_batched": ([u8(128, K), u8(1, 2), of(bf, T, K), 1, None, None], lambda a: rt.fp8_e4m3_gemv_batched(*a)),
+        "fp8_shared_swiglu": ([shared, x, 10.0, 0.0, out, u8(2 * H), None], lambda a: rt.fp8_shared_swiglu(*a)),
+        "grouped_gemv": ([*stack, x, of(f32, E), out, u8(1 << 16)], lambda a: rt.mxfp4_grouped_gemv(*a[:3], None, *a[3:])),
+        "grouped_gemv_ids": ([bank, of(i32, 6), x, of(f32, 6), out, u8(1 << 16), 3], lambda a: rt.mxfp4_grouped_gemv_ids(*a)),
+        "route_topk": ([of(f32, T, E), 2, "softmax", 1e-20, 1.0, of(i32, T, 2), of(f32, T, 2)], lambda a: rt.moe_route_topk(*a)),
+        "decode_layer": ([bank, of(f32, E), x, 2, "softmax", 1e-20, 1.0, out, u8(1 << 16)], lambda a: rt.moe_decode_layer(*a)),
+        "moe_forward": ([bank, of(bf, T, K), of(i32, T, 2), of(f32, T, 2), of(bf, T, K), u8(1 << 20), -1],
+                        lambda a: rt.moe_forward(*a[:6])),
+    }
+
+
+NAMES = ["mxfp4_gemv", "fp8_gemv", "fp8_gemv_f32scale", "fp8_gemv_batched", "fp8_shared_swiglu", "grouped_gemv", "grouped_gemv_ids",
+         "route_topk", "decode_layer", "moe_forward"]
+
+
+@pytest.mark.parametrize("name", NAMES)
+def test_tensors_of_two_devices(rt, name):
+    capi = importlib.import_module("dsv4_b200.runtime._capi")
+    for key in capi.SIGNATURES:
+        capi.load(key)
+    native = getattr(capi.host(), name)
+    makers, operator = cases(rt)[name]
+    places = []
+    for i, m in enumerate(makers):
+        places += [(i, k) for k in m] if isinstance(m, dict) else [(i, None)] if callable(m) else []
+    for moved in places:
+        def build(i, m):
+            if isinstance(m, dict):
+                return {k: v("cuda:1" if (i, k) == moved else "cuda:0") for k, v in m.items()}
+            return m("cuda:1" if (i, None) == moved else "cuda:0") if callable(m) else m
+
+        with FakeTensorMode():
+            args = [build(i, m) for i, m in enumerate(makers)]
+        assert native(*args) is None, moved
+        with pytest.raises((RuntimeError, ValueError), match="CUDA device"):
+            operator(args)
