@@ -12,6 +12,7 @@
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <cstdint>
@@ -105,8 +106,9 @@ enum { kW1p, kW3p, kW2p, kW1s, kW3s, kW2s, kW1, kW3, kW2, kPacked, kScale };
 PyObject* get(PyObject* dict, int key) { return PyDict_Check(dict) ? PyDict_GetItem(dict, kKeys[key]) : nullptr; }
 
 #define FAST(name) PyObject* name(PyObject*, PyObject* const* a, Py_ssize_t n)
-#define ORDINARY(cond) do { if (!(cond)) Py_RETURN_NONE; } while (0)
-#define GUARD(...) try { __VA_ARGS__ } catch (const std::exception& e) { PyErr_SetString(PyExc_RuntimeError, e.what()); return nullptr; }
+#define ORDINARY(cond) do { if (!(cond)) { PyErr_Clear(); Py_RETURN_NONE; } } while (0)      // (an integer beyond 64 bits is an error that is pending)
+// C++ exceptions become the Python ones that torch raises for them (torch.OutOfMemoryError for an allocation).
+#define GUARD(...) HANDLE_TH_ERRORS __VA_ARGS__ END_HANDLE_TH_ERRORS
 
 FAST(bind) {
     if (n != 2) { PyErr_SetString(PyExc_TypeError, "bind(name, address)"); return nullptr; }

@@ -70,3 +70,11 @@ def test_interpreter_lock_is_released_around_the_call(ops, capi, name):
     finally:
         for lib in capi._loaded.values():
             capi._bind(lib)
+
+
+def test_failed_allocation_raises_what_torch_raises(rt, ops):
+    logits = torch.zeros(1, 8, device=DEV)
+    with pytest.raises(torch.OutOfMemoryError):
+        rt.moe_route_topk(logits, k=1 << 42)        # 16 TB of ids
+    ids, _ = rt.moe_route_topk(logits, k=2)
+    assert ids.tolist() == [[0, 1]]

@@ -63,3 +63,19 @@ def test_tensors_of_two_devices(rt, name):
         assert native(*args) is None, moved
         with pytest.raises((RuntimeError, ValueError), match="CUDA device"):
             operator(args)
+
+
+def test_integers_beyond_64_bits_are_declined(rt):
+    capi = importlib.import_module("dsv4_b200.runtime._capi")
+    for key in capi.SIGNATURES:
+        capi.load(key)
+    makers, _ = cases(rt)["fp8_gemv_batched"]
+    with FakeTensorMode():
+        args = [m("cuda:0") if callable(m) else m for m in makers]
+    args[3] = 1 << 70
+    assert capi.host().fp8_gemv_batched(*args) is None
+    makers, _ = cases(rt)["route_topk"]
+    with FakeTensorMode():
+        args = [m("cuda:0") if callable(m) else m for m in makers]
+    args[1] = 1 << 70
+    assert capi.host().route_topk(*args) is None
