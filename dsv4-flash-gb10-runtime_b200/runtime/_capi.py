@@ -3,9 +3,10 @@ from __future__ import annotations
 
 import ctypes
 import os
+import warnings
 from ctypes import c_int, c_int64, c_longlong, c_size_t, c_void_p, c_float
 
-from .. import HOST_FILE, LIB_DIR, lib_path
+from .. import LIB_DIR, host_file, lib_path
 
 _P = c_void_p
 
@@ -59,19 +60,30 @@ _loaded: dict[str, ctypes.CDLL] = {}
 _host = None
 
 
+class _Declines:
+    """In the place of the call path's module where that cannot be loaded: declines every call."""
+
+    def __getattr__(self, name):
+        return lambda *args: None
+
+
 def host():
     """The extension module with the operators' call path.  Its functions do the ordinary call and return None for
-    anything else, which then takes the checks in Python; it knows an entry point once that library has been loaded."""
+    anything else, which then takes the checks in Python and ctypes; it knows an entry point once that library has been
+    loaded.  Without the module (not built, or for another torch) every call goes that way."""
     global _host
     if _host is None:
         import importlib.util
         import torch  # noqa: F401  (the module links against its libraries)
-        path = os.path.join(LIB_DIR, HOST_FILE)
-        if not os.path.exists(path):
-            raise FileNotFoundError(f"{HOST_FILE} not found at {path}: build it with `make` in the package directory")
-        spec = importlib.util.spec_from_file_location("dsv4_host", path)
-        mod = importlib.util.module_from_spec(spec)
-        spec.loader.exec_module(mod)
+        path = os.path.join(LIB_DIR, host_file() or "dsv4_host")
+        try:
+            spec = importlib.util.spec_from_file_location("dsv4_host", path)
+            mod = importlib.util.module_from_spec(spec)
+            spec.loader.exec_module(mod)
+        except (ImportError, OSError, AttributeError) as e:
+            warnings.warn(f"{path} cannot be loaded ({e}); the operators make their calls through ctypes, with some 15 us more "
+                          "host time each: build it with `make` in the package directory", RuntimeWarning)
+            mod = _Declines()
         _host = mod
         for lib in _loaded.values():
             _bind(lib)

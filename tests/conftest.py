@@ -19,7 +19,7 @@ def pytest_configure(config):
 def pkg():
     """The package, with its libraries built (nvcc cross-compiles without a GPU)."""
     p = entry.load_package()
-    if not all(os.path.exists(p.lib_path(k)) for k in p.LIB_FILES):
+    if not all(os.path.exists(f) for f in [*(p.lib_path(k) for k in p.LIB_FILES), os.path.join(p.LIB_DIR, p.host_file())]):
         p.build()
     return p
 

@@ -78,3 +78,16 @@ def test_failed_allocation_raises_what_torch_raises(rt, ops):
         rt.moe_route_topk(logits, k=1 << 42)        # 16 TB of ids
     ids, _ = rt.moe_route_topk(logits, k=2)
     assert ids.tolist() == [[0, 1]]
+
+
+@pytest.mark.parametrize("name", OPS)
+def test_same_bits_through_ctypes(ops, capi, monkeypatch, name):
+    def tensors(result):
+        return list(result) if isinstance(result, tuple) else [result]
+
+    native = tensors(ops[name][1]())
+    with monkeypatch.context() as m:
+        m.setattr(capi, "_host", capi._Declines())
+        through_ctypes = tensors(ops[name][1]())
+    assert [(t.dtype, t.shape, t.device) for t in native] == [(t.dtype, t.shape, t.device) for t in through_ctypes]
+    assert all(torch.equal(a.view(torch.uint8), b.view(torch.uint8)) for a, b in zip(native, through_ctypes))

@@ -79,3 +79,22 @@ def test_integers_beyond_64_bits_are_declined(rt):
         args = [m("cuda:0") if callable(m) else m for m in makers]
     args[1] = 1 << 70
     assert capi.host().route_topk(*args) is None
+
+
+@pytest.mark.parametrize("content", [None, b"not a library"])
+def test_operators_do_without_the_module(rt, pkg, monkeypatch, tmp_path, content):
+    """A lib/ without the module, or with one that does not load: one warning, then the checks in Python and ctypes."""
+    capi = importlib.import_module("dsv4_b200.runtime._capi")
+    if content is not None:
+        (tmp_path / pkg.host_file()).write_bytes(content)
+    monkeypatch.setattr(capi, "LIB_DIR", str(tmp_path))
+    monkeypatch.setattr(capi, "_host", None)
+    with pytest.warns(RuntimeWarning, match="ctypes"):
+        with pytest.raises(RuntimeError, match="CUDA device"):
+            rt.mxfp4_gemv(torch.zeros(8, 32, dtype=torch.uint8), torch.zeros(8, 2, dtype=torch.uint8), torch.zeros(64, dtype=torch.bfloat16))
+    assert capi.host().moe_forward(None) is None
+    capi.load("mxfp4")
+
+
+def test_module_is_named_for_its_torch(pkg):
+    assert torch.__version__ in pkg.host_file()
