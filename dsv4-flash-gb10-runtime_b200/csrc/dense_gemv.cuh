@@ -251,11 +251,16 @@ inline bool dense_pdl_enabled() {
 }
 
 // CTAs per group: one CTA per SM over all groups (two successive launches share each SM), more where a CTA's partial sums would
-// not fit.
+// not fit.  Groups that do not divide the SMs leave a few SMs with two CTAs (rounded up; rounded down, a few SMs idle: slower still),
+// and everyone waits for those: with more than kRowSmall bytes of weights per SM as many CTAs as fit two per SM are faster.  Eight
+// groups of 1024 x 4096 10.2 -> 8.4 us (rounded down 11.2), twelve 13.8 -> 10.1, eight of 1024 x 1024 4.1 -> 3.6; below, one per SM is: eight
+// of 512 x 512 2.5 us, with two 2.8.  Groups that divide the SMs keep one: two of 1024 x 4096 3.0 us, with two CTAs per SM 3.6.
 inline long long dense_grid(const DenseArgs& a, int mats, const RowPlan& p, int n_groups) {
     const long long cap = kDenseParts / (4 * mats * p.n_slices);          // rows per CTA
-    const long long sms = (dense_sm_count() + n_groups - 1) / n_groups, need = ((long long)a.N + cap - 1) / cap;
-    const long long grid = sms < need ? need : sms;
+    const long long sms = dense_sm_count(), need = ((long long)a.N + cap - 1) / cap;
+    long long grid = (sms + n_groups - 1) / n_groups;
+    if (sms % n_groups != 0 && (long long)n_groups * a.N * p.row_bytes > sms * kRowSmall && 2 * sms / n_groups > grid) grid = 2 * sms / n_groups;
+    if (grid < need) grid = need;
     return grid < a.N ? grid : a.N;
 }
 // Needs 16-byte aligned x, weights and row strides.

@@ -88,3 +88,24 @@ def test_fp8_several_tokens(rt, qz, K, N, G, S, gap):
         r, b = slice(grp * N, (grp + 1) * N), slice(grp * N // 128, (grp + 1) * N // 128)
         full = w[r].view(torch.float8_e4m3fn).float() * torch.repeat_interleave(torch.repeat_interleave(scale[b], 128, 0), 128, 1)
         close(y[:, r], (x[:, grp * K:(grp + 1) * K].float() @ full.T).numpy(), f"group {grp} of {G}x{N}x{K}, {S} tokens")
+
+
+@pytest.mark.parametrize("G,N,K", [
+    (2, 1024, 512), (37, 128, 512),    # groups that divide 148 SMs
+    (3, 2048, 896), (3, 2048, 1024),   # others, either side of 40 KB per SM
+    (8, 1024, 4096), (147, 128, 512), (149, 128, 512), (300, 128, 384),
+])
+def test_fp8_groups_one_token(rt, qz, G, N, K):
+    """One launch over G groups equals the G single calls bit for bit (the split of the reduction depends on K alone)."""
+    g = torch.Generator().manual_seed(G)
+    w, s = qz.quantize_fp8_block128(torch.randn(G * N, K, generator=g) * 0.02, "e8m0")
+    s = (s.int() + torch.arange(s.numel()).view(s.shape) % 3).to(torch.uint8)
+    x = torch.randn(G * K, generator=g).to(torch.bfloat16)
+    w, s, x = w.to(DEV), s.to(DEV), x.to(DEV)
+    y = rt.fp8_e4m3_gemv_batched(w, s, x, n_groups=G)
+    single = [rt.fp8_e4m3_gemv(w[i * N:(i + 1) * N], s[i * N // 128:(i + 1) * N // 128], x[i * K:(i + 1) * K]) for i in range(G)]
+    assert torch.equal(y.view(torch.int16), torch.cat(single).view(torch.int16))
+    full = w[:N].cpu().view(torch.float8_e4m3fn).float()
+    tiles = torch.ldexp(torch.ones(N // 128, K // 128), s[:N // 128].cpu().int() - 127)
+    full = full * torch.repeat_interleave(torch.repeat_interleave(tiles, 128, 0), 128, 1)
+    close(y[:N], (full @ x[:K].float().cpu()).numpy(), f"group 0 of {G}x{N}x{K}")
