@@ -6,7 +6,7 @@ The directory name carries a hyphen, so it cannot be imported by name; load it w
 
 Layout
 ------
-csrc/      CUDA sources of the three shared libraries (Makefile in this directory builds them into lib/)
+csrc/      CUDA sources of the shared libraries (Makefile in this directory builds them into lib/)
 lib/       built libraries: libmxfp4_grouped_gemv.so, libmxfp4_gemv.so, libfp8_e4m3_gemv.so, libmxfp4_moe.so,
            and dsv4_host.<python>.torch-<version>.so (the operators' call path)
 runtime/   host-side mirror of the reference's ctypes bindings (same function names and argument meaning),
@@ -53,7 +53,7 @@ LIB_ENV = {
 
 
 def lib_path(key: str) -> str:
-    """Path of one of the three libraries, honouring the reference's environment overrides."""
+    """Path of one of the libraries, honouring the reference's environment overrides."""
     return os.path.abspath(os.environ.get(LIB_ENV[key], os.path.join(LIB_DIR, LIB_FILES[key])))
 
 

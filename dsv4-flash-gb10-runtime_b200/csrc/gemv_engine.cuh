@@ -1,12 +1,12 @@
 // Shared device-side building blocks of the B200 (sm_100a) quantized-weight GEMV kernels.
 //
 // Design (decode is HBM-bound: every weight byte is read exactly once):
-//   * one lane owns ONE 16-byte weight block of the reduction axis (32 E2M1 nibbles or
-//     16 E4M3 bytes) and keeps the matching activation block in registers as fp16x2,
-//     pre-scaled by a per-block power of two so that fp16 never overflows or flushes;
-//   * a warp therefore streams 512 contiguous bytes of a weight row per 128-bit load,
-//     and walks DOWN the rows of the matrix with many such loads in flight
-//     (two register buffers: the next batch is requested before the current is consumed);
+//   * weight rows stream through shared memory by bulk copies, requested far ahead of their use
+//     (row_stream.cuh, stream_ring.cuh);
+//   * a lane owns 16-byte weight blocks of the reduction axis (32 E2M1 nibbles or 16 E4M3
+//     bytes) and keeps the matching activation blocks in registers as fp16x2, pre-scaled by
+//     a power of two so that fp16 never overflows or flushes; a warp reads 512 contiguous
+//     bytes of a row per 128-bit load;
 //   * E2M1 / E4M3 are decoded by the hardware converters (cvt.rn.f16x2.e2m1x2 /
 //     cvt.rn.f16x2.e4m3x2): one instruction per two weights, no LUT traffic;
 //   * products of a block are summed in four short fp16x2 chains (each E2M1 x bf16 product

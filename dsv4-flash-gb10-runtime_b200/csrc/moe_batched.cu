@@ -95,10 +95,15 @@ bool pdl_enabled() {
     return v == 1;
 }
 
-// Every kernel of this library executes griddepcontrol.launch_dependents early and reads or writes global memory only
-// after griddepcontrol.wait, so consecutive kernels are launched with programmatic stream serialisation: the
-// next kernel's CTAs are scheduled while the previous kernel drains, and its prologue (barrier set-up, tensor
-// memory allocation) overlaps the tail.
+// Consecutive kernels are launched with programmatic stream serialisation: a kernel's CTAs are scheduled while the one before it
+// drains, and what they do before griddepcontrol.wait (barrier set-up, tensor memory allocation, first reads) overlaps its tail.
+// What a kernel may read before its wait follows from when the one before it triggers (griddepcontrol.launch_dependents):
+//   * A kernel that triggers only AFTER its own wait tells its successor that everything before itself is complete.  That holds
+//     for the grouping kernel (behind it the activation kernels read x), the activation kernels (behind them the gate/up GEMM reads
+//     the tile tables and requests weights) and the gate/up GEMM (behind it the down GEMM does).  Their triggers must stay there.
+//   * The combine kernels, moe_ep_gather_meta_kernel and moe_ep_sum_kernel trigger first; what follows them (the grouping
+//     kernel, or another call) reads nothing of theirs, nor of what is before them, until its own wait.
+// Every kernel writes global memory only after its wait.
 template <class... Params, class... Args>
 cudaError_t launch_k(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int cluster,
                      Args&&... args) {
@@ -211,8 +216,8 @@ DSV4_API int mxfp4_moe_stage_times(float* us_out) {
     return 0;
 }
 
-// Bytes of workspace mxfp4_moe_forward needs (normalised activations, grouping tables, the fp16 intermediate
-// [n_tokens * k, hidden] and the FP32 per-pair outputs [n_tokens * k, out_dim]).
+// Bytes of workspace mxfp4_moe_forward needs: grouping tables, the FP32 per-pair outputs [n_tokens * k, out_dim], and the
+// activations and the intermediate of every pair in the form of the path that needs more (three MXFP4 terms; fp16).
 DSV4_API size_t mxfp4_moe_forward_workspace_bytes(int n_tokens, int k, int K_in, int hidden, int out_dim,
                                                   int n_experts) {
     if (n_tokens <= 0 || k <= 0 || K_in <= 0 || hidden <= 0 || out_dim <= 0 || n_experts <= 0) return 0;
@@ -266,6 +271,8 @@ static int moe_forward_impl(int path, const __nv_bfloat16* x, const uint8_t* ban
     ga.ids = ids; ga.weights = weights; ga.n_pairs = P; ga.n_experts = n_experts; ga.g = g; ga.status = status;
     const int rows_up = path == 1 ? kQTileRowsUp : kMoeTileRows, rows_down = path == 1 ? kQTileRowsDown : 2 * kMoeTileRows;
     ga.m_tiles_up = hidden / rows_up; ga.m_tiles_down = (out_dim + rows_down - 1) / rows_down;
+    // (Pairs of the whole batch: where ids are negative, as under expert parallelism, the experts here have fewer, and the larger tiles
+    // are taken although the smaller would do.  Eight ranks emulated on one GPU, 128 to 1024 tokens: 1 % of the layer's time.)
     const int cap16 = P <= (long long)kTmFewTokens * n_experts ? 64 : kMoeTileTokens;      // tokens per tile, fp16 path
     const bool few = P <= (long long)kQFewTokens * n_experts;
     const int cap_q = few ? 32 : kQTok;                                                    // tokens per tile, block-scaled path

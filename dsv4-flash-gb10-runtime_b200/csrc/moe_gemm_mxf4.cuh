@@ -418,7 +418,7 @@ __global__ void __launch_bounds__(kQThreads, 1) moe_gemm_mxf4_kernel(const __gri
                     RingPos p;
                     for (int s = 0; s < s0; ++s, p.next(kQStages)) weights(s, p);
                     pdl_wait();
-                    pdl_launch_dependents();
+                    pdl_launch_dependents();                  // after the wait: the next kernel reads the tile tables before its own
                     waited = true;
                     for (int s = 0; s < s0; ++s, pos.next(kQStages)) tokens(s, pos);
                 }

@@ -1,5 +1,6 @@
-// Small kernels around the batched routed-expert GEMMs: activations to normalised fp16, grouping of
-// (token, expert) pairs by expert, and the final per-token sum.
+// What the batched routed-expert layer's kernels share: tile widths, work descriptors, the three-term MXFP4 quantiser; and its
+// small kernels behind the GEMMs, the per-token sum and the expert-parallel exchange (grouping and activations:
+// moe_prep_kernel.cuh).
 #pragma once
 
 #include "gemv_engine.cuh"

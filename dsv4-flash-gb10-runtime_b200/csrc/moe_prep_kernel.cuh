@@ -27,7 +27,7 @@ struct MoeGroupArgs {
 __global__ void __launch_bounds__(kPrepThreads) moe_group_kernel(const MoeGroupArgs a) {
     __shared__ int count[kMoeMaxExperts], cursor[kMoeMaxExperts], warp_sums[2][32];
     pdl_wait();
-    pdl_launch_dependents();
+    pdl_launch_dependents();                               // after the wait: the next kernel reads x before its own
     const int e = threadIdx.x, lane = e & 31, wid = e >> 5;
     const int blocks = gridDim.x, blk = blockIdx.x;
     count[e] = 0;
@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(256, 6) moe_act_mxf4_kernel(const MoeActArgs a
     int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     fetch(w, cur);
     if (!PEER) pdl_wait();
-    pdl_launch_dependents();
+    pdl_launch_dependents();                               // after the wait: the next kernel reads the tile tables before its own
     int slots = slots_of(w);
     for (; w < n_chunks; w += warps) {
         fetch(w + warps, nxt);

@@ -1,4 +1,4 @@
-"""ctypes loading of the three shared libraries, with the exact C signatures of include/dsv4_b200.h."""
+"""ctypes loading of the shared libraries, with the exact C signatures of include/dsv4_b200.h."""
 from __future__ import annotations
 
 import ctypes

@@ -98,7 +98,7 @@ def mxfp4_grouped_gemv_static(W1: Dict[str, torch.Tensor], W3: Dict[str, torch.T
     """The routed-expert FFN through the entry point that takes no workspace and allocates nothing.
 
     For hosts that cannot get device memory at call time (everything already committed to the expert bank and the
-    KV cache, or a thread that must not enter cudaMalloc): the intermediate sits in a fixed 96 KB array inside the
+    KV cache, or a thread that must not enter cudaMalloc): the intermediate sits in a fixed 192 KB array inside the
     library, shared by every call on the device, so calls that overlap on the GPU must be serialised by the caller.
     `out` (bfloat16 [out_dim]) is mandatory so that this wrapper allocates nothing either.  hidden <= 4096,
     six experts.  Make the first call on a device before capturing a stream there."""

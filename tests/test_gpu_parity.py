@@ -195,7 +195,7 @@ def run_grouped(rt, bank_dev, x, r, dev):
 
 
 # (1024, 1024), (2048, 1024), (4096, 2048): shapes served by the shared-memory ring kernels; the others by the
-# register-streaming kernels
+# row-streaming kernels
 @pytest.mark.parametrize("K,H", [(32, 32), (64, 96), (256, 128), (512, 512), (1024, 992), (1024, 1024), (2048, 1024),
                                  (1024, 1536), (2048, 4096), (4096, 2048)])
 def test_grouped_gemv(rt, qz, dev, K, H):

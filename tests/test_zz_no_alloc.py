@@ -29,7 +29,7 @@ def _sets(bank_dev):
             {"packed": bank_dev["w2p"], "scale": bank_dev["w2s"]})
 
 
-@pytest.mark.parametrize("K,H", [(4096, 2048), (256, 96)])      # the ring kernels and the register-streaming ones
+@pytest.mark.parametrize("K,H", [(4096, 2048), (256, 96)])      # the ring kernels and the row-streaming ones
 def test_static_entry_matches_workspace_entry_twice(rt, qz, K, H):
     assert torch.cuda.is_available(), "GPU tests need a CUDA device"
     dev = torch.device("cuda:0")
