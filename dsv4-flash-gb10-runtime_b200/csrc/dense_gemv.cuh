@@ -117,22 +117,29 @@ __global__ void __launch_bounds__(kRowThreads, 2) dense_stream_kernel(const Dens
         bool ok[SPW];
 #pragma unroll
         for (int q = 0; q < SPW; ++q) { blk[q] = (ks0 + q * w_slices) * 32 + lane; ok[q] = blk[q] < n_blk; }
-        bool alive = Sc::kPerRow || __all_sync(kFullMask, row_wait(p, ring.x, 0, 2));
-        if (MATS == 2 && !alive) failed = 1;
+        auto give_up = [&](int st) {
+#pragma unroll 1
+            for (int m = 0; m < MATS; ++m)
+#pragma unroll 1
+                for (int ks = ks0; ks < p.n_slices; ks += w_slices)
+                    row_give_up(p, st * p.rows + rg, n_local, lane, part + m * n_local * p.n_slices + ks, p.n_slices);
+            if (MATS == 2) failed = 1;
+        };
+        const bool got_x = Sc::kPerRow || __all_sync(kFullMask, row_wait(p, ring.x, 0, 2));
         ActBlock<Fmt> xb[SPW];
 #pragma unroll
         for (int q = 0; q < SPW; ++q) {
             if constexpr (Sc::kPerRow) row_act_block(smem + p.off_x, n_blk, blk[q], ok[q], xb[q]);
             else row_act_block_bf16<Fmt>(smem + p.off_x, blk[q], ok[q], xb[q]);
             if (!ok[q]) blk[q] = 0;
-            if (!Sc::kPerRow && !alive) xb[q].scale = row_nan();
+            if (!got_x) xb[q].scale = row_nan();
         }
+        if (MATS == 2 && !got_x) failed = 1;
         RowPos pos;
         for (int st = 0; st < n_stages; ++st) {
-            if (alive && !__all_sync(kFullMask, row_wait(p, ring.full[pos.slot], pos.round, 2))) {
-                alive = false;
-                for (int q = 0; q < SPW; ++q) xb[q].scale = row_nan();
-                if (MATS == 2) failed = 1;
+            if (!__all_sync(kFullMask, row_wait(p, ring.full[pos.slot], pos.round, 2))) {
+                give_up(st);
+                break;
             }
             const uint32_t stage = smem + pos.slot * p.stage_bytes;
             const int row = st * p.rows + rg, left = n_local - row;
@@ -165,7 +172,7 @@ __global__ void __launch_bounds__(kRowThreads, 2) dense_stream_kernel(const Dens
                     for (int i = 0; i < RPW; ++i) v[m * row_pow2(RPW) + i] = Fmt::dot(w[m * RPW + i], xb[q].h) * (sc[m * RPW + i] * xb[q].scale);
                 row_store<RPW>(v, left, p.n_groups, lane, part + row * p.n_slices + ks0 + q * w_slices, p.n_slices, n_local * p.n_slices);
             }
-            row_release(ring, p, pos, lane, alive);
+            row_release(ring, p, pos, lane);
         }
     }
     __syncthreads();

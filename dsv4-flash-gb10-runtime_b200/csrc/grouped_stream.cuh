@@ -98,16 +98,15 @@ __global__ void __launch_bounds__(kRowThreads, 2) grouped_gate_stream_kernel(con
         if (warp < p.warps) {
             const int ks = warp % p.n_slices, rg = warp / p.n_slices, blk = ks * 32 + lane;
             const bool ok = blk < row_s;
-            bool alive = true;
             ActBlock<Fp4Format> xb;
             row_act_block(smem + p.off_x, row_s, blk, ok, xb);
             const uint32_t blk_r = ok ? blk : 0;               // lanes past the row's end: block 0 against zeros
             RowPos pos;
             Walk c = walk_start();
             for (int st = 0; st < n_stages; ++st, walk_next(c)) {
-                if (alive && !__all_sync(kFullMask, row_wait(p, ring.full[pos.slot], pos.round, 1))) {
-                    alive = false;
-                    xb.scale = row_nan();
+                if (!__all_sync(kFullMask, row_wait(p, ring.full[pos.slot], pos.round, 1))) {      // (NaN for the gate is enough)
+                    row_give_up(p, st * p.rows + rg, n_local, lane, part + ks, p.n_slices);
+                    break;
                 }
                 walk_stage(c, st);
                 const uint32_t stage = smem + pos.slot * p.stage_bytes;
@@ -129,7 +128,7 @@ __global__ void __launch_bounds__(kRowThreads, 2) grouped_gate_stream_kernel(con
 #pragma unroll
                 for (int k = 0; k < 2 * kGateRpw; ++k) v[k] = Fp4Format::dot(w[k], xb.h) * (sc[k] * xb.scale);
                 row_store<kGateRpw>(v, n_local - row, p.n_groups, lane, part + row * p.n_slices + ks, p.n_slices, n_local * p.n_slices);
-                row_release(ring, p, pos, lane, alive);
+                row_release(ring, p, pos, lane);
             }
         }
     }
@@ -221,7 +220,7 @@ __global__ void __launch_bounds__(kRowThreads, 2) grouped_down_stream_kernel(con
             RowPos pos;
             bool alive = true;
             const int blk_r = ok ? blk : 0;
-            for (int e = 0; e < a.E; ++e) {
+            for (int e = 0; e < a.E && alive; ++e) {
                 {
                     const int b = e * n_blk + blk_r;
 #pragma unroll
@@ -230,13 +229,14 @@ __global__ void __launch_bounds__(kRowThreads, 2) grouped_down_stream_kernel(con
                         if (!ok) q = make_uint4(0, 0, 0, 0);
                         *reinterpret_cast<uint4*>(&xb.h[4 * c]) = q;
                     }
-                    xb.scale = alive ? mid_scale[b] : row_nan();
+                    xb.scale = mid_scale[b];
                 }
                 const uint32_t s_first = (uint32_t)reinterpret_cast<uintptr_t>(scales_of(e, 0));
                 for (int row0 = 0; row0 < n_local; row0 += p.rows) {
-                    if (alive && !__all_sync(kFullMask, row_wait(p, ring.full[pos.slot], pos.round, 2))) {
+                    if (!__all_sync(kFullMask, row_wait(p, ring.full[pos.slot], pos.round, 2))) {      // (the last expert's product is enough)
+                        row_give_up(p, (e == a.E - 1 ? row0 : 0) + rg, n_local, lane, part + (a.E - 1) * p.n_slices + ks, a.E * p.n_slices);
                         alive = false;
-                        xb.scale = row_nan();
+                        break;
                     }
                     const uint32_t stage = smem + pos.slot * p.stage_bytes, sbase = stage + p.rows * p.row_bytes + blk_r;
                     const uint32_t s_addr = s_first + row0 * n_blk;
@@ -252,7 +252,7 @@ __global__ void __launch_bounds__(kRowThreads, 2) grouped_down_stream_kernel(con
 #pragma unroll
                     for (int j = 0; j < RPW; ++j) v[j] = Fp4Format::dot(w[j], xb.h) * (sc[j] * xb.scale);
                     row_store<RPW>(v, n_local - row, p.n_groups, lane, part + (row * a.E + e) * p.n_slices + ks, a.E * p.n_slices, 0);
-                    row_release(ring, p, pos, lane, alive);
+                    row_release(ring, p, pos, lane);
                 }
             }
         }

@@ -13,10 +13,10 @@
 // these finish.  Nothing is loaded by the consumers inside the loop: a load queues behind the SM's own weight copies, one to
 // four microseconds (scale bytes fetched that way, two stages ahead, made 33.6 MB of FP8 take 11.1 us).
 //
-// Every wait has a poll budget.  A consumer warp whose wait runs out records a status, takes NaN for its activations' scale - so
-// that the rows it did not get come out as NaN - and goes through its remaining stages without waiting and without freeing a slot.
-// Nothing is requested past the ring then, and what was requested landed long before the last role has given up: no copy is on
-// its way when the CTA leaves.  (A flag for the whole CTA, looked at behind the last stage, made every launch 0.05 to 0.1 us longer.)
+// Every wait has a poll budget.  A consumer warp whose wait runs out records a status, writes NaN for its share of the rows it did
+// not get and stops, without freeing another slot.  Nothing is requested past the ring then, and what was requested landed long
+// before the last role has given up: no copy is on its way when the CTA leaves.  (A flag for the whole CTA, looked at behind the
+// last stage, made every launch 0.05 to 0.1 us longer.)
 #pragma once
 
 #include "gemv_engine.cuh"
@@ -173,9 +173,13 @@ __device__ __forceinline__ bool row_wait_free(RowRing& r, const RowPlan& p, cons
     return row_wait(p, r.empty[pos.slot], pos.round - 1, code);
 }
 __device__ __forceinline__ float row_nan() { return __uint_as_float(0x7fffffffu); }
-__device__ __forceinline__ void row_release(RowRing& r, const RowPlan& p, RowPos& pos, int lane, bool alive) {
+// NaN for a warp's rows from `first` on (its every n_groups-th), by its lanes.
+__device__ __forceinline__ void row_give_up(const RowPlan& p, int first, int n_local, int lane, float* part, int part_stride) {
+    for (int t = first + lane * p.n_groups; t < n_local; t += 32 * p.n_groups) part[t * part_stride] = row_nan();
+}
+__device__ __forceinline__ void row_release(RowRing& r, const RowPlan& p, RowPos& pos, int lane) {
     __syncwarp();
-    if (lane == 0 && alive) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&r.empty[pos.slot])) : "memory");
+    if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&r.empty[pos.slot])) : "memory");
     pos.next(p.slots);
 }
 
