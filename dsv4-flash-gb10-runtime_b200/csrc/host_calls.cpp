@@ -3,14 +3,14 @@
 //
 // A call through ctypes with its checks in Python took 17 us of host time, more than the kernel of every dense operator;
 // this takes about 3 (most of it the launch itself).  A function returns None when anything is out of the ordinary (tensors of
-// several devices, a stride, a shape that does not fit, an explicit stream): the caller then goes through the checks in Python,
-// which name what is wrong, or copy what may be copied.  Entry addresses come from the ctypes-loaded libraries (bind), so the
+// several devices or of one that is not current, a stride, a shape that does not fit, an explicit stream): the caller then goes
+// through the checks in Python, which name what is wrong, copy what may be copied, or make the device current.  Entry addresses come from the ctypes-loaded libraries (bind), so the
 // environment overrides of the library paths hold here too.
 #include <Python.h>
 
 #include <ATen/ATen.h>
 #include <ATen/cuda/EmptyTensor.h>
-#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
@@ -67,13 +67,16 @@ const Tensor* dense(PyObject* o, ScalarType type) {
 bool shape(const Tensor& t, std::initializer_list<int64_t> want) {
     return t.sizes() == at::IntArrayRef(want);
 }
-// All on the device of the first one.
+// All on one device.
 bool together(std::initializer_list<const Tensor*> tensors) {
     const auto device = (*tensors.begin())->device();
     for (const Tensor* t : tensors)
         if (t->device() != device) return false;
     return true;
 }
+// That device is the current one, which allocation, stream and launch are meant for.  (A guard that makes it so cost every call
+// about 0.1 us.)
+bool current(const Tensor* t) { return c10::cuda::current_device() == t->device().index(); }
 // An optional output or workspace: on that device, or not on a GPU at all (mapped host memory, where an operator takes it).
 bool reachable(PyObject* given, const Tensor* like) {
     if (given == Py_None) return true;
@@ -81,11 +84,6 @@ bool reachable(PyObject* given, const Tensor* like) {
     const Tensor& t = THPVariable_Unpack(given);
     return !t.is_cuda() || t.device() == like->device();
 }
-// Allocation, stream and launch on the device of the tensors, whichever is current.
-struct OnDevice {
-    c10::cuda::CUDAGuard guard;
-    explicit OnDevice(const Tensor* t) : guard(t->device()) {}
-};
 P ptr(const Tensor* t) { return t->const_data_ptr(); }
 void* stream_of(const Tensor* t) { return c10::cuda::getCurrentCUDAStream(t->device().index()).stream(); }
 Tensor empty(at::IntArrayRef size, ScalarType type, const Tensor* like) {
@@ -108,7 +106,7 @@ PyObject* get(PyObject* dict, int key) { return PyDict_Check(dict) ? PyDict_GetI
 #define FAST(name) PyObject* name(PyObject*, PyObject* const* a, Py_ssize_t n)
 #define ORDINARY(cond) do { if (!(cond)) { PyErr_Clear(); Py_RETURN_NONE; } } while (0)      // (an integer beyond 64 bits is an error that is pending)
 // C++ exceptions become the Python ones that torch raises for them (torch.OutOfMemoryError for an allocation).
-#define GUARD(...) HANDLE_TH_ERRORS __VA_ARGS__ END_HANDLE_TH_ERRORS
+#define GUARD(...) try { __VA_ARGS__ } catch (...) { torch::translate_exception_to_python(std::current_exception()); return nullptr; }
 
 FAST(bind) {
     if (n != 2) { PyErr_SetString(PyExc_TypeError, "bind(name, address)"); return nullptr; }
@@ -135,7 +133,7 @@ PyObject* dense_gemv(void* f, const char* what, PyObject* const* a, Py_ssize_t n
     const bool fp4 = tile == 1;
     ORDINARY(K % per_block_k == 0 && N % tile == 0 && w->size(1) == (fp4 ? K / 2 : K) && s->size(0) == N / tile &&
              s->size(1) == K / per_block_k && w->stride(1) == 1 && s->stride(1) == 1 && together({x, w, s}) && good_out(a[3], {N}, x));
-    OnDevice here(x);
+    ORDINARY(current(x));
     Tensor made;
     void* y;
     if (a[3] == Py_None) { made = empty({N}, kBf16, x); y = made.mutable_data_ptr(); }
@@ -159,7 +157,7 @@ FAST(fp8_gemv_batched) { GUARD(
     const int64_t S = single ? 1 : x->size(0), row = single ? x->size(0) : x->size(1);
     ORDINARY(G >= 1 && row == G * K && rows % G == 0 && K % 128 == 0 && (rows / G) % 128 == 0 && s->size(0) == rows / 128 &&
              s->size(1) == K / 128 && w->stride(1) == 1 && s->stride(1) == 1 && x->stride(-1) == 1 && a[4] == Py_None && together({x, w, s}));
-    OnDevice here(x);
+    ORDINARY(current(x));
     Tensor y = single ? empty({rows}, kBf16, x) : empty({S, rows}, kBf16, x);
     const int rc = call(fn<int (*)(P, P, P, int, int, int64_t, int64_t, int, int, int64_t, int64_t, void*, void*)>(entry.fp8_e4m3_gemv_batched),
         ptr(x), ptr(w), ptr(s), (int)K, (int)(rows / G), w->stride(0), s->stride(0), (int)G, (int)S,
@@ -178,7 +176,7 @@ FAST(fp8_shared_swiglu) { GUARD(
     const int64_t K = x->size(0), H = w1->size(0), O = w2->size(0);
     ORDINARY(shape(*w1, {H, K}) && shape(*w3, {H, K}) && shape(*w2, {O, H}) && shape(*s1, {H / 128, K / 128}) &&
              shape(*s3, {H / 128, K / 128}) && shape(*s2, {O / 128, H / 128}) && together({x, w1, w3, w2, s1, s3, s2}) && good_out(a[4], {O}, x) && reachable(a[5], x));
-    OnDevice here(x);
+    ORDINARY(current(x));
     const double lg = PyFloat_AsDouble(a[2]), lu = PyFloat_AsDouble(a[3]);
     if (PyErr_Occurred()) return nullptr;
     const size_t need = fn<size_t (*)(int)>(entry.fp8_e4m3_shared_swiglu_workspace_bytes)((int)H);
@@ -230,7 +228,7 @@ FAST(grouped_gemv) { GUARD(
                  dense(get(a[0], kScale), kByte), dense(get(a[1], kScale), kByte), dense(get(a[2], kScale), kByte), 0, 0, 0};
     const Tensor *x = dense(a[3], kBf16), *r = dense(a[4], kF32);
     ORDINARY(x && r && e.ok(x, x->numel()) && shape(*r, {e.E}) && together({x, r}) && reachable(a[5], x) && reachable(a[6], x));
-    OnDevice here(x);
+    ORDINARY(current(x));
     Tensor out, ws;
     void* y = take(a[5], e.O, kBf16, x, out);
     void* w = take(a[6], (int64_t)fn<size_t (*)(int, int, int)>(entry.mxfp4_grouped_workspace_bytes)((int)e.E, (int)e.H, (int)e.O), kByte, x, ws);
@@ -247,7 +245,7 @@ FAST(grouped_gemv_ids) { GUARD(
     Experts e = bank_of(a[0]);
     const Tensor *ids = dense(a[1], kI32), *x = dense(a[2], kBf16), *r = dense(a[3], kF32);
     ORDINARY(ids && x && r && e.ok(x, x->numel()) && shape(*r, {ids->numel()}) && together({x, ids, r}) && reachable(a[4], x) && reachable(a[5], x));
-    OnDevice here(x);
+    ORDINARY(current(x));
     Tensor out, ws;
     const int k = (int)ids->numel();
     void* y = take(a[4], e.O, kBf16, x, out);
@@ -271,7 +269,7 @@ FAST(route_topk) { GUARD(
     if (PyErr_Occurred()) return nullptr;
     Tensor ids; Tensor w;
     ORDINARY(reachable(a[5], l) && reachable(a[6], l));
-    OnDevice here(l);
+    ORDINARY(current(l));
     ids = a[5] == Py_None ? empty({T, k}, kI32, l) : THPVariable_Unpack(a[5]);
     w = a[6] == Py_None ? empty({T, k}, kF32, l) : THPVariable_Unpack(a[6]);
     const int rc = call(fn<int (*)(P, int, int, int, int, float, float, void*, void*, void*)>(entry.mxfp4_moe_route_topk),
@@ -294,7 +292,7 @@ FAST(decode_layer) { GUARD(
     const double eps = PyFloat_AsDouble(a[5]), scaling = PyFloat_AsDouble(a[6]);
     if (PyErr_Occurred()) return nullptr;
     ORDINARY(k > 0);
-    OnDevice here(x);
+    ORDINARY(current(x));
     Tensor out, ws;
     void* y = take(a[7], e.O, kBf16, x, out);
     void* w = take(a[8], (int64_t)fn<size_t (*)(int, int, int)>(entry.mxfp4_moe_decode_workspace_bytes)(k, (int)e.H, (int)e.O), kByte, x, ws);
@@ -311,7 +309,7 @@ FAST(moe_forward) { GUARD(
     Experts e = bank_of(a[0]);
     const Tensor *x = dense(a[1], kBf16), *ids = dense(a[2], kI32), *w = dense(a[3], kF32);
     ORDINARY(x && ids && w && x->dim() == 2 && ids->dim() == 2 && e.ok(x, x->size(1)) && together({x, ids, w}) && reachable(a[4], x) && reachable(a[5], x));
-    OnDevice here(x);
+    ORDINARY(current(x));
     const int64_t T = x->size(0), K = x->size(1), k = ids->size(1);
     ORDINARY(shape(*ids, {T, k}) && shape(*w, {T, k}));
     Tensor out, ws;

@@ -1,10 +1,13 @@
 """ctypes loading of the shared libraries, with the exact C signatures of include/dsv4_b200.h."""
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import os
 import warnings
 from ctypes import c_int, c_int64, c_longlong, c_size_t, c_void_p, c_float
+
+import torch
 
 from .. import LIB_DIR, host_file, lib_path
 
@@ -74,7 +77,6 @@ def host():
     global _host
     if _host is None:
         import importlib.util
-        import torch  # noqa: F401  (the module links against its libraries)
         path = os.path.join(LIB_DIR, host_file() or "dsv4_host")
         try:
             spec = importlib.util.spec_from_file_location("dsv4_host", path)
@@ -128,19 +130,21 @@ BANK = ("w1p", "w3p", "w2p", "w1s", "w3s", "w2s")
 
 def elsewhere(x, **tensors):
     """Name of the first tensor that lives on another GPU than x, or None (None and host tensors are passed over)."""
+    here = x.get_device()
     for name, t in tensors.items():
-        if t is not None and t.is_cuda and t.device != x.device:
+        if t is not None and t.is_cuda and t.get_device() != here:
             return name
     return None
 
 
+_CURRENT = contextlib.nullcontext()
+
+
 def on_device(x):
     """Context in which the GPU of x is the current one: a launch goes to the current device, whatever its stream."""
-    import torch
-    return torch.cuda.device(x.device)
+    return _CURRENT if torch.cuda.current_device() == x.get_device() else torch.cuda.device(x.device)
 
 
 def stream_ptr(device, stream=None) -> c_void_p:
-    import torch
     s = stream if stream is not None else torch.cuda.current_stream(device)
     return c_void_p(s.cuda_stream)

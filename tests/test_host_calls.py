@@ -98,3 +98,18 @@ def test_operators_do_without_the_module(rt, pkg, monkeypatch, tmp_path, content
 
 def test_module_is_named_for_its_torch(pkg):
     assert torch.__version__ in pkg.host_file()
+
+
+def test_device_that_is_not_current_is_made_so(rt, monkeypatch):
+    """The call then goes through Python, which enters the tensors' device; on the current one it enters nothing."""
+    capi = importlib.import_module("dsv4_b200.runtime._capi")
+    entered = []
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 0)
+    monkeypatch.setattr(torch.cuda, "device", lambda d: entered.append(d))
+    with FakeTensorMode():
+        here, other = torch.empty(1, device="cuda:0"), torch.empty(1, device="cuda:1")
+    with capi.on_device(here):
+        assert not entered
+    capi.on_device(other)
+    assert entered == [torch.device("cuda:1")]
+    assert capi.elsewhere(here, a=None, b=here, c=torch.zeros(1), d=other) == "d"
