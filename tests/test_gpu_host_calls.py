@@ -91,3 +91,47 @@ def test_same_bits_through_ctypes(ops, capi, monkeypatch, name):
         through_ctypes = tensors(ops[name][1]())
     assert [(t.dtype, t.shape, t.device) for t in native] == [(t.dtype, t.shape, t.device) for t in through_ctypes]
     assert all(torch.equal(a.view(torch.uint8), b.view(torch.uint8)) for a, b in zip(native, through_ctypes))
+
+
+@pytest.mark.parametrize("kind", ["mxfp4", "fp8", "fp8_batched"])
+def test_calls_out_of_the_ordinary(rt, qz, capi, kind):
+    """Strides, an explicit stream and given outputs give the ordinary call's bits, whichever way they take; what does not fit
+    raises."""
+    g = torch.Generator(device=DEV).manual_seed(9)
+    w = torch.randn(256, K, generator=g, device=DEV) * 0.02
+    p, s = qz.quantize_mxfp4(w.to(torch.bfloat16)) if kind == "mxfp4" else qz.quantize_fp8_block128(w)
+    op = {"mxfp4": rt.mxfp4_gemv, "fp8": rt.fp8_e4m3_gemv, "fp8_batched": rt.fp8_e4m3_gemv_batched}[kind]
+    x = torch.randn(K, generator=g, device=DEV).to(torch.bfloat16)
+    want = op(p, s, x).view(torch.int16)
+    apart = torch.zeros(256, p.shape[1] + 48, dtype=p.dtype, device=DEV)[:, : p.shape[1]].copy_(p)      # rows with gaps
+    column = torch.zeros(K, 2, dtype=x.dtype, device=DEV)[:, 0].copy_(x)                                # every second element
+    turned = torch.zeros(p.shape[1], 256, dtype=p.dtype, device=DEV).t().copy_(p)                       # rows not dense
+    odd = torch.zeros(K + 1, dtype=x.dtype, device=DEV)[1:].copy_(x)                                    # not 16-byte aligned
+    side = torch.cuda.Stream(device=DEV)
+    side.wait_stream(torch.cuda.current_stream(DEV))
+    out = torch.empty(256, dtype=torch.bfloat16, device=DEV)
+    results = [op(apart, s, x), op(p, s, column), op(turned, s, x), op(p, s, x, stream=side), op(p, s, x, out=out)]
+    torch.cuda.synchronize()
+    assert results[-1].data_ptr() == out.data_ptr()
+    assert all(torch.equal(r.view(torch.int16), want) for r in results)
+    if kind == "fp8_batched":
+        with pytest.raises(RuntimeError):
+            op(p, s, odd)
+    else:
+        err = (op(p, s, odd).float() - want.view(torch.bfloat16).float()).abs().max()      # the byte-wise kernel: FP32 sums, where the other's are fp16 inside a block; bf16 rounding of both is 2^-8
+        assert err <= 2 ** -7 * want.view(torch.bfloat16).float().abs().max()
+    for bad in (dict(out=out.float()), dict(out=out[:128]), dict(out=out.cpu())):
+        with pytest.raises(RuntimeError):
+            op(p, s, x, **bad)
+    for args in ((p, s[:1], x), (p, s, x[:-128]), (p.int(), s, x), (p, s, x.float()), (p.cpu(), s, x)):
+        with pytest.raises(RuntimeError):
+            op(*args)
+
+
+def test_workspace_that_is_too_small_is_refused(rt, qz, ops):
+    call = ops["fp8_shared_swiglu"][1]
+    good = call(workspace=torch.empty(2 * H, dtype=torch.uint8, device=DEV))
+    assert torch.equal(good.view(torch.int16), call().view(torch.int16))
+    for ws in (torch.empty(2 * H - 1, dtype=torch.uint8, device=DEV), torch.empty(2 * H, dtype=torch.uint8)):
+        with pytest.raises(RuntimeError):
+            call(workspace=ws)
