@@ -56,3 +56,31 @@ def test_grouping_by_one_block_and_by_a_cluster(rt, qz, path, n_pairs):
 def test_tiles_of_few_tokens(rt, qz, counts, K, H):
     """At most 16 pairs per expert on average: tiles of up to 32 tokens, five stages, more tiles than one for a busy expert."""
     run_case(rt, qz, "mxf4", counts, K=K, H=H, O=K, seed=sum(counts) + K)
+
+
+@pytest.mark.parametrize("K,H", [(256, 256), (1280, 512), (2304, 768)])
+@pytest.mark.parametrize("counts", [[24] * 4, [25] * 4, [33, 1, 0, 60], [0] * 7 + [97]])
+def test_five_terms_on_either_side_of_the_small_tiles(rt, qz, counts, K, H):
+    """The path "fp16": tiles of up to 32 tokens to an average of 24 pairs per expert, of up to 96 beyond, reduction lengths whose
+    scale rows are 8-byte aligned only; scale bytes 0xFF contribute nothing, and a token that is not finite leaves the others alone."""
+    g = torch.Generator().manual_seed(sum(counts) + K)
+    E, T = len(counts), sum(counts)
+    bank = qz.make_expert_bank(E, K, H, "cpu", seed=K)
+    bank["w1s"][:, 1::5, 2], bank["w2s"][:, ::7, 1] = 255, 255
+    ids = torch.repeat_interleave(torch.arange(E), torch.tensor(counts)).to(torch.int32)[:, None].contiguous()
+    w = torch.rand(T, 1, generator=g) + 0.5
+    x = torch.randn(T, K, generator=g).to(torch.bfloat16)
+    x[T // 2, 7] = float("inf")
+    out = rt.moe_forward({n: v.to(DEV) for n, v in bank.items()}, x.to(DEV), ids.to(DEV), w.to(DEV), path="fp16").float().cpu()
+    assert rt.moe_device_status() == 0
+    assert not torch.isfinite(out[T // 2]).any()
+    rest = torch.arange(T) != T // 2
+    clean = {n: v.clone() for n, v in bank.items()}
+    for n in ("w1", "w2"):                               # the same weights with those blocks zero
+        zero = (clean[n + "s"] == 255).repeat_interleave(16, -1)
+        clean[n + "p"][zero] = 0
+        clean[n + "s"][clean[n + "s"] == 255] = 127
+    ref = oracle.moe_layer_ref(x[rest], clean, ids[rest].numpy(), w[rest].numpy())
+    got = out[rest].numpy()
+    err, cos = oracle.max_abs_rel(got, ref), oracle.cosine(got, ref)
+    assert err <= 5e-3 and cos >= 0.99999, f"{counts}: max-abs/inf {err:.3e} cosine {cos:.7f}"       # bf16 output rounding: 2^-9 of a value
