@@ -262,11 +262,14 @@ static int moe_forward_impl(int path, const __nv_bfloat16* x, const uint8_t* ban
     aa.q = ws + m.xq; aa.s = ws + m.xs;
     const MoePeerIn no_peers = {};
     const MoePeerIn& pin = peer_in ? *peer_in : no_peers;
-    // a warp per 256 elements, at most eight blocks of eight warps per SM
-    const long long blocks = ((long long)n_tokens * (K_in / 256) + 7) / 8;
-    const dim3 agrid((unsigned)(blocks < 8LL * grid ? blocks : 8LL * grid)), ablock(256);
-    if (path == 1) launch_k(peer_in ? moe_act_mxf4_kernel<true, 3> : moe_act_mxf4_kernel<false, 3>, agrid, ablock, 0, stream, 1, aa, pin);
-    else launch_k(peer_in ? moe_act_mxf4_kernel<true, 5> : moe_act_mxf4_kernel<false, 5>, agrid, ablock, 0, stream, 1, aa, pin);
+    // A warp per 256 elements, at most eight blocks of eight warps per SM; where that fills the SMs, a warp per 1024, two blocks.
+    const bool many = n_tokens >= kActManyTokens;
+    const long long pieces = (long long)n_tokens * (many ? (K_in + 1023) / 1024 : K_in / 256), blocks = (pieces + 7) / 8, most = (many ? 2LL : 8LL) * grid;
+    const dim3 agrid((unsigned)(blocks < most ? blocks : most)), ablock(256);
+#define DSV4_ACT(KERNEL, TERMS) launch_k(peer_in ? KERNEL<true, TERMS> : KERNEL<false, TERMS>, agrid, ablock, 0, stream, 1, aa, pin)
+    if (path == 1) { if (many) DSV4_ACT(moe_act_blocks_kernel, 3); else DSV4_ACT(moe_act_mxf4_kernel, 3); }
+    else { if (many) DSV4_ACT(moe_act_blocks_kernel, 5); else DSV4_ACT(moe_act_mxf4_kernel, 5); }
+#undef DSV4_ACT
     stage_mark(stream, 2);
     MoeQMaps up_maps, down_maps;
     cudaError_t err = weight_map(&up_maps.wa, bank_W1_packed, (long long)n_experts * hidden, K_in);

@@ -184,4 +184,34 @@ __device__ __forceinline__ void moe_quantize_mxfp4(float (&v)[8], uint32_t (&wor
     }
 }
 
+// The same of a whole block by one lane.
+template <int TERMS>
+__device__ __forceinline__ void moe_quantize_block(float (&v)[32], uint4 (&word)[TERMS], uint32_t (&scale)[TERMS]) {
+#pragma unroll
+    for (int t = 0; t < TERMS; ++t) {
+        uint32_t m = 0;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) m = max(m, __float_as_uint(v[i]) & 0x7fffffffu);
+        int e = (int)((m + 0x003fffffu) >> 23) - 129;
+        e = min(max(e, -127), 127);
+        const float inv = __uint_as_float((uint32_t)min(max(127 - e, 1), 254) << 23);
+        const float sc = __uint_as_float((uint32_t)max(e + 127, 1) << 23);
+        uint32_t r[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            uint16_t packed;
+            asm("{\n .reg .b8 b;\n cvt.rn.satfinite.e2m1x2.f32 b, %2, %1;\n mov.b16 %0, {b, 0};\n}"
+                : "=h"(packed) : "f"(v[2 * i] * inv), "f"(v[2 * i + 1] * inv));
+            if (t + 1 < TERMS) {
+                const float2 back = e2m1x2_to_float2(packed);
+                v[2 * i] = fmaf(-back.x, sc, v[2 * i]);
+                v[2 * i + 1] = fmaf(-back.y, sc, v[2 * i + 1]);
+            }
+            r[i >> 2] |= (uint32_t)(packed & 0xff) << (8 * (i & 3));
+        }
+        word[t] = make_uint4(r[0], r[1], r[2], r[3]);
+        scale[t] = TERMS > 3 && t == 0 && m >= 0x7f800000u ? 255u : (uint32_t)(e + 127);
+    }
+}
+
 }  // namespace dsv4

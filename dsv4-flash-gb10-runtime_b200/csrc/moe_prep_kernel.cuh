@@ -204,4 +204,71 @@ __global__ void __launch_bounds__(256, 6) moe_act_mxf4_kernel(const MoeActArgs a
     }
 }
 
+// The same for many tokens: a lane takes a whole block of 32 elements, a warp 1024 of a row.  What bounds it: HBM, 2 K bytes in and
+// terms x 17 K / 32 bytes out per pair.  The form above spends the time on its stores (four bytes per lane, term and pair) and on the
+// maxima of a block, two shuffles per term; here a term of a pair is one 16-byte store per lane and a block has no shuffles.  Measured
+// (K 4096, six pairs a token, the form above -> this one): 4 096 tokens, three terms 57 -> 41 us, five 77 -> 63; 16 384 tokens, three
+// terms 197 -> 156 (1.3 GB out and 0.13 in: 9.3 TB/s, part of the output still in L2).
+// kActManyTokens: a quarter of the warps, each with four times the work, has to fill the SMs: 64 tokens 7.0 us above, 9.0 here (five
+// terms 8.2, 10.2), 128 tokens 8.2-9.0 and 9.0, 256 tokens 10.2-10.7 and 9.1 (five terms 11.0-12.3, 10.2-11.2).
+constexpr int kActManyTokens = 256;
+
+// The same bytes as above.
+template <bool PEER, int TERMS>
+__global__ void __launch_bounds__(256, 2) moe_act_blocks_kernel(const MoeActArgs a, const MoePeerIn in) {
+    const int lane = threadIdx.x & 31;
+    const int per_row = (a.K + 1023) >> 10, warps = gridDim.x * (blockDim.x >> 5), n_pieces = a.n_tokens * per_row;
+    const long long term_q = a.n_pairs * (a.K >> 1), term_s = a.n_pairs * (a.K >> 5);
+    auto slots_of = [&](int w) -> int {                        // lane j: slot of the j-th pair of the piece's token
+        return w < n_pieces && lane < a.k ? __ldcg(a.pair_slot + (long long)(w / per_row) * a.k + lane) : -1;
+    };
+    auto fetch = [&](int w, uint4 (&u)[4]) {
+        const int row = w / per_row, at = (w - row * per_row) * 1024 + lane * 32;
+        if (w < n_pieces && at < a.K && (!PEER || moe_act_wanted(a, row))) {
+            const uint4* src = reinterpret_cast<const uint4*>(moe_act_row<PEER>(a, in, row) + at);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) u[i] = __ldcs(src + i);
+        }
+    };
+    if (PEER) pdl_wait();
+    uint4 cur[4] = {}, nxt[4] = {};
+    int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    fetch(w, cur);
+    if (!PEER) pdl_wait();
+    pdl_launch_dependents();                               // after the wait: the next kernel reads the tile tables before its own
+    int slots = slots_of(w);
+    for (; w < n_pieces; w += warps) {
+        fetch(w + warps, nxt);
+        const int next_slots = slots_of(w + warps);
+        float v[32];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const uint32_t u[4] = {cur[i].x, cur[i].y, cur[i].z, cur[i].w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                v[8 * i + 2 * j] = __uint_as_float(u[j] << 16);
+                v[8 * i + 2 * j + 1] = __uint_as_float(u[j] & 0xffff0000u);
+            }
+        }
+        uint4 word[TERMS];
+        uint32_t scale[TERMS];
+        moe_quantize_block<TERMS>(v, word, scale);
+        const int row = w / per_row, at = (w - row * per_row) * 1024 + lane * 32;
+        for (int j = 0; j < a.k; ++j) {
+            const int slot = j < 32 ? __shfl_sync(kFullMask, slots, j) : __ldcg(a.pair_slot + (long long)row * a.k + j);
+            if (slot < 0 || at >= a.K) continue;
+            uint8_t* q = a.q + (long long)slot * (a.K >> 1) + (at >> 1);
+            uint8_t* sb = a.s + (long long)slot * (a.K >> 5) + (at >> 5);
+#pragma unroll
+            for (int t = 0; t < TERMS; ++t) {
+                *reinterpret_cast<uint4*>(q + t * term_q) = word[t];
+                sb[t * term_s] = (uint8_t)scale[t];
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) cur[i] = nxt[i];
+        slots = next_slots;
+    }
+}
+
 }  // namespace dsv4

@@ -84,3 +84,31 @@ def test_five_terms_on_either_side_of_the_small_tiles(rt, qz, counts, K, H):
     got = out[rest].numpy()
     err, cos = oracle.max_abs_rel(got, ref), oracle.cosine(got, ref)
     assert err <= 5e-3 and cos >= 0.99999, f"{counts}: max-abs/inf {err:.3e} cosine {cos:.7f}"       # bf16 output rounding: 2^-9 of a value
+
+
+@pytest.mark.parametrize("path", ["mxf4", "fp16"])
+@pytest.mark.parametrize("T,K", [(256, 256), (256, 1280), (257, 4096), (700, 2304)])
+def test_quantised_activations_of_many_tokens(rt, qz, path, T, K):
+    """From 256 tokens on x is quantised 1024 elements to a warp: rows that are less than that or not a multiple of it.  A token's result
+    is bit for bit that of a call with 255 tokens, which takes the other kernel (same tiles otherwise: more than 128 pairs an expert)."""
+    g = torch.Generator().manual_seed(T + K)
+    bank = qz.make_expert_bank(4, K, 256, "cpu", seed=K)
+    ids = torch.stack([torch.randperm(4, generator=g)[:3] for _ in range(T)]).to(torch.int32)
+    w = torch.rand(T, 3, generator=g) + 0.5
+    x = (torch.randn(T, K, generator=g) * torch.randn(T, 1, generator=g).mul(3).exp2()).to(torch.bfloat16)
+    x[3, :64], x[4] = 0, 0
+    x[5, 33] = float("inf")
+    dev = {n: v.to(DEV) for n, v in bank.items()}
+    run = lambda n: rt.moe_forward(dev, x[:n].to(DEV), ids[:n].contiguous().to(DEV), w[:n].contiguous().to(DEV), path=path).float().cpu()
+    many, few = run(T), run(255)
+    assert rt.moe_device_status() == 0
+    assert torch.equal(torch.nan_to_num(many[:255], nan=1.5), torch.nan_to_num(few, nan=1.5))      # the infinite token too
+    rest = torch.arange(T) != 5
+    assert torch.isfinite(many[rest]).all()
+    ref = oracle.moe_layer_ref(x[rest], bank, ids[rest].numpy(), w[rest].numpy())
+    got = many[rest].numpy()
+    scale = abs(ref).max(axis=1, keepdims=True) + 1e-30          # every token by itself: their sizes differ by powers of two
+    # bf16 output rounding, 2^-9 of a value; with three terms also five standard deviations of 2.2e-3 of a row's rms (1e-3 of x and 2e-3
+    # of the intermediate), the row's largest value being at least twice the rms: 2e-3 + 5.5e-3
+    err, tight = (abs(got - ref) / scale).max(), 5e-3 if path == "fp16" else 8e-3
+    assert err <= tight, f"{path} {T}: max-abs/inf of a token {err:.3e}"
