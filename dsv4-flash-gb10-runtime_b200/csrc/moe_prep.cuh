@@ -11,10 +11,11 @@ constexpr int kMoeMaxExperts = 1024;
 constexpr int kMoeTileRows = 128;      // weight rows per tensor-core tile (the MMA's M)
 constexpr int kMoeTileTokens = 128;    // tokens per tile at most, fp16 path
 
-// The tokens of a tile are padded to one of five column counts (the boxes the activation copies are encoded for).
-constexpr int kMoeWidths = 5;
-__host__ __device__ __forceinline__ int moe_width_index(int n) { return n <= 16 ? 0 : n <= 32 ? 1 : n <= 64 ? 2 : n <= 96 ? 3 : 4; }
-__host__ __device__ __forceinline__ int moe_width(int index, int cap) { return index == 4 ? cap : index == 3 ? 96 : 16 << index; }
+// The tokens of a tile are padded to one of seven column counts (the boxes the activation copies are encoded for): a multiple of 16, or
+// all that a tile may have.  (48 and 80 among them: 256 experts of 4096, 2048, top 6, 1 800 tokens 724 -> 687 us, 2 800 tokens 831 -> 795.)
+constexpr int kMoeWidths = 7;
+__host__ __device__ __forceinline__ int moe_width_index(int n) { return n <= 16 ? 0 : n <= 96 ? (n - 1) >> 4 : 6; }
+__host__ __device__ __forceinline__ int moe_width(int index, int cap) { return index == 6 ? cap : 16 * (index + 1); }
 // The n tokens of an expert are cut into the fewest tiles of at most `cap`, all but the last of one size: tiles of one
 // size finish together.
 __host__ __device__ __forceinline__ int moe_token_tiles(int n, int cap) { return (n + cap - 1) / cap; }
