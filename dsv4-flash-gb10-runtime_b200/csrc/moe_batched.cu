@@ -5,7 +5,8 @@
 // Pipeline on the caller's stream: pairs grouped by expert; grouped GEMM 1 (gate/up + SwiGLU) and grouped GEMM 2
 // (down, router weight applied) on tcgen05 tensor cores; per-token sum in the router's order.  Two tensor-core
 // paths: block-scaled MXFP4 MMAs fed with the packed weights as stored (moe_gemm_mxf4.cuh; activations as three
-// MXFP4 terms; the default), and fp16 MMAs with the weights dequantised into tensor memory (moe_gemm_kernel.cuh).
+// MXFP4 terms; the default), and "fp16" for more precise activations: the same kernel with three E4M3 terms, or fp16 MMAs with the
+// weights dequantised into tensor memory (moe_gemm_kernel.cuh).
 // Nothing is allocated; all scratch lives in the caller's workspace.
 #include "moe_gemm_kernel.cuh"
 #include "moe_prep_kernel.cuh"
@@ -28,6 +29,8 @@ struct WorkspaceMap {
     size_t offsets, tiles_up, tiles_down, pair_slot, slot_w, y;      // both paths
     size_t xq, xs, mq, ms;                                          // block-scaled path
     size_t xh, xexp, typical, mid, mid_exp;                         // fp16 path (the same bytes)
+    size_t xq8, xs8, mq8, ms8;                                      // its form on the block-scaled MMAs (the same bytes; x in those of y)
+    bool fits8;                                                     // which hold it
     size_t total;
 };
 
@@ -55,6 +58,15 @@ WorkspaceMap map_workspace(long long T, int k, int K, int H, int O, int E) {
     m.mid = c.take((size_t)P * H * 2);
     m.mid_exp = c.take((size_t)P * 4);
     m.total = c.off > mxf4_end ? c.off : mxf4_end;
+    // three E4M3 terms: x is done with before the down GEMM writes y
+    c.off = m.y;
+    m.xq8 = c.take((size_t)3 * P * K);
+    m.xs8 = c.take((size_t)3 * P * K / 32);
+    m.fits8 = c.off <= shared;
+    c.off = shared;
+    m.mq8 = c.take((size_t)3 * P * H);
+    m.ms8 = c.take((size_t)3 * P * H / 32);
+    m.fits8 = m.fits8 && c.off <= m.total;
     return m;
 }
 
@@ -133,7 +145,7 @@ cudaError_t launch_k(void (*kernel)(Params...), dim3 grid, dim3 block, size_t sm
 typedef CUresult (*EncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                 const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                 CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-cudaError_t box_map(CUtensorMap* map, CUtensorMapDataType type, int elem, const void* base, int rank, const cuuint64_t* dim,
+cudaError_t box_map(CUtensorMap* map, CUtensorMapDataType type, int row_bytes, const void* base, int rank, const cuuint64_t* dim,
                     const cuuint32_t* box) {
     static EncodeTiled encode = [] {
         void* p = nullptr;
@@ -142,7 +154,7 @@ cudaError_t box_map(CUtensorMap* map, CUtensorMapDataType type, int elem, const 
         return reinterpret_cast<EncodeTiled>(p);
     }();
     if (!encode) return cudaErrorNotSupported;
-    const cuuint64_t stride[2] = {dim[0] * elem, dim[0] * elem * dim[1]};
+    const cuuint64_t stride[2] = {(cuuint64_t)row_bytes, (cuuint64_t)row_bytes * dim[1]};
     const cuuint32_t step[3] = {1, 1, 1};
     const CUresult r = encode(map, type, (cuuint32_t)rank, const_cast<void*>(base), dim, stride, box, step,
                               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -153,15 +165,21 @@ cudaError_t box_map(CUtensorMap* map, CUtensorMapDataType type, int elem, const 
 cudaError_t weight_map(CUtensorMap* map, const uint8_t* base, long long rows, int K) {
     const cuuint64_t dim[2] = {(cuuint64_t)(K / 2), (cuuint64_t)rows};
     const cuuint32_t box[2] = {128, kMoeTileRows};
-    return box_map(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, base, 2, dim, box);
+    return box_map(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, K / 2, base, 2, dim, box);
 }
-// three MXFP4 terms [3][P][K / 2]: half a tile's columns of every term
-cudaError_t term_maps(CUtensorMap (&map)[kMoeWidths], const uint8_t* base, long long P, int K, int cap) {
+// the same laid down in groups of 8 bytes and 8 of padding: 128 elements a row (base 32-byte aligned)
+cudaError_t weight_map_padded(CUtensorMap* map, const uint8_t* base, long long rows, int K) {
+    const cuuint64_t dim[2] = {(cuuint64_t)K, (cuuint64_t)rows};
+    const cuuint32_t box[2] = {128, kMoeTileRows};
+    return box_map(map, CU_TENSOR_MAP_DATA_TYPE_16U4_ALIGN16B, K / 2, base, 2, dim, box);
+}
+// three terms [3][P][row_bytes]: half a tile's columns of every term
+cudaError_t term_maps(CUtensorMap (&map)[kMoeWidths], const uint8_t* base, long long P, int row_bytes, int cap) {
     cudaError_t err = cudaSuccess;
     for (int i = 0; i < kMoeWidths && err == cudaSuccess; ++i) {
-        const cuuint64_t dim[3] = {(cuuint64_t)(K / 2), (cuuint64_t)P, kQTerms};
+        const cuuint64_t dim[3] = {(cuuint64_t)row_bytes, (cuuint64_t)P, kQTerms};
         const cuuint32_t box[3] = {128, (cuuint32_t)moe_width(i, cap) / 2, kQTerms};
-        err = box_map(&map[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, base, 3, dim, box);
+        err = box_map(&map[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, row_bytes, base, 3, dim, box);
     }
     return err;
 }
@@ -171,7 +189,7 @@ cudaError_t half_maps(CUtensorMap (&map)[kMoeWidths], const __half* base, long l
     for (int i = 0; i < kMoeWidths && err == cudaSuccess; ++i) {
         const cuuint64_t dim[2] = {(cuuint64_t)K, (cuuint64_t)P};
         const cuuint32_t box[2] = {64, (cuuint32_t)moe_width(i, cap)};
-        err = box_map(&map[i], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, base, 2, dim, box);
+        err = box_map(&map[i], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, K * 2, base, 2, dim, box);
     }
     return err;
 }
@@ -268,14 +286,18 @@ static int moe_forward_impl(int path, const __nv_bfloat16* x, const uint8_t* ban
 
     MoeGroupArgs ga;
     ga.ids = ids; ga.weights = weights; ga.n_pairs = P; ga.n_experts = n_experts; ga.g = g; ga.status = status;
-    const int rows_up = path == 1 ? kQTileRowsUp : kMoeTileRows, rows_down = path == 1 ? kQTileRowsDown : 2 * kMoeTileRows;
+    // Path 0 runs on the block-scaled MMAs too, with E4M3 terms, where its operands have room and the TMA can lay the weights down.
+    const bool fp8 = path == 0 && !peer_in && m.fits8 && P <= (long long)kQMostTokensFp8 * n_experts &&
+                     ((reinterpret_cast<uintptr_t>(bank_W1_packed) | reinterpret_cast<uintptr_t>(bank_W3_packed) | reinterpret_cast<uintptr_t>(bank_W2_packed)) & 31u) == 0;
+    const bool pairs = path == 1 || fp8;                   // tiles of CTA pairs
+    const int rows_up = pairs ? kQTileRowsUp : kMoeTileRows, rows_down = pairs ? kQTileRowsDown : 2 * kMoeTileRows;
     ga.m_tiles_up = hidden / rows_up; ga.m_tiles_down = (out_dim + rows_down - 1) / rows_down;
     // (Pairs of the whole batch: where ids are negative, as under expert parallelism, the experts here have fewer, and the larger tiles
     // are taken although the smaller would do.  Eight ranks emulated on one GPU, 128 to 1024 tokens: 1 % of the layer's time.)
     const int cap16 = P <= (long long)kTmFewTokens * n_experts ? 64 : kMoeTileTokens;      // tokens per tile, fp16 path
-    const bool few = P <= (long long)kQFewTokens * n_experts;
+    const bool few = P <= (long long)(fp8 ? kQFewTokensFp8 : kQFewTokens) * n_experts;
     const int cap_q = few ? 32 : kQTok;                                                    // tokens per tile, block-scaled path
-    ga.tile_tokens = path == 1 ? cap_q : cap16;
+    ga.tile_tokens = pairs ? cap_q : cap16;
     launch_k(moe_group_kernel, dim3(P > kGroupOneBlockPairs ? kGroupCluster : 1), dim3(kPrepThreads), 0, stream, P > kGroupOneBlockPairs ? kGroupCluster : 1, ga);
     stage_mark(stream, 1);
 
@@ -287,42 +309,55 @@ static int moe_forward_impl(int path, const __nv_bfloat16* x, const uint8_t* ban
     const MoePeerIn no_peers = {};
     const MoePeerIn& pin = peer_in ? *peer_in : no_peers;
     cudaError_t err = cudaSuccess;
-    if (path == 1) {
+    if (pairs) {
         // ---- block-scaled MXFP4 tensor-core path; a warp per 256 elements, at most eight blocks of eight warps per SM; where that
         // fills the SMs, a warp per 1024, two blocks
         const bool many = !peer_in && moe_act_by_blocks(n_tokens, K_in);
-        const long long pieces = (long long)n_tokens * (many ? (K_in + 1023) / 1024 : K_in / 256), blocks = (pieces + 7) / 8;
-        const long long most = (many ? 2LL : 8LL) * grid;
+        const long long pieces = (long long)n_tokens * (fp8 ? (K_in + 511) / 512 : many ? (K_in + 1023) / 1024 : K_in / 256), blocks = (pieces + 7) / 8;
+        const long long most = (fp8 ? 4LL : many ? 2LL : 8LL) * grid;
+        uint8_t* const mid_q = ws + (fp8 ? m.mq8 : m.mq);
+        uint8_t* const mid_s = ws + (fp8 ? m.ms8 : m.ms);
+        if (fp8) { aa.q = ws + m.xq8; aa.s = ws + m.xs8; }
         const dim3 agrid((unsigned)(blocks < most ? blocks : most)), ablock(256);
-        if (many) launch_k(moe_act_blocks_kernel, agrid, ablock, 0, stream, 1, aa);
+        if (fp8) launch_k(moe_act_fp8_kernel, agrid, ablock, 0, stream, 1, aa);
+        else if (many) launch_k(moe_act_blocks_kernel, agrid, ablock, 0, stream, 1, aa);
         else launch_k(peer_in ? moe_act_mxf4_kernel<true> : moe_act_mxf4_kernel<false>, agrid, ablock, 0, stream, 1, aa, pin);
         stage_mark(stream, 2);
         MoeQMaps up_maps, down_maps;
-        err = weight_map(&up_maps.wa, bank_W1_packed, (long long)n_experts * hidden, K_in);
-        if (err == cudaSuccess) err = weight_map(&up_maps.wb, bank_W3_packed, (long long)n_experts * hidden, K_in);
-        if (err == cudaSuccess) err = term_maps(up_maps.act, aa.q, P, K_in, cap_q);
-        if (err == cudaSuccess) err = weight_map(&down_maps.wa, bank_W2_packed, (long long)n_experts * out_dim, hidden);
+        auto weights = [&](CUtensorMap* map, const uint8_t* base, long long rows, int K) {
+            if (err == cudaSuccess) err = fp8 ? weight_map_padded(map, base, rows, K) : weight_map(map, base, rows, K);
+        };
+        weights(&up_maps.wa, bank_W1_packed, (long long)n_experts * hidden, K_in);
+        weights(&up_maps.wb, bank_W3_packed, (long long)n_experts * hidden, K_in);
+        weights(&down_maps.wa, bank_W2_packed, (long long)n_experts * out_dim, hidden);
         down_maps.wb = down_maps.wa;
-        if (err == cudaSuccess) err = term_maps(down_maps.act, ws + m.mq, P, hidden, cap_q);
+        if (err == cudaSuccess) err = term_maps(up_maps.act, aa.q, P, fp8 ? K_in : K_in / 2, cap_q);
+        if (err == cudaSuccess) err = term_maps(down_maps.act, mid_q, P, fp8 ? hidden : hidden / 2, cap_q);
         MoeQGemmArgs qu;
         qu.wa_s = bank_W1_scale; qu.wb_s = bank_W3_scale; qu.rows = hidden; qu.K = K_in; qu.n_experts = n_experts;
-        qu.act_s = aa.s; qu.n_pairs = P; qu.g = g; qu.mid_q = ws + m.mq; qu.mid_s = ws + m.ms; qu.y = nullptr;
+        qu.act_s = aa.s; qu.n_pairs = P; qu.g = g; qu.mid_q = mid_q; qu.mid_s = mid_s; qu.y = nullptr;
         MoeQGemmArgs qd = qu;
-        qd.wa_s = bank_W2_scale; qd.wb_s = nullptr; qd.rows = out_dim; qd.K = hidden; qd.act_s = ws + m.ms; qd.y = y;
-        auto gemms = [&](auto up_kernel, auto down_kernel, uint32_t smem, uint32_t most, int (&up_done)[64], int (&down_done)[64]) {
-            if (err == cudaSuccess) err = allow_smem(up_kernel, most, up_done);
-            if (err == cudaSuccess) err = allow_smem(down_kernel, most, down_done);
+        qd.wa_s = bank_W2_scale; qd.wb_s = nullptr; qd.rows = out_dim; qd.K = hidden; qd.act_s = mid_s; qd.y = y;
+        auto gemms = [&](auto format, auto cap) {
+            using F = decltype(format);
+            constexpr int CAP = decltype(cap)::value;
+            auto up_kernel = moe_gemm_mxf4_kernel<0, CAP, F>;
+            auto down_kernel = moe_gemm_mxf4_kernel<1, CAP, F>;
+            static int up_done[64] = {0}, down_done[64] = {0};
+            const uint32_t smem = MoeQShape<F, CAP>::smem(n_experts), most_smem = MoeQShape<F, CAP>::smem(kMoeMaxExperts);
+            if (err == cudaSuccess) err = allow_smem(up_kernel, most_smem, up_done);
+            if (err == cudaSuccess) err = allow_smem(down_kernel, most_smem, down_done);
             if (err != cudaSuccess) return;
             launch_k(up_kernel, dim3(grid & ~1), dim3(kQThreads), smem, stream, 2, up_maps, qu);
             stage_mark(stream, 3);
             stage_mark(stream, 4);
             launch_k(down_kernel, dim3(grid & ~1), dim3(kQThreads), smem, stream, 2, down_maps, qd);
         };
-        static int up_few[64] = {0}, down_few[64] = {0}, up_most[64] = {0}, down_most[64] = {0};
-        if (few) gemms(moe_gemm_mxf4_kernel<0, 32>, moe_gemm_mxf4_kernel<1, 32>, MoeQShape<32>::smem(n_experts),
-                       MoeQShape<32>::smem(kMoeMaxExperts), up_few, down_few);
-        else gemms(moe_gemm_mxf4_kernel<0, kQTok>, moe_gemm_mxf4_kernel<1, kQTok>, MoeQShape<kQTok>::smem(n_experts),
-                   MoeQShape<kQTok>::smem(kMoeMaxExperts), up_most, down_most);
+        const std::integral_constant<int, 32> cap_few;
+        const std::integral_constant<int, kQTok> cap_most;
+        if (fp8) { if (few) gemms(MoeQFp8(), cap_few); else gemms(MoeQFp8(), cap_most); }
+        else if (few) gemms(MoeQFp4(), cap_few);
+        else gemms(MoeQFp4(), cap_most);
     } else {
         // ---- fp16 tensor-core path: weights dequantised into tensor memory
         const int blocks = (n_tokens + kActRows - 1) / kActRows;
@@ -396,8 +431,8 @@ DSV4_API int mxfp4_moe_forward(const __nv_bfloat16* x, const uint8_t* bank_W1_pa
                             stream);
 }
 
-// The same with the tensor-core path chosen by the caller: 0 = fp16 MMAs with in-kernel dequantisation (moe_gemm.cuh
-// says what they hold exactly), 1 = block-scaled MXFP4 MMAs (weights as stored, activations as three MXFP4 terms).
+// The same with the tensor-core path chosen by the caller: 0 = "fp16" (moe_gemm.cuh says what its two forms
+// hold exactly), 1 = block-scaled MXFP4 MMAs (weights as stored, activations as three MXFP4 terms).
 DSV4_API int mxfp4_moe_forward_path(int path, const __nv_bfloat16* x, const uint8_t* bank_W1_packed,
                                     const uint8_t* bank_W3_packed, const uint8_t* bank_W2_packed,
                                     const uint8_t* bank_W1_scale, const uint8_t* bank_W3_scale,

@@ -1,5 +1,5 @@
 // Batched routed-expert GEMMs on the 5th-generation tensor cores (tcgen05, accumulators in tensor memory): what the
-// two tensor-core paths share, and the number formats of the fp16 path (moe_gemm_kernel.cuh).
+// two tensor-core paths share, and the number formats of the path "fp16".
 //
 // For every expert e with its n_e tokens (pairs sorted by expert, "slots"):
 //   up   : G[h, t] = W1_e[h, :] . x_t,  U[h, t] = W3_e[h, :] . x_t,  mid[slot, h] = silu(G) * U
@@ -7,7 +7,15 @@
 // Weights are the MMA's A operand (M = 128 weight rows per tile), tokens its B operand (N = 16 .. 128 tokens),
 // so a weight tile is read from HBM and dequantised ONCE for all tokens of the tile.
 //
-// Numbers of the fp16 path.  Operands are fp16, products and sums FP32 in the tensor core.
+// Numbers of the path "fp16", two forms of it.  Products are exact and sums FP32 in both.
+// (a) Block-scaled MMAs (moe_gemm_mxf4.cuh, MoeQFp8), up to kQMostTokensFp8 pairs per expert: the weights are E2M1 with their scale bytes, exact
+//   (0xFF counts as 2^-127); x and the intermediate are three E4M3 terms with a scale per 32 elements (moe_quantize_e4m3x3): x exact down to
+//   2^-18 of the largest of its 32, the intermediate 12 bits and more.  A token with an infinity or a NaN gives NaN.  Error beside the bf16
+//   output's rounding, against 64 bits: 1.4e-5 of the norm, and 3.4e-5 with one channel of 32 a factor 2^14 larger and its weights zero; (b) has
+//   2.1e-4 and 8e-2.
+// (b) fp16 MMAs (moe_gemm_kernel.cuh): more tokens, rows of other ranks, weights that are 16- but not 32-byte aligned, and shapes where (a)'s
+//   operands have no room in the workspace (its x lies in the bytes of y, which is written when x is done with).
+// Of (b):
 //   * weights: E2M1 * 2^(s - c_row), c_row = largest E8M0 byte of the row.  E2M1 times a power of two is exact in fp16
 //     down to 2^-24, i.e. blocks up to 2^23 times smaller than the row's largest are exact, smaller ones vanish; scale
 //     byte 0xFF contributes 0.

@@ -9,7 +9,8 @@
 // x up to 112 tokens, one tile per PAIR of CTAs (cta_group::2): each CTA holds 128 rows of both blocks and half of the
 // tokens.  A stage covers 256 K-elements (one 128-byte swizzled row per operand row = 4 MMAs of K = 64).
 //
-// How the terms are multiplied.  Each term is an MMA of its own into the SAME accumulator columns, with the weight tile
+// How the terms are multiplied (FP8 tiles of few tokens apart, whose three terms lie side by side along N: a third of the MMAs, 44 to 56
+// clocks each; FP4 tiles that way were slower, 64 tokens 428 -> 458 us).  Each term is an MMA of its own into the SAME accumulator columns, with the weight tile
 // kept in the collector between the three: 3 x N / 2 clocks for N tokens (N >= 96), the full rate of the tensor pipe;
 // a stage's 24 MMAs and 10 scale copies take 1 170 clocks at N = 96 and 580 at N = 16.  Without the collector every MMA
 // reads its A tile again, 32 clocks at 128 bytes a clock.  Two accumulator sets of 2 x 112 columns fit into tensor memory,
@@ -39,35 +40,64 @@
 
 #include "moe_gemm.cuh"
 
+#include <type_traits>
+
 namespace dsv4 {
 
-constexpr int kQKBlock = 256;                        // K-elements per stage
+// How the operands are held.  A stage is one 128-byte swizzled row per operand row, four MMAs.
+//
+// FP8 is the form of the path "fp16" (moe_gemm.cuh says what it holds exactly): the tensor cores multiply E2M1 weights by E4M3 terms, the TMA
+// spreading the packed weights over twice their bytes as it writes them.  What bounds it: that write, 4.2 clocks a row of 64 packed bytes
+// and SM, i.e. 4.4 TB/s of weights (7.0 as stored; boxes of 64 bytes as stored are as slow), and from some 80 tokens an expert on the MMAs, half as fast
+// as FP4 ones.  The kernel before it (moe_gemm_kernel.cuh, which dequantises into tensor memory) waits for its handshakes: 256 experts of
+// 4096, 2048, top 6, us that one -> this: 2 tokens 116 -> 80, 64 tokens (Zipf) 495 -> 408, 1 003 tokens 1 133 -> 988, 2 048 tokens 1 349 ->
+// 1 257, 3 300 tokens 1 592 -> 1 574; 32 experts of 2048, 1024, 300 tokens 92 -> 63.
+struct MoeQFp4 {                                     // kind::mxf4: activations as three MXFP4 terms
+    static constexpr int kKBlock = 256;              // K-elements per stage
+    static constexpr uint32_t kBoxBytes = 128 * 128; // bytes that a box of 128 weight rows brings in
+    static constexpr int kAtoms128 = 2;              // pieces of 128 K-elements (scale atoms of an operand's 128 rows) per stage
+    static constexpr bool kWide = false;             // few tokens: the three terms side by side along N
+};
+struct MoeQFp8 {                                     // kind::mxf8f6f4: activations as three E4M3 terms, weights E2M1 in 16-byte groups
+    static constexpr int kKBlock = 128;              // of 16 (8 bytes, 8 bytes of padding), which is how the TMA lays them down
+    static constexpr uint32_t kBoxBytes = 128 * 64;
+    static constexpr int kAtoms128 = 1;
+    static constexpr bool kWide = true;
+};
 constexpr int kQTerms = 3;                           // activation terms
 constexpr int kQTok = 112;                           // tokens per tile at most
 constexpr uint32_t kQTile = 128 * 128;               // bytes of one packed weight tile (128 rows x 128 B)
-constexpr uint32_t kQSfStage = 2 * 2 * 512 + 2 * kQTerms * 512;      // scale atoms: [mat][atom], then [atom][term]
 // Tiles of up to CAP tokens.  Where experts have few tokens the weights' way from HBM is what a tile waits for: five stages of 32
 // tokens instead of three of 112 keep more of them on it (256 experts of 4096, 2048, top 6: 17 tokens 216 -> 209.5 us, 64 zipf 278 ->
 // 270, 300 579 -> 567; below ten tokens no difference).  Taken up to kQFewTokens pairs per expert, where next to no expert has more
 // than 32.
 constexpr int kQFewTokens = 16;
-template <int CAP>
+// FP8: the tiles of 32 tokens (terms side by side) against those of 112, pairs per expert: 14 765 / 802 us, 19 811 / 855, 23.5 844 / 877, 29
+// 1 010 / 929.  Above kQMostTokensFp8 pairs per expert dequantising takes over: 70 1 395 there, 1 265 here; 96 1 650 / 1 674; 250 (2048, 1024)
+// 223 / 227.
+constexpr int kQFewTokensFp8 = 24, kQMostTokensFp8 = 80;
+constexpr int kQEpiWarps = 12, kQScaleWarps = 8;
+constexpr int kQEpiGroups = kQEpiWarps / 4;          // warps per lane quadrant of tensor memory
+template <class F, int CAP>
 struct MoeQShape {
     static constexpr int kStages = CAP <= 32 ? 5 : 3;
+    static constexpr bool kWide = F::kWide && CAP <= 32;                     // the terms side by side along N
+    static constexpr int kAtoms = kWide ? 1 : kQTerms;                       // scale atoms of B per 128 K-elements
+    static constexpr uint32_t kMatCols = kQTok, kAccCols = 2 * kMatCols;     // accumulator columns of a matrix; of a set
+    static_assert((kWide ? kQTerms * CAP : CAP) <= kQTok, "accumulator columns");
+    static constexpr uint32_t kSfCol = 2 * kAccCols;                         // scale columns: A [mat][piece] x 4, B [piece][term] x 4
     static constexpr uint32_t kBStage = kQTerms * (CAP / 2) * 128;           // activation rows of one stage and CTA
-    static constexpr uint32_t kOffB = kStages * 2 * kQTile, kOffSf = kOffB + kStages * kBStage, kOffTables = kOffSf + kStages * kQSfStage;
+    static constexpr int kPieces = F::kAtoms128;
+    static constexpr uint32_t kSfB = 2 * kPieces * 512, kSfStage = kSfB + kPieces * kAtoms * 512;      // scale atoms: [mat][piece], then [piece][term]
+    static constexpr int kEpiRounds = (CAP + 16 * kQEpiGroups - 1) / (16 * kQEpiGroups);
+    static constexpr uint32_t kOffB = kStages * 2 * kQTile, kOffSf = kOffB + kStages * kBStage, kOffTables = kOffSf + kStages * kSfStage;
+    static_assert(kSfCol + 16 + 8 * kAtoms <= 512, "tensor memory overflow");
     // dynamic shared memory: stages, then the tile and offset tables of the experts
     static __host__ __device__ __forceinline__ uint32_t smem(int n_experts) { return kOffTables + 8 * (uint32_t)(n_experts + 1) + 1024; }
     static_assert(kOffTables + 8 * (kMoeMaxExperts + 1) + 1024 + 1024 <= 227 * 1024, "shared memory overflow");
 };
-constexpr int kQEpiWarps = 12, kQScaleWarps = 8;
-constexpr int kQEpiGroups = kQEpiWarps / 4;          // warps per lane quadrant of tensor memory
-constexpr int kQEpiRounds = (kQTok + 16 * kQEpiGroups - 1) / (16 * kQEpiGroups);
 constexpr int kQMmaWarp = 0, kQProducerWarp = 1, kQEpiWarp = 4, kQScaleWarp = kQEpiWarp + kQEpiWarps;    // warps 2, 3: idle
 constexpr int kQThreads = (kQScaleWarp + kQScaleWarps) * 32;
-constexpr uint32_t kQAccCols = 2 * kQTok;            // per accumulator set
-constexpr uint32_t kQSfCol = 2 * kQAccCols, kQSfCols = 16 + 8 * kQTerms;
-static_assert(kQSfCol + kQSfCols <= 512, "tensor memory overflow");
 
 struct MoeQGemmArgs {
     const uint8_t* wa_s; const uint8_t* wb_s;        // E8M0 scales: up W1, W3; down W2 (wb unused)
@@ -128,31 +158,54 @@ __device__ __forceinline__ void tma_pair_load_3d(uint32_t dst, const CUtensorMap
 // copies and MMAs of one thread execute in the order they are issued.
 struct MoeQStage {
     uint64_t w, b;                                   // descriptors of the first weight tile and of term 1
-    uint32_t sf, acc, sfa, b_term, idesc[2];
+    uint32_t sf, acc, sfa, b_term, idesc[4];         // (idesc: by K-step; FP4 by its parity)
     bool fresh;                                      // first stage of a tile: overwrite the accumulators
 };
-template <int MATS>
+template <class F, class Q, int MATS>
 __device__ __forceinline__ void moe_q_issue(const MoeQStage& q) {
-    const uint32_t sfb = q.sfa + 16;                 // columns: A [mat][atom] x 4, B [atom][term] x 4
+    constexpr bool FP8 = F::kAtoms128 == 1;
+    const uint32_t sfb = q.sfa + 16;
 #pragma unroll
-    for (int at = 0; at < 2; ++at) {
+    for (int at = 0; at < Q::kPieces; ++at) {
 #pragma unroll
-        for (int m = 0; m < MATS; ++m) tc05_pair_copy_scale_atom(q.sfa + m * 8 + at * 4, q.sf + m * 1024 + at * 512);
+        for (int m = 0; m < MATS; ++m) tc05_pair_copy_scale_atom(q.sfa + (m * Q::kPieces + at) * 4, q.sf + (m * Q::kPieces + at) * 512);
 #pragma unroll
-        for (int i = 0; i < kQTerms; ++i)
-            tc05_pair_copy_scale_atom(sfb + (at * kQTerms + i) * 4, q.sf + 2048 + (at * kQTerms + i) * 512);
+        for (int i = 0; i < Q::kAtoms; ++i)
+            tc05_pair_copy_scale_atom(sfb + (at * Q::kAtoms + i) * 4, q.sf + Q::kSfB + (at * Q::kAtoms + i) * 512);
     }
 #pragma unroll
-    for (int j = 0; j < 4; ++j)                      // K-steps of 64 (32 bytes)
+    for (int j = 0; j < 4; ++j)                      // K-steps of 32 bytes
 #pragma unroll
         for (int m = 0; m < MATS; ++m) {
+            const int at = FP8 ? 0 : j >> 1;
             const uint64_t da = q.w + m * (kQTile >> 4) + 2 * j;
-            const uint32_t d = q.acc + m * kQTok, sa = q.sfa + m * 8 + (j >> 1) * 4, sb = sfb + (j >> 1) * kQTerms * 4;
+            const uint32_t d = q.acc + m * Q::kMatCols, sa = q.sfa + (m * Q::kPieces + at) * 4, sb = sfb + at * Q::kAtoms * 4;
+            if (Q::kWide) {
+                tc05_pair_mma_mx<FP8, kAOnce>(d, da, q.b + 2 * j, q.idesc[FP8 ? j : j & 1], sa, sb, (j > 0 || !q.fresh) ? 1u : 0u);
+                continue;
+            }
             // the three terms multiply the same A: read once, kept in the collector
-            tc05_pair_mma_mxf4<kAFill>(d, da, q.b + 2 * j, q.idesc[j & 1], sa, sb, (j > 0 || !q.fresh) ? 1u : 0u);
-            tc05_pair_mma_mxf4<kAUse>(d, da, q.b + q.b_term + 2 * j, q.idesc[j & 1], sa, sb + 4, 1u);
-            tc05_pair_mma_mxf4<kALast>(d, da, q.b + 2 * q.b_term + 2 * j, q.idesc[j & 1], sa, sb + 8, 1u);
+            tc05_pair_mma_mx<FP8, kAFill>(d, da, q.b + 2 * j, q.idesc[FP8 ? j : j & 1], sa, sb, (j > 0 || !q.fresh) ? 1u : 0u);
+            tc05_pair_mma_mx<FP8, kAUse>(d, da, q.b + q.b_term + 2 * j, q.idesc[FP8 ? j : j & 1], sa, sb + 4, 1u);
+            tc05_pair_mma_mx<FP8, kALast>(d, da, q.b + 2 * q.b_term + 2 * j, q.idesc[FP8 ? j : j & 1], sa, sb + 8, 1u);
         }
+}
+
+// Terms side by side (N = 3 x tokens): column i * half + j of CTA r's half of the columns (they start at 3 half r) is term i of token
+// r * half + j, half = 8 or 16.  Both ways the 48 columns from 3 c on are those of the 16 tokens from c on: their sums.
+__device__ __forceinline__ void moe_q_sum_terms(uint32_t tcol, int half, uint32_t (&p)[16]) {
+    uint32_t q[kQTerms][16];
+#pragma unroll
+    for (int i = 0; i < kQTerms; ++i) tc05_ld16_issue(tcol + 16 * i, q[i]);
+    tc05_wait_ld();
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+        const int w = (j >> 3) * 24 + (j & 7);
+        const float a = __uint_as_float(half == 8 ? q[w >> 4][w & 15] : q[0][j]);
+        const float b = __uint_as_float(half == 8 ? q[(w + 8) >> 4][(w + 8) & 15] : q[1][j]);
+        const float c = __uint_as_float(half == 8 ? q[(w + 16) >> 4][(w + 16) & 15] : q[2][j]);
+        p[j] = __float_as_uint((a + b) + c);
+    }
 }
 
 // Tokens and lanes trade places: on entry v[i] is token i of row `lane` of a 32-row block, on return v[j] is row
@@ -207,17 +260,27 @@ __device__ __forceinline__ void moe_quantize_half_block(float (&v)[16], uint2 (&
     }
 }
 
-template <int MODE, int CAP>
-__global__ void __launch_bounds__(kQThreads, 1) moe_gemm_mxf4_kernel(const __grid_constant__ MoeQMaps maps,
-                                                                                              const MoeQGemmArgs a) {
-    using Q = MoeQShape<CAP>;
-    constexpr int kQStages = Q::kStages;
+// The same -> three E4M3 terms (moe_quantize_e4m3x3), 16 bytes each.
+__device__ __forceinline__ void moe_quantize_half_block_fp8(float (&v)[16], uint4 (&packed)[kQTerms], uint32_t (&scale)[kQTerms]) {
+    uint32_t m = 0;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) m = max(m, __float_as_uint(v[i]) & 0x7fffffffu);
+    m = max(m, __shfl_xor_sync(kFullMask, m, 16));
+    moe_quantize_e4m3x3<kE4m3MidStep>(v, m, packed, scale);
+}
+
+template <int MODE, int CAP, class F>
+__global__ void __launch_bounds__(kQThreads, 1) moe_gemm_mxf4_kernel(const __grid_constant__ MoeQMaps maps, const MoeQGemmArgs a) {
+    using Q = MoeQShape<F, CAP>;
+    constexpr bool FP8 = F::kAtoms128 == 1;
+    constexpr int kQStages = Q::kStages, kQEpiRounds = Q::kEpiRounds;
+    constexpr uint32_t kQSfStage = Q::kSfStage;
     extern __shared__ __align__(1024) uint8_t gemm_smem[];
     __shared__ __align__(8) uint64_t full[kQStages], empty[kQStages], acc_full[2], acc_free[2];
     __shared__ uint32_t tmem_holder;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int n_st = a.K / kQKBlock, row_s = a.K >> 5;
+    const int n_st = a.K / F::kKBlock, row_s = a.K >> 5;
     const uint32_t smem_w = smem_u32(gemm_smem), smem_b = smem_w + Q::kOffB, smem_sf = smem_w + Q::kOffSf;
     int* const s_tiles = reinterpret_cast<int*>(gemm_smem + Q::kOffTables);
     int* const s_offsets = s_tiles + a.n_experts + 1;
@@ -270,17 +333,21 @@ __global__ void __launch_bounds__(kQThreads, 1) moe_gemm_mxf4_kernel(const __gri
                 }
             wait(acc_full[buf], tc >> 1, 6);
             tc05_fence_after_sync();
-            const uint32_t trow = tmem + ((uint32_t)(quad * 32) << 16) + buf * kQAccCols;
+            const uint32_t trow = tmem + ((uint32_t)(quad * 32) << 16) + buf * Q::kAccCols;
             // the warps of a lane quadrant take chunks of 16 tokens in turn
 #pragma unroll
             for (int k = 0; k < kQEpiRounds; ++k) {
                 const int c = (((warp - kQEpiWarp) >> 2) + kQEpiGroups * k) * 16;
                 if (c >= t.n_valid || !alive) break;
                 const int n = min(16, t.n_valid - c);
+                auto sums = [&](int m, uint32_t (&p)[16]) {   // of block m; wide: complete on return
+                    if constexpr (Q::kWide) moe_q_sum_terms(trow + m * Q::kMatCols + 3 * c, moe_width(t.width, CAP) >> 1, p);
+                    else tc05_ld16_issue(trow + m * Q::kMatCols + c, p);
+                };
                 uint32_t p0[16], p1[16];
-                tc05_ld16_issue(trow + c, p0);
-                tc05_ld16_issue(trow + kQTok + c, p1);        // stale, and not used, in a half tile
-                tc05_wait_ld();
+                sums(0, p0);
+                if (MODE == 0 || !Q::kWide) sums(1, p1);      // (stale, and not used, in a half tile)
+                if (!Q::kWide) tc05_wait_ld();
                 if (MODE == 0) {
                     float g[16];
 #pragma unroll
@@ -289,29 +356,34 @@ __global__ void __launch_bounds__(kQThreads, 1) moe_gemm_mxf4_kernel(const __gri
                         g[i] = i < n ? __fdividef(gate, 1.0f + __expf(-gate)) * __uint_as_float(p1[i]) : 0.f;
                     }
                     moe_transpose16(g, lane);
-                    uint2 packed[kQTerms];
+                    typename std::conditional<FP8, uint4, uint2>::type packed[kQTerms];
                     uint32_t scale[kQTerms];
-                    moe_quantize_half_block(g, packed, scale);
+                    if constexpr (FP8) moe_quantize_half_block_fp8(g, packed, scale);
+                    else moe_quantize_half_block(g, packed, scale);
                     const int i = lane & 15;
                     const long long slot = t.slot0 + c + i;
                     if (i < n) {
                         const int h0 = m0 + quad * 32;
 #pragma unroll
                         for (int q = 0; q < kQTerms; ++q) {
-                            *reinterpret_cast<uint2*>(a.mid_q + (q * a.n_pairs + slot) * (a.rows >> 1) + (h0 >> 1) + (lane >> 4) * 8) = packed[q];
+                            const long long at = (q * a.n_pairs + slot) * a.rows + h0;          // element
+                            if constexpr (FP8) *reinterpret_cast<uint4*>(a.mid_q + at + (lane >> 4) * 16) = packed[q];
+                            else *reinterpret_cast<uint2*>(a.mid_q + (at >> 1) + (lane >> 4) * 8) = packed[q];
                             if (lane < 16) a.mid_s[(q * a.n_pairs + slot) * (a.rows >> 5) + (h0 >> 5)] = (uint8_t)scale[q];
                         }
                     }
                 } else {
+                    auto put = [&](const uint32_t (&p)[16], int row) {
+                        if (row >= a.rows) return;                                                        // (a.rows is a multiple of 128)
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) {
-                        const float wi = __shfl_sync(kFullMask, w[k], i);
-                        if (i < n) {
-                            float* yrow = a.y + (size_t)(t.slot0 + c + i) * a.rows + m0 + r;
-                            if (m0 < a.rows) yrow[0] = __uint_as_float(p0[i]) * wi;                  // (a.rows is a multiple of 128)
-                            if (m0 + kQRows < a.rows) yrow[kQRows] = __uint_as_float(p1[i]) * wi;
+                        for (int i = 0; i < 16; ++i) {
+                            const float wi = __shfl_sync(kFullMask, w[k], i);
+                            if (i < n) a.y[(size_t)(t.slot0 + c + i) * a.rows + row + r] = __uint_as_float(p[i]) * wi;
                         }
-                    }
+                    };
+                    put(p0, m0);
+                    if (Q::kWide && t.mats == 2) sums(1, p1);
+                    put(p1, m0 + kQRows);
                 }
             }
             tc05_fence_before_sync();
@@ -319,15 +391,19 @@ __global__ void __launch_bounds__(kQThreads, 1) moe_gemm_mxf4_kernel(const __gri
             if (lane == 0) mbar_arrive_cluster(leader(acc_free[buf]));
         }
     } else if (warp >= kQScaleWarp) {
-        // ---- scale bytes: 8 per row and stage.  Thread st of a group holds weight row st of both matrices and token st of
-        // every term.  A group takes every second pair of stages (16 bytes of a row per load); its next pair is loaded
-        // before the current one is stored, whichever tile it belongs to.
+        // ---- scale bytes: a word per row and 128 K-elements.  Thread st of a group holds weight row st of both matrices and token st of
+        // every term.  A load, 16 bytes of a row or 8, is a run of kRun stages; a group takes every second run, and its next run is loaded
+        // before the current one is stored, whichever tile it belongs to.  Between a group's runs lies one of the other's: only with more
+        // stages in the ring than kRun has it seen the slot's last but one use end, without which a parity says nothing.
+        constexpr int kRun = 4 / Q::kPieces < kQStages ? 4 / Q::kPieces : 2;
+        static_assert(kQStages > kRun, "a scale group may not run ahead of a slot by two phases");
         const int st = (tid - kQScaleWarp * 32) & 127, group = (warp - kQScaleWarp) >> 2;
-        const int n_prs = (n_st + 1) >> 1;
-        int tile = pair, count = 0, pr = group;               // next pair to load: pr of tile number `count`
+        const int n_prs = (n_st + kRun - 1) / kRun;
+        int tile = pair, count = 0, pr = group;               // next run to load: pr of tile number `count`
         const uint8_t* src[2 + kQTerms] = {};
         bool fresh = true;
-        struct Loaded { uint4 v[2 + kQTerms]; uint32_t has; uint32_t it; bool two; };
+        struct Loaded { uint4 v[2 + kQTerms]; uint32_t has; uint32_t it; int stages, half; };
+        int half = 0;                                          // token columns of a CTA
         auto load = [&](Loaded& l) -> bool {
             while (pr >= n_prs) { pr -= n_prs; tile += n_pairs; ++count; fresh = true; }
             if (tile >= n_tiles) return false;
@@ -340,45 +416,67 @@ __global__ void __launch_bounds__(kQThreads, 1) moe_gemm_mxf4_kernel(const __gri
 #pragma unroll
                 for (int i = 0; i < kQTerms; ++i)
                     src[2 + i] = st < t.n_valid ? a.act_s + (i * a.n_pairs + t.slot0 + st) * row_s : nullptr;
+                half = moe_width(t.width, CAP) >> 1;
                 fresh = false;
             }
+            l.half = half;
             l.has = 0;
-            l.it = (uint32_t)count * n_st + 2 * pr;
-            l.two = 2 * pr + 1 < n_st;
+            l.it = (uint32_t)count * n_st + kRun * pr;
+            l.stages = min(kRun, n_st - kRun * pr);
 #pragma unroll
             for (int i = 0; i < 2 + kQTerms; ++i) {
                 if (!src[i]) continue;
                 l.has |= 1u << i;
-                if ((row_s & 15) == 0) {                       // otherwise the rows are 8-byte aligned
+                if (kRun * Q::kPieces == 2) {
+                    const uint2 v = __ldcg(reinterpret_cast<const uint2*>(src[i]) + pr);
+                    l.v[i] = make_uint4(v.x, v.y, 0, 0);
+                } else if ((row_s & 15) == 0) {                // otherwise the rows are 8-byte aligned
                     l.v[i] = __ldcg(reinterpret_cast<const uint4*>(src[i]) + pr);
                 } else {
                     const uint2* p = reinterpret_cast<const uint2*>(src[i]) + 2 * pr;
-                    const uint2 lo = __ldcg(p), hi = l.two ? __ldcg(p + 1) : make_uint2(0, 0);
+                    const uint2 lo = __ldcg(p), hi = l.stages == kRun ? __ldcg(p + 1) : make_uint2(0, 0);
                     l.v[i] = make_uint4(lo.x, lo.y, hi.x, hi.y);
+                }
+                if (FP8 && i < 2) {                            // a weight's scale byte 0xFF contributes nothing on this path: 2^-127
+                    l.v[i].x &= ~__vcmpeq4(l.v[i].x, 0xffffffffu); l.v[i].y &= ~__vcmpeq4(l.v[i].y, 0xffffffffu);
+                    l.v[i].z &= ~__vcmpeq4(l.v[i].z, 0xffffffffu); l.v[i].w &= ~__vcmpeq4(l.v[i].w, 0xffffffffu);
                 }
             }
             pr += 2;
             return true;
         };
         const uint32_t atom = tc05_scale_atom_offset(st, 0);
-        auto put_stage = [&](const Loaded& l, uint32_t it, bool second) {
+        // Stage n of a run.  (Written as a loop over the run, unrolled, this role held up the gate/up GEMM of few tokens: 64 tokens 280 ->
+        // 302 us, 600 tokens 374 -> 406.)
+        auto put_stage = [&](const Loaded& l, uint32_t it, int n) {
             const uint32_t slot = it % kQStages, round = it / kQStages;
             if (round > 0) wait(empty[slot], round - 1, 4);
-            const uint32_t sf = smem_sf + slot * kQSfStage + atom;
+            const uint32_t sf = smem_sf + slot * kQSfStage;
 #pragma unroll
             for (int i = 0; i < 2 + kQTerms; ++i)
-                if (l.has & (1u << i)) {                       // scales 0..3 -> atom 0, 4..7 -> atom 1
-                    const uint32_t at = sf + (i < 2 ? i * 1024u : 2048u + (i - 2) * 512u);
-                    asm volatile("st.shared.u32 [%0], %1;" ::"r"(at), "r"(second ? l.v[i].z : l.v[i].x) : "memory");
-                    asm volatile("st.shared.u32 [%0], %1;" ::"r"(at + (i < 2 ? 512u : kQTerms * 512u)), "r"(second ? l.v[i].w : l.v[i].y) : "memory");
+                if (l.has & (1u << i)) {
+                    uint32_t at = sf + atom + (i < 2 ? i * Q::kPieces * 512u : Q::kSfB + (i - 2) * 512u);
+                    if (Q::kWide && i >= 2)                    // a column per term and token: see moe_q_sum_terms
+                        at = sf + Q::kSfB + tc05_scale_atom_offset(st + (i - 2 + (st >= l.half ? kQTerms - 1 : 0)) * l.half, 0);
+                    const uint4& v = l.v[i];
+                    if (FP8) {                                 // one piece of 128 K-elements, or two
+                        asm volatile("st.shared.u32 [%0], %1;" ::"r"(at), "r"(n == 0 ? v.x : n == 1 ? v.y : n == 2 ? v.z : v.w) : "memory");
+                    } else {
+                        asm volatile("st.shared.u32 [%0], %1;" ::"r"(at), "r"(n == 1 ? v.z : v.x) : "memory");
+                        asm volatile("st.shared.u32 [%0], %1;" ::"r"(at + (i < 2 ? 512u : Q::kAtoms * 512u)), "r"(n == 1 ? v.w : v.y) : "memory");
+                    }
                 }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(leader(full[slot]));
         };
         auto put = [&](const Loaded& l) {
-            put_stage(l, l.it, false);
-            if (l.two) put_stage(l, l.it + 1, true);
+            put_stage(l, l.it, 0);
+            if (l.stages > 1) put_stage(l, l.it + 1, 1);
+            if (kRun == 4 && l.stages > 2) {                   // (an even number of stages a tile)
+                put_stage(l, l.it + 2, 2);
+                put_stage(l, l.it + 3, 3);
+            }
         };
         pdl_wait();
         Loaded l0, l1;
@@ -402,7 +500,7 @@ __global__ void __launch_bounds__(kQThreads, 1) moe_gemm_mxf4_kernel(const __gri
                 const int first = t.e * a.rows + t.m0 + rank * kMoeTileRows;      // past the expert in a half tile: loaded, not used
                 const int half = moe_width(t.width, CAP) >> 1, slot = t.slot0 + rank * half;
                 const CUtensorMap* act = &maps.act[t.width];
-                const uint32_t bytes = t.mats * kQTile + kQTerms * half * 128u;
+                const uint32_t bytes = t.mats * F::kBoxBytes + kQTerms * half * 128u;
                 auto weights = [&](int s, const RingPos& p) {
                     const uint32_t bar = leader(full[p.slot]), dst = smem_w + p.slot * 2 * kQTile;
                     mbar_arrive_expect_tx_cluster(bar, bytes);
@@ -443,11 +541,14 @@ __global__ void __launch_bounds__(kQThreads, 1) moe_gemm_mxf4_kernel(const __gri
                 const uint32_t buf = tc & 1u;
                 const int n = moe_width(t.width, CAP);
                 MoeQStage q;
-                q.acc = tmem + buf * kQAccCols;
-                q.sfa = tmem + kQSfCol;
+                q.acc = tmem + buf * Q::kAccCols;
+                q.sfa = tmem + Q::kSfCol;
                 q.b_term = (uint32_t)n * 4;                   // 128 n / 2 bytes, in the descriptor's units
-                q.idesc[0] = tc05_idesc_mxf4(256, n, 0, 0);
-                q.idesc[1] = tc05_idesc_mxf4(256, n, 2, 2);
+#pragma unroll
+                for (int j = 0; j < (FP8 ? 4 : 2); ++j) {     // scale bytes of K-step j: two of every four, or one
+                    const int id = FP8 ? j : 2 * j;
+                    q.idesc[j] = FP8 ? tc05_idesc_mxf8f6f4(256, Q::kWide ? kQTerms * n : n, id, id) : tc05_idesc_mxf4(256, Q::kWide ? kQTerms * n : n, id, id);
+                }
                 if (tc >= 2) wait_one(acc_free[buf], (tc >> 1) - 1, 7);
                 for (int s = 0; s < n_st; ++s, pos.next(kQStages)) {
                     wait_one(full[pos.slot], pos.round, 5);
@@ -457,7 +558,7 @@ __global__ void __launch_bounds__(kQThreads, 1) moe_gemm_mxf4_kernel(const __gri
                     q.b = tc05_desc_k_sw128(smem_b + pos.slot * Q::kBStage);
                     q.sf = smem_sf + pos.slot * kQSfStage;
                     q.fresh = s == 0;
-                    if (t.mats == 2) moe_q_issue<2>(q); else moe_q_issue<1>(q);
+                    if (t.mats == 2) moe_q_issue<F, Q, 2>(q); else moe_q_issue<F, Q, 1>(q);
                     tc05_pair_commit(smem_u32(&empty[pos.slot]));
                     if (s == n_st >> 1 && tile + n_pairs < n_tiles) next = decode(tile + n_pairs);
                     if (s == n_st - 1) tc05_pair_commit(smem_u32(&acc_full[buf]));

@@ -213,4 +213,47 @@ __device__ __forceinline__ void moe_quantize_block_x3(float (&v)[32], uint4 (&wo
     }
 }
 
+// 16 elements of a 32-element block whose largest magnitude is m (float bits) -> three E4M3 terms,
+//   v ~ 2^e (q1 + 2^-4 q2 + 2^-(4 + STEP) q3),   2^e such that the largest q1 is in [128, 256),
+// each term rounding what the ones before it left: a term takes four significant bits and leaves at most half a step of its last, so the
+// next in units 16 times smaller is below 256.  STEP = kE4m3MidStep (FP32 values): 12 bits and more of an element down to 2^-14 of the
+// block's largest.  STEP = kE4m3BfStep (bf16 values): two terms hold such an element exactly, and the third is kept for smaller ones, whose
+// first two terms are subnormal: exact down to 2^-18 of the block's largest, four bits far below.
+// A block with an infinity or a NaN gets scale byte 0xFF, E8M0's NaN.
+constexpr int kE4m3MidStep = 4, kE4m3BfStep = 14;
+template <int STEP>
+__device__ __forceinline__ void moe_quantize_e4m3x3(float (&v)[16], uint32_t m, uint4 (&packed)[3], uint32_t (&scale)[3]) {
+    const int e = max((int)(m >> 23) - 7, 4 + STEP + 2);                    // biased
+    const bool finite = m < 0x7f800000u;
+    const float inv = __uint_as_float((uint32_t)max(254 - e, 1) << 23);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] *= inv;
+#pragma unroll
+    for (int t = 0; t < 3; ++t) {
+        uint32_t r[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            uint32_t half[2];
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                float &lo = v[4 * i + 2 * j], &hi = v[4 * i + 2 * j + 1];
+                uint16_t q;
+                asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(q) : "f"(hi), "f"(lo));
+                half[j] = q;
+                if (t < 2) {
+                    uint32_t h;
+                    asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(h) : "h"(q));
+                    const float2 back = __half22float2(*reinterpret_cast<const __half2*>(&h));
+                    const float up = t == 0 ? 16.f : (float)(1 << STEP);
+                    lo = (lo - back.x) * up;
+                    hi = (hi - back.y) * up;
+                }
+            }
+            r[i] = half[0] | (half[1] << 16);
+        }
+        packed[t] = make_uint4(r[0], r[1], r[2], r[3]);
+        scale[t] = finite ? (uint32_t)(t == 0 ? e : t == 1 ? e - 4 : e - 4 - STEP) : 255u;
+    }
+}
+
 }  // namespace dsv4

@@ -277,6 +277,65 @@ __global__ void __launch_bounds__(256, 2) moe_act_blocks_kernel(const MoeActArgs
     }
 }
 
+// Three E4M3 terms, of rows of this GPU.  A lane takes half a block, a warp 512 elements of a row; the next piece and the slots of its row
+// are on their way while this one is quantised.  2 K bytes of a token come in, 99 K / 32 of each of its pairs go out.
+__global__ void __launch_bounds__(256, 4) moe_act_fp8_kernel(const MoeActArgs a) {
+    const int lane = threadIdx.x & 31;
+    const int per_row = (a.K + 511) >> 9, warps = gridDim.x * (blockDim.x >> 5), n_pieces = a.n_tokens * per_row;
+    const long long term_q = a.n_pairs * a.K, term_s = a.n_pairs * (a.K >> 5);
+    auto slots_of = [&](int w) -> int {                        // lane j: slot of the j-th pair of the piece's token
+        return w < n_pieces && lane < a.k ? __ldcg(a.pair_slot + (long long)(w / per_row) * a.k + lane) : -1;
+    };
+    auto fetch = [&](int w, uint4 (&u)[2]) {
+        const int row = w / per_row, at = (w - row * per_row) * 512 + lane * 16;
+        if (w < n_pieces && at < a.K) {
+            const uint4* src = reinterpret_cast<const uint4*>(a.x + (long long)row * a.K + at);
+            u[0] = __ldcs(src);
+            u[1] = __ldcs(src + 1);
+        }
+    };
+    uint4 cur[2] = {}, nxt[2] = {};
+    int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    fetch(w, cur);
+    pdl_wait();
+    pdl_launch_dependents();                               // after the wait: the next kernel reads the tile tables before its own
+    int slots = slots_of(w);
+    for (; w < n_pieces; w += warps) {
+        fetch(w + warps, nxt);
+        const int next_slots = slots_of(w + warps);
+        float v[16];
+        uint32_t m = 0;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const uint32_t u[4] = {cur[i].x, cur[i].y, cur[i].z, cur[i].w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                v[8 * i + 2 * j] = __uint_as_float(u[j] << 16);
+                v[8 * i + 2 * j + 1] = __uint_as_float(u[j] & 0xffff0000u);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 16; ++i) m = max(m, __float_as_uint(v[i]) & 0x7fffffffu);
+        m = max(m, __shfl_xor_sync(kFullMask, m, 1));
+        uint4 word[3];
+        uint32_t scale[3];
+        moe_quantize_e4m3x3<kE4m3BfStep>(v, m, word, scale);
+        const int row = w / per_row, at = (w - row * per_row) * 512 + lane * 16;
+        for (int j = 0; j < a.k; ++j) {
+            const int slot = j < 32 ? __shfl_sync(kFullMask, slots, j) : __ldcg(a.pair_slot + (long long)row * a.k + j);
+            if (slot < 0 || at >= a.K) continue;
+#pragma unroll
+            for (int t = 0; t < 3; ++t) {
+                *reinterpret_cast<uint4*>(a.q + t * term_q + (long long)slot * a.K + at) = word[t];
+                if ((lane & 1) == 0) a.s[t * term_s + (long long)slot * (a.K >> 5) + (at >> 5)] = (uint8_t)scale[t];
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i) cur[i] = nxt[i];
+        slots = next_slots;
+    }
+}
+
 constexpr int kActRowThreads = 256;                        // threads per activation row (four rows per block)
 constexpr int kActRows = kPrepThreads / kActRowThreads;
 constexpr int kActMaxChunks = 16384 / 8 / kActRowThreads;  // 16-byte chunks per thread at the largest K

@@ -117,6 +117,12 @@ __device__ __forceinline__ uint32_t tc05_idesc_mxf4(int m, int n, int a_sf_id, i
            ((uint32_t)(m >> 4) << 24) | ((uint32_t)a_sf_id << 29);
 }
 
+// The same of kind::mxf8f6f4 (one scale per MMA of K = 32: ids 0 .. 3) with A E2M1 (format 5), held as 8 bytes of values and 8 of padding
+// per 16 elements, and B E4M3 (format 0).
+__device__ __forceinline__ uint32_t tc05_idesc_mxf8f6f4(int m, int n, int a_sf_id, int b_sf_id) {
+    return ((uint32_t)b_sf_id << 4) | (5u << 7) | ((uint32_t)(n >> 3) << 17) | (1u << 23) | ((uint32_t)(m >> 4) << 24) | ((uint32_t)a_sf_id << 29);
+}
+
 // Shared-memory descriptor of one scale atom: 32 rows x 16 bytes, no swizzle, 8-row groups 128 bytes apart.
 __device__ __forceinline__ uint64_t tc05_desc_scale_atom(uint32_t smem_addr) {
     uint64_t d = 0;
@@ -167,21 +173,26 @@ __device__ __forceinline__ void tc05_pair_commit(uint32_t mbar_addr) {
 }
 
 // A_USE says what happens to the A tile in the tensor core's collector buffer: kAFill (read and keep), kAUse (take the
-// kept one), kALast (take it and drop it).  MMAs that multiply the same A one after another read it from shared memory once
+// kept one), kALast (take it and drop it), kAOnce (read, not kept).  MMAs that multiply the same A one after another read it from shared memory once
 // this way.
-enum { kAFill, kAUse, kALast };
-template <int A_USE>
-__device__ __forceinline__ void tc05_pair_mma_mxf4(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
-                                                   uint32_t tmem_sfa, uint32_t tmem_sfb, uint32_t accumulate) {
-#define DSV4_MMA_MXF4(COLLECTOR)                                                                                        \
+enum { kAFill, kAUse, kALast, kAOnce };
+template <bool FP8, int A_USE>
+__device__ __forceinline__ void tc05_pair_mma_mx(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
+                                                 uint32_t tmem_sfa, uint32_t tmem_sfb, uint32_t accumulate) {
+#define DSV4_MMA_MX(KIND, COLLECTOR)                                                                                    \
     asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %6, 0;\n"                                                          \
-                 " tcgen05.mma.cta_group::2.kind::mxf4.block_scale.scale_vec::2X" COLLECTOR                              \
+                 " tcgen05.mma.cta_group::2.kind::" KIND COLLECTOR                                                       \
                  " [%0], %1, %2, %3, [%4], [%5], p;\n}\n" ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc),           \
                  "r"(tmem_sfa), "r"(tmem_sfb), "r"(accumulate) : "memory")
-    if (A_USE == kAFill) DSV4_MMA_MXF4(".collector::a::fill");
-    else if (A_USE == kAUse) DSV4_MMA_MXF4(".collector::a::use");
-    else DSV4_MMA_MXF4(".collector::a::lastuse");
-#undef DSV4_MMA_MXF4
+#define DSV4_MMA_MX_USE(KIND)                                                                                           \
+    if (A_USE == kAFill) DSV4_MMA_MX(KIND, ".collector::a::fill");                                                       \
+    else if (A_USE == kAUse) DSV4_MMA_MX(KIND, ".collector::a::use");                                                    \
+    else if (A_USE == kALast) DSV4_MMA_MX(KIND, ".collector::a::lastuse");                                               \
+    else DSV4_MMA_MX(KIND, "")
+    if (FP8) { DSV4_MMA_MX_USE("mxf8f6f4.block_scale.scale_vec::1X"); }
+    else { DSV4_MMA_MX_USE("mxf4.block_scale.scale_vec::2X"); }
+#undef DSV4_MMA_MX_USE
+#undef DSV4_MMA_MX
 }
 
 // Byte offset of scale (row r, scale j of 4) inside a scale atom.

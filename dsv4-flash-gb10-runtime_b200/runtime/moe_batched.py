@@ -28,8 +28,8 @@ def moe_forward(bank: Dict[str, torch.Tensor], x: torch.Tensor, ids: torch.Tenso
                 out: Optional[torch.Tensor] = None, workspace: Optional[torch.Tensor] = None,
                 path: Optional[str] = None) -> torch.Tensor:
     """`path`: None = the library's default (block-scaled MXFP4 MMAs unless DSV4_B200_MOE_PATH=fp16), 'mxf4' =
-    block-scaled MMAs fed with the packed weights (activations as three MXFP4 terms), 'fp16' = fp16 MMAs with
-    in-kernel dequantisation (x and weights exact within fp16's range of their row's largest, the intermediate in fp16)."""
+    block-scaled MMAs fed with the packed weights (activations as three MXFP4 terms), 'fp16' = operands of fp16's
+    precision and more (x exact down to 2^-17 of its row's largest, the intermediate to 11 bits: E4M3 terms or fp16)."""
     code = -1 if path is None else _PATHS[path]
     done = (_capi._host or _capi.host()).moe_forward(bank, x, ids, weights, out, workspace, code)
     if done is not None:

@@ -206,8 +206,8 @@ int mxfp4_moe_forward(const uint16_t* x, const uint8_t* bank_W1_packed, const ui
                       int K_in, int hidden, int out_dim, int k, uint16_t* out, void* workspace, void* stream);
 /* The same with the tensor-core path chosen by the caller: 1 = block-scaled MXFP4 MMAs fed with the packed weights as
  * stored, activations as three MXFP4 terms (what mxfp4_moe_forward uses unless DSV4_B200_MOE_PATH=fp16 is set);
- * 0 = fp16 MMAs with in-kernel dequantisation: x is exact down to 2^-17 of its row's largest element, weights down to
- * scales 2^-23 of their row's largest, the intermediate is rounded to fp16. */
+ * 0 ("fp16") = x exact down to 2^-17 of its row's largest element and the intermediate to 11 bits or more: E4M3 terms on block-scaled
+ * MMAs, or fp16 MMAs with in-kernel dequantisation (weights down to scales 2^-23 of their row's largest). */
 int mxfp4_moe_forward_path(int path, const uint16_t* x, const uint8_t* bank_W1_packed, const uint8_t* bank_W3_packed,
                            const uint8_t* bank_W2_packed, const uint8_t* bank_W1_scale, const uint8_t* bank_W3_scale,
                            const uint8_t* bank_W2_scale, const int* ids, const float* weights, int n_tokens,

@@ -1,0 +1,91 @@
+"""The batched layer's path "fp16" in both its forms, E4M3 terms on block-scaled MMAs and fp16 MMAs, at the edges of the rule that chooses
+between them and of the tiles of the first, against 64 bits and against each other."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = torch.device("cuda:0")
+LUT = torch.tensor([0, .5, 1, 1.5, 2, 3, 4, 6, -0., -.5, -1, -1.5, -2, -3, -4, -6], dtype=torch.float64)
+
+
+def dense(p, s):
+    v = torch.stack([LUT.to(p.device)[(p & 15).long()], LUT.to(p.device)[(p >> 4).long()]], -1).flatten(-2)
+    return v * torch.ldexp(torch.ones(s.shape, dtype=torch.float64, device=p.device), s.int() - 127).repeat_interleave(32, -1)
+
+
+def layer64(bank, x, ids, w):
+    out = torch.zeros(x.shape[0], bank["w2p"].shape[1], dtype=torch.float64, device=x.device)
+    for e in range(bank["w1p"].shape[0]):
+        t, j = (ids == e).nonzero(as_tuple=True)
+        if len(t):
+            a, b = (x[t].double() @ dense(bank[n + "p"][e], bank[n + "s"][e]).T for n in ("w1", "w3"))
+            out.index_add_(0, t, ((a * torch.sigmoid(a) * b) @ dense(bank["w2p"][e], bank["w2s"][e]).T) * w[t, j].double()[:, None])
+    return out
+
+
+def at_odd_16_bytes(t):
+    """The same bytes at an address that is 16 modulo 32: the TMA cannot lay such weights down padded."""
+    buf = torch.empty(t.numel() + 48, dtype=t.dtype, device=t.device)
+    shift = (16 - buf.data_ptr() % 32) % 32
+    view = buf[shift:shift + t.numel()].view(t.shape)
+    assert view.data_ptr() % 32 == 16
+    return view.copy_(t)
+
+
+@pytest.mark.parametrize("counts,K,H,O", [
+    ([1, 0, 15, 16], 256, 256, 256),             # two stages a tile, one run of scale bytes cut short
+    ([24, 24, 24, 24], 1280, 512, 1280),         # the most pairs for tiles of 32 tokens
+    ([25, 24, 24, 24], 1280, 512, 1280),         # one more
+    ([17, 31, 32, 33] + [0] * 4, 2304, 768, 2304),
+    ([64, 65, 1, 30] + [0] * 4, 4096, 2048, 4096),          # three tokens tiles of an expert
+    ([80, 80, 80, 80], 768, 1280, 768),          # the most for the E4M3 form
+    ([112, 97, 48, 62], 512, 256, 640),          # a quarter tile of output rows
+    ([130, 33, 96, 49], 4096, 512, 4096),
+    ([81, 80, 80, 80], 512, 256, 512),           # fp16 MMAs
+    ([40, 9], 256, 1280, 256),                   # no room for the terms of the intermediate
+    ([40, 9], 1280, 256, 384),                   # nor of x
+])
+def test_forms_agree(rt, qz, counts, K, H, O):
+    g = torch.Generator(device=DEV).manual_seed(sum(counts) + K)
+    E, T = len(counts), sum(counts)
+    bank = qz.make_expert_bank(E, K, H, DEV, seed=K)
+    if O != K:
+        bank["w2p"], bank["w2s"] = qz.quantize_mxfp4((torch.randn(E, O, H, generator=g, device=DEV) * 0.02).to(torch.bfloat16))
+    bank["w1s"] += (torch.arange(bank["w1s"].numel(), device=DEV).view(bank["w1s"].shape) % 5).to(torch.uint8)        # scales that differ along K
+    ids = torch.repeat_interleave(torch.arange(E, device=DEV), torch.tensor(counts, device=DEV))[torch.randperm(T, generator=g, device=DEV)].to(torch.int32)[:, None].contiguous()
+    w = torch.rand(T, 1, generator=g, device=DEV) + 0.5
+    x = (torch.randn(T, K, generator=g, device=DEV) * torch.exp2(torch.randn(T, 1, generator=g, device=DEV) * 3)).to(torch.bfloat16)
+    x[T // 2, :64] = 0
+    one = rt.moe_forward(bank, x, ids, w, path="fp16")
+    other = rt.moe_forward({n: at_odd_16_bytes(t) for n, t in bank.items()}, x, ids, w, path="fp16")
+    again = rt.moe_forward(bank, x, ids, w, path="fp16")
+    assert rt.moe_device_status() == 0
+    assert torch.equal(one.view(torch.int16), again.view(torch.int16))
+    ref = layer64(bank, x, ids, w)
+    rounding = (ref.to(torch.bfloat16).double() - ref).norm(dim=1)
+    terms = T <= 80 * E and 99 * (K // 32) <= 128 * (O // 32) and 99 * H <= 64 * (K + H)
+    # beside the output's rounding: the intermediate in 11 bits (fp16, and a bit more where a row lies low in its range), or in three
+    # terms of four bits, which leave 2^-13 of a value
+    for out, bound in ((one, 2.0 ** -13 if terms else 2 * 2.0 ** -11 / 3 ** 0.5), (other, 2 * 2.0 ** -11 / 3 ** 0.5)):
+        err = (out.double() - ref).norm(dim=1)
+        worst = ((err ** 2 - rounding ** 2).clamp(min=0).sqrt() / (ref.norm(dim=1) + 1e-300)).max().item()
+        assert worst <= bound, f"{counts} {K} {H} {O}: {worst:.2e} of a token's norm beside the rounding, {bound:.2e} allowed"
+
+
+@pytest.mark.parametrize("counts", [[24] * 4, [60] * 4])
+def test_wide_range_of_x(rt, qz, counts):
+    """Elements 2^14 below the largest of their 32 keep their eight bits: one channel of 32 that much larger, its weights zero."""
+    g = torch.Generator(device=DEV).manual_seed(len(counts))
+    K, H, E, T = 1024, 512, len(counts), sum(counts)
+    bank = qz.make_expert_bank(E, K, H, DEV, seed=3)
+    x = torch.randn(T, K, generator=g, device=DEV)
+    x[:, 5::32] *= 2.0 ** 14
+    x = x.to(torch.bfloat16)
+    for n in ("w1p", "w3p"):
+        bank[n][:, :, 2::16] &= 0x0f                       # odd elements are the high nibbles
+    ids = torch.repeat_interleave(torch.arange(E, device=DEV), torch.tensor(counts, device=DEV)).to(torch.int32)[:, None].contiguous()
+    w = torch.ones(T, 1, device=DEV)
+    out = rt.moe_forward(bank, x, ids, w, path="fp16").double()
+    ref = layer64(bank, x, ids, w)
+    rounding = (ref.to(torch.bfloat16).double() - ref).norm() / ref.norm()
+    assert ((out - ref).norm() / ref.norm()) ** 2 <= rounding ** 2 + 2.0 ** -26
