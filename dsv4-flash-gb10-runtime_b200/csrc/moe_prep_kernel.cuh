@@ -1,5 +1,5 @@
 // Preparation of the batched layer, two launches: the pairs grouped by expert, then the activations in the form the
-// tensor-core path wants - three MXFP4 terms, or normalised fp16 - written once per PAIR in slot order, so that the rows
+// tensor-core path wants - three MXFP4 or E4M3 terms, or normalised fp16 - written once per PAIR in slot order, so that the rows
 // of a tile are neighbours and the GEMM fetches them with one copy per stage instead of one gather per four rows.
 #pragma once
 
