@@ -29,7 +29,7 @@ struct WorkspaceMap {
     size_t offsets, tiles_up, tiles_down, pair_slot, slot_w, y;      // both paths
     size_t xq, xs, mq, ms;                                          // block-scaled path
     size_t xh, xexp, typical, mid, mid_exp;                         // fp16 path (the same bytes)
-    size_t xq8, xs8, mq8, ms8;                                      // its form on the block-scaled MMAs (the same bytes; x in those of y)
+    size_t xq8, xs8, mq8, ms8, row_exp8, typical8;                  // its form on the block-scaled MMAs (the same bytes; x in those of y)
     bool fits8;                                                     // which hold it
     size_t total;
 };
@@ -66,6 +66,8 @@ WorkspaceMap map_workspace(long long T, int k, int K, int H, int O, int E) {
     c.off = shared;
     m.mq8 = c.take((size_t)3 * P * H);
     m.ms8 = c.take((size_t)3 * P * H / 32);
+    m.row_exp8 = c.take((size_t)P * 4);
+    m.typical8 = c.take((size_t)E * 4);
     m.fits8 = m.fits8 && c.off <= m.total;
     return m;
 }
@@ -298,28 +300,38 @@ static int moe_forward_impl(int path, const __nv_bfloat16* x, const uint8_t* ban
     const bool few = P <= (long long)(fp8 ? kQFewTokensFp8 : kQFewTokens) * n_experts;
     const int cap_q = few ? 32 : kQTok;                                                    // tokens per tile, block-scaled path
     ga.tile_tokens = pairs ? cap_q : cap16;
-    launch_k(moe_group_kernel, dim3(P > kGroupOneBlockPairs ? kGroupCluster : 1), dim3(kPrepThreads), 0, stream, P > kGroupOneBlockPairs ? kGroupCluster : 1, ga);
+    ga.typical.w1_s = bank_W1_scale; ga.typical.w3_s = bank_W3_scale; ga.typical.K = K_in; ga.typical.hidden = hidden;
+    ga.typical.n_experts = n_experts; ga.typical.typical = reinterpret_cast<int*>(ws + (fp8 ? m.typical8 : m.typical));
+    ga.blocks = P > kGroupOneBlockPairs ? kGroupCluster : 1;
+    // E4M3 terms: further blocks of the grouping kernel look for the typical scales (fp16 MMAs: blocks of the activation kernel do)
+    const int scale_blocks = (n_experts + kTypicalExperts - 1) / kTypicalExperts;
+    const int ggrid = ga.blocks + (fp8 ? (scale_blocks + ga.blocks - 1) / ga.blocks * ga.blocks : 0);
+    launch_k(moe_group_kernel, dim3(ggrid), dim3(kPrepThreads), 0, stream, ga.blocks, ga);
     stage_mark(stream, 1);
 
     MoeActArgs aa;
     aa.x = x; aa.pair_slot = g.pair_slot; aa.n_tokens = n_tokens; aa.k = k; aa.K = K_in; aa.n_pairs = P;
     aa.q = ws + m.xq; aa.s = ws + m.xs; aa.xh = reinterpret_cast<__half*>(ws + m.xh);
-    aa.xexp = reinterpret_cast<int2*>(ws + m.xexp); aa.typical = reinterpret_cast<int*>(ws + m.typical);
-    aa.w1_s = bank_W1_scale; aa.w3_s = bank_W3_scale; aa.hidden = hidden; aa.n_experts = n_experts;
+    aa.xexp = reinterpret_cast<int2*>(ws + m.xexp); aa.ids = ids; aa.row_exp = reinterpret_cast<int*>(ws + m.row_exp8);
+    aa.typical = ga.typical;
     const MoePeerIn no_peers = {};
     const MoePeerIn& pin = peer_in ? *peer_in : no_peers;
     cudaError_t err = cudaSuccess;
     if (pairs) {
-        // ---- block-scaled MXFP4 tensor-core path; a warp per 256 elements, at most eight blocks of eight warps per SM; where that
-        // fills the SMs, a warp per 1024, two blocks
+        // ---- block-scaled MMAs.  MXFP4 terms of x: a warp per 256 elements, at most eight blocks of eight warps per SM; where that
+        // fills the SMs, a warp per 1024, two blocks.  E4M3 terms: blocks of whole rows, as many as the registers of an SM hold.
         const bool many = !peer_in && moe_act_by_blocks(n_tokens, K_in);
-        const long long pieces = (long long)n_tokens * (fp8 ? (K_in + 511) / 512 : many ? (K_in + 1023) / 1024 : K_in / 256), blocks = (pieces + 7) / 8;
-        const long long most = (fp8 ? 4LL : many ? 2LL : 8LL) * grid;
+        const long long pieces = (long long)n_tokens * (many ? (K_in + 1023) / 1024 : K_in / 256);
+        const int act8_rows = kAct8Warps / moe_act8_row_warps(K_in), act8_pieces = (K_in + 512 * kAct8Warps - 1) / (512 * kAct8Warps);
+        const long long blocks = fp8 ? (n_tokens + act8_rows - 1) / act8_rows : (pieces + 7) / 8;
+        const long long most = (fp8 ? (act8_pieces == 1 ? 4LL : act8_pieces == 2 ? 3LL : 2LL) : many ? 2LL : 8LL) * grid;
         uint8_t* const mid_q = ws + (fp8 ? m.mq8 : m.mq);
         uint8_t* const mid_s = ws + (fp8 ? m.ms8 : m.ms);
         if (fp8) { aa.q = ws + m.xq8; aa.s = ws + m.xs8; }
         const dim3 agrid((unsigned)(blocks < most ? blocks : most)), ablock(256);
-        if (fp8) launch_k(moe_act_fp8_kernel, agrid, ablock, 0, stream, 1, aa);
+        if (fp8)
+            launch_k(act8_pieces == 1 ? moe_act_fp8_kernel<1> : act8_pieces == 2 ? moe_act_fp8_kernel<2> : moe_act_fp8_kernel<4>, agrid,
+                     ablock, 0, stream, 1, aa);
         else if (many) launch_k(moe_act_blocks_kernel, agrid, ablock, 0, stream, 1, aa);
         else launch_k(peer_in ? moe_act_mxf4_kernel<true> : moe_act_mxf4_kernel<false>, agrid, ablock, 0, stream, 1, aa, pin);
         stage_mark(stream, 2);
@@ -335,7 +347,7 @@ static int moe_forward_impl(int path, const __nv_bfloat16* x, const uint8_t* ban
         if (err == cudaSuccess) err = term_maps(down_maps.act, mid_q, P, fp8 ? hidden : hidden / 2, cap_q);
         MoeQGemmArgs qu;
         qu.wa_s = bank_W1_scale; qu.wb_s = bank_W3_scale; qu.rows = hidden; qu.K = K_in; qu.n_experts = n_experts;
-        qu.act_s = aa.s; qu.n_pairs = P; qu.g = g; qu.mid_q = mid_q; qu.mid_s = mid_s; qu.y = nullptr;
+        qu.act_s = aa.s; qu.row_exp = aa.row_exp; qu.n_pairs = P; qu.g = g; qu.mid_q = mid_q; qu.mid_s = mid_s; qu.y = nullptr;
         MoeQGemmArgs qd = qu;
         qd.wa_s = bank_W2_scale; qd.wb_s = nullptr; qd.rows = out_dim; qd.K = hidden; qd.act_s = mid_s; qd.y = y;
         auto gemms = [&](auto format, auto cap) {
@@ -361,7 +373,7 @@ static int moe_forward_impl(int path, const __nv_bfloat16* x, const uint8_t* ban
     } else {
         // ---- fp16 tensor-core path: weights dequantised into tensor memory
         const int blocks = (n_tokens + kActRows - 1) / kActRows;
-        const dim3 agrid((n_experts + 31) / 32 + (blocks < 2 * grid ? blocks : 2 * grid)), ablock(kPrepThreads);
+        const dim3 agrid(scale_blocks + (blocks < 2 * grid ? blocks : 2 * grid)), ablock(kPrepThreads);
         launch_k(peer_in ? moe_act_fp16_kernel<true> : moe_act_fp16_kernel<false>, agrid, ablock, 0, stream, 1, aa, pin);
         stage_mark(stream, 2);
         __half* mid = reinterpret_cast<__half*>(ws + m.mid);
@@ -374,7 +386,7 @@ static int moe_forward_impl(int path, const __nv_bfloat16* x, const uint8_t* ban
         if (err == cudaSuccess) err = half_maps(down_maps.act, mid, P, hidden, cap16);
         MoeGemmArgs up;
         up.wa_s = bank_W1_scale; up.wb_s = bank_W3_scale; up.rows = hidden; up.K = K_in; up.n_experts = n_experts;
-        up.xexp = aa.xexp; up.typical = aa.typical; up.g = g;
+        up.xexp = aa.xexp; up.typical = aa.typical.typical; up.g = g;
         up.mid_log = 2;
         while ((2 << (up.mid_log - 2)) <= K_in) ++up.mid_log;                // floor(log2(K)) + 2
         up.mid = mid; up.mid_exp = reinterpret_cast<int*>(ws + m.mid_exp); up.y = y;

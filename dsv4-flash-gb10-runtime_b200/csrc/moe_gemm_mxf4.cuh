@@ -103,9 +103,10 @@ struct MoeQGemmArgs {
     const uint8_t* wa_s; const uint8_t* wb_s;        // E8M0 scales: up W1, W3; down W2 (wb unused)
     int rows, K, n_experts;
     const uint8_t* act_s;                            // [3][P][K / 32]
+    const int* row_exp;                              // E4M3 terms: [P], exponent taken out of a slot's x (moe_act_fp8_kernel)
     long long n_pairs;
     MoeGroups g;
-    uint8_t* mid_q; uint8_t* mid_s;                  // up output [3][P][rows / 2], [3][P][rows / 32]
+    uint8_t* mid_q; uint8_t* mid_s;                  // up output [3][P][rows / 2] (MXFP4) or [3][P][rows] (E4M3), [3][P][rows / 32]
     float* y;                                        // down output [P, rows] FP32
 };
 // Weight boxes of 128 rows; activation boxes of 3 terms x half a tile's columns, one per column count.
@@ -323,13 +324,15 @@ __global__ void __launch_bounds__(kQThreads, 1) moe_gemm_mxf4_kernel(const __gri
             const MoeQTile t = decode(tile);
             const uint32_t buf = tc & 1u;
             const int m0 = t.m0 + rank * kMoeTileRows;        // first row of this CTA in block 0
-            // router weights (down): lanes i and i + 16 hold that of token i of each of this warp's chunks
-            float w[kQEpiRounds];
-            if (MODE == 1)
+            // lanes i and i + 16 hold, for token i of each of this warp's chunks: down, the router weight; of E4M3 terms, the power of two
+            // that was taken out of x, and so of G and of U - once for the gate, twice for y (with the weight and by itself)
+            float w[kQEpiRounds], unit[kQEpiRounds];
+            if (MODE == 1 || FP8)
 #pragma unroll
                 for (int i = 0; i < kQEpiRounds; ++i) {
                     const int n = (((warp - kQEpiWarp) >> 2) + kQEpiGroups * i) * 16 + (lane & 15);
-                    w[i] = n < t.n_valid ? __ldcg(a.g.slot_w + t.slot0 + n) : 0.f;
+                    if (FP8) unit[i] = n < t.n_valid ? float_pow2(__ldcg(a.row_exp + t.slot0 + n)) : 1.f;
+                    if (MODE == 1) w[i] = n < t.n_valid ? __ldcg(a.g.slot_w + t.slot0 + n) * (FP8 ? unit[i] : 1.f) : 0.f;
                 }
             wait(acc_full[buf], tc >> 1, 6);
             tc05_fence_after_sync();
@@ -340,6 +343,7 @@ __global__ void __launch_bounds__(kQThreads, 1) moe_gemm_mxf4_kernel(const __gri
                 const int c = (((warp - kQEpiWarp) >> 2) + kQEpiGroups * k) * 16;
                 if (c >= t.n_valid || !alive) break;
                 const int n = min(16, t.n_valid - c);
+                const bool scaled = FP8 && __any_sync(kFullMask, unit[k] != 1.f);
                 auto sums = [&](int m, uint32_t (&p)[16]) {   // of block m; wide: complete on return
                     if constexpr (Q::kWide) moe_q_sum_terms(trow + m * Q::kMatCols + 3 * c, moe_width(t.width, CAP) >> 1, p);
                     else tc05_ld16_issue(trow + m * Q::kMatCols + c, p);
@@ -350,10 +354,20 @@ __global__ void __launch_bounds__(kQThreads, 1) moe_gemm_mxf4_kernel(const __gri
                 if (!Q::kWide) tc05_wait_ld();
                 if (MODE == 0) {
                     float g[16];
+                    if (!scaled) {
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) {
-                        const float gate = __uint_as_float(p0[i]);
-                        g[i] = i < n ? __fdividef(gate, 1.0f + __expf(-gate)) * __uint_as_float(p1[i]) : 0.f;
+                        for (int i = 0; i < 16; ++i) {
+                            const float gate = __uint_as_float(p0[i]);
+                            const float v = __fdividef(gate, 1.0f + __expf(-gate)) * __uint_as_float(p1[i]);
+                            g[i] = i < n ? (FP8 ? saturate_finite(v) : v) : 0.f;
+                        }
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) {
+                            const float gate = saturate_finite(__uint_as_float(p0[i])), true_gate = gate * __shfl_sync(kFullMask, unit[k], i);
+                            const float v = __fdividef(gate, 1.0f + __expf(-true_gate)) * __uint_as_float(p1[i]);
+                            g[i] = i < n ? saturate_finite(v) : 0.f;
+                        }
                     }
                     moe_transpose16(g, lane);
                     typename std::conditional<FP8, uint4, uint2>::type packed[kQTerms];
@@ -373,8 +387,12 @@ __global__ void __launch_bounds__(kQThreads, 1) moe_gemm_mxf4_kernel(const __gri
                         }
                     }
                 } else {
-                    auto put = [&](const uint32_t (&p)[16], int row) {
+                    auto put = [&](uint32_t (&p)[16], int row) {
                         if (row >= a.rows) return;                                                        // (a.rows is a multiple of 128)
+                        if (scaled) {
+#pragma unroll
+                            for (int i = 0; i < 16; ++i) p[i] = __float_as_uint(__uint_as_float(p[i]) * __shfl_sync(kFullMask, unit[k], i));
+                        }
 #pragma unroll
                         for (int i = 0; i < 16; ++i) {
                             const float wi = __shfl_sync(kFullMask, w[k], i);

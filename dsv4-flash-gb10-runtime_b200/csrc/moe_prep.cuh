@@ -216,7 +216,7 @@ __device__ __forceinline__ void moe_quantize_block_x3(float (&v)[32], uint4 (&wo
 // 16 elements of a 32-element block whose largest magnitude is m (float bits) -> three E4M3 terms,
 //   v ~ 2^e (q1 + 2^-4 q2 + 2^-(4 + STEP) q3),   2^e such that the largest q1 is in [128, 256),
 // each term rounding what the ones before it left: a term takes four significant bits and leaves at most half a step of its last, so the
-// next in units 16 times smaller is below 256.  STEP = kE4m3MidStep (FP32 values): 12 bits and more of an element down to 2^-14 of the
+// next in units 16 times smaller is below 256.  STEP = kE4m3MidStep (FP32 values): 11 bits and more of an element down to 2^-13 of the
 // block's largest.  STEP = kE4m3BfStep (bf16 values): two terms hold such an element exactly, and the third is kept for smaller ones, whose
 // first two terms are subnormal: exact down to 2^-18 of the block's largest, four bits far below.
 // A block with an infinity or a NaN gets scale byte 0xFF, E8M0's NaN.

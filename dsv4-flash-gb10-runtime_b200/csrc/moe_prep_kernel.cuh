@@ -13,10 +13,60 @@ constexpr int kPrepThreads = 1024;
 constexpr int kGroupOneBlockPairs = 2048;
 constexpr int kGroupCluster = 8;
 
+constexpr int kTypicalRows = 16;                           // weight rows looked at per expert and matrix
+constexpr int kTypicalExperts = kPrepThreads / 32 / 4;     // experts of a block: four warps each
+
+// The typical scale byte of W1 and of W3 of a few experts, by a block: the mean E8M0 byte of some of their rows (bytes 0 and 255, i.e.
+// zero blocks and NaN, left out).  It only centres the range of the intermediate; any value near the truth will do.  A warp takes half of
+// an expert's rows of one matrix.  (Short code: a warp for a whole expert, unrolled, is as many loads but 12 us of instruction fetches.)
+struct MoeTypicalArgs {
+    const uint8_t* w1_s; const uint8_t* w3_s;              // E8M0 bytes [E, hidden, K / 32]
+    int K, hidden, n_experts;
+    int* typical;                                          // [E] out: typical byte of W1 | of W3 << 8
+};
+__device__ __forceinline__ void moe_typical_scales(const MoeTypicalArgs& a, int block) {
+    __shared__ int part[kPrepThreads / 32][2];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int e = block * kTypicalExperts + (warp >> 2);
+    const int row_s = a.K >> 5, words = row_s >> 2, step = max(1, a.hidden / kTypicalRows);
+    int sum = 0, n = 0;
+    if (e < a.n_experts) {
+        const uint8_t* base = (warp & 2 ? a.w3_s : a.w1_s) + (long long)e * a.hidden * row_s;
+        const int r0 = (warp & 1) * (kTypicalRows / 2);
+        for (int c = lane; c < words; c += 32) {
+            uint32_t w[kTypicalRows / 2];
+#pragma unroll
+            for (int i = 0; i < kTypicalRows / 2; ++i)
+                w[i] = __ldg(reinterpret_cast<const uint32_t*>(base + (long long)min((r0 + i) * step, a.hidden - 1) * row_s) + c);
+#pragma unroll
+            for (int i = 0; i < kTypicalRows / 2; ++i) {
+                const uint32_t f = w[i] & ~__vcmpeq4(w[i], 0xffffffffu);           // 0xFF and 0 add nothing
+                sum = __dp4a(f, 0x01010101u, (uint32_t)sum);
+                n += __popc((((f & 0x7f7f7f7fu) + 0x7f7f7f7fu) | f) & 0x80808080u);
+            }
+        }
+    }
+    sum = __reduce_add_sync(kFullMask, sum);
+    n = __reduce_add_sync(kFullMask, n);
+    if (lane == 0) { part[warp][0] = sum; part[warp][1] = n; }
+    __syncthreads();
+    if (threadIdx.x >= kTypicalExperts || block * kTypicalExperts + (int)threadIdx.x >= a.n_experts) return;
+    int typ[2];
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+        const int* p = part[4 * threadIdx.x + 2 * m];
+        const int s = p[0] + p[2], c = p[1] + p[3];
+        typ[m] = c > 0 ? (s + c / 2) / c : 127;
+    }
+    a.typical[block * kTypicalExperts + threadIdx.x] = typ[0] | (typ[1] << 8);
+}
+
 struct MoeGroupArgs {
     const int* ids;                  // [P] expert of every pair, negative = skip
     const float* weights;            // [P]
     int n_pairs, n_experts, m_tiles_up, m_tiles_down, tile_tokens;
+    int blocks;                      // that sort; where the grid has more, they look for the typical scales
+    MoeTypicalArgs typical;
     MoeGroups g;
     int* status;
 };
@@ -29,7 +79,11 @@ __global__ void __launch_bounds__(kPrepThreads) moe_group_kernel(const MoeGroupA
     pdl_wait();
     pdl_launch_dependents();                               // after the wait: the next kernel reads x before its own
     const int e = threadIdx.x, lane = e & 31, wid = e >> 5;
-    const int blocks = gridDim.x, blk = blockIdx.x;
+    const int blocks = a.blocks, blk = blockIdx.x;
+    if (blk >= blocks) {                                   // (whole clusters of them)
+        moe_typical_scales(a.typical, blk - blocks);
+        return;
+    }
     count[e] = 0;
     __syncthreads();
     const int per = (a.n_pairs + blocks - 1) / blocks;
@@ -127,12 +181,12 @@ struct MoeActArgs {
     const int* pair_slot;            // [T, k]
     int n_tokens, k, K;
     long long n_pairs;
-    uint8_t* q; uint8_t* s;          // block-scaled path, out: [3][P][K / 2], [3][P][K / 32]
-    __half* xh;                      // fp16 path, out: [P, K]
-    int2* xexp;                      // [P] out: {exponent removed from x, floor(log2(rms of what is left))}
-    const uint8_t* w1_s; const uint8_t* w3_s;   // fp16 path: E8M0 bytes [E, hidden, K / 32]
-    int hidden, n_experts;
-    int* typical;                    // [E] out: typical scale byte of W1 | of W3 << 8
+    uint8_t* q; uint8_t* s;          // block-scaled MMAs, out: terms [3][P][K / 2] (MXFP4) or [3][P][K] (E4M3), scales [3][P][K / 32]
+    __half* xh;                      // fp16 MMAs, out: [P, K]
+    int2* xexp;                      // fp16 MMAs, [P] out: {exponent removed from x, floor(log2(rms of what is left))}
+    const int* ids;                  // E4M3 terms: [T, k]
+    int* row_exp;                    // E4M3 terms, [P] out: exponent removed from x
+    MoeTypicalArgs typical;          // fp16 MMAs: the first blocks write them; E4M3 terms: read
 };
 
 template <bool PEER>
@@ -277,69 +331,136 @@ __global__ void __launch_bounds__(256, 2) moe_act_blocks_kernel(const MoeActArgs
     }
 }
 
-// Three E4M3 terms, of rows of this GPU.  A lane takes half a block, a warp 512 elements of a row; the next piece and the slots of its row
-// are on their way while this one is quantised.  2 K bytes of a token come in, 99 K / 32 of each of its pairs go out.
-__global__ void __launch_bounds__(256, 4) moe_act_fp8_kernel(const MoeActArgs a) {
-    const int lane = threadIdx.x & 31;
-    const int per_row = (a.K + 511) >> 9, warps = gridDim.x * (blockDim.x >> 5), n_pieces = a.n_tokens * per_row;
+// Exponent taken out of a row whose largest magnitude is m (float bits): floor(log2 m), 0 for a row of zeros.
+__device__ __forceinline__ int moe_row_exponent(uint32_t m) { return m == 0 ? 0 : min(max((int)(m >> 23) - 127, -100), 126); }
+
+// Three E4M3 terms, of rows of this GPU.  FP32 is to hold G, U and silu(G) * U whatever the scales of x and of the weights, so the larger
+// and the smaller ones are normalised: x is multiplied by 2^-(its row's exponent), and the scale bytes of a pair are lower by its expert's
+// typical scale exponent, the mean of W1's and W3's, from -kAct8Down to kAct8Up (the bytes of a normalised row, 120 and less, leave room for
+// that).  row_exp is the sum of the two.  Exponents of up to kAct8Plain either way are left alone: in ordinary use row_exp is 0 and the GEMMs'
+// epilogues have nothing to multiply by (1 003 tokens of 256 experts, gate/up: 490 us without row_exp, 508 with, 502 this way), and the
+// worst of them, 16 384 products of 2^17 and 6 * 2^16, are 2^100 when squared.
+// A lane takes half a block of 32, a warp 512 elements of a row in each of PIECES (one up to K 4096, two, four), so that a row is read
+// once between its maximum and its terms; a block takes as many rows as its warps cover.  The next rows and their slots are on their way
+// while these are quantised.  2 K bytes of a token come in, 99 K / 32 of each of its pairs go out.
+constexpr int kAct8Warps = 8, kAct8Down = 100, kAct8Up = 60, kAct8Plain = 16;
+__host__ __device__ __forceinline__ int moe_act8_row_warps(int K) { return K >= 512 * kAct8Warps ? kAct8Warps : (K + 511) >> 9; }
+__device__ __forceinline__ int moe_act8_plain(int e) { return abs(e) <= kAct8Plain ? 0 : e; }
+template <int PIECES>
+__global__ void __launch_bounds__(32 * kAct8Warps, PIECES == 1 ? 4 : PIECES == 2 ? 3 : 2) moe_act_fp8_kernel(const MoeActArgs a) {
+    __shared__ uint32_t warp_max[2][kAct8Warps];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int row_warps = moe_act8_row_warps(a.K), rows = kAct8Warps / row_warps;      // rows of a block
+    const int sub = warp / row_warps, first_warp = sub * row_warps, w = warp - first_warp;
+    const int stride = (int)gridDim.x * rows;
     const long long term_q = a.n_pairs * a.K, term_s = a.n_pairs * (a.K >> 5);
-    auto slots_of = [&](int w) -> int {                        // lane j: slot of the j-th pair of the piece's token
-        return w < n_pieces && lane < a.k ? __ldcg(a.pair_slot + (long long)(w / per_row) * a.k + lane) : -1;
-    };
-    auto fetch = [&](int w, uint4 (&u)[2]) {
-        const int row = w / per_row, at = (w - row * per_row) * 512 + lane * 16;
-        if (w < n_pieces && at < a.K) {
-            const uint4* src = reinterpret_cast<const uint4*>(a.x + (long long)row * a.K + at);
-            u[0] = __ldcs(src);
-            u[1] = __ldcs(src + 1);
+    auto here = [&](int row) { return sub < rows && row < a.n_tokens; };
+    auto at_of = [&](int i) { return (w + i * row_warps) * 512 + lane * 16; };
+    auto fetch = [&](int row, uint4 (&u)[PIECES][2]) {
+#pragma unroll
+        for (int i = 0; i < PIECES; ++i) {
+            u[i][0] = u[i][1] = make_uint4(0, 0, 0, 0);
+            if (here(row) && at_of(i) < a.K) {
+                const uint4* src = reinterpret_cast<const uint4*>(a.x + (long long)row * a.K + at_of(i));
+                u[i][0] = __ldcs(src);
+                u[i][1] = __ldcs(src + 1);
+            }
         }
     };
-    uint4 cur[2] = {}, nxt[2] = {};
-    int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    fetch(w, cur);
+    // slot and expert of pair j of a row; -1 for a dropped pair
+    auto pair_of = [&](int row, int j) -> int2 {
+        const long long p = (long long)row * a.k + j;
+        return here(row) && j < a.k ? make_int2(__ldcg(a.pair_slot + p), __ldcg(a.ids + p)) : make_int2(-1, 0);
+    };
+    auto shift_of = [&](const int2& pair) -> int {
+        if (pair.x < 0) return 0;
+        const int typ = __ldcg(a.typical.typical + pair.y);
+        return moe_act8_plain(min(max((((typ & 255) + (typ >> 8)) >> 1) - 127, -kAct8Down), kAct8Up));
+    };
+    uint4 cur[PIECES][2], nxt[PIECES][2];
+    int row0 = (int)blockIdx.x * rows, buf = 0;
+    fetch(row0 + sub, cur);
     pdl_wait();
     pdl_launch_dependents();                               // after the wait: the next kernel reads the tile tables before its own
-    int slots = slots_of(w);
-    for (; w < n_pieces; w += warps) {
-        fetch(w + warps, nxt);
-        const int next_slots = slots_of(w + warps);
-        float v[16];
+    int2 pair = pair_of(row0 + sub, lane);                 // lane j: the j-th pair of the row
+    int shift = shift_of(pair);
+    for (; row0 < a.n_tokens; row0 += stride, buf ^= 1) {      // the same number of times in every warp of the block
+        const int row = row0 + sub;
+        fetch(row + stride, nxt);
+        const int2 next_pair = pair_of(row + stride, lane);
         uint32_t m = 0;
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const uint32_t u[4] = {cur[i].x, cur[i].y, cur[i].z, cur[i].w};
+        for (int i = 0; i < PIECES; ++i)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                v[8 * i + 2 * j] = __uint_as_float(u[j] << 16);
-                v[8 * i + 2 * j + 1] = __uint_as_float(u[j] & 0xffff0000u);
+            for (int h = 0; h < 2; ++h) {
+                const uint32_t u[4] = {cur[i][h].x, cur[i][h].y, cur[i][h].z, cur[i][h].w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) m = max(m, max((u[j] << 16) & 0x7fffffffu, u[j] & 0x7fff0000u));
+            }
+        m = __reduce_max_sync(kFullMask, m);
+        if (lane == 0) warp_max[buf][warp] = m;
+        __syncthreads();                                       // (two buffers: one barrier a row)
+        for (int i = 0; i < row_warps && sub < rows; ++i) m = max(m, warp_max[buf][first_warp + i]);
+        const int e = moe_act8_plain(moe_row_exponent(m));
+        const float inv = __uint_as_float((uint32_t)(127 - e) << 23);
+#pragma unroll
+        for (int i = 0; i < PIECES; ++i) {
+            float v[16];
+            uint32_t bm = 0;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const uint32_t u[4] = {cur[i][h].x, cur[i][h].y, cur[i][h].z, cur[i][h].w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    v[8 * h + 2 * j] = __uint_as_float(u[j] << 16) * inv;
+                    v[8 * h + 2 * j + 1] = __uint_as_float(u[j] & 0xffff0000u) * inv;
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < 16; ++j) bm = max(bm, __float_as_uint(v[j]) & 0x7fffffffu);
+            bm = max(bm, __shfl_xor_sync(kFullMask, bm, 1));
+            uint4 word[3];
+            uint32_t scale[3];
+            moe_quantize_e4m3x3<kE4m3BfStep>(v, bm, word, scale);
+            const int at = at_of(i);
+            for (int j = 0; j < a.k; ++j) {
+                int slot, sh;
+                if (j < 32) {
+                    slot = __shfl_sync(kFullMask, pair.x, j);
+                    sh = __shfl_sync(kFullMask, shift, j);
+                } else {
+                    const int2 p = pair_of(row, j);
+                    slot = p.x;
+                    sh = shift_of(p);
+                }
+                if (slot < 0 || at >= a.K) continue;
+#pragma unroll
+                for (int t = 0; t < 3; ++t) {
+                    *reinterpret_cast<uint4*>(a.q + t * term_q + (long long)slot * a.K + at) = word[t];
+                    const int byte = scale[t] == 255 ? 255 : max((int)scale[t] - sh, 0);
+                    if ((lane & 1) == 0) a.s[t * term_s + (long long)slot * (a.K >> 5) + (at >> 5)] = (uint8_t)byte;
+                }
+            }
+        }
+        if (w == 0) {
+            if (pair.x >= 0) a.row_exp[pair.x] = e + shift;
+            for (int j = 32 + lane; j < a.k; j += 32) {
+                const int2 p = pair_of(row, j);
+                if (p.x >= 0) a.row_exp[p.x] = e + shift_of(p);
             }
         }
 #pragma unroll
-        for (int i = 0; i < 16; ++i) m = max(m, __float_as_uint(v[i]) & 0x7fffffffu);
-        m = max(m, __shfl_xor_sync(kFullMask, m, 1));
-        uint4 word[3];
-        uint32_t scale[3];
-        moe_quantize_e4m3x3<kE4m3BfStep>(v, m, word, scale);
-        const int row = w / per_row, at = (w - row * per_row) * 512 + lane * 16;
-        for (int j = 0; j < a.k; ++j) {
-            const int slot = j < 32 ? __shfl_sync(kFullMask, slots, j) : __ldcg(a.pair_slot + (long long)row * a.k + j);
-            if (slot < 0 || at >= a.K) continue;
+        for (int i = 0; i < PIECES; ++i)
 #pragma unroll
-            for (int t = 0; t < 3; ++t) {
-                *reinterpret_cast<uint4*>(a.q + t * term_q + (long long)slot * a.K + at) = word[t];
-                if ((lane & 1) == 0) a.s[t * term_s + (long long)slot * (a.K >> 5) + (at >> 5)] = (uint8_t)scale[t];
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < 2; ++i) cur[i] = nxt[i];
-        slots = next_slots;
+            for (int h = 0; h < 2; ++h) cur[i][h] = nxt[i][h];
+        pair = next_pair;
+        shift = shift_of(pair);
     }
 }
 
 constexpr int kActRowThreads = 256;                        // threads per activation row (four rows per block)
 constexpr int kActRows = kPrepThreads / kActRowThreads;
 constexpr int kActMaxChunks = 16384 / 8 / kActRowThreads;  // 16-byte chunks per thread at the largest K
-constexpr int kActSampleRows = 16;                         // weight rows looked at per expert and matrix
 
 // Normalised fp16 (and, in the first blocks, the typical weight scale of every expert).
 template <bool PEER>
@@ -349,38 +470,11 @@ __global__ void __launch_bounds__(kPrepThreads) moe_act_fp16_kernel(const MoeAct
     __shared__ int slots[kActRows][32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     int blk = blockIdx.x;
-    const int scale_blocks = (a.n_experts + 31) / 32;
+    const int scale_blocks = (a.typical.n_experts + kTypicalExperts - 1) / kTypicalExperts;
     if (blk < scale_blocks) {
-        // One warp per expert: the mean E8M0 byte of a few rows of W1 and of W3 (bytes 0 and 255, i.e. zero blocks and
-        // NaN, left out).  It only centres the fp16 range of the intermediate; any value near the truth will do.
         pdl_wait();
         pdl_launch_dependents();
-        const int e = blk * 32 + warp;
-        if (e >= a.n_experts) return;
-        const int row_s = a.K >> 5, words = row_s >> 2, step = max(1, a.hidden / kActSampleRows);
-        int typ[2];
-#pragma unroll
-        for (int m = 0; m < 2; ++m) {
-            const uint8_t* base = (m == 0 ? a.w1_s : a.w3_s) + (long long)e * a.hidden * row_s;
-            int sum = 0, n = 0;
-            for (int c = lane; c < words; c += 32) {
-                uint32_t w[kActSampleRows];
-#pragma unroll
-                for (int i = 0; i < kActSampleRows; ++i)
-                    w[i] = __ldg(reinterpret_cast<const uint32_t*>(base + (long long)min(i * step, a.hidden - 1) * row_s) + c);
-#pragma unroll
-                for (int i = 0; i < kActSampleRows; ++i)
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const int b = (w[i] >> (8 * j)) & 255;
-                        if (b != 0 && b != 255) { sum += b; ++n; }
-                    }
-            }
-            sum = __reduce_add_sync(kFullMask, sum);
-            n = __reduce_add_sync(kFullMask, n);
-            typ[m] = n > 0 ? (sum + n / 2) / n : 127;
-        }
-        if (lane == 0) a.typical[e] = typ[0] | (typ[1] << 8);
+        moe_typical_scales(a.typical, blk);
         return;
     }
     blk -= scale_blocks;
@@ -417,9 +511,7 @@ __global__ void __launch_bounds__(kPrepThreads) moe_act_fp16_kernel(const MoeAct
         const int w0 = sub * (kActRowThreads / 32);
 #pragma unroll
         for (int w = 0; w < kActRowThreads / 32; ++w) m = max(m, red_max[w0 + w]);
-        int e = (int)(m >> 23) - 127;                      // floor(log2(amax))
-        if (m == 0) e = 0;
-        e = min(max(e, -100), 126);
+        const int e = moe_row_exponent(m);
         const float inv = __uint_as_float((uint32_t)(127 - e) << 23);
         float ss = 0.f;
 #pragma unroll

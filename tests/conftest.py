@@ -39,3 +39,18 @@ def qz(pkg):
 @pytest.fixture(scope="session")
 def golden():
     return np.load(os.path.join(ROOT, "tests", "golden", "reference_vectors.npz"))
+
+
+@pytest.fixture(scope="session")
+def odd_bank():
+    """A bank's tensors at addresses that are 16 modulo 32: the TMA cannot lay such weights down padded, so the batched layer's path "fp16"
+    dequantises them."""
+    import torch
+
+    def at_odd_16_bytes(t):
+        buf = torch.empty(t.numel() + 48, dtype=t.dtype, device=t.device)
+        shift = (16 - buf.data_ptr() % 32) % 32
+        view = buf[shift:shift + t.numel()].view(t.shape)
+        assert view.data_ptr() % 32 == 16
+        return view.copy_(t)
+    return lambda bank: {n: at_odd_16_bytes(t) for n, t in bank.items()}

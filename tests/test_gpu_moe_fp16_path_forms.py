@@ -23,15 +23,6 @@ def layer64(bank, x, ids, w):
     return out
 
 
-def at_odd_16_bytes(t):
-    """The same bytes at an address that is 16 modulo 32: the TMA cannot lay such weights down padded."""
-    buf = torch.empty(t.numel() + 48, dtype=t.dtype, device=t.device)
-    shift = (16 - buf.data_ptr() % 32) % 32
-    view = buf[shift:shift + t.numel()].view(t.shape)
-    assert view.data_ptr() % 32 == 16
-    return view.copy_(t)
-
-
 @pytest.mark.parametrize("counts,K,H,O", [
     ([1, 0, 15, 16], 256, 256, 256),             # two stages a tile, one run of scale bytes cut short
     ([24, 24, 24, 24], 1280, 512, 1280),         # the most pairs for tiles of 32 tokens
@@ -45,7 +36,7 @@ def at_odd_16_bytes(t):
     ([40, 9], 256, 1280, 256),                   # no room for the terms of the intermediate
     ([40, 9], 1280, 256, 384),                   # nor of x
 ])
-def test_forms_agree(rt, qz, counts, K, H, O):
+def test_forms_agree(rt, qz, odd_bank, counts, K, H, O):
     g = torch.Generator(device=DEV).manual_seed(sum(counts) + K)
     E, T = len(counts), sum(counts)
     bank = qz.make_expert_bank(E, K, H, DEV, seed=K)
@@ -57,7 +48,7 @@ def test_forms_agree(rt, qz, counts, K, H, O):
     x = (torch.randn(T, K, generator=g, device=DEV) * torch.exp2(torch.randn(T, 1, generator=g, device=DEV) * 3)).to(torch.bfloat16)
     x[T // 2, :64] = 0
     one = rt.moe_forward(bank, x, ids, w, path="fp16")
-    other = rt.moe_forward({n: at_odd_16_bytes(t) for n, t in bank.items()}, x, ids, w, path="fp16")
+    other = rt.moe_forward(odd_bank(bank), x, ids, w, path="fp16")
     again = rt.moe_forward(bank, x, ids, w, path="fp16")
     assert rt.moe_device_status() == 0
     assert torch.equal(one.view(torch.int16), again.view(torch.int16))
@@ -89,3 +80,34 @@ def test_wide_range_of_x(rt, qz, counts):
     ref = layer64(bank, x, ids, w)
     rounding = (ref.to(torch.bfloat16).double() - ref).norm() / ref.norm()
     assert ((out - ref).norm() / ref.norm()) ** 2 <= rounding ** 2 + 2.0 ** -26
+
+
+@pytest.mark.parametrize("n", [24, 60])
+@pytest.mark.parametrize("up,down,of_x", [
+    (64, -100, [0]), (0, -110, [66]), (100, -110, [-30]),       # silu(G) * U beyond FP32
+    (-70, 100, [0]), (-30, 100, [-40]),                         # below its smallest normal value
+    (8, 0, [30, -30, 0, 17, -17, 16]),                          # normalised tokens beside others
+])
+def test_range_of_the_intermediate(rt, qz, odd_bank, n, up, down, of_x):
+    """Scales of x (powers of two, token by token) and of W1 and W3 that take silu(G) * U out of the range of FP32, and scales of W2 that
+    bring the result back into that of bf16."""
+    E, K, H = 4, 1024, 512
+    T = E * n
+    g = torch.Generator(device=DEV).manual_seed(n)
+    bank = qz.make_expert_bank(E, K, H, DEV, seed=5)
+    for name, d in (("w1s", up), ("w3s", up), ("w2s", down)):
+        bank[name] = (bank[name].int() + d).to(torch.uint8)
+    ids = torch.repeat_interleave(torch.arange(E, device=DEV), n).to(torch.int32)[:, None].contiguous()
+    w = torch.rand(T, 1, generator=g, device=DEV) + 0.5
+    e = torch.tensor(of_x, device=DEV)[torch.arange(T, device=DEV) % len(of_x)]
+    x = (torch.randn(T, K, generator=g, device=DEV) * torch.exp2(e.float())[:, None]).to(torch.bfloat16)
+    ref = layer64(bank, x, ids, w)
+    assert 1e-37 < ref.norm(dim=1).min() and ref.abs().max() < 2.0 ** 127
+    rounding = (ref.to(torch.bfloat16).double() - ref).norm(dim=1)
+    # the bounds of test_forms_agree
+    for b, bound in ((bank, 2.0 ** -13), (odd_bank(bank), 2 * 2.0 ** -11 / 3 ** 0.5)):
+        out = rt.moe_forward(b, x, ids, w, path="fp16").double()
+        assert torch.isfinite(out).all()
+        worst = (((out - ref).norm(dim=1) ** 2 - rounding ** 2).clamp(min=0).sqrt() / ref.norm(dim=1)).max().item()
+        assert worst <= bound, f"{worst:.2e} of a token's norm beside the rounding, {bound:.2e} allowed"
+    assert rt.moe_device_status() == 0
