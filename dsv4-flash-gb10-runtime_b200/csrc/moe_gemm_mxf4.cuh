@@ -455,10 +455,6 @@ __global__ void __launch_bounds__(kQThreads, 1) moe_gemm_mxf4_kernel(const __gri
                     const uint2 lo = __ldcg(p), hi = l.stages == kRun ? __ldcg(p + 1) : make_uint2(0, 0);
                     l.v[i] = make_uint4(lo.x, lo.y, hi.x, hi.y);
                 }
-                if (FP8 && i < 2) {                            // a weight's scale byte 0xFF contributes nothing on this path: 2^-127
-                    l.v[i].x &= ~__vcmpeq4(l.v[i].x, 0xffffffffu); l.v[i].y &= ~__vcmpeq4(l.v[i].y, 0xffffffffu);
-                    l.v[i].z &= ~__vcmpeq4(l.v[i].z, 0xffffffffu); l.v[i].w &= ~__vcmpeq4(l.v[i].w, 0xffffffffu);
-                }
             }
             pr += 2;
             return true;
@@ -478,7 +474,9 @@ __global__ void __launch_bounds__(kQThreads, 1) moe_gemm_mxf4_kernel(const __gri
                         at = sf + Q::kSfB + tc05_scale_atom_offset(st + (i - 2 + (st >= l.half ? kQTerms - 1 : 0)) * l.half, 0);
                     const uint4& v = l.v[i];
                     if (FP8) {                                 // one piece of 128 K-elements, or two
-                        asm volatile("st.shared.u32 [%0], %1;" ::"r"(at), "r"(n == 0 ? v.x : n == 1 ? v.y : n == 2 ? v.z : v.w) : "memory");
+                        uint32_t word = n == 0 ? v.x : n == 1 ? v.y : n == 2 ? v.z : v.w;
+                        if (i < 2) word &= ~__vcmpeq4(word, 0xffffffffu);      // a weight's 0xFF contributes nothing on this path: 2^-127
+                        asm volatile("st.shared.u32 [%0], %1;" ::"r"(at), "r"(word) : "memory");
                     } else {
                         asm volatile("st.shared.u32 [%0], %1;" ::"r"(at), "r"(n == 1 ? v.z : v.x) : "memory");
                         asm volatile("st.shared.u32 [%0], %1;" ::"r"(at + (i < 2 ? 512u : Q::kAtoms * 512u)), "r"(n == 1 ? v.w : v.y) : "memory");
