@@ -175,20 +175,20 @@ cudaError_t weight_map_padded(CUtensorMap* map, const uint8_t* base, long long r
     const cuuint32_t box[2] = {128, kMoeTileRows};
     return box_map(map, CU_TENSOR_MAP_DATA_TYPE_16U4_ALIGN16B, K / 2, base, 2, dim, box);
 }
-// three terms [3][P][row_bytes]: half a tile's columns of every term
+// three terms [3][P][row_bytes]: half a tile's columns of every term; boxes of the column counts that tiles of up to `cap` tokens have
 cudaError_t term_maps(CUtensorMap (&map)[kMoeWidths], const uint8_t* base, long long P, int row_bytes, int cap) {
     cudaError_t err = cudaSuccess;
-    for (int i = 0; i < kMoeWidths && err == cudaSuccess; ++i) {
+    for (int i = 0; i <= moe_width_index(cap) && err == cudaSuccess; ++i) {
         const cuuint64_t dim[3] = {(cuuint64_t)row_bytes, (cuuint64_t)P, kQTerms};
         const cuuint32_t box[3] = {128, (cuuint32_t)moe_width(i, cap) / 2, kQTerms};
         err = box_map(&map[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, row_bytes, base, 3, dim, box);
     }
     return err;
 }
-// fp16 activations [P, K]: a tile's columns
+// fp16 activations [P, K]: a tile's columns, likewise
 cudaError_t half_maps(CUtensorMap (&map)[kMoeWidths], const __half* base, long long P, int K, int cap) {
     cudaError_t err = cudaSuccess;
-    for (int i = 0; i < kMoeWidths && err == cudaSuccess; ++i) {
+    for (int i = 0; i <= moe_width_index(cap) && err == cudaSuccess; ++i) {
         const cuuint64_t dim[2] = {(cuuint64_t)K, (cuuint64_t)P};
         const cuuint32_t box[2] = {64, (cuuint32_t)moe_width(i, cap)};
         err = box_map(&map[i], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, K * 2, base, 2, dim, box);
