@@ -325,14 +325,17 @@ __global__ void __launch_bounds__(kQThreads, 1) moe_gemm_mxf4_kernel(const __gri
             const uint32_t buf = tc & 1u;
             const int m0 = t.m0 + rank * kMoeTileRows;        // first row of this CTA in block 0
             // lanes i and i + 16 hold, for token i of each of this warp's chunks: down, the router weight; of E4M3 terms, the power of two
-            // that was taken out of x, and so of G and of U - once for the gate, twice for y (with the weight and by itself)
-            float w[kQEpiRounds], unit[kQEpiRounds];
+            // that was taken out of x and so of G and of U.  G gets it back before the sigmoid, y with the weight.
+            float w[kQEpiRounds];
             if (MODE == 1 || FP8)
 #pragma unroll
                 for (int i = 0; i < kQEpiRounds; ++i) {
                     const int n = (((warp - kQEpiWarp) >> 2) + kQEpiGroups * i) * 16 + (lane & 15);
-                    if (FP8) unit[i] = n < t.n_valid ? float_pow2(__ldcg(a.row_exp + t.slot0 + n)) : 1.f;
-                    if (MODE == 1) w[i] = n < t.n_valid ? __ldcg(a.g.slot_w + t.slot0 + n) * (FP8 ? unit[i] : 1.f) : 0.f;
+                    w[i] = MODE == 1 ? 0.f : 1.f;
+                    if (n < t.n_valid) {
+                        if (MODE == 1) w[i] = __ldcg(a.g.slot_w + t.slot0 + n);
+                        if (FP8) w[i] *= float_pow2(__ldcg(a.row_exp + t.slot0 + n));
+                    }
                 }
             wait(acc_full[buf], tc >> 1, 6);
             tc05_fence_after_sync();
@@ -343,7 +346,6 @@ __global__ void __launch_bounds__(kQThreads, 1) moe_gemm_mxf4_kernel(const __gri
                 const int c = (((warp - kQEpiWarp) >> 2) + kQEpiGroups * k) * 16;
                 if (c >= t.n_valid || !alive) break;
                 const int n = min(16, t.n_valid - c);
-                const bool scaled = FP8 && __any_sync(kFullMask, unit[k] != 1.f);
                 auto sums = [&](int m, uint32_t (&p)[16]) {   // of block m; wide: complete on return
                     if constexpr (Q::kWide) moe_q_sum_terms(trow + m * Q::kMatCols + 3 * c, moe_width(t.width, CAP) >> 1, p);
                     else tc05_ld16_issue(trow + m * Q::kMatCols + c, p);
@@ -354,20 +356,16 @@ __global__ void __launch_bounds__(kQThreads, 1) moe_gemm_mxf4_kernel(const __gri
                 if (!Q::kWide) tc05_wait_ld();
                 if (MODE == 0) {
                     float g[16];
-                    if (!scaled) {
+                    if (FP8 && __any_sync(kFullMask, w[k] != 1.f)) {
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) {
-                            const float gate = __uint_as_float(p0[i]);
-                            const float v = __fdividef(gate, 1.0f + __expf(-gate)) * __uint_as_float(p1[i]);
-                            g[i] = i < n ? (FP8 ? saturate_finite(v) : v) : 0.f;
-                        }
-                    } else {
+                        for (int i = 0; i < 16; ++i)
+                            p0[i] = __float_as_uint(saturate_finite(__uint_as_float(p0[i]) * __shfl_sync(kFullMask, w[k], i)));
+                    }
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) {
-                            const float gate = saturate_finite(__uint_as_float(p0[i])), true_gate = gate * __shfl_sync(kFullMask, unit[k], i);
-                            const float v = __fdividef(gate, 1.0f + __expf(-true_gate)) * __uint_as_float(p1[i]);
-                            g[i] = i < n ? saturate_finite(v) : 0.f;
-                        }
+                    for (int i = 0; i < 16; ++i) {
+                        const float gate = __uint_as_float(p0[i]);
+                        const float v = __fdividef(gate, 1.0f + __expf(-gate)) * __uint_as_float(p1[i]);
+                        g[i] = i < n ? (FP8 ? saturate_finite(v) : v) : 0.f;
                     }
                     moe_transpose16(g, lane);
                     typename std::conditional<FP8, uint4, uint2>::type packed[kQTerms];
@@ -387,12 +385,8 @@ __global__ void __launch_bounds__(kQThreads, 1) moe_gemm_mxf4_kernel(const __gri
                         }
                     }
                 } else {
-                    auto put = [&](uint32_t (&p)[16], int row) {
+                    auto put = [&](const uint32_t (&p)[16], int row) {
                         if (row >= a.rows) return;                                                        // (a.rows is a multiple of 128)
-                        if (scaled) {
-#pragma unroll
-                            for (int i = 0; i < 16; ++i) p[i] = __float_as_uint(__uint_as_float(p[i]) * __shfl_sync(kFullMask, unit[k], i));
-                        }
 #pragma unroll
                         for (int i = 0; i < 16; ++i) {
                             const float wi = __shfl_sync(kFullMask, w[k], i);

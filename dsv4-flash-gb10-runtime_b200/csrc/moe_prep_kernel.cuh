@@ -334,15 +334,17 @@ __global__ void __launch_bounds__(256, 2) moe_act_blocks_kernel(const MoeActArgs
 // Exponent taken out of a row whose largest magnitude is m (float bits): floor(log2 m), 0 for a row of zeros.
 __device__ __forceinline__ int moe_row_exponent(uint32_t m) { return m == 0 ? 0 : min(max((int)(m >> 23) - 127, -100), 126); }
 
-// Three E4M3 terms, of rows of this GPU.  FP32 is to hold G, U and silu(G) * U whatever the scales of x and of the weights, so the larger
-// and the smaller ones are normalised: x is multiplied by 2^-(its row's exponent), and the scale bytes of a pair are lower by its expert's
-// typical scale exponent, the mean of W1's and W3's, from -kAct8Down to kAct8Up (the bytes of a normalised row, 120 and less, leave room for
-// that).  row_exp is the sum of the two.  Exponents of up to kAct8Plain either way are left alone: in ordinary use row_exp is 0 and the GEMMs'
-// epilogues have nothing to multiply by (1 003 tokens of 256 experts, gate/up: 490 us without row_exp, 508 with, 502 this way), and the
-// worst of them, 16 384 products of 2^17 and 6 * 2^16, are 2^100 when squared.
-// A lane takes half a block of 32, a warp 512 elements of a row in each of PIECES (one up to K 4096, two, four), so that a row is read
-// once between its maximum and its terms; a block takes as many rows as its warps cover.  The next rows and their slots are on their way
-// while these are quantised.  2 K bytes of a token come in, 99 K / 32 of each of its pairs go out.
+// Three E4M3 terms, of rows of this GPU.  The accumulators of the gate/up GEMM are to be within FP32 whatever the scales of x and of the
+// weights, so the larger and the smaller ones are normalised: x is multiplied by 2^-(its row's exponent), and the scale bytes of a pair are
+// lower by its expert's typical scale exponent, the mean of W1's and W3's, from -kAct8Down to kAct8Up (the bytes of a normalised row, 120 and
+// less, leave room for that).  row_exp is the sum of the two; G gets it back before the sigmoid, U keeps it out until y is written, so that
+// silu(G) * U overflows hardly before G does.  Exponents of up to kAct8Plain either way are left alone: in ordinary use row_exp is 0 and the
+// gate/up epilogue has nothing to multiply (1 003 tokens of 256 experts: 490 to 494 us with no exponents at all, 508 with a multiplication for each
+// value, 502 this way), and the worst of them, 16 384 products of 2^17 and 6 * 2^16, are 2^100 when squared.
+// A lane takes half a block of 32, a warp 512 elements of a row in each of PIECES (one up to K 4096, two up to 8192, four), so that a row is
+// read once between its maximum and its terms; a block takes as many rows as its warps cover.  The next rows and their slots are on their way
+// while these are quantised.  2 K bytes of a token come in, 99 K / 32 of each of its pairs go out.  Us of the stage between two events, a warp
+// for 512 elements without the maximum -> this: 2 and 64 tokens of K 4096 8.3 -> 8.5, 1 003 18.5 -> 20, 2 048 35 -> 37.6; 400 of K 6144 10 -> 12.3.
 constexpr int kAct8Warps = 8, kAct8Down = 100, kAct8Up = 60, kAct8Plain = 16;
 __host__ __device__ __forceinline__ int moe_act8_row_warps(int K) { return K >= 512 * kAct8Warps ? kAct8Warps : (K + 511) >> 9; }
 __device__ __forceinline__ int moe_act8_plain(int e) { return abs(e) <= kAct8Plain ? 0 : e; }

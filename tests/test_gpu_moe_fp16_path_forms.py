@@ -95,8 +95,8 @@ def test_wide_range_of_x(rt, qz, counts):
 
 @pytest.mark.parametrize("n", [24, 60])
 @pytest.mark.parametrize("up,down,of_x", [
-    (64, -100, [0]), (0, -110, [66]), (100, -110, [-30]),       # silu(G) * U beyond FP32
-    (-70, 100, [0]), (-30, 100, [-40]),                         # below its smallest normal value
+    (64, -100, [0]), (0, -110, [66]), (100, -110, [-30]),       # silu(G) * U beyond FP32,
+    (0, -110, [100]), (-70, 100, [0]), (-30, 100, [-40]), (0, 110, [-90]),      # and below its smallest normal value
     (8, 0, [30, -30, 0, 17, -17, 16]),                          # normalised tokens beside others
 ])
 def test_range_of_the_intermediate(rt, qz, odd_bank, n, up, down, of_x):
