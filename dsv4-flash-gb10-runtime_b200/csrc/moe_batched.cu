@@ -236,7 +236,8 @@ DSV4_API int mxfp4_moe_stage_times(float* us_out) {
 }
 
 // Bytes of workspace mxfp4_moe_forward needs: grouping tables, the FP32 per-pair outputs [n_tokens * k, out_dim], and the
-// activations and the intermediate of every pair in the form of the path that needs more (three MXFP4 terms; fp16).
+// activations and the intermediate of every pair in the form that needs more (three MXFP4 terms; fp16).  Three E4M3 terms of the intermediate
+// lie in the same bytes, those of x in the bytes of the outputs, where there is room for them.
 DSV4_API size_t mxfp4_moe_forward_workspace_bytes(int n_tokens, int k, int K_in, int hidden, int out_dim,
                                                   int n_experts) {
     if (n_tokens <= 0 || k <= 0 || K_in <= 0 || hidden <= 0 || out_dim <= 0 || n_experts <= 0) return 0;
@@ -289,13 +290,15 @@ static int moe_forward_impl(int path, const __nv_bfloat16* x, const uint8_t* ban
     MoeGroupArgs ga;
     ga.ids = ids; ga.weights = weights; ga.n_pairs = P; ga.n_experts = n_experts; ga.g = g; ga.status = status;
     // Path 0 runs on the block-scaled MMAs too, with E4M3 terms, where its operands have room and the TMA can lay the weights down.
-    const bool fp8 = path == 0 && !peer_in && m.fits8 && P <= (long long)kQMostTokensFp8 * n_experts &&
-                     ((reinterpret_cast<uintptr_t>(bank_W1_packed) | reinterpret_cast<uintptr_t>(bank_W3_packed) | reinterpret_cast<uintptr_t>(bank_W2_packed)) & 31u) == 0;
+    auto aligned32 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 31u) == 0; };
+    const bool fp8 = path == 0 && !peer_in && m.fits8 && P <= (long long)kQMostTokensFp8 * n_experts && aligned32(bank_W1_packed) &&
+                     aligned32(bank_W3_packed) && aligned32(bank_W2_packed);
     const bool pairs = path == 1 || fp8;                   // tiles of CTA pairs
     const int rows_up = pairs ? kQTileRowsUp : kMoeTileRows, rows_down = pairs ? kQTileRowsDown : 2 * kMoeTileRows;
     ga.m_tiles_up = hidden / rows_up; ga.m_tiles_down = (out_dim + rows_down - 1) / rows_down;
-    // (Pairs of the whole batch: where ids are negative, as under expert parallelism, the experts here have fewer, and the larger tiles
-    // are taken although the smaller would do.  Eight ranks emulated on one GPU, 128 to 1024 tokens: 1 % of the layer's time.)
+    // (Pairs of the whole batch: where ids are negative, as under expert parallelism, the experts here have fewer.  Eight ranks emulated on
+    // one GPU, 32 experts of 4096, 2048 each, top 6: the larger tiles although the smaller would do cost 1 % of the layer's time from 128 to 1024
+    // tokens; fp16 MMAs although E4M3 terms would do, path 0, 512 tokens 178 us where 144 would do, 1 024 194 / 156, 2 048 222 / 184.)
     const int cap16 = P <= (long long)kTmFewTokens * n_experts ? 64 : kMoeTileTokens;      // tokens per tile, fp16 path
     const bool few = P <= (long long)(fp8 ? kQFewTokensFp8 : kQFewTokens) * n_experts;
     const int cap_q = few ? 32 : kQTok;                                                    // tokens per tile, block-scaled path

@@ -9,12 +9,12 @@
 // x up to 112 tokens, one tile per PAIR of CTAs (cta_group::2): each CTA holds 128 rows of both blocks and half of the
 // tokens.  A stage covers 256 K-elements (one 128-byte swizzled row per operand row = 4 MMAs of K = 64).
 //
-// How the terms are multiplied (FP8 tiles of few tokens apart, whose three terms lie side by side along N: a third of the MMAs, 44 to 56
-// clocks each; FP4 tiles that way were slower, 64 tokens 428 -> 458 us).  Each term is an MMA of its own into the SAME accumulator columns, with the weight tile
+// How the terms are multiplied.  Each term is an MMA of its own into the SAME accumulator columns, with the weight tile
 // kept in the collector between the three: 3 x N / 2 clocks for N tokens (N >= 96), the full rate of the tensor pipe;
 // a stage's 24 MMAs and 10 scale copies take 1 170 clocks at N = 96 and 580 at N = 16.  Without the collector every MMA
 // reads its A tile again, 32 clocks at 128 bytes a clock.  Two accumulator sets of 2 x 112 columns fit into tensor memory,
-// so the MMAs of a tile run while the one before it is read out.
+// so the MMAs of a tile run while the one before it is read out.  (E4M3 tiles of few tokens: the three terms lie side by side
+// along N, a third of the MMAs, 44 to 56 clocks each.  FP4 tiles that way were slower, 64 tokens 428 -> 458 us.)
 //
 // What bounds it: the weights.  A CTA takes in 34 KB of weights and scales per stage, 1 400 clocks of its share of 7 TB/s,
 // so everything else has to keep out of the way of that stream, above all instruction issue: with six roles on a CTA an
@@ -48,10 +48,11 @@ namespace dsv4 {
 //
 // FP8 is the form of the path "fp16" (moe_gemm.cuh says what it holds exactly): the tensor cores multiply E2M1 weights by E4M3 terms, the TMA
 // spreading the packed weights over twice their bytes as it writes them.  What bounds it: that write, 4.2 clocks a row of 64 packed bytes
-// and SM, i.e. 4.4 TB/s of weights (7.0 as stored; boxes of 64 bytes as stored are as slow), and from some 80 tokens an expert on the MMAs, half as fast
-// as FP4 ones.  The kernel before it (moe_gemm_kernel.cuh, which dequantises into tensor memory) waits for its handshakes: 256 experts of
-// 4096, 2048, top 6, us that one -> this: 2 tokens 116 -> 80, 64 tokens (Zipf) 495 -> 408, 1 003 tokens 1 133 -> 988, 2 048 tokens 1 349 ->
-// 1 257, 3 300 tokens 1 592 -> 1 574; 32 experts of 2048, 1024, 300 tokens 92 -> 63.
+// and SM, i.e. 4.4 TB/s of weights (7.0 as stored; boxes of 64 bytes as stored are as slow), and from some 80 tokens an expert on the MMAs,
+// half as fast as FP4 ones.  moe_gemm_kernel.cuh, which dequantises into tensor memory, waits for its handshakes: 256 experts of 4096, 2048,
+// top 6, us a layer there -> here: 2 tokens 112 -> 80, 64 tokens (Zipf) 482 -> 368, 300 tokens 924 -> 719, 1 003 tokens 995 -> 846, 2 048
+// tokens 1 160 -> 1 075, 3 300 tokens 1 379 -> 1 345 (from 1 003 on at the power limit: up to 15 % more on other boxes); 32 experts of 2048,
+// 1024, top 4, 300 tokens 87 -> 66.
 struct MoeQFp4 {                                     // kind::mxf4: activations as three MXFP4 terms
     static constexpr int kKBlock = 256;              // K-elements per stage
     static constexpr uint32_t kBoxBytes = 128 * 128; // bytes that a box of 128 weight rows brings in
@@ -72,9 +73,15 @@ constexpr uint32_t kQTile = 128 * 128;               // bytes of one packed weig
 // 270, 300 579 -> 567; below ten tokens no difference).  Taken up to kQFewTokens pairs per expert, where next to no expert has more
 // than 32.
 constexpr int kQFewTokens = 16;
-// FP8: the tiles of 32 tokens (terms side by side) against those of 112, pairs per expert: 14 765 / 802 us, 19 811 / 855, 23.5 844 / 877, 29
-// 1 010 / 929.  Above kQMostTokensFp8 pairs per expert dequantising takes over: 70 1 395 there, 1 265 here; 96 1 650 / 1 674; 250 (2048, 1024)
-// 223 / 227.
+// E4M3 terms.  Us a layer, tiles of 32 tokens (terms side by side) / of 112 / dequantising (moe_gemm_kernel.cuh), one box, by pairs per expert:
+//   256 experts of 4096, 2048, top 6, uniform: 8 727 / 780 / 933,  16 805 / 850 / 1 005,  20 821 / 876 / 1 031,  24 917 / 915 / 1 052,
+//     28 1 025 / 936 / 1 104,  64 - / 1 180 / 1 390,  79 - / 1 490 / 1 573,  90 - / 1 690 / 1 650,  100 - / 1 755 / 1 758
+//   the same, Zipf(1.1): 8 720 / 870 / 910,  12 850 / 832 / 1 003,  16 958 / 892 / 1 096,  20 1 046 / 948 / 1 156,  24 1 140 / 986 / 1 216,
+//     64 - / 1 460 / 1 575,  79 - / 1 805 / 1 824,  100 - / 2 010 / 2 060
+//   32 experts, top 2, uniform: 24 148 / 153 / 185,  28 164 / 156 / 186,  79 - / 198 / 241,  100 - / 229 / 262;  Zipf: 12 136 / 158 / 173,
+//     24 157 / 155 / 179,  79 - / 218 / 252,  100 - / 262 / 266
+// The line at 24 is where uniform routing changes over; under Zipf, whose busy experts take several tiles of 32, it is at 10, and tiles of 112
+// are 5 to 13 % faster from there to 24.  The line at 80 is where dequantising is as fast for the largest bank.
 constexpr int kQFewTokensFp8 = 24, kQMostTokensFp8 = 80;
 constexpr int kQEpiWarps = 12, kQScaleWarps = 8;
 constexpr int kQEpiGroups = kQEpiWarps / 4;          // warps per lane quadrant of tensor memory
@@ -88,7 +95,7 @@ struct MoeQShape {
     static constexpr uint32_t kSfCol = 2 * kAccCols;                         // scale columns: A [mat][piece] x 4, B [piece][term] x 4
     static constexpr uint32_t kBStage = kQTerms * (CAP / 2) * 128;           // activation rows of one stage and CTA
     static constexpr int kPieces = F::kAtoms128;
-    static constexpr uint32_t kSfB = 2 * kPieces * 512, kSfStage = kSfB + kPieces * kAtoms * 512;      // scale atoms: [mat][piece], then [piece][term]
+    static constexpr uint32_t kSfB = 2 * kPieces * 512, kSfStage = kSfB + kPieces * kAtoms * 512;      // scale atoms: [mat][piece], [piece][term]
     static constexpr int kEpiRounds = (CAP + 16 * kQEpiGroups - 1) / (16 * kQEpiGroups);
     static constexpr uint32_t kOffB = kStages * 2 * kQTile, kOffSf = kOffB + kStages * kBStage, kOffTables = kOffSf + kStages * kSfStage;
     static_assert(kSfCol + 16 + 8 * kAtoms <= 512, "tensor memory overflow");
@@ -557,7 +564,8 @@ __global__ void __launch_bounds__(kQThreads, 1) moe_gemm_mxf4_kernel(const __gri
 #pragma unroll
                 for (int j = 0; j < (FP8 ? 4 : 2); ++j) {     // scale bytes of K-step j: two of every four, or one
                     const int id = FP8 ? j : 2 * j;
-                    q.idesc[j] = FP8 ? tc05_idesc_mxf8f6f4(256, Q::kWide ? kQTerms * n : n, id, id) : tc05_idesc_mxf4(256, Q::kWide ? kQTerms * n : n, id, id);
+                    const int cols = Q::kWide ? kQTerms * n : n;
+                    q.idesc[j] = FP8 ? tc05_idesc_mxf8f6f4(256, cols, id, id) : tc05_idesc_mxf4(256, cols, id, id);
                 }
                 if (tc >= 2) wait_one(acc_free[buf], (tc >> 1) - 1, 7);
                 for (int s = 0; s < n_st; ++s, pos.next(kQStages)) {

@@ -12,7 +12,7 @@ constexpr int kMoeTileRows = 128;      // weight rows per tensor-core tile (the 
 constexpr int kMoeTileTokens = 128;    // tokens per tile at most, fp16 path
 
 // The tokens of a tile are padded to one of seven column counts (the boxes the activation copies are encoded for): a multiple of 16, or
-// all that a tile may have.  (48 and 80 among them: 256 experts of 4096, 2048, top 6, 1 800 tokens 724 -> 687 us, 2 800 tokens 831 -> 795.)
+// all that a tile may have.  (48 and 80 among them: 256 experts of 4096, 2048, top 6, 1 800 tokens 724 -> 692 us, 2 800 tokens 824 -> 795.)
 constexpr int kMoeWidths = 7;
 __host__ __device__ __forceinline__ int moe_width_index(int n) { return n <= 16 ? 0 : n <= 96 ? (n - 1) >> 4 : 6; }
 __host__ __device__ __forceinline__ int moe_width(int index, int cap) { return index == 6 ? cap : 16 * (index + 1); }

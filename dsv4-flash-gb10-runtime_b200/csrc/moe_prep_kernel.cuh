@@ -18,7 +18,7 @@ constexpr int kTypicalExperts = kPrepThreads / 32 / 4;     // experts of a block
 
 // The typical scale byte of W1 and of W3 of a few experts, by a block: the mean E8M0 byte of some of their rows (bytes 0 and 255, i.e.
 // zero blocks and NaN, left out).  It only centres the range of the intermediate; any value near the truth will do.  A warp takes half of
-// an expert's rows of one matrix.  (Short code: a warp for a whole expert, unrolled, is as many loads but 12 us of instruction fetches.)
+// an expert's rows of one matrix.  (A warp for a whole expert, its bytes counted one by one, made the launch 12 us longer.)
 struct MoeTypicalArgs {
     const uint8_t* w1_s; const uint8_t* w3_s;              // E8M0 bytes [E, hidden, K / 32]
     int K, hidden, n_experts;

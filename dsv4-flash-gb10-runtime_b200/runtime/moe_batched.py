@@ -29,7 +29,8 @@ def moe_forward(bank: Dict[str, torch.Tensor], x: torch.Tensor, ids: torch.Tenso
                 path: Optional[str] = None) -> torch.Tensor:
     """`path`: None = the library's default (block-scaled MXFP4 MMAs unless DSV4_B200_MOE_PATH=fp16), 'mxf4' =
     block-scaled MMAs fed with the packed weights (activations as three MXFP4 terms), 'fp16' = operands of fp16's
-    precision and more (x exact down to 2^-17 of its row's largest, the intermediate to 11 bits: E4M3 terms or fp16)."""
+    precision and more (x exact down to 2^-17 of its row's largest, the intermediate to 11 bits: E4M3 terms up to 80 pairs an
+    expert, fp16 above; include/dsv4_b200.h says what differs between the two)."""
     code = -1 if path is None else _PATHS[path]
     done = (_capi._host or _capi.host()).moe_forward(bank, x, ids, weights, out, workspace, code)
     if done is not None:

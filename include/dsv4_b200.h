@@ -199,15 +199,22 @@ int fp8_e4m3_gemv_test_wait_limits(long long polls, int withheld_stages);
  * x bf16 [n_tokens, K_in]; bank tensors as in mxfp4_grouped_gemv_topk_ids; ids int32 [n_tokens, k]; weights FP32
  * [n_tokens, k]; out bf16 [n_tokens, out_dim].  A negative id marks a pair to skip (an expert-parallel caller masks
  * the experts of other ranks this way); an id >= n_experts is dropped and reported by mxfp4_moe_device_status().
- * K_in, hidden multiples of 256; out_dim multiple of 128; n_experts <= 1024.  Returns -1 bad shape, -2 null / misaligned pointer, -3 launch failure. */
+ * K_in, hidden multiples of 256; out_dim multiple of 128; n_experts <= 1024.  Returns -1 bad shape, -2 null / misaligned
+ * pointer, -3 launch failure. */
 int mxfp4_moe_forward(const uint16_t* x, const uint8_t* bank_W1_packed, const uint8_t* bank_W3_packed,
                       const uint8_t* bank_W2_packed, const uint8_t* bank_W1_scale, const uint8_t* bank_W3_scale,
                       const uint8_t* bank_W2_scale, const int* ids, const float* weights, int n_tokens, int n_experts,
                       int K_in, int hidden, int out_dim, int k, uint16_t* out, void* workspace, void* stream);
 /* The same with the tensor-core path chosen by the caller: 1 = block-scaled MXFP4 MMAs fed with the packed weights as
  * stored, activations as three MXFP4 terms (what mxfp4_moe_forward uses unless DSV4_B200_MOE_PATH=fp16 is set);
- * 0 ("fp16") = x exact down to 2^-17 of its row's largest element and the intermediate to 11 bits or more: E4M3 terms on block-scaled
- * MMAs, or fp16 MMAs with in-kernel dequantisation (weights down to scales 2^-23 of their row's largest). */
+ * 0 ("fp16") = x exact down to 2^-17 of its row's largest element, the intermediate to 11 bits and more.  Path 0 has two forms:
+ *   E4M3 terms on block-scaled MMAs: n_tokens * k <= 80 * n_experts, packed weights 32-byte aligned, x of this GPU (not
+ *     mxfp4_moe_forward_ep2), and shapes for whose terms the workspace has room (about 99 K_in <= 128 out_dim and 99 hidden <= 64 (K_in +
+ *     hidden)).  The intermediate has its 11 bits down to 2^-13 of the largest of 32 neighbours; a token with an infinity or a NaN is NaN
+ *     throughout; a weight's scale byte 0xFF counts as 2^-127;
+ *   fp16 MMAs with in-kernel dequantisation otherwise: weights down to scales 2^-23 of their row's largest; an element of the intermediate
+ *     more than about 2^8 times the usual for its token and expert saturates; a token with an infinity or a NaN gives a mix of NaN, infinities
+ *     and finite values; a scale byte 0xFF counts as 0. */
 int mxfp4_moe_forward_path(int path, const uint16_t* x, const uint8_t* bank_W1_packed, const uint8_t* bank_W3_packed,
                            const uint8_t* bank_W2_packed, const uint8_t* bank_W1_scale, const uint8_t* bank_W3_scale,
                            const uint8_t* bank_W2_scale, const int* ids, const float* weights, int n_tokens,
