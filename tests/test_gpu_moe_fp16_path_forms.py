@@ -58,7 +58,8 @@ def test_forms_agree(rt, qz, odd_bank, counts, K, H, O):
     if O != K:
         bank["w2p"], bank["w2s"] = qz.quantize_mxfp4((torch.randn(E, O, H, generator=g, device=DEV) * 0.02).to(torch.bfloat16))
     bank["w1s"] += (torch.arange(bank["w1s"].numel(), device=DEV).view(bank["w1s"].shape) % 5).to(torch.uint8)        # scales that differ along K
-    ids = torch.repeat_interleave(torch.arange(E, device=DEV), torch.tensor(counts, device=DEV))[torch.randperm(T, generator=g, device=DEV)].to(torch.int32)[:, None].contiguous()
+    ids = torch.repeat_interleave(torch.arange(E, device=DEV), torch.tensor(counts, device=DEV))
+    ids = ids[torch.randperm(T, generator=g, device=DEV)].to(torch.int32)[:, None].contiguous()
     w = torch.rand(T, 1, generator=g, device=DEV) + 0.5
     x = (torch.randn(T, K, generator=g, device=DEV) * torch.exp2(torch.randn(T, 1, generator=g, device=DEV) * 3)).to(torch.bfloat16)
     x[T // 2, :64] = 0
